@@ -1,0 +1,671 @@
+// Exact digit contraction (exact_gemm.cuh): operand checks and digits, the
+// tcgen05 kernel, and the FP64 epilogue.
+//
+// The contraction kernel.  A CTA takes one (128 rows x 80 B' rows x K range)
+// item at a time.  Per 16-K tile the 21 digit products run as nine MMAs: the
+// B slices are stacked along N, so A_i times [B_j .. B_k] fills the adjacent
+// accumulators s = i + j .. i + k in one instruction (N up to 240), which
+// reads A from shared memory once for up to three products (107 bytes per
+// clock of the 128 available; one MMA per product would need 166).  TMEM
+// holds the six accumulators (480 of 512 columns).  They live 128 K values;
+// the nine MMAs are issued as two groups (s = 0..2, then s = 3..5) over pairs
+// of tiles, so that one group's accumulators are read while the other
+// group's products run.  Eight drain warps convert the FP32 integers and add
+// them to 64-bit integer sums (s <= 3) and FP32 sums (s = 4, 5) in registers,
+// no FP64 operation (2 per clock per SM on this part); an item ends with its
+// raw sums written out, and exact_finish_kernel forms the weighted FP64 sums.
+//
+// Measured: the FF contraction of 512 x (15 x 820) x 16384 in 13.8 ms, 555 ms
+// with FP64 multiply-adds (ff_fp64.cu); normwise error 2.8e-15 (5e-15).
+//
+// Roles (352 threads): warps 0-7 drain, warp 8 streams 39 KB tiles (one bulk
+// copy per operand) into a five-stage ring, warp 10 waits for the stages and
+// the accumulators and releases warp 9, which issues the MMAs (the issuing
+// thread polls no shared memory, which would stall the tensor pipe).
+#include <algorithm>
+#include <climits>
+
+#include "exact_gemm.cuh"
+
+namespace sigma {
+namespace {
+
+using namespace tma;
+
+constexpr int kThreadsEx = 352;
+constexpr int kCopyWarp = 8, kIssueWarp = 9, kGateWarpEx = 10;
+constexpr uint32_t kStageEx = kExABytes + kExBBytes;  // 39 KB
+constexpr int kStagesEx = 5;
+constexpr uint32_t kSmemEx = kStagesEx * kStageEx + 1024;
+constexpr int kBlockTiles = 8;  // K tiles per accumulator lifetime (128 K values)
+constexpr int kColsHalf = kExCols / 2;
+
+// 32-byte swizzle: rows of 16 elements (32 B), 8-row groups of 256 B (layout
+// code 6 in bits 61-63).
+__device__ __forceinline__ uint64_t sw32_desc(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)1u << 16;
+  d |= (uint64_t)(256u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)6u << 61;
+  return d;
+}
+
+__device__ __forceinline__ void arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// The gate and the issuing warp meet; the gate's failure flag is passed on.
+__device__ __forceinline__ bool gate_sync(bool flag) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "bar.red.or.pred p, 2, 64, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)flag)
+      : "memory");
+  return r != 0;
+}
+
+// 8 consecutive TMEM columns of this warp's 32 lanes (no wait).
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+struct ExItem {
+  int rb, cb, t0, nst;
+  size_t pidx;
+};
+// Band blocks vary fastest (the CTAs of one time share A tiles), then the row
+// blocks of one K split, the splits slowest.
+__device__ __forceinline__ ExItem ex_decode(const ExactPrep& ex, int item) {
+  ExItem t;
+  t.cb = item % ex.n_col_blocks;
+  const int4 e = ex.entries[item / ex.n_col_blocks];
+  t.rb = e.x;
+  t.t0 = e.z;
+  t.nst = e.w;
+  t.pidx = ((size_t)t.rb * ex.n_col_blocks + t.cb) * ex.max_pieces + e.y;
+  return t;
+}
+
+constexpr uint32_t idesc_n(int n) { return idesc_bf16_f32(128, n); }
+
+__global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex, int* status) {
+  extern __shared__ unsigned char smem_raw[];
+  // full[5], empty[5], lo full, hi full, lo empty, hi empty, done
+  __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
+  __shared__ uint32_t tmem_slot;
+  if (*ex.flag) return;  // operands outside the split's range: the FP64 kernel runs instead
+
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t sbase = (raw + 1023u) & ~1023u;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kStagesEx]);
+  const uint32_t accf = smem_u32(&bars[2 * kStagesEx]), acce = smem_u32(&bars[2 * kStagesEx + 2]);
+  const uint32_t done0 = smem_u32(&bars[2 * kStagesEx + 4]);
+
+  if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 512);
+  if (tid == 0) {
+    for (int i = 0; i < 2 * kStagesEx + 2; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    mbar_init(acce, 8);
+    mbar_init(acce + 8u, 8);
+    mbar_init(done0, 1);
+    fence_mbar_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  if (warp == kCopyWarp) {
+    if (lane == 0) {
+      uint32_t g = 0;  // tiles issued by this CTA
+      bool ok = true;
+      for (int item = blockIdx.x; ok && item < ex.n_items; item += gridDim.x) {
+        const ExItem it = ex_decode(ex, item);
+        const size_t kts = (size_t)ex.halves * ex.kt;
+        const unsigned char* a = ex.a_tiles + ((size_t)it.rb * kts + it.t0) * kExABytes;
+        const unsigned char* b = ex.b_tiles + ((size_t)it.cb * kts + it.t0) * kExBBytes;
+        for (int s = 0; s < it.nst; ++s, ++g) {
+          const uint32_t st = g % kStagesEx, use = g / kStagesEx;
+          if (use > 0 && !mbar_wait(empty0 + 8u * st, (use - 1) & 1u, status)) {
+            ok = false;
+            break;
+          }
+          const uint32_t bar = full0 + 8u * st, dst = sbase + st * kStageEx;
+          mbar_expect_tx(bar, kStageEx);
+          bulk_load(dst, a + (size_t)s * kExABytes, kExABytes, bar);
+          bulk_load(dst + kExABytes, b + (size_t)s * kExBBytes, kExBBytes, bar);
+        }
+      }
+      // after a failure: the copies still landing end before the CTA does
+      if (!ok)
+        for (uint32_t t = g > (uint32_t)kStagesEx ? g - kStagesEx : 0u; t < g; ++t)
+          mbar_wait_own(full0 + 8u * (t % kStagesEx), (t / kStagesEx) & 1u);
+    }
+    __syncwarp();
+  } else if (warp == kGateWarpEx) {
+    // per pair of tiles: both stages full; at a block's first pair also the
+    // lo accumulators drained, and (second meeting) the hi accumulators
+    bool failed = false;
+    uint32_t g = 0, blk = 0;  // tiles and accumulator lifetimes so far
+    for (int item = blockIdx.x; item < ex.n_items; item += gridDim.x) {
+      const int nst = ex_decode(ex, item).nst;
+      for (int s = 0; s < nst; s += 2, g += 2) {
+        const bool first = s % kBlockTiles == 0;
+        if (lane == 0 && !failed) {
+          if (first && blk > 0) failed = !mbar_wait(acce, (blk - 1) & 1u, status);
+          for (uint32_t t = g; t < g + 2 && !failed; ++t)
+            failed = !mbar_wait(full0 + 8u * (t % kStagesEx), (t / kStagesEx) & 1u, status);
+        }
+        __syncwarp();
+        gate_sync(failed);
+        if (first) {
+          if (lane == 0 && !failed && blk > 0) failed = !mbar_wait(acce + 8u, (blk - 1) & 1u, status);
+          __syncwarp();
+          gate_sync(failed);
+          ++blk;
+        }
+      }
+    }
+    // the last lifetime drained
+    if (lane == 0 && !failed && blk > 0) {
+      mbar_wait(acce, (blk - 1) & 1u, status);
+      mbar_wait(acce + 8u, (blk - 1) & 1u, status);
+    }
+    __syncwarp();
+  } else if (warp == kIssueWarp) {
+    uint32_t g = 0;
+    bool failed = false;
+    for (int item = blockIdx.x; item < ex.n_items; item += gridDim.x) {
+      const int nst = ex_decode(ex, item).nst;
+      for (int s = 0; s < nst; s += 2, g += 2) {
+        const bool first = s % kBlockTiles == 0;
+        const bool last = s % kBlockTiles == kBlockTiles - 2 || s + 2 >= nst;
+        failed = gate_sync(false) || failed;
+        if (lane == 0 && !failed) {
+          tc_fence_after();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const uint32_t a = sbase + ((g + q) % kStagesEx) * kStageEx, b = a + kExABytes;
+            const uint64_t b0 = sw32_desc(b);
+            mma_f16(tmem, sw32_desc(a), b0, idesc_n(3 * kExCols), first && q == 0 ? 0u : 1u);
+            mma_f16(tmem + kExCols, sw32_desc(a + kExASlice), b0, idesc_n(2 * kExCols), 1u);
+            mma_f16(tmem + 2 * kExCols, sw32_desc(a + 2 * kExASlice), b0, idesc_n(kExCols), 1u);
+          }
+          if (last) mma_commit(accf);
+        }
+        __syncwarp();
+        if (first) failed = gate_sync(false) || failed;
+        if (lane == 0 && !failed) {
+          tc_fence_after();
+          const uint32_t d = tmem + 3 * kExCols;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const uint32_t st = (g + q) % kStagesEx;
+            const uint32_t a = sbase + st * kStageEx, b = a + kExABytes;
+            mma_f16(d, sw32_desc(a), sw32_desc(b + 3 * kExBSlice), idesc_n(3 * kExCols), first && q == 0 ? 0u : 1u);
+            mma_f16(d, sw32_desc(a + kExASlice), sw32_desc(b + 2 * kExBSlice), idesc_n(3 * kExCols), 1u);
+            mma_f16(d, sw32_desc(a + 2 * kExASlice), sw32_desc(b + kExBSlice), idesc_n(3 * kExCols), 1u);
+            mma_f16(d, sw32_desc(a + 3 * kExASlice), sw32_desc(b), idesc_n(3 * kExCols), 1u);
+            mma_f16(d + kExCols, sw32_desc(a + 4 * kExASlice), sw32_desc(b), idesc_n(2 * kExCols), 1u);
+            mma_f16(d + 2 * kExCols, sw32_desc(a + 5 * kExASlice), sw32_desc(b), idesc_n(kExCols), 1u);
+            mma_commit(empty0 + 8u * st);
+          }
+          if (last) mma_commit(accf + 8u);
+        }
+        __syncwarp();
+      }
+    }
+    // after a failure: the MMAs already issued end before the tensor memory
+    // is released
+    if (lane == 0 && failed) {
+      mma_commit(done0);
+      mbar_wait_own(done0, 0);
+    }
+    __syncwarp();
+  } else {
+    const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+    const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + half * kColsHalf;
+    uint32_t blk = 0;
+    for (int item = blockIdx.x; item < ex.n_items; item += gridDim.x) {
+      const ExItem it = ex_decode(ex, item);
+      long long hi[kColsHalf];
+      float lo[kColsHalf];
+#pragma unroll
+      for (int i = 0; i < kColsHalf; ++i) {
+        hi[i] = 0;
+        lo[i] = 0.f;
+      }
+      const int nblk = (it.nst + kBlockTiles - 1) / kBlockTiles;
+#pragma unroll 1
+      for (int c = 0; c < nblk; ++c, ++blk) {
+        mbar_wait(accf, blk & 1u, status);
+        tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < kColsHalf / 8; ++q) {
+          float v0[8], v1[8], v2[8];
+          tmem_ld8(tl + q * 8, v0);
+          tmem_ld8(tl + kExCols + q * 8, v1);
+          tmem_ld8(tl + 2 * kExCols + q * 8, v2);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int u = __float2int_rn(v0[i]) * 512 + __float2int_rn(v1[i]);  // below 2^31
+            hi[q * 8 + i] += (long long)u * (1 << 18) + (long long)__float2int_rn(v2[i]) * 512;
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive(acce);
+        mbar_wait(accf + 8u, blk & 1u, status);
+        tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < kColsHalf / 8; ++q) {
+          float v3[8], v4[8], v5[8];
+          tmem_ld8(tl + 3 * kExCols + q * 8, v3);
+          tmem_ld8(tl + 4 * kExCols + q * 8, v4);
+          tmem_ld8(tl + 5 * kExCols + q * 8, v5);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            hi[q * 8 + i] += __float2int_rn(v3[i]);
+            lo[q * 8 + i] = fmaf(fmaf(v5[i], 1.f / 512.f, v4[i]), 1.f / 512.f, lo[q * 8 + i]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive(acce + 8u);
+      }
+      const size_t base = (it.pidx * kExCols + half * kColsHalf) * kExRows + row;
+#pragma unroll
+      for (int i = 0; i < kColsHalf; ++i) {
+        ex.raw_hi[base + (size_t)i * kExRows] = hi[i];
+        ex.raw_lo[base + (size_t)i * kExRows] = lo[i];
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------- operand checks
+// One CTA per row of complex values: its exponent (largest part below 2^e)
+// and, per 512-value segment, how many elements are large.  Bands (kB) lower
+// seg_min to their counts; A rows add up how many large elements must
+// coincide with large elements of every band and raise the flag when they
+// are too few.  Zero rows are exact and pass.
+template <bool kB>
+__global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const double2* x, int nc, const int* kend) {
+  __shared__ unsigned s_max[8];
+  __shared__ int s_sum[8];
+  const int row = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int k_eff = kend ? min(kend[row], nc) : nc;
+  const int4* v = reinterpret_cast<const int4*>(x + (size_t)row * nc);
+  unsigned m = 0, any = 0;
+  for (int k = tid; k < k_eff; k += 256) {
+    const int4 d = v[k];
+    const unsigned r = (unsigned)d.y & 0x7FFFFFFFu, i = (unsigned)d.w & 0x7FFFFFFFu;
+    m = max(m, max(r, i));
+    any |= (unsigned)(d.x | d.z);
+  }
+  if (any) m = max(m, 1u);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 0) s_max[warp] = m;
+  __syncthreads();
+  m = s_max[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) m = max(m, s_max[i]);
+  const int exm = (int)(m >> 20);
+  if (tid == 0) {
+    (kB ? ex.eb : ex.ea)[row] = m ? exm - 1022 : 0;
+    if (m && (exm < 1023 - 400 || exm > 1023 + 400)) *ex.flag = 1;
+  }
+  if (m == 0) return;
+  const unsigned thr = (unsigned)max(exm - (kB ? kExSlackB : kExSlackA), 1) << 20;
+  int sum = 0;
+  for (int s = warp; s < ex.n_kseg; s += 8) {
+    int c = 0;
+    const int k1 = min(k_eff, (s + 1) * kExSeg);
+    for (int k = s * kExSeg + lane; k < k1; k += 32) {
+      const int4 d = v[k];
+      c += max((unsigned)d.y & 0x7FFFFFFFu, (unsigned)d.w & 0x7FFFFFFFu) >= thr ? 1 : 0;
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) {
+      if (kB)
+        atomicMin(&ex.seg_min[s], c);
+      else
+        sum += max(0, c + min(ex.seg_min[s], kExSeg) - min(kExSeg, nc - s * kExSeg));
+    }
+  }
+  if (kB) return;
+  if (lane == 0) s_sum[warp] = sum;
+  __syncthreads();
+  if (tid == 0) {
+    int t = 0;
+    for (int i = 0; i < 8; ++i) t += s_sum[i];
+    if ((long long)t * kExOverlap < k_eff) *ex.flag = 1;
+  }
+}
+
+// ---------------------------------------------------------------- digits
+// Element t: (row block, K tile pair, row, 8-value chunk of the 32 K values).
+__global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const double2* a, int rows, int nc) {
+  if (*ex.flag) return;
+  const int pairs = ex.kt / 2;
+  const long long total = (long long)ex.n_row_blocks * pairs * kExRows * 4;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int ch = (int)(t & 3), r = (int)(t >> 2) & (kExRows - 1);
+    const long long rest = t / (4 * kExRows);
+    const int kp = (int)(rest % pairs), rb = (int)(rest / pairs);
+    if (2 * kp >= ex.kt_lim[rb]) continue;  // zero tiles, not read by the contraction
+    const int R = rb * kExRows + r, k0 = kp * 32 + ch * 8;
+    double re[8], im[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double2 d = R < rows && k0 + j < nc ? a[(size_t)R * nc + k0 + j] : make_double2(0.0, 0.0);
+      re[j] = d.x;
+      im[j] = d.y;
+    }
+    const int e = R < rows ? ex.ea[R] : 0;
+    unsigned char* tile = ex.a_tiles + ((size_t)rb * 2 * ex.kt + 2 * kp + (ch >> 1)) * kExABytes;
+    ex_store(tile, kExASlice, r, ch & 1, ex_chunk(re, e));
+    ex_store(tile + (size_t)ex.kt * kExABytes, kExASlice, r, ch & 1, ex_chunk(im, e));
+  }
+}
+
+__global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const double2* b, int nb, int nc) {
+  if (*ex.flag) return;
+  const int pairs = ex.kt / 2;
+  const long long total = (long long)ex.n_col_blocks * pairs * ex.bands * 4;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int ch = (int)(t & 3), nl = (int)((t >> 2) % ex.bands);
+    const long long rest = t / (4 * ex.bands);
+    const int kp = (int)(rest % pairs), cb = (int)(rest / pairs);
+    const int n = cb * ex.bands + nl, k0 = kp * 32 + ch * 8;
+    double re[8], im[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double2 d = n < nb && k0 + j < nc ? b[(size_t)n * nc + k0 + j] : make_double2(0.0, 0.0);
+      re[j] = d.x;
+      im[j] = d.y;
+    }
+    const int e = n < nb ? ex.eb[n] : 0;
+    unsigned char* tile = ex.b_tiles + ((size_t)cb * 2 * ex.kt + 2 * kp + (ch >> 1)) * kExBBytes;
+    unsigned char* upper = tile + (size_t)ex.kt * kExBBytes;  // K' >= K
+    const ExChunk cr = ex_chunk(re, e), ci = ex_chunk(im, e);
+    ex_store(tile, kExBSlice, 2 * nl, ch & 1, cr);
+    ex_store(tile, kExBSlice, 2 * nl + 1, ch & 1, ci);
+    ex_store(upper, kExBSlice, 2 * nl, ch & 1, ex_negate(ci));
+    ex_store(upper, kExBSlice, 2 * nl + 1, ch & 1, cr);
+  }
+}
+
+// ---------------------------------------------------------------- epilogue
+// (hi + lo) 2^(e - 41): the 64-bit sum and the FP32 tail in FP64.
+__device__ __forceinline__ double ex_value(long long hi, double lo, int e) {
+  return scalbn((double)hi + lo, e - 41);
+}
+
+// One CTA per (row block, band block): tempz of 128 rows x 40 bands from the
+// pieces' raw sums (added as integers, so their order does not matter), times
+// weight * conj(aqsm[n1][igp]), summed over the rows of each frequency in a
+// fixed order.
+constexpr int kFinRow = kExRows + 1;
+__global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex) {
+  extern __shared__ double2 s_prod[];  // [40][129]
+  if (*ex.flag) return;
+  const int rb = blockIdx.x, cb = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rows = p.nf * p.ng, r = tid & (kExRows - 1), R = rb * kExRows + r;
+  const int g = R < rows ? R % p.ng : 0, igp = R < rows ? p.igp_of[g] : -1;
+  const double wgt = ff_column_weight(p, igp);
+  const int e_row = R < rows ? ex.ea[R] : 0, np = ex.pieces[rb];
+  const size_t base = ((size_t)rb * ex.n_col_blocks + cb) * ex.max_pieces * kExCols * kExRows + r;
+  for (int b = tid >> 7; b < 40; b += 2) {
+    const int n = cb * 40 + b;
+    double2 v = make_double2(0.0, 0.0);
+    if (igp >= 0 && n < p.nb) {
+      long long hr = 0, hi = 0;
+      double lr = 0.0, li = 0.0;
+      for (int q = 0; q < np; ++q) {
+        const size_t o = base + ((size_t)q * kExCols + 2 * b) * kExRows;
+        hr += ex.raw_hi[o];
+        hi += ex.raw_hi[o + kExRows];
+        lr += ex.raw_lo[o];
+        li += ex.raw_lo[o + kExRows];
+      }
+      const int e = e_row + ex.eb[n];
+      const double zr = ex_value(hr, lr, e), zi = ex_value(hi, li, e);
+      const double2 m = p.aqsm[(size_t)n * p.nc + igp];
+      v = make_double2((zr * m.x + zi * m.y) * wgt, (zi * m.x - zr * m.y) * wgt);
+    }
+    s_prod[b * kFinRow + r] = v;
+  }
+  __syncthreads();
+  const int f0 = rb * kExRows / p.ng, f1 = (min((rb + 1) * kExRows, rows) - 1) / p.ng;
+  for (int o = warp; o < 40 * (f1 - f0 + 1); o += 8) {
+    const int b = o % 40, f = f0 + o / 40;
+    const int lo = max(f * p.ng - rb * kExRows, 0), hi = min((f + 1) * p.ng - rb * kExRows, kExRows);
+    double sx = 0.0, sy = 0.0, tx = 0.0, ty = 0.0;
+    for (int q = lo + lane; q < hi; q += 32) {
+      const double2 v = s_prod[b * kFinRow + q];
+      sx += v.x;
+      sy += v.y;
+      if (p.vcoul2) {
+        const int ig2 = p.igp_of[(rb * kExRows + q) % p.ng];
+        const double w2 = ig2 >= 0 ? p.vfac2 * p.vcoul2[ig2] : 0.0;
+        tx += v.x * w2;
+        ty += v.y * w2;
+      }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      sx += __shfl_xor_sync(0xffffffffu, sx, d);
+      sy += __shfl_xor_sync(0xffffffffu, sy, d);
+      if (p.vcoul2) {
+        tx += __shfl_xor_sync(0xffffffffu, tx, d);
+        ty += __shfl_xor_sync(0xffffffffu, ty, d);
+      }
+    }
+    if (lane == 0) {
+      const size_t i = (((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (f - f0)) * 40 + b;
+      ex.partial[i] = make_double2(sx, sy);
+      if (p.vcoul2) ex.partial2[i] = make_double2(tx, ty);
+    }
+  }
+}
+
+// out[n][f]: one warp per entry, fixed-order compensated sum over the row blocks.
+__global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, const double2* partial, double2* out) {
+  if (*ex.flag) return;
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= p.nb * p.nf) return;
+  const int n = w / p.nf, f = w % p.nf, cb = n / 40, b = n % 40;
+  const int lo = f * p.ng / kExRows, hi = ((f + 1) * p.ng - 1) / kExRows;
+  Comp sx, sy;
+  for (int rb = lo + lane; rb <= hi; rb += 32) {
+    const double2 v = partial[(((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (f - rb * kExRows / p.ng)) * 40 + b];
+    sx.add(v.x);
+    sy.add(v.y);
+  }
+  const double x = warp_sum_comp(sx), y = warp_sum_comp(sy);
+  if (lane == 0) out[(size_t)n * p.nf + f] = make_double2(x, y);
+}
+
+size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+struct ExSizes {
+  size_t a, b, ea, eb, seg, ent, pcs, lim, hi, lo, part;
+};
+ExSizes ex_sizes(const ExactPrep& ex) {
+  ExSizes z;
+  const size_t kts = (size_t)ex.halves * ex.kt;
+  const size_t slots = (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_pieces * kExCols * kExRows;
+  z.a = up256((size_t)ex.n_row_blocks * kts * kExABytes);
+  z.b = up256((size_t)ex.n_col_blocks * kts * kExBBytes);
+  z.ea = up256(sizeof(int) * (size_t)ex.n_row_blocks * kExRows);
+  z.eb = up256(sizeof(int) * (size_t)ex.n_col_blocks * ex.bands);
+  z.seg = up256(sizeof(int) * (size_t)(ex.n_kseg + 1));
+  z.ent = up256(sizeof(int4) * (size_t)std::max(ex.n_entries, 1));
+  z.pcs = up256(sizeof(int) * (size_t)ex.n_row_blocks);
+  z.lim = z.pcs;
+  z.hi = up256(sizeof(long long) * slots);
+  z.lo = up256(sizeof(float) * slots);
+  z.part = up256(sizeof(double2) * (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_seg * ex.bands);
+  return z;
+}
+
+}  // namespace
+
+void exact_size(ExactPrep& ex, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
+                ExactTables* tables) {
+  const int rows = nf * ng;
+  ex.halves = cplx ? 2 : 1;
+  ex.bands = cplx ? kExCols / 2 : kExCols;
+  ex.kt = (nc + 31) / 32 * 2;
+  ex.n_row_blocks = (rows + kExRows - 1) / kExRows;
+  ex.n_col_blocks = (nb + ex.bands - 1) / ex.bands;
+  ex.max_seg = (kExRows + ng - 2) / ng + 1;
+  ex.n_kseg = (nc + kExSeg - 1) / kExSeg;
+  std::vector<int> kl(ex.n_row_blocks, ex.kt);
+  long long active = 0;
+  for (int rb = 0; rb < ex.n_row_blocks; ++rb) {
+    if (row_kend) {
+      int k = 0;
+      for (int r = rb * kExRows; r < std::min(rows, (rb + 1) * kExRows); ++r) k = std::max(k, std::min(row_kend[r], nc));
+      kl[rb] = (k + 31) / 32 * 2;
+    }
+    active += (long long)ex.halves * kl[rb];
+  }
+  // K splits: as few as fill the grid's waves well.  An item costs its tiles
+  // plus about 6 tiles' time for its raw sums and the ring's refill.  Ragged
+  // row limits (items of different lengths) take at least 10 items per CTA.
+  const int all = ex.halves * ex.kt;
+  const long long blocks = (long long)ex.n_row_blocks * ex.n_col_blocks;
+  long long best = LLONG_MAX;
+  int splits = 1;
+  for (int s = 1; s <= std::min(all / 2, 96); ++s) {
+    const long long items = blocks * s;
+    if (row_kend && items < 10LL * grid && s < std::min(all / 2, 96)) continue;
+    const int len = (all / 2 + s - 1) / s * 2;
+    const long long cost = (items + grid - 1) / grid * (len + 6LL);
+    if (cost < best) {
+      best = cost;
+      splits = s;
+    }
+    if (row_kend) break;
+  }
+  ex.split_tiles = (all / 2 + splits - 1) / splits * 2;
+  ex.n_splits = (all + ex.split_tiles - 1) / ex.split_tiles;
+  std::vector<int4> ent;
+  std::vector<int> pieces;
+  k_entries(ex.n_row_blocks, ex.halves, ex.kt, ex.split_tiles, ex.n_splits, kl, ent, pieces);
+  ex.n_entries = (int)ent.size();
+  ex.n_items = ex.n_entries * ex.n_col_blocks;
+  ex.max_pieces = std::max(1, *std::max_element(pieces.begin(), pieces.end()));
+  if (tables) {
+    tables->entries = std::move(ent);
+    tables->pieces = std::move(pieces);
+    tables->kt_lim = std::move(kl);
+  }
+}
+
+size_t exact_bytes(const ExactPrep& ex) {
+  const ExSizes z = ex_sizes(ex);
+  return z.a + z.b + z.ea + z.eb + z.seg + z.ent + z.pcs + z.lim + z.hi + z.lo + 2 * z.part + 1024;
+}
+
+void exact_bind(ExactPrep& ex, void* base) {
+  const ExSizes z = ex_sizes(ex);
+  char* p = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + 1023) & ~uintptr_t(1023));
+  auto take = [&](size_t bytes) {
+    char* q = p;
+    p += bytes;
+    return q;
+  };
+  ex.a_tiles = reinterpret_cast<unsigned char*>(take(z.a));
+  ex.b_tiles = reinterpret_cast<unsigned char*>(take(z.b));
+  ex.ea = reinterpret_cast<int*>(take(z.ea));
+  ex.eb = reinterpret_cast<int*>(take(z.eb));
+  ex.flag = reinterpret_cast<int*>(take(z.seg));
+  ex.seg_min = ex.flag + 1;
+  ex.entries = reinterpret_cast<const int4*>(take(z.ent));
+  ex.pieces = reinterpret_cast<const int*>(take(z.pcs));
+  ex.kt_lim = reinterpret_cast<const int*>(take(z.lim));
+  ex.raw_hi = reinterpret_cast<long long*>(take(z.hi));
+  ex.raw_lo = reinterpret_cast<float*>(take(z.lo));
+  ex.partial = reinterpret_cast<double2*>(take(z.part));
+  ex.partial2 = reinterpret_cast<double2*>(take(z.part));
+}
+
+cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t) {
+  auto up = [](const void* dst, const void* src, size_t n) {
+    return n ? cudaMemcpy(const_cast<void*>(dst), src, n, cudaMemcpyHostToDevice) : cudaSuccess;
+  };
+  cudaError_t e = up(ex.entries, t.entries.data(), sizeof(int4) * t.entries.size());
+  if (e == cudaSuccess) e = up(ex.pieces, t.pieces.data(), sizeof(int) * t.pieces.size());
+  if (e == cudaSuccess) e = up(ex.kt_lim, t.kt_lim.data(), sizeof(int) * t.kt_lim.size());
+  return e;
+}
+
+cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(ex.flag, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * (size_t)ex.n_kseg, s);
+}
+
+cudaError_t launch_exact_b(const ExactPrep& ex, const double2* b, int nb, int nc, cudaStream_t s) {
+  exact_stats_kernel<true><<<nb, 256, 0, s>>>(ex, b, nc, nullptr);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  exact_slice_b_kernel<<<152 * 8, 256, 0, s>>>(ex, b, nb, nc);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int nc, const int* row_kend,
+                           cudaStream_t s) {
+  exact_stats_kernel<false><<<rows, 256, 0, s>>>(ex, a, nc, row_kend);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  exact_slice_a_kernel<<<152 * 16, 256, 0, s>>>(ex, a, rows, nc);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(exact_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemEx);
+  if (e != cudaSuccess) return e;
+  exact_gemm_kernel<<<std::min(grid, ex.n_items), kThreadsEx, kSmemEx, s>>>(ex, status);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s) {
+  const int smem = 40 * kFinRow * (int)sizeof(double2);
+  cudaError_t e = cudaFuncSetAttribute(exact_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  exact_finish_kernel<<<dim3(ex.n_row_blocks, ex.n_col_blocks), 256, smem, s>>>(d, ex);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int blocks = (d.nb * d.nf * 32 + 255) / 256;
+  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, ex.partial, out);
+  e = cudaGetLastError();
+  if (e != cudaSuccess || !out2) return e;
+  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, ex.partial2, out2);
+  return cudaGetLastError();
+}
+
+}  // namespace sigma

@@ -6,16 +6,19 @@
 #include "sigma_ff.h"
 #include "ff_internal.cuh"
 #include "ff_ozaki.cuh"
+#include "exact_gemm.cuh"
 #include "ff_plan.h"
 #include "runtime.h"
 
 struct sigma_ff_plan_s {
   int device = 0;
   int nb = 0, nc = 0, ng = 0, nf = 0, mode = 0;
-  int grid = 0;
+  int grid = 0, ex_grid = 0;
   sigma::FfDev dev{};
   sigma::FfWork work{};
   sigma::OzakiPrep oz{};
+  sigma::ExactPrep ex{};       // FP64 form on the tensor cores (ex_block set)
+  void* ex_block = nullptr;
   void* block = nullptr;
   bool timing = false;
   std::vector<cudaEvent_t> events;  // 3 per recorded execution
@@ -39,6 +42,10 @@ int ff_map_columns(int nc, int ng, const int* inv, const int* indinv, std::vecto
   }
   return SIGMA_OK;
 }
+
+// FP64 contractions from this size on run as exact digit products on the
+// tensor cores.
+constexpr double kExactMin = 1 << 22;
 
 int ff_check_shape(int nb, int nc, int ng, int nf) {
   // ngpown > ncouls is rejected as FFKer_cori/ffKernel.cpp:320-325 rejects it
@@ -141,6 +148,25 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
     delete p;
     return SIGMA_ERR_CUDA;
   }
+  if (mode == SIGMA_FF_FP64 && (double)number_bands * ncouls * ngpown * nfreq >= kExactMin) {
+    ExactTables et;
+    exact_size(p->ex, number_bands, ncouls, ngpown, nfreq, true, sms, row_kend, &et);
+    // without room for the digits the FP64 kernel keeps the work
+    if (cudaMalloc(&p->ex_block, exact_bytes(p->ex)) != cudaSuccess) {
+      cudaGetLastError();
+      p->ex_block = nullptr;
+    } else {
+      exact_bind(p->ex, p->ex_block);
+      e = exact_upload_tables(p->ex, et);
+      if (e != cudaSuccess) {
+        set_last_cuda_error(e, "cudaMemcpy(exact tables)", __LINE__);
+        sigma_ff_plan_destroy(p);
+        return SIGMA_ERR_CUDA;
+      }
+      w.run_if = p->ex.flag;
+      p->ex_grid = sms;
+    }
+  }
   *out = p;
   return SIGMA_OK;
 }
@@ -169,6 +195,7 @@ extern "C" int sigma_ff_plan_destroy(sigma_ff_plan plan) {
   cudaSetDevice(plan->device);
   for (cudaEvent_t ev : plan->events) cudaEventDestroy(ev);
   if (plan->block) cudaFree(plan->block);
+  if (plan->ex_block) cudaFree(plan->ex_block);
   cudaSetDevice(cur);
   delete plan;
   return SIGMA_OK;
@@ -256,8 +283,8 @@ int ff_execute_weighted(sigma_ff_plan plan, const sigma_complex128* I_epsR,
   if ((epsr32 || reuse_a || operands_ready) && plan->mode != SIGMA_FF_OZAKI_BF16) return SIGMA_ERR_UNSUPPORTED;
   if (operands_ready && !reuse_a) return SIGMA_ERR_UNSUPPORTED;
   if ((out2 != nullptr) != (vcoul2 != nullptr) || (out2 && vcoul)) return SIGMA_ERR_UNSUPPORTED;
-  if (out2 && plan->mode == SIGMA_FF_FP64) {
-    // the FP64 form contracts twice
+  if (out2 && plan->mode == SIGMA_FF_FP64 && !plan->ex_block) {
+    // the plain FP64 form contracts twice
     const int r = ff_execute_weighted(plan, I_epsR, aqsntemp, aqsmtemp, nullptr, vfac, schDt_matrix, stream);
     if (r != SIGMA_OK) return r;
     return ff_execute_weighted(plan, I_epsR, aqsntemp, aqsmtemp, vcoul2, vfac * vfac2, out2, stream);
@@ -281,10 +308,33 @@ int ff_execute_weighted(sigma_ff_plan plan, const sigma_complex128* I_epsR,
   if (plan->timing && plan->recorded < kFfMaxTimed) ev = &plan->events[3 * plan->recorded++];
   SIGMA_CUDA_TRY(cudaMemsetAsync(plan->work.counter, 0, 2 * sizeof(int), s));
   if (plan->mode == SIGMA_FF_FP64) {
-    if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
+    const ExactPrep& ex = plan->ex;
+    if (plan->ex_block) {
+      SIGMA_CUDA_TRY(exact_begin(ex, s));
+      SIGMA_CUDA_TRY(launch_exact_b(ex, d.aqsn, d.nb, d.nc, s));
+      SIGMA_CUDA_TRY(launch_exact_a(ex, d.epsr, d.nf * d.ng, d.nc, nullptr, s));
+      if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
+      SIGMA_CUDA_TRY(launch_exact_gemm(ex, plan->ex_grid, plan->work.status, s));
+    } else if (ev) {
+      SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
+    }
+    // with the exact form planned these run only when its flag is raised
     SIGMA_CUDA_TRY(launch_ff_fp64(d, plan->work, plan->grid, s));
     if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[1], s));
+    if (plan->ex_block)
+      SIGMA_CUDA_TRY(launch_exact_finish(d, ex, reinterpret_cast<double2*>(schDt_matrix),
+                                         reinterpret_cast<double2*>(out2), s));
     SIGMA_CUDA_TRY(launch_ff_reduce(d, plan->work, reinterpret_cast<double2*>(schDt_matrix), s));
+    if (out2) {
+      // the second output of the flagged case, with the weights multiplied
+      FfDev d2 = d;
+      d2.vcoul = vcoul2;
+      d2.vfac = vfac * vfac2;
+      d2.vcoul2 = nullptr;
+      SIGMA_CUDA_TRY(cudaMemsetAsync(plan->work.counter, 0, sizeof(int), s));
+      SIGMA_CUDA_TRY(launch_ff_fp64(d2, plan->work, plan->grid, s));
+      SIGMA_CUDA_TRY(launch_ff_reduce(d2, plan->work, reinterpret_cast<double2*>(out2), s));
+    }
   } else {
     // operands_ready: the A and B slices and the epilogue factors were
     // written by the caller's producer pass

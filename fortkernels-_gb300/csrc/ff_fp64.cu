@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) ff_fp64_kernel(FfDev p, FfWork 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FfSmem& sm = *reinterpret_cast<FfSmem*>(smem_raw);
   __shared__ int s_item;
+  if (w.run_if && !*w.run_if) return;
   const int tid = threadIdx.x, tc = tid & 15, tr = tid >> 4;
   const int blocks_per_freq = p.ngp / kFfRows;
 
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) ff_fp64_kernel(FfDev p, FfWork 
 __global__ void ff_reduce_kernel(FfDev p, FfWork w, double2* schdt) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= p.nb * p.nf) return;
+  if (warp >= p.nb * p.nf || (w.run_if && !*w.run_if)) return;
   const int n = warp / p.nf, f = warp % p.nf;
   const int blocks_per_freq = p.ngp / kFfRows;
   const int cb = n / kFfCols, c = n % kFfCols;

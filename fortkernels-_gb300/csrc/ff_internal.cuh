@@ -1,6 +1,8 @@
 // Internal declarations of the FF schDt contraction.
 #pragma once
 
+#include <vector>
+
 #include "sigma_internal.cuh"
 
 namespace sigma {
@@ -46,6 +48,8 @@ struct FfWork {
   int* counter;
   double2* partial;        // [row block][col block][split][kFfCols]
   int* status;
+  // FP64 kernels: run only when this device word is nonzero (null: always)
+  const int* run_if = nullptr;
 };
 
 // item -> (row block, band block, split); band blocks vary fastest so that
@@ -63,6 +67,14 @@ __device__ __forceinline__ FfItem ff_decode(const FfWork& w, int item) {
   t.pidx = ((size_t)t.rb * w.n_col_blocks + t.cb) * w.n_splits + t.s;
   return t;
 }
+
+// Work entries of a tiled contraction whose row blocks hold nonzero values in
+// the first kl[rb] K tiles of each of `halves` halves of kt tiles: per K split
+// (n_splits ranges of split_tiles tiles), per row block, the split's runs of
+// such tiles, (row block, piece, first tile, tiles); pieces counts each row
+// block's.
+void k_entries(int n_row_blocks, int halves, int kt, int split_tiles, int n_splits, const std::vector<int>& kl,
+               std::vector<int4>& entries, std::vector<int>& pieces);
 
 cudaError_t launch_ff_fp64(const FfDev& p, const FfWork& w, int grid, cudaStream_t s);
 int ff_fp64_blocks_per_sm();

@@ -149,6 +149,32 @@ __global__ void ozaki_group_reduce_kernel(OzGroup g) {
 
 }  // namespace
 
+// Per split, per row block: the split's tiles within [0, kl) and
+// [kt, kt + kl) (one run when they touch).
+void k_entries(int n_row_blocks, int halves, int kt, int split_tiles, int n_splits, const std::vector<int>& kl,
+               std::vector<int4>& entries, std::vector<int>& pieces) {
+  entries.clear();
+  pieces.assign(n_row_blocks, 0);
+  for (int sp = 0; sp < n_splits; ++sp) {
+    const int a = sp * split_tiles, b = std::min(halves * kt, a + split_tiles);
+    for (int rb = 0; rb < n_row_blocks; ++rb) {
+      int lo[2], hi[2], n = 0;
+      for (int h = 0; h < halves; ++h) {
+        const int x = std::max(a, h * kt), y = std::min(b, h * kt + kl[rb]);
+        if (x >= y) continue;
+        if (n > 0 && hi[n - 1] == x) {
+          hi[n - 1] = y;
+        } else {
+          lo[n] = x;
+          hi[n] = y;
+          ++n;
+        }
+      }
+      for (int i = 0; i < n; ++i) entries.push_back(make_int4(rb, pieces[rb]++, lo[i], hi[i] - lo[i]));
+    }
+  }
+}
+
 void ozaki_size(OzakiPrep& oz, const FfDev& d, int grid, const int* row_kend, OzakiTables* tables,
                 int split_tiles_hint, int items_per_cta) {
   oz.kt = (d.nc + kOzKTile - 1) / kOzKTile;
@@ -177,29 +203,9 @@ void ozaki_size(OzakiPrep& oz, const FfDev& d, int grid, const int* row_kend, Oz
   if (s > two_kt) s = two_kt;
   oz.split_tiles = (int)((two_kt + s - 1) / s);
   oz.n_splits = (two_kt + oz.split_tiles - 1) / oz.split_tiles;
-  // entries: per split, per row block, the split's tiles within [0, kl) and
-  // [kt, kt + kl) (one run when they touch)
   std::vector<int4> ent;
-  std::vector<int> pieces(oz.n_row_blocks, 0);
-  for (int sp = 0; sp < oz.n_splits; ++sp) {
-    const int a = sp * oz.split_tiles, b = std::min(two_kt, a + oz.split_tiles);
-    for (int rb = 0; rb < oz.n_row_blocks; ++rb) {
-      const int runs[2][2] = {{0, kl[rb]}, {oz.kt, oz.kt + kl[rb]}};
-      int lo[2], hi[2], n = 0;
-      for (const auto& run : runs) {
-        const int x = std::max(a, run[0]), y = std::min(b, run[1]);
-        if (x >= y) continue;
-        if (n > 0 && hi[n - 1] == x) {
-          hi[n - 1] = y;
-        } else {
-          lo[n] = x;
-          hi[n] = y;
-          ++n;
-        }
-      }
-      for (int i = 0; i < n; ++i) ent.push_back(make_int4(rb, pieces[rb]++, lo[i], hi[i] - lo[i]));
-    }
-  }
+  std::vector<int> pieces;
+  k_entries(oz.n_row_blocks, 2, oz.kt, oz.split_tiles, oz.n_splits, kl, ent, pieces);
   oz.n_entries = (int)ent.size();
   oz.n_items = oz.n_entries * oz.n_col_blocks;
   oz.max_pieces = std::max(1, *std::max_element(pieces.begin(), pieces.end()));

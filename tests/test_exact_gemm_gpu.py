@@ -1,0 +1,81 @@
+"""FP64 contractions as exact digit products on the tensor cores
+(csrc/exact_gemm.cu), at the edges of its tiles and of its operand range.
+
+Bar: 1e-14 normwise on uniform inputs.  A product's error is at most ~2^-52
+of the product of its rows' maxima, i.e. ~2^-50.5 of a uniform product's rms;
+the sums over K are exact and the FP64 epilogue adds a few 2^-53.  Inputs
+outside the split's range take the FP64 kernel, whose sums of K ~ 5000 terms
+in 16-wide chunks stay within 1e-12 of max|schDt|.
+"""
+import numpy as np
+import pytest
+
+import workload as W
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _norm(g, o):
+    return np.linalg.norm(g - o) / np.linalg.norm(o)
+
+
+@pytest.mark.parametrize("case", [
+    # number_bands, ncouls, ngpown, nfreq: band blocks of 40, row blocks of 128, K tiles of 32, blocks of 128
+    (1, 32768, 128, 1), (39, 4099, 127, 1), (40, 4096, 64, 2), (41, 4097, 43, 3), (80, 2015, 129, 1),
+    (81, 1985, 10, 26), (3, 20011, 71, 1), (200, 129, 129, 5), (513, 512, 20, 3),
+], ids=lambda c: "x".join(map(str, c)))
+def test_exact_contraction_edges(sigma_lib, case):
+    p = W.ff_random(*case, seed=31 + case[0])
+    assert case[0] * case[1] * case[2] * case[3] >= 1 << 22
+    o = O.ff_schdt(p).reshape(p.number_bands, p.nfreq)
+    assert _norm(sigma_lib.ff_host(p, sigma_lib.FF_MODE_FP64), o) <= 1e-14
+
+
+@pytest.mark.parametrize("kind", ["coherent", "decaying", "scaled_rows", "zero_rows"])
+def test_exact_contraction_value_ranges(sigma_lib, kind):
+    p = W.ff_random(45, 5003, 67, 2, seed=7)
+    k = np.arange(p.ncouls)
+    if kind == "coherent":        # every digit sum at its largest: all elements alike, no zero digits
+        p.I_epsR[:] = 0.7 + 0.9j / 1.1
+        p.aqsntemp[:] = 1 / 3 - 0.8j / 1.3
+    elif kind == "decaying":      # both operands fall off over 2^-20
+        p.I_epsR *= 2.0 ** (-20.0 * k / p.ncouls)
+        p.aqsntemp *= 2.0 ** (-20.0 * k / p.ncouls)
+    elif kind == "scaled_rows":   # rows of very different size
+        p.I_epsR *= (10.0 ** np.linspace(-30, 30, p.ngpown))[None, :, None]
+        p.aqsntemp *= (10.0 ** np.linspace(40, -40, p.number_bands))[:, None]
+    else:
+        p.I_epsR[0, 5] = 0
+        p.aqsntemp[7] = 0
+    o = O.ff_schdt(p).reshape(p.number_bands, p.nfreq)
+    g = sigma_lib.ff_host(p, sigma_lib.FF_MODE_FP64)
+    if kind == "scaled_rows":
+        assert max(_norm(g[n], o[n]) for n in range(p.number_bands)) <= 1e-14
+    else:
+        assert _norm(g, o) <= 1e-14
+    if kind == "zero_rows":
+        assert np.all(g[7] == 0)
+
+
+@pytest.mark.parametrize("kind", ["outlier", "opposed", "huge", "nan"])
+def test_out_of_range_operands_take_the_fp64_kernel(sigma_lib, kind):
+    p = W.ff_random(45, 5003, 67, 2, seed=8)
+    half = p.ncouls // 2
+    if kind == "outlier":         # one element 2^40 above its row
+        p.I_epsR[1, 3, 17] *= 2.0 ** 40
+        p.aqsntemp[4, 17] = 0.0
+    elif kind == "opposed":       # large elements never meet
+        p.I_epsR[:, :, :half] *= 1e-9
+        p.aqsntemp[:, half:] *= 1e-9
+    elif kind == "huge":
+        p.I_epsR *= 1e150
+    else:
+        p.I_epsR[0, 11, 100] = np.nan
+    g = sigma_lib.ff_host(p, sigma_lib.FF_MODE_FP64)
+    if kind == "nan":
+        assert np.all(np.isnan(g[:, 0].real)) and np.all(np.isfinite(g[:, 1]))
+        return
+    o = O.ff_schdt(p).reshape(p.number_bands, p.nfreq)
+    assert np.abs(g - o).max(axis=0).max() / np.abs(o).max() <= 1e-12
+    assert np.linalg.norm(g[:, 0] - o[:, 0]) / np.linalg.norm(o[:, 0]) <= 1e-12
