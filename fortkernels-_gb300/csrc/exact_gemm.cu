@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const do
   for (int i = 1; i < 8; ++i) m = max(m, s_max[i]);
   const int exm = (int)(m >> 20);
   if (tid == 0) {
-    (kB ? ex.eb : ex.ea)[row] = m ? exm - 1022 : 0;
+    (kB ? ex.eb : ex.ea)[row] = m ? exm - 1022 : kExZeroRow;
     if (m && (exm < 1023 - 400 || exm > 1023 + 400)) *ex.flag = 1;
   }
   if (m == 0) return;
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const 
       re[j] = d.x;
       im[j] = d.y;
     }
-    const int e = R < rows ? ex.ea[R] : 0;
+    const int e = R < rows ? ex.ea[R] : kExZeroRow;
     unsigned char* tile = ex.a_tiles + ((size_t)rb * 2 * ex.kt + 2 * kp + (ch >> 1)) * kExABytes;
     ex_store(tile, kExASlice, r, ch & 1, ex_chunk(re, e));
     ex_store(tile + (size_t)ex.kt * kExABytes, kExASlice, r, ch & 1, ex_chunk(im, e));
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const 
       re[j] = d.x;
       im[j] = d.y;
     }
-    const int e = n < nb ? ex.eb[n] : 0;
+    const int e = n < nb ? ex.eb[n] : kExZeroRow;
     unsigned char* tile = ex.b_tiles + ((size_t)cb * 2 * ex.kt + 2 * kp + (ch >> 1)) * kExBBytes;
     unsigned char* upper = tile + (size_t)ex.kt * kExBBytes;  // K' >= K
     const ExChunk cr = ex_chunk(re, e), ci = ex_chunk(im, e);

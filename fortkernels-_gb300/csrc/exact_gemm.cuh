@@ -47,6 +47,7 @@ constexpr uint32_t kExBBytes = kExSlices * kExBSlice;           // 15 KB
 // larger part is within 2^-slack of its row's maximum.
 constexpr int kExSlackA = 5, kExSlackB = 3;
 constexpr int kExOverlap = 16;   // a row pair needs K / kExOverlap coinciding large elements
+constexpr int kExZeroRow = 4096; // exponent of a row without a nonzero value (its digits are zero)
 
 // Operand layout.  halves = 2: complex, the real and imaginary parts laid
 // along K' as in the split-BF16 form,
@@ -88,6 +89,10 @@ void exact_size(ExactPrep& ex, int nb, int nc, int ng, int nf, bool cplx, int gr
 size_t exact_bytes(const ExactPrep& ex);
 void exact_bind(ExactPrep& ex, void* base);
 cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t);
+
+// Plans take the exact form from this many products on (rows x bands x K): below it
+// its ten launches cost more than the FP64 kernel.
+constexpr double kExactMin = 1 << 22;
 
 // One contraction, in order:
 //   exact_begin       clears the flag and the overlap counts
@@ -159,6 +164,15 @@ __device__ __forceinline__ void ex_store(unsigned char* tile, uint32_t slice_byt
   unsigned char* p = tile + sw32_offset(r, ch);
 #pragma unroll
   for (int i = 0; i < kExSlices; ++i) *reinterpret_cast<uint4*>(p + i * slice_bytes) = c.s[i];
+}
+
+// The same for 8 values whose digits come from a plane of doubles in shared
+// memory (a factor pass's staging).
+__device__ __forceinline__ void ex_put(unsigned char* tile, uint32_t slice_bytes, int r, int ch, const double* v, int e) {
+  double x[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) x[j] = v[j];
+  ex_store(tile, slice_bytes, r, ch, ex_chunk(x, e));
 }
 
 }  // namespace sigma

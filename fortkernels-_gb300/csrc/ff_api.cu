@@ -43,10 +43,6 @@ int ff_map_columns(int nc, int ng, const int* inv, const int* indinv, std::vecto
   return SIGMA_OK;
 }
 
-// FP64 contractions from this size on run as exact digit products on the
-// tensor cores.
-constexpr double kExactMin = 1 << 22;
-
 int ff_check_shape(int nb, int nc, int ng, int nf) {
   // ngpown > ncouls is rejected as FFKer_cori/ffKernel.cpp:320-325 rejects it
   if (nb <= 0 || nc <= 0 || ng <= 0 || nf <= 0 || ng > nc) return SIGMA_ERR_INVALID_SHAPE;

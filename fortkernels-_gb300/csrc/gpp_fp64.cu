@@ -671,6 +671,7 @@ template <int BN, int BP>
 __global__ void __launch_bounds__(kThreads, 2) sch_fp64y_kernel(GppDev p, GppWork w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
+  if (w.run_if && !*w.run_if) return;
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();

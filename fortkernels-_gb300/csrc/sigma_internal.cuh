@@ -74,6 +74,9 @@ struct GppWork {
   int ready_first = 0, ready_gs = 1;
   const unsigned* ready_m = nullptr;
   int* ready_status = nullptr;
+  // Run (kernel) / sum the partials (reduction) only when this device word is
+  // nonzero: the FP64 pass behind an exact contraction's flag (null: always).
+  const int* run_if = nullptr;
   int ready_polls = 1 << 22;   // polls of a gate word (256 ns apart) before a wait gives up
 };
 
@@ -189,6 +192,7 @@ cudaError_t launch_tensor_factors(const GppDev& p, const GppWork& w, const Mixed
 struct ReduceArgs {
   int sch_rows;       // bands whose sums come from sch partials (0: acht_n1 already holds them)
   const double2* sch_partial;
+  const int* sch_run_if;  // nonnull: acht_n1 already holds the band sums unless this word is nonzero
   int sch_ncb, sch_splits, sch_bn;
   const double2* ssx_partial;
   int ssx_ncb, ssx_splits;

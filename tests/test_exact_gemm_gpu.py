@@ -79,3 +79,40 @@ def test_out_of_range_operands_take_the_fp64_kernel(sigma_lib, kind):
     o = O.ff_schdt(p).reshape(p.number_bands, p.nfreq)
     assert np.abs(g - o).max(axis=0).max() / np.abs(o).max() <= 1e-12
     assert np.linalg.norm(g[:, 0] - o[:, 0]) / np.linalg.norm(o[:, 0]) <= 1e-12
+
+
+# GPP band sums (csrc/gpp_exact.cu).  Bars as the FP64 parity tests: 1e-12 per
+# achtemp / asxtemp output, 1e-12 of the largest band value.
+@pytest.mark.parametrize("case", [
+    # number_bands, nvband, ncouls, ngpown, stress: 16-column tiles, 64- and 512-g-vector segments, padding rows
+    (40, 1, 4096, 64, False), (39, 2, 1985, 43, True), (41, 0, 513, 129, False), (100, 3, 511, 85, False),
+    (1, 1, 32767, 43, False), (81, 8, 2049, 17, True), (300, 2, 4000, 3, False), (512, 0, 63, 63, False),
+], ids=lambda c: "x".join(map(str, c[:4])) + ("s" if c[4] else ""))
+def test_gpp_band_sums_edges(sigma_lib, case):
+    nb, nvb, nc, ng, stress = case
+    assert 3 * nb * nc * ng >= 1 << 22
+    p = W.gpp_random(nb, nvb, nc, ng, 90 + nb, stress=stress)
+    p.vcoul = np.abs(p.vcoul)
+    o, g = O.gpp(p), sigma_lib.gpp_host(p, sigma_lib.PREC_FP64)
+    assert np.all(np.abs(g[0] - o[0]) <= 1e-12 * np.abs(o[0]))
+    assert np.all(np.abs(g[1] - o[1]) <= 1e-12 * np.abs(o[1]))
+    assert np.abs(g[2] - o[2]).max() <= 1e-12 * np.abs(o[2]).max()
+
+
+@pytest.mark.parametrize("kind", ["outlier_wtilde", "outlier_aqsn", "huge_wtilde", "all_dropped", "tiny"])
+def test_gpp_band_sums_out_of_range(sigma_lib, kind):
+    p = W.gpp_random(45, 2, 3001, 37, 5)
+    if kind == "outlier_wtilde":
+        p.wtilde_array[3, 100] = complex(2.0 ** 50, 1.0)
+        p.I_eps_array[3, 100] = 2.0 ** 45
+    elif kind == "outlier_aqsn":
+        p.aqsntemp[7, 11] *= 2.0 ** 30
+    elif kind == "huge_wtilde":
+        p.wtilde_array[:] *= 1e25
+    elif kind == "all_dropped":     # one column's terms all inside the guard
+        p.wtilde_array[5, :] = 4.0 + 0.1j
+    else:
+        p.I_eps_array[:] *= 1e-60
+    o, g = O.gpp(p), sigma_lib.gpp_host(p, sigma_lib.PREC_FP64)
+    assert np.all(np.abs(g[0] - o[0]) <= 1e-12 * np.abs(o[0]))
+    assert np.abs(g[2] - o[2]).max() <= 1e-12 * np.abs(o[2]).max()
