@@ -34,11 +34,10 @@ using namespace tma;
 
 constexpr int kThreadsEx = 352;
 constexpr int kCopyWarp = 8, kIssueWarp = 9, kGateWarpEx = 10;
-constexpr uint32_t kStageEx = kExABytes + kExBBytes;  // 39 KB
 constexpr int kStagesEx = 5;
-constexpr uint32_t kSmemEx = kStagesEx * kStageEx + 1024;
+constexpr uint32_t ex_stage(int S) { return ex_a_bytes(S) + ex_b_bytes(S); }  // 39 / 42 KB
+constexpr uint32_t ex_smem(int S) { return kStagesEx * ex_stage(S) + 1024; }
 constexpr int kBlockTiles = 8;  // K tiles per accumulator lifetime (128 K values)
-constexpr int kColsHalf = kExCols / 2;
 
 // 32-byte swizzle: rows of 16 elements (32 B), 8-row groups of 256 B (layout
 // code 6 in bits 61-63).
@@ -100,7 +99,11 @@ __device__ __forceinline__ ExItem ex_decode(const ExactPrep& ex, int item) {
 
 constexpr uint32_t idesc_n(int n) { return idesc_bf16_f32(128, n); }
 
+template <int S>
 __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex, int* status) {
+  constexpr int kCols = ex_cols(S), kColsHalf = kCols / 2, kHi = S - 3;  // kHi accumulators from s = 3 on
+  constexpr uint32_t kStage = ex_stage(S), kABytes = ex_a_bytes(S), kBBytes = ex_b_bytes(S), kBSlice = ex_b_slice(S);
+  static_assert(S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
   extern __shared__ unsigned char smem_raw[];
   // full[5], empty[5], lo full, hi full, lo empty, hi empty, done
   __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
@@ -134,18 +137,18 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
       for (int item = blockIdx.x; ok && item < ex.n_items; item += gridDim.x) {
         const ExItem it = ex_decode(ex, item);
         const size_t kts = (size_t)ex.halves * ex.kt;
-        const unsigned char* a = ex.a_tiles + ((size_t)it.rb * kts + it.t0) * kExABytes;
-        const unsigned char* b = ex.b_tiles + ((size_t)it.cb * kts + it.t0) * kExBBytes;
+        const unsigned char* a = ex.a_tiles + ((size_t)it.rb * kts + it.t0) * kABytes;
+        const unsigned char* b = ex.b_tiles + ((size_t)it.cb * kts + it.t0) * kBBytes;
         for (int s = 0; s < it.nst; ++s, ++g) {
           const uint32_t st = g % kStagesEx, use = g / kStagesEx;
           if (use > 0 && !mbar_wait(empty0 + 8u * st, (use - 1) & 1u, status)) {
             ok = false;
             break;
           }
-          const uint32_t bar = full0 + 8u * st, dst = sbase + st * kStageEx;
-          mbar_expect_tx(bar, kStageEx);
-          bulk_load(dst, a + (size_t)s * kExABytes, kExABytes, bar);
-          bulk_load(dst + kExABytes, b + (size_t)s * kExBBytes, kExBBytes, bar);
+          const uint32_t bar = full0 + 8u * st, dst = sbase + st * kStage;
+          mbar_expect_tx(bar, kStage);
+          bulk_load(dst, a + (size_t)s * kABytes, kABytes, bar);
+          bulk_load(dst + kABytes, b + (size_t)s * kBBytes, kBBytes, bar);
         }
       }
       // after a failure: the copies still landing end before the CTA does
@@ -197,11 +200,11 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
           tc_fence_after();
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            const uint32_t a = sbase + ((g + q) % kStagesEx) * kStageEx, b = a + kExABytes;
+            const uint32_t a = sbase + ((g + q) % kStagesEx) * kStage, b = a + kABytes;
             const uint64_t b0 = sw32_desc(b);
-            mma_f16(tmem, sw32_desc(a), b0, idesc_n(3 * kExCols), first && q == 0 ? 0u : 1u);
-            mma_f16(tmem + kExCols, sw32_desc(a + kExASlice), b0, idesc_n(2 * kExCols), 1u);
-            mma_f16(tmem + 2 * kExCols, sw32_desc(a + 2 * kExASlice), b0, idesc_n(kExCols), 1u);
+            mma_f16(tmem, sw32_desc(a), b0, idesc_n(3 * kCols), first && q == 0 ? 0u : 1u);
+            mma_f16(tmem + kCols, sw32_desc(a + kExASlice), b0, idesc_n(2 * kCols), 1u);
+            mma_f16(tmem + 2 * kCols, sw32_desc(a + 2 * kExASlice), b0, idesc_n(kCols), 1u);
           }
           if (last) mma_commit(accf);
         }
@@ -209,17 +212,18 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         if (first) failed = gate_sync(false) || failed;
         if (lane == 0 && !failed) {
           tc_fence_after();
-          const uint32_t d = tmem + 3 * kExCols;
+          const uint32_t d = tmem + 3 * kCols;
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             const uint32_t st = (g + q) % kStagesEx;
-            const uint32_t a = sbase + st * kStageEx, b = a + kExABytes;
-            mma_f16(d, sw32_desc(a), sw32_desc(b + 3 * kExBSlice), idesc_n(3 * kExCols), first && q == 0 ? 0u : 1u);
-            mma_f16(d, sw32_desc(a + kExASlice), sw32_desc(b + 2 * kExBSlice), idesc_n(3 * kExCols), 1u);
-            mma_f16(d, sw32_desc(a + 2 * kExASlice), sw32_desc(b + kExBSlice), idesc_n(3 * kExCols), 1u);
-            mma_f16(d, sw32_desc(a + 3 * kExASlice), sw32_desc(b), idesc_n(3 * kExCols), 1u);
-            mma_f16(d + kExCols, sw32_desc(a + 4 * kExASlice), sw32_desc(b), idesc_n(2 * kExCols), 1u);
-            mma_f16(d + 2 * kExCols, sw32_desc(a + 5 * kExASlice), sw32_desc(b), idesc_n(kExCols), 1u);
+            const uint32_t a = sbase + st * kStage, b = a + kABytes;
+            // A_i times the B slices j with 3 <= i + j < S
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+              const int j0 = i < 3 ? 3 - i : 0, n = S - i - j0;
+              mma_f16(d + (i + j0 - 3) * kCols, sw32_desc(a + i * kExASlice), sw32_desc(b + j0 * kBSlice),
+                      idesc_n(n * kCols), first && q == 0 && i == 0 ? 0u : 1u);
+            }
             mma_commit(empty0 + 8u * st);
           }
           if (last) mma_commit(accf + 8u);
@@ -256,8 +260,8 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         for (int q = 0; q < kColsHalf / 8; ++q) {
           float v0[8], v1[8], v2[8];
           tmem_ld8(tl + q * 8, v0);
-          tmem_ld8(tl + kExCols + q * 8, v1);
-          tmem_ld8(tl + 2 * kExCols + q * 8, v2);
+          tmem_ld8(tl + kCols + q * 8, v1);
+          tmem_ld8(tl + 2 * kCols + q * 8, v2);
           tmem_wait_ld();
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -272,22 +276,24 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         tc_fence_after();
 #pragma unroll
         for (int q = 0; q < kColsHalf / 8; ++q) {
-          float v3[8], v4[8], v5[8];
-          tmem_ld8(tl + 3 * kExCols + q * 8, v3);
-          tmem_ld8(tl + 4 * kExCols + q * 8, v4);
-          tmem_ld8(tl + 5 * kExCols + q * 8, v5);
+          float v[kHi][8];
+#pragma unroll
+          for (int d = 0; d < kHi; ++d) tmem_ld8(tl + (3 + d) * kCols + q * 8, v[d]);
           tmem_wait_ld();
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            hi[q * 8 + i] += __float2int_rn(v3[i]);
-            lo[q * 8 + i] = fmaf(fmaf(v5[i], 1.f / 512.f, v4[i]), 1.f / 512.f, lo[q * 8 + i]);
+            hi[q * 8 + i] += __float2int_rn(v[0][i]);
+            float t = v[kHi - 1][i];
+#pragma unroll
+            for (int d = kHi - 2; d >= 1; --d) t = fmaf(t, 1.f / 512.f, v[d][i]);
+            lo[q * 8 + i] = fmaf(t, 1.f / 512.f, lo[q * 8 + i]);
           }
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive(acce + 8u);
       }
-      const size_t base = (it.pidx * kExCols + half * kColsHalf) * kExRows + row;
+      const size_t base = (it.pidx * kCols + half * kColsHalf) * kExRows + row;
 #pragma unroll
       for (int i = 0; i < kColsHalf; ++i) {
         ex.raw_hi[base + (size_t)i * kExRows] = hi[i];
@@ -302,24 +308,37 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
 }
 
 // ---------------------------------------------------------------- operand checks
-// One CTA per row of complex values: its exponent (largest part below 2^e)
-// and, per 512-value segment, how many elements are large.  Bands (kB) lower
-// seg_min to their counts; A rows add up how many large elements must
-// coincide with large elements of every band and raise the flag when they
-// are too few.  Zero rows are exact and pass.
-template <bool kB>
-__global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const double2* x, int nc, const int* kend) {
+// Magnitude bits (upper word without sign) of a value's larger part.
+template <bool kReal>
+__device__ __forceinline__ unsigned ex_mag(const int2* v, size_t k, unsigned& low) {
+  if (kReal) {
+    const int2 d = v[k];
+    low = (unsigned)d.x;
+    return (unsigned)d.y & 0x7FFFFFFFu;
+  }
+  const int4 d = reinterpret_cast<const int4*>(v)[k];
+  low = (unsigned)(d.x | d.z);
+  return max((unsigned)d.y & 0x7FFFFFFFu, (unsigned)d.w & 0x7FFFFFFFu);
+}
+
+// One CTA per row of values: its exponent (largest part below 2^e) and, per
+// 512-value segment, how many elements are large.  Bands (kB) lower seg_min
+// to their counts and seg_pow to their sums of squares (of the larger parts);
+// A rows add up how many large elements must coincide with large elements of
+// every band and raise the flag when they are too few.  Zero rows are exact
+// and pass.
+template <bool kB, bool kReal>
+__global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const void* x0, int n0, const void* x1,
+                                                          int nc) {
   __shared__ unsigned s_max[8];
   __shared__ int s_sum[8];
   const int row = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int k_eff = kend ? min(kend[row], nc) : nc;
-  const int4* v = reinterpret_cast<const int4*>(x + (size_t)row * nc);
+  const int2* v = static_cast<const int2*>(row < n0 ? x0 : x1) + (size_t)(row < n0 ? row : row - n0) * nc * (kReal ? 1 : 2);
   unsigned m = 0, any = 0;
-  for (int k = tid; k < k_eff; k += 256) {
-    const int4 d = v[k];
-    const unsigned r = (unsigned)d.y & 0x7FFFFFFFu, i = (unsigned)d.w & 0x7FFFFFFFu;
-    m = max(m, max(r, i));
-    any |= (unsigned)(d.x | d.z);
+  for (int k = tid; k < nc; k += 256) {
+    unsigned low;
+    m = max(m, ex_mag<kReal>(v, k, low));
+    any |= low;
   }
   if (any) m = max(m, 1u);
   m = __reduce_max_sync(0xffffffffu, m);
@@ -331,24 +350,37 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const do
   const int exm = (int)(m >> 20);
   if (tid == 0) {
     (kB ? ex.eb : ex.ea)[row] = m ? exm - 1022 : kExZeroRow;
-    if (m && (exm < 1023 - 400 || exm > 1023 + 400)) *ex.flag = 1;
+    if (m && (exm < 1023 - 400 || exm > 1023 + 400)) ex_raise(ex);
   }
   if (m == 0) return;
   const unsigned thr = (unsigned)max(exm - (kB ? kExSlackB : kExSlackA), 1) << 20;
   int sum = 0;
   for (int s = warp; s < ex.n_kseg; s += 8) {
     int c = 0;
-    const int k1 = min(k_eff, (s + 1) * kExSeg);
+    float q = 0.f;
+    const int k1 = min(nc, (s + 1) * kExSeg);
     for (int k = s * kExSeg + lane; k < k1; k += 32) {
-      const int4 d = v[k];
-      c += max((unsigned)d.y & 0x7FFFFFFFu, (unsigned)d.w & 0x7FFFFFFFu) >= thr ? 1 : 0;
+      unsigned low;
+      const unsigned d = ex_mag<kReal>(v, k, low);
+      c += d >= thr ? 1 : 0;
+      if (kB) {
+        // the larger part over 2^e to 20 bits: exponent d >> 20 against exm + 1
+        const int sh = exm + 1 - (int)(d >> 20);
+        const float f = sh < 100 ? __uint_as_float(((unsigned)(127 - sh) << 23) | ((d & 0xFFFFFu) << 3)) : 0.f;
+        q = fmaf(f, f, q);
+      }
     }
     c = __reduce_add_sync(0xffffffffu, c);
+    if (kB)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
     if (lane == 0) {
-      if (kB)
+      if (kB) {
         atomicMin(&ex.seg_min[s], c);
-      else
+        atomicMin(&ex.seg_pow[s], __float_as_int(q));
+      } else {
         sum += max(0, c + min(ex.seg_min[s], kExSeg) - min(kExSeg, nc - s * kExSeg));
+      }
     }
   }
   if (kB) return;
@@ -357,13 +389,14 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const do
   if (tid == 0) {
     int t = 0;
     for (int i = 0; i < 8; ++i) t += s_sum[i];
-    if ((long long)t * kExOverlap < k_eff) *ex.flag = 1;
+    if ((long long)t * kExOverlap < nc) ex_raise(ex);
   }
 }
 
 // ---------------------------------------------------------------- digits
 // Element t: (row block, K tile pair, row, 8-value chunk of the 32 K values).
 __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const double2* a, int rows, int nc) {
+  constexpr int S = 6;
   if (*ex.flag) return;
   const int pairs = ex.kt / 2;
   const long long total = (long long)ex.n_row_blocks * pairs * kExRows * 4;
@@ -382,37 +415,55 @@ __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const 
       im[j] = d.y;
     }
     const int e = R < rows ? ex.ea[R] : kExZeroRow;
-    unsigned char* tile = ex.a_tiles + ((size_t)rb * 2 * ex.kt + 2 * kp + (ch >> 1)) * kExABytes;
-    ex_store(tile, kExASlice, r, ch & 1, ex_chunk(re, e));
-    ex_store(tile + (size_t)ex.kt * kExABytes, kExASlice, r, ch & 1, ex_chunk(im, e));
+    unsigned char* tile = ex.a_tiles + ((size_t)rb * 2 * ex.kt + 2 * kp + (ch >> 1)) * ex_a_bytes(S);
+    ex_store<S>(tile, kExASlice, r, ch & 1, ex_chunk<S>(re, e));
+    ex_store<S>(tile + (size_t)ex.kt * ex_a_bytes(S), kExASlice, r, ch & 1, ex_chunk<S>(im, e));
   }
 }
 
-__global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const double2* b, int nb, int nc) {
+template <int S, bool kReal>
+__global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const void* b0, int nb0, const void* b1,
+                                                            int nb, int nc) {
   if (*ex.flag) return;
+  constexpr int kW = kReal ? 1 : 2, kBands = kReal ? ex_cols(S) : ex_cols(S) / 2;
+  constexpr uint32_t kSlice = ex_b_slice(S), kBytes = ex_b_bytes(S);
   const int pairs = ex.kt / 2;
-  const long long total = (long long)ex.n_col_blocks * pairs * ex.bands * 4;
+  const long long total = (long long)ex.n_col_blocks * pairs * kBands * 4;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(t & 3), nl = (int)((t >> 2) % ex.bands);
-    const long long rest = t / (4 * ex.bands);
+    const int ch = (int)(t & 3), nl = (int)((t >> 2) % kBands);
+    const long long rest = t / (4 * kBands);
     const int kp = (int)(rest % pairs), cb = (int)(rest / pairs);
-    const int n = cb * ex.bands + nl, k0 = kp * 32 + ch * 8;
+    const int n = cb * kBands + nl, k0 = kp * 32 + ch * 8;
+    const double* src =
+        static_cast<const double*>(n < nb0 ? b0 : b1) + ((size_t)(n < nb0 ? n : n - nb0) * nc + k0) * kW;
     double re[8], im[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const double2 d = n < nb && k0 + j < nc ? b[(size_t)n * nc + k0 + j] : make_double2(0.0, 0.0);
-      re[j] = d.x;
-      im[j] = d.y;
+      re[j] = im[j] = 0.0;
+      if (n < nb && k0 + j < nc) {
+        if (kReal) {
+          re[j] = src[j];
+        } else {
+          const double2 d = reinterpret_cast<const double2*>(src)[j];
+          re[j] = d.x;
+          im[j] = d.y;
+        }
+      }
     }
     const int e = n < nb ? ex.eb[n] : kExZeroRow;
-    unsigned char* tile = ex.b_tiles + ((size_t)cb * 2 * ex.kt + 2 * kp + (ch >> 1)) * kExBBytes;
-    unsigned char* upper = tile + (size_t)ex.kt * kExBBytes;  // K' >= K
-    const ExChunk cr = ex_chunk(re, e), ci = ex_chunk(im, e);
-    ex_store(tile, kExBSlice, 2 * nl, ch & 1, cr);
-    ex_store(tile, kExBSlice, 2 * nl + 1, ch & 1, ci);
-    ex_store(upper, kExBSlice, 2 * nl, ch & 1, ex_negate(ci));
-    ex_store(upper, kExBSlice, 2 * nl + 1, ch & 1, cr);
+    unsigned char* tile = ex.b_tiles + ((size_t)cb * ex.halves * ex.kt + 2 * kp + (ch >> 1)) * kBytes;
+    const ExChunk<S> cr = ex_chunk<S>(re, e);
+    if (kReal) {
+      ex_store<S>(tile, kSlice, nl, ch & 1, cr);
+      continue;
+    }
+    unsigned char* upper = tile + (size_t)ex.kt * kBytes;  // K' >= K
+    const ExChunk<S> ci = ex_chunk<S>(im, e);
+    ex_store<S>(tile, kSlice, 2 * nl, ch & 1, cr);
+    ex_store<S>(tile, kSlice, 2 * nl + 1, ch & 1, ci);
+    ex_store<S>(upper, kSlice, 2 * nl, ch & 1, ex_negate<S>(ci));
+    ex_store<S>(upper, kSlice, 2 * nl + 1, ch & 1, cr);
   }
 }
 
@@ -422,48 +473,69 @@ __device__ __forceinline__ double ex_value(long long hi, double lo, int e) {
   return scalbn((double)hi + lo, e - 41);
 }
 
-// One CTA per (row block, band block): tempz of 128 rows x 40 bands from the
-// pieces' raw sums (added as integers, so their order does not matter), times
-// weight * conj(aqsm[n1][igp]), summed over the rows of each frequency in a
-// fixed order.
+// Epilogue weights: conj(aqsm[n][igp]) times the column weight.  With
+// pair_bands set (the half sum's second band set), bands from pair_bands on
+// take band n - pair_bands, and in the last frequency aqsn's.
+__device__ __forceinline__ double2 ex_weight(const FfDev& p, int n, int f, int igp) {
+  const bool second = p.pair_bands > 0 && n >= p.pair_bands;
+  const double2* m = second && f == p.nf - 1 && p.pair_static ? p.aqsn : p.aqsm;
+  return m[(size_t)(second ? n - p.pair_bands : n) * p.nc + igp];
+}
+
+// One CTA per (row block, band block): tempz of 128 rows x the block's bands from the pieces' raw sums (added as integers, so their order does not
+// matter), times weight * conj(aqsm[n1][igp]), summed over the rows of each
+// frequency in a fixed order.
 constexpr int kFinRow = kExRows + 1;
+template <bool kReal>
 __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex) {
-  extern __shared__ double2 s_prod[];  // [40][129]
+  const int kBands = ex.bands, kCols = ex.cols;
+  extern __shared__ double2 s_prod[];  // [bands][129], complex or real
+  double* s_real = reinterpret_cast<double*>(s_prod);
   if (*ex.flag) return;
   const int rb = blockIdx.x, cb = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rows = p.nf * p.ng, r = tid & (kExRows - 1), R = rb * kExRows + r;
-  const int g = R < rows ? R % p.ng : 0, igp = R < rows ? p.igp_of[g] : -1;
+  const int f = R / p.ng, igp = R < rows ? p.igp_of[R % p.ng] : -1;
   const double wgt = ff_column_weight(p, igp);
   const int e_row = R < rows ? ex.ea[R] : 0, np = ex.pieces[rb];
-  const size_t base = ((size_t)rb * ex.n_col_blocks + cb) * ex.max_pieces * kExCols * kExRows + r;
-  for (int b = tid >> 7; b < 40; b += 2) {
-    const int n = cb * 40 + b;
+  const size_t base = ((size_t)rb * ex.n_col_blocks + cb) * ex.max_pieces * kCols * kExRows + r;
+  for (int b = tid >> 7; b < kBands; b += 2) {
+    const int n = cb * kBands + b;
     double2 v = make_double2(0.0, 0.0);
     if (igp >= 0 && n < p.nb) {
       long long hr = 0, hi = 0;
       double lr = 0.0, li = 0.0;
       for (int q = 0; q < np; ++q) {
-        const size_t o = base + ((size_t)q * kExCols + 2 * b) * kExRows;
+        const size_t o = base + ((size_t)q * kCols + (kReal ? b : 2 * b)) * kExRows;
         hr += ex.raw_hi[o];
-        hi += ex.raw_hi[o + kExRows];
         lr += ex.raw_lo[o];
-        li += ex.raw_lo[o + kExRows];
+        if (!kReal) {
+          hi += ex.raw_hi[o + kExRows];
+          li += ex.raw_lo[o + kExRows];
+        }
       }
       const int e = e_row + ex.eb[n];
-      const double zr = ex_value(hr, lr, e), zi = ex_value(hi, li, e);
-      const double2 m = p.aqsm[(size_t)n * p.nc + igp];
-      v = make_double2((zr * m.x + zi * m.y) * wgt, (zi * m.x - zr * m.y) * wgt);
+      const double zr = ex_value(hr, lr, e);
+      if (kReal) {
+        v.x = zr * reinterpret_cast<const double*>(p.aqsm)[(size_t)n * p.nc + igp] * wgt;
+      } else {
+        const double zi = ex_value(hi, li, e);
+        const double2 m = ex_weight(p, n, f, igp);
+        v = make_double2((zr * m.x + zi * m.y) * wgt, (zi * m.x - zr * m.y) * wgt);
+      }
     }
-    s_prod[b * kFinRow + r] = v;
+    if (kReal)
+      s_real[b * kFinRow + r] = v.x;
+    else
+      s_prod[b * kFinRow + r] = v;
   }
   __syncthreads();
   const int f0 = rb * kExRows / p.ng, f1 = (min((rb + 1) * kExRows, rows) - 1) / p.ng;
-  for (int o = warp; o < 40 * (f1 - f0 + 1); o += 8) {
-    const int b = o % 40, f = f0 + o / 40;
-    const int lo = max(f * p.ng - rb * kExRows, 0), hi = min((f + 1) * p.ng - rb * kExRows, kExRows);
+  for (int o = warp; o < kBands * (f1 - f0 + 1); o += 8) {
+    const int b = o % kBands, fo = f0 + o / kBands;
+    const int lo = max(fo * p.ng - rb * kExRows, 0), hi = min((fo + 1) * p.ng - rb * kExRows, kExRows);
     double sx = 0.0, sy = 0.0, tx = 0.0, ty = 0.0;
     for (int q = lo + lane; q < hi; q += 32) {
-      const double2 v = s_prod[b * kFinRow + q];
+      const double2 v = kReal ? make_double2(s_real[b * kFinRow + q], 0.0) : s_prod[b * kFinRow + q];
       sx += v.x;
       sy += v.y;
       if (p.vcoul2) {
@@ -483,7 +555,7 @@ __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex
       }
     }
     if (lane == 0) {
-      const size_t i = (((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (f - f0)) * 40 + b;
+      const size_t i = (((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (fo - f0)) * kBands + b;
       ex.partial[i] = make_double2(sx, sy);
       if (p.vcoul2) ex.partial2[i] = make_double2(tx, ty);
     }
@@ -495,11 +567,11 @@ __global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, const double2* partia
   if (*ex.flag) return;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= p.nb * p.nf) return;
-  const int n = w / p.nf, f = w % p.nf, cb = n / 40, b = n % 40;
+  const int n = w / p.nf, f = w % p.nf, cb = n / ex.bands, b = n % ex.bands;
   const int lo = f * p.ng / kExRows, hi = ((f + 1) * p.ng - 1) / kExRows;
   Comp sx, sy;
   for (int rb = lo + lane; rb <= hi; rb += 32) {
-    const double2 v = partial[(((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (f - rb * kExRows / p.ng)) * 40 + b];
+    const double2 v = partial[(((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (f - rb * kExRows / p.ng)) * ex.bands + b];
     sx.add(v.x);
     sy.add(v.y);
   }
@@ -510,33 +582,36 @@ __global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, const double2* partia
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 struct ExSizes {
-  size_t a, b, ea, eb, seg, ent, pcs, lim, hi, lo, part;
+  size_t a, b, ea, eb, seg, hi, lo, part;  // work
+  size_t flag, ent, pcs;                   // own
 };
 ExSizes ex_sizes(const ExactPrep& ex) {
   ExSizes z;
   const size_t kts = (size_t)ex.halves * ex.kt;
-  const size_t slots = (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_pieces * kExCols * kExRows;
-  z.a = up256((size_t)ex.n_row_blocks * kts * kExABytes);
-  z.b = up256((size_t)ex.n_col_blocks * kts * kExBBytes);
+  const size_t slots = (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_pieces * ex.cols * kExRows;
+  z.a = up256((size_t)ex.n_row_blocks * kts * ex_a_bytes(ex.slices));
+  z.b = up256((size_t)ex.n_col_blocks * kts * ex_b_bytes(ex.slices));
   z.ea = up256(sizeof(int) * (size_t)ex.n_row_blocks * kExRows);
   z.eb = up256(sizeof(int) * (size_t)ex.n_col_blocks * ex.bands);
-  z.seg = up256(sizeof(int) * (size_t)(ex.n_kseg + 1));
-  z.ent = up256(sizeof(int4) * (size_t)std::max(ex.n_entries, 1));
-  z.pcs = up256(sizeof(int) * (size_t)ex.n_row_blocks);
-  z.lim = z.pcs;
+  z.seg = up256(sizeof(int) * 2 * (size_t)ex.n_kseg);
   z.hi = up256(sizeof(long long) * slots);
   z.lo = up256(sizeof(float) * slots);
   z.part = up256(sizeof(double2) * (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_seg * ex.bands);
+  z.flag = 256;
+  z.ent = up256(sizeof(int4) * (size_t)std::max(ex.n_entries, 1));
+  z.pcs = up256(sizeof(int) * (size_t)ex.n_row_blocks);
   return z;
 }
 
 }  // namespace
 
-void exact_size(ExactPrep& ex, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
+void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
                 ExactTables* tables) {
   const int rows = nf * ng;
   ex.halves = cplx ? 2 : 1;
-  ex.bands = cplx ? kExCols / 2 : kExCols;
+  ex.slices = slices;
+  ex.cols = ex_cols(slices);
+  ex.bands = cplx ? ex.cols / 2 : ex.cols;
   ex.kt = (nc + 31) / 32 * 2;
   ex.n_row_blocks = (rows + kExRows - 1) / kExRows;
   ex.n_col_blocks = (nb + ex.bands - 1) / ex.bands;
@@ -585,32 +660,43 @@ void exact_size(ExactPrep& ex, int nb, int nc, int ng, int nf, bool cplx, int gr
   }
 }
 
-size_t exact_bytes(const ExactPrep& ex) {
+size_t exact_work_bytes(const ExactPrep& ex) {
   const ExSizes z = ex_sizes(ex);
-  return z.a + z.b + z.ea + z.eb + z.seg + z.ent + z.pcs + z.lim + z.hi + z.lo + 2 * z.part + 1024;
+  return z.a + z.b + z.ea + z.eb + z.seg + z.hi + z.lo + 2 * z.part + 1024;
+}
+size_t exact_own_bytes(const ExactPrep& ex) {
+  const ExSizes z = ex_sizes(ex);
+  return z.flag + z.ent + 2 * z.pcs + 256;
 }
 
-void exact_bind(ExactPrep& ex, void* base) {
+void exact_bind(ExactPrep& ex, void* work, void* own) {
   const ExSizes z = ex_sizes(ex);
-  char* p = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + 1023) & ~uintptr_t(1023));
+  char* p = nullptr;
+  auto from = [&](void* base, uintptr_t align) {
+    p = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + align - 1) & ~(align - 1));
+  };
   auto take = [&](size_t bytes) {
     char* q = p;
     p += bytes;
     return q;
   };
+  from(work, 1024);
   ex.a_tiles = reinterpret_cast<unsigned char*>(take(z.a));
   ex.b_tiles = reinterpret_cast<unsigned char*>(take(z.b));
   ex.ea = reinterpret_cast<int*>(take(z.ea));
   ex.eb = reinterpret_cast<int*>(take(z.eb));
-  ex.flag = reinterpret_cast<int*>(take(z.seg));
-  ex.seg_min = ex.flag + 1;
-  ex.entries = reinterpret_cast<const int4*>(take(z.ent));
-  ex.pieces = reinterpret_cast<const int*>(take(z.pcs));
-  ex.kt_lim = reinterpret_cast<const int*>(take(z.lim));
+  ex.seg_min = reinterpret_cast<int*>(take(z.seg));
+  ex.seg_pow = ex.seg_min + ex.n_kseg;
   ex.raw_hi = reinterpret_cast<long long*>(take(z.hi));
   ex.raw_lo = reinterpret_cast<float*>(take(z.lo));
   ex.partial = reinterpret_cast<double2*>(take(z.part));
   ex.partial2 = reinterpret_cast<double2*>(take(z.part));
+  from(own, 256);
+  ex.flag = reinterpret_cast<int*>(take(z.flag));
+  ex.entries = reinterpret_cast<const int4*>(take(z.ent));
+  ex.pieces = reinterpret_cast<const int*>(take(z.pcs));
+  ex.kt_lim = reinterpret_cast<const int*>(take(z.pcs));
+  ex.any = nullptr;
 }
 
 cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t) {
@@ -626,20 +712,29 @@ cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t) {
 cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(ex.flag, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
-  return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * (size_t)ex.n_kseg, s);
+  return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * 2 * (size_t)ex.n_kseg, s);
 }
 
-cudaError_t launch_exact_b(const ExactPrep& ex, const double2* b, int nb, int nc, cudaStream_t s) {
-  exact_stats_kernel<true><<<nb, 256, 0, s>>>(ex, b, nc, nullptr);
+cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const void* b1, int nb1, int nc,
+                           cudaStream_t s) {
+  const int nb = nb0 + nb1;
+  if (ex.halves == 1)
+    exact_stats_kernel<true, true><<<nb, 256, 0, s>>>(ex, b0, nb0, b1, nc);
+  else
+    exact_stats_kernel<true, false><<<nb, 256, 0, s>>>(ex, b0, nb0, b1, nc);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  exact_slice_b_kernel<<<152 * 8, 256, 0, s>>>(ex, b, nb, nc);
+  if (ex.halves == 1)
+    exact_slice_b_kernel<6, true><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
+  else if (ex.slices == 7)
+    exact_slice_b_kernel<7, false><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
+  else
+    exact_slice_b_kernel<6, false><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
   return cudaGetLastError();
 }
 
-cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int nc, const int* row_kend,
-                           cudaStream_t s) {
-  exact_stats_kernel<false><<<rows, 256, 0, s>>>(ex, a, nc, row_kend);
+cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int nc, cudaStream_t s) {
+  exact_stats_kernel<false, false><<<rows, 256, 0, s>>>(ex, a, rows, nullptr, nc);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   exact_slice_a_kernel<<<152 * 16, 256, 0, s>>>(ex, a, rows, nc);
@@ -647,17 +742,20 @@ cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int 
 }
 
 cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(exact_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemEx);
+  auto* kernel = ex.slices == 7 ? exact_gemm_kernel<7> : exact_gemm_kernel<6>;
+  const uint32_t smem = ex_smem(ex.slices);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  exact_gemm_kernel<<<std::min(grid, ex.n_items), kThreadsEx, kSmemEx, s>>>(ex, status);
+  kernel<<<std::min(grid, ex.n_items), kThreadsEx, smem, s>>>(ex, status);
   return cudaGetLastError();
 }
 
 cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s) {
-  const int smem = 40 * kFinRow * (int)sizeof(double2);
-  cudaError_t e = cudaFuncSetAttribute(exact_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int smem = ex.cols / 2 * kFinRow * (int)sizeof(double2);
+  auto* kernel = ex.halves == 1 ? exact_finish_kernel<true> : exact_finish_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  exact_finish_kernel<<<dim3(ex.n_row_blocks, ex.n_col_blocks), 256, smem, s>>>(d, ex);
+  kernel<<<dim3(ex.n_row_blocks, ex.n_col_blocks), 256, smem, s>>>(d, ex);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int blocks = (d.nb * d.nf * 32 + 255) / 256;

@@ -146,13 +146,14 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
   }
   if (mode == SIGMA_FF_FP64 && (double)number_bands * ncouls * ngpown * nfreq >= kExactMin) {
     ExactTables et;
-    exact_size(p->ex, number_bands, ncouls, ngpown, nfreq, true, sms, row_kend, &et);
+    exact_size(p->ex, 6, number_bands, ncouls, ngpown, nfreq, true, sms, row_kend, &et);
     // without room for the digits the FP64 kernel keeps the work
-    if (cudaMalloc(&p->ex_block, exact_bytes(p->ex)) != cudaSuccess) {
+    const size_t work = exact_work_bytes(p->ex);
+    if (cudaMalloc(&p->ex_block, work + exact_own_bytes(p->ex)) != cudaSuccess) {
       cudaGetLastError();
       p->ex_block = nullptr;
     } else {
-      exact_bind(p->ex, p->ex_block);
+      exact_bind(p->ex, p->ex_block, static_cast<char*>(p->ex_block) + work);
       e = exact_upload_tables(p->ex, et);
       if (e != cudaSuccess) {
         set_last_cuda_error(e, "cudaMemcpy(exact tables)", __LINE__);
@@ -307,8 +308,8 @@ int ff_execute_weighted(sigma_ff_plan plan, const sigma_complex128* I_epsR,
     const ExactPrep& ex = plan->ex;
     if (plan->ex_block) {
       SIGMA_CUDA_TRY(exact_begin(ex, s));
-      SIGMA_CUDA_TRY(launch_exact_b(ex, d.aqsn, d.nb, d.nc, s));
-      SIGMA_CUDA_TRY(launch_exact_a(ex, d.epsr, d.nf * d.ng, d.nc, nullptr, s));
+      SIGMA_CUDA_TRY(launch_exact_b(ex, d.aqsn, d.nb, nullptr, 0, d.nc, s));
+      SIGMA_CUDA_TRY(launch_exact_a(ex, d.epsr, d.nf * d.ng, d.nc, s));
       if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
       SIGMA_CUDA_TRY(launch_exact_gemm(ex, plan->ex_grid, plan->work.status, s));
     } else if (ev) {

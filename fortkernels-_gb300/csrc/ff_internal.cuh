@@ -32,6 +32,10 @@ struct FfDev {
   // extra column factor vfac2 * vcoul2[igp]
   const double* vcoul2 = nullptr;
   double vfac2 = 1.0;
+  // Exact form, half sum: bands n >= pair_bands (> 0) weight as band
+  // n - pair_bands; with pair_static the last frequency's take aqsn
+  int pair_bands = 0;
+  bool pair_static = false;
 };
 
 // Column weight of the contraction epilogue (0 for a column left out).

@@ -36,7 +36,7 @@ struct sigma_gpp_plan_s {
   sigma::FactorJob fac{};
   int fac_grid = 0;
 
-  // FP64 with one frequency set: the band sums on the tensor cores (block
+  // FP64 with one frequency set: the band sums on the tensor cores (when
   // set); schy then runs only when its flag is raised
   sigma::GppExact exact{};
   sigma::MixedPrep prep{};    // FP32 operands of the mixed path (unused for FP64)
@@ -266,7 +266,7 @@ extern "C" int sigma_gpp_plan_create(sigma_gpp_plan* plan_out, int number_bands,
     delete p;
     return SIGMA_ERR_CUDA;
   }
-  if (!mixed) gpp_exact_create(p->exact, number_bands, ncouls, ngpown, sms);
+  if (!mixed) gpp_exact_create(p->exact, kGxGpp, number_bands, ncouls, ngpown, kNW, igp_of, sms);
   p->host_inv.assign(inv_igp_index, inv_igp_index + ngpown);
   p->host_indinv.assign(indinv, indinv + ncouls);
   *plan_out = p;
@@ -405,10 +405,10 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
     SIGMA_CUDA_TRY(launch_prep_mixed(p, plan->prepw, plan->prep, s));
   GppWork main = ypath ? plan->schy : (mypath ? plan->schmy : plan->sch);
   if (tensor) main.partial = nullptr;  // band sums land in acht_n1 directly
-  const bool exact = ypath && plan->exact.block;
+  const bool exact = ypath && plan->exact;
   if (exact) {
     main.run_if = plan->exact.ex.flag;  // unless it is raised, acht_n1 too
-    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, p, s));
+    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, gx_dev(p), s));
   }
   if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
   if (tensor && plan->fused) {
@@ -436,7 +436,7 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
                                        true);
     if (st != SIGMA_OK) return st;
   } else if (ypath) {
-    if (exact) SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, p, plan->prep.status, plan->acht_n1, s));
+    if (exact) SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, gx_dev(p), plan->prep.status, plan->acht_n1, s));
     SIGMA_CUDA_TRY(launch_sch_fp64y(p, main, plan->schy_grid, s));
   }
   else if (mypath)
@@ -621,7 +621,7 @@ int gpp_host(int precision, int nb, int nvband, int nc, int ng, int nstart, int 
   if (st != SIGMA_OK) return st;
   char* a = static_cast<char*>(arena);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (precision == SIGMA_PREC_FP64 && plan->schy.n_items > 0 && !plan->exact.block) {
+  if (precision == SIGMA_PREC_FP64 && plan->schy.n_items > 0 && !plan->exact) {
     // FP64 with the shared-frequency pass: the inputs travel on a copy
     // stream while the sum runs, each piece followed by a gate word the
     // pass's items wait for.  The items run with the K split slowest, and

@@ -43,6 +43,7 @@
 #include "sigma_gpp.h"
 #include "sigma_internal.cuh"
 #include "floatfloat.cuh"
+#include "gpp_exact.cuh"
 #include "ff_plan.h"
 #include "ff_ozaki.cuh"
 #include "runtime.h"
@@ -197,6 +198,7 @@ static __device__ __noinline__ void half_wide_chunk(const HalfDev& p, double2 (*
 
 template <int NF>
 __global__ void __launch_bounds__(kThreads, 1) half_main_kernel(HalfDev p, GppWork w) {
+  if (w.run_if && !*w.run_if) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   HalfSmem<NF>& sm = *reinterpret_cast<HalfSmem<NF>*>(smem_raw);
   __shared__ int s_item, s_kmax;
@@ -701,6 +703,7 @@ struct HalfReduceArgs {
   const double2* stat_part;  // all bands, 1 per row (null without the static remainder)
   int stat_count;
   const double2* occ_ach;    // [nvband][ng][3]
+  const int* run_if;         // nonnull: only when this word is nonzero
   const double2* occ_asx;
   double2* acht_n1;  // [nb][3]
   double2* asx_n1;   // [nvband][3]
@@ -712,7 +715,7 @@ __global__ void half_reduce_bands_kernel(HalfReduceArgs a) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int n_ach = a.nb * kNW, n_asx = a.nvband * kNW, n_stat = a.stat_part ? a.nb : 0;
-  if (warp >= n_ach + n_asx + n_stat) return;
+  if (warp >= n_ach + n_asx + n_stat || (a.run_if && !*a.run_if)) return;
   Comp sx, sy;
   double2* dst;
   if (warp < n_ach) {
@@ -940,10 +943,11 @@ __global__ void __launch_bounds__(256) half_zs_slices_kernel(HalfDev p, OzakiPre
 //   stat_n1[n1]     = Ts + conj(Us) + unpaired       (static remainder)
 constexpr int kRowWarps = 8;
 __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
-    HalfDev p, const double2* t3, const double2* u3, const double2* ts, const double2* us,
-    const double2* occ_ach, const double2* occ_asx, double2* acht_n1, double2* asx_n1, double2* stat_n1) {
+    HalfDev p, const double2* t3, const double2* u3, const double2* ts, const double2* us, int stride3, int stride1,
+    const int* skip_if, const double2* occ_ach, const double2* occ_asx, double2* acht_n1, double2* asx_n1, double2* stat_n1) {
   constexpr int kVals = 4 * kNW + 2;  // ax, ay, sx, sy per frequency; qx, qy
   __shared__ double part[kRowWarps][kVals];
+  if (skip_if && *skip_if) return;
   const int n1 = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool occ = n1 < p.nvband;
@@ -1017,11 +1021,14 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
       acht_n1[n1 * kNW + iw] = make_double2(rx, ry);
       asx_n1[n1 * kNW + iw] = make_double2(ux, uy);
     } else {
-      const double2 a = t3[(size_t)n1 * kNW + iw], b = u3[(size_t)n1 * kNW + iw];
+      const double2 a = t3[(size_t)n1 * stride3 + iw], b = u3[(size_t)n1 * stride3 + iw];
       acht_n1[n1 * kNW + iw] = make_double2(rx + a.x + b.x, ry + a.y - b.y);
     }
   }
-  if (ts) stat_n1[n1] = make_double2(tot[4 * kNW] + ts[n1].x + us[n1].x, tot[4 * kNW + 1] + ts[n1].y - us[n1].y);
+  if (ts) {
+    const double2 a = ts[(size_t)n1 * stride1], b = us[(size_t)n1 * stride1];
+    stat_n1[n1] = make_double2(tot[4 * kNW] + a.x + b.x, tot[4 * kNW + 1] + a.y - b.y);
+  }
 }
 
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
@@ -1055,6 +1062,11 @@ struct sigma_gpp_halfsum_plan_s {
   sigma_ff_plan ff3 = nullptr, ff1 = nullptr;
   void* tblock = nullptr;
   float2 *m32 = nullptr, *n32 = nullptr;  // occupied bands' aqsm / aqsn rows in FP32
+  // FP64 form: T and U of the three frequencies (and the static pair) as one
+  // exact contraction over the bands of aqsn and aqsm; the FP64 passes then
+  // run only when its flag is raised
+  sigma::GppExact exact{};
+  double2* tu = nullptr;  // [2 nb][3 or 4]
   double2 *t3 = nullptr, *u3 = nullptr, *ts = nullptr, *us = nullptr;  // [nb][3], [nb][1]
 };
 
@@ -1193,6 +1205,16 @@ extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int nu
       return st;
     }
   }
+  if (!tensor) {
+    const int nf = (flags & SIGMA_HALFSUM_STATIC) ? kNW + 1 : kNW;
+    if (gpp_exact_create(p->exact, kGxHalf, number_bands, ncouls, ngpown, nf, igp_of, sms) &&
+        cudaMalloc(&p->tblock, sizeof(double2) * 2 * (size_t)number_bands * nf) != cudaSuccess) {
+      cudaGetLastError();
+      p->tblock = nullptr;
+      gpp_exact_destroy(p->exact);
+    }
+    p->tu = static_cast<double2*>(p->tblock);
+  }
   *out = p;
   return SIGMA_OK;
 }
@@ -1206,6 +1228,7 @@ extern "C" int sigma_gpp_halfsum_plan_destroy(sigma_gpp_halfsum_plan p) {
   if (p->ff3) sigma_ff_plan_destroy(p->ff3);
   if (p->ff1) sigma_ff_plan_destroy(p->ff1);
   if (p->tblock) cudaFree(p->tblock);
+  sigma::gpp_exact_destroy(p->exact);
   cudaSetDevice(cur);
   delete p;
   return SIGMA_OK;
@@ -1246,7 +1269,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
   }
   HalfDev p{plan->nb, plan->nvband, plan->nc, plan->ng, occ, aqsm, aqsn, ieps, wt,
             vcoul, wx_array, plan->igp_of, plan->brk};
-  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 2 * sizeof(int), s));
+  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 3 * sizeof(int), s));
   if (plan->nvband > 0) {
     half_brk_kernel<<<plan->ng, kThreads, 0, s>>>(p, plan->brk);
     SIGMA_CUDA_TRY(cudaGetLastError());
@@ -1288,7 +1311,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
     }
     if (st != SIGMA_OK) return st;
     half_tensor_rows_kernel<<<plan->nb, kRowWarps * 32, 0, s>>>(
-        p, plan->t3, plan->u3, stat ? plan->ts : nullptr, plan->us, plan->occ_ach, plan->occ_asx,
+        p, plan->t3, plan->u3, stat ? plan->ts : nullptr, plan->us, kNW, 1, nullptr, plan->occ_ach, plan->occ_asx,
         plan->acht_n1, plan->asx_n1, plan->stat_n1);
     SIGMA_CUDA_TRY(cudaGetLastError());
     half_reduce_total_kernel<<<1, 256, 0, s>>>(plan->acht_n1, plan->asx_n1, plan->stat_n1, plan->nb,
@@ -1299,10 +1322,26 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
     SIGMA_CUDA_TRY(cudaGetLastError());
     return SIGMA_OK;
   }
-  if (plan->wm.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<3>(p, plan->wm, plan->main_grid, s));
   const bool stat = plan->ws.partial && achstemp;
-  if (stat && plan->ws.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<1>(p, plan->ws, plan->stat_grid, s));
+  GppWork wm = plan->wm, ws = plan->ws;
+  const int* flag = nullptr;
+  if (plan->exact) {
+    auto D = [](const double2* x) { return reinterpret_cast<const double*>(x); };
+    const GxDev x{plan->nb, plan->nc, plan->ng, D(aqsm), D(aqsn), D(ieps), D(wt), vcoul, wx_array, plan->igp_of};
+    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s));
+    SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->tu, s));
+    const int nf = plan->exact.nf;
+    const double2* u = plan->tu + (size_t)plan->nb * nf;
+    wm.run_if = ws.run_if = flag = plan->exact.ex.flag;
+    half_tensor_rows_kernel<<<plan->nb, kRowWarps * 32, 0, s>>>(
+        p, plan->tu, u, stat ? plan->tu + kNW : nullptr, u + kNW, nf, nf, flag, plan->occ_ach, plan->occ_asx,
+        plan->acht_n1, plan->asx_n1, plan->stat_n1);
+    SIGMA_CUDA_TRY(cudaGetLastError());
+  }
+  if (plan->wm.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<3>(p, wm, plan->main_grid, s));
+  if (stat && plan->ws.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<1>(p, ws, plan->stat_grid, s));
   HalfReduceArgs a;
+  a.run_if = flag;
   a.nb = plan->nb;
   a.nvband = plan->nvband;
   a.ng = plan->ng;

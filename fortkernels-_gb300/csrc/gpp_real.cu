@@ -32,6 +32,7 @@
 #include "sigma_gpp.h"
 #include "sigma_internal.cuh"
 #include "floatfloat.cuh"
+#include "gpp_exact.cuh"
 #include "runtime.h"
 
 namespace sigma {
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(kThreads, 2) sch_real_kernel(GppRealDev p, Gpp
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RealSmem& sm = *reinterpret_cast<RealSmem*>(smem_raw);
   __shared__ int s_item;
+  if (w.run_if && !*w.run_if) return;
   constexpr int TB = kRBN / 16, TC = kRBP / 16;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const double wx0 = p.wx[0], wx1 = p.wx[1], wx2 = p.wx[2];
@@ -341,6 +343,7 @@ struct sigma_gpp_real_plan_s {
   int device = 0, nb = 0, nvband = 0, nc = 0, ng = 0;
   int sch_grid = 0, ssx_grid = 0;
   sigma::GppWork sch{}, ssx{};
+  sigma::GppExact exact{};  // when set, sch runs only when its flag is raised
   void* block = nullptr;
   int* igp_of = nullptr;
   int* counters = nullptr;
@@ -409,6 +412,7 @@ extern "C" int sigma_gpp_real_plan_create(sigma_gpp_real_plan* out, int number_b
     delete p;
     return SIGMA_ERR_CUDA;
   }
+  gpp_exact_create(p->exact, kGxReal, number_bands, ncouls, ngpown, kNW, igp_of, sms);
   *out = p;
   return SIGMA_OK;
 }
@@ -419,6 +423,7 @@ extern "C" int sigma_gpp_real_plan_destroy(sigma_gpp_real_plan p) {
   cudaGetDevice(&cur);
   cudaSetDevice(p->device);
   if (p->block) cudaFree(p->block);
+  sigma::gpp_exact_destroy(p->exact);
   cudaSetDevice(cur);
   delete p;
   return SIGMA_OK;
@@ -440,14 +445,21 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GppRealDev p{plan->nb, plan->nvband, plan->nc, plan->ng, occ, aqsmtemp, aqsntemp, I_eps_array,
                wtilde_array, vcoul, wx_array, plan->igp_of};
-  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 2 * sizeof(int), s));
+  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 3 * sizeof(int), s));
+  GppWork sch = plan->sch;
+  if (plan->exact) {
+    const GxDev x{p.nb, p.nc, p.ng, p.aqsm, p.aqsn, p.ieps, p.wt, p.vcoul, p.wx, p.igp_of};
+    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s));
+    SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->acht_n1, s));
+    sch.run_if = plan->exact.ex.flag;
+  }
   if (plan->sch.n_items > 0) {
     SIGMA_CUDA_TRY(cudaFuncSetAttribute(sch_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sizeof(RealSmem)));
     // two CTAs per SM hold ~180 KB of shared memory between them
     SIGMA_CUDA_TRY(cudaFuncSetAttribute(sch_real_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared));
-    sch_real_kernel<<<plan->sch_grid, kThreads, sizeof(RealSmem), s>>>(p, plan->sch);
+    sch_real_kernel<<<plan->sch_grid, kThreads, sizeof(RealSmem), s>>>(p, sch);
     SIGMA_CUDA_TRY(cudaGetLastError());
   }
   if (plan->ssx.n_items > 0) {
@@ -457,7 +469,7 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
   double2* ach_c = plan->outc;
   double2* asx_c = plan->outc + kNW;
   double2* n1_c = plan->outc + 2 * kNW;
-  SIGMA_CUDA_TRY(launch_gpp_reduce(plan->sch, plan->ssx, plan->nb, plan->acht_n1, ach_c, asx_c,
+  SIGMA_CUDA_TRY(launch_gpp_reduce(sch, plan->ssx, plan->nb, plan->acht_n1, ach_c, asx_c,
                                    acht_n1_loc ? n1_c : nullptr, s));
   const int nthreads = 256, n = std::max(plan->nb, kNW);
   real_parts_kernel<<<(n + nthreads - 1) / nthreads, nthreads, 0, s>>>(ach_c, asx_c, n1_c, plan->nb,

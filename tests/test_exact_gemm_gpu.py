@@ -116,3 +116,34 @@ def test_gpp_band_sums_out_of_range(sigma_lib, kind):
     o, g = O.gpp(p), sigma_lib.gpp_host(p, sigma_lib.PREC_FP64)
     assert np.all(np.abs(g[0] - o[0]) <= 1e-12 * np.abs(o[0]))
     assert np.abs(g[2] - o[2]).max() <= 1e-12 * np.abs(o[2]).max()
+
+
+# Real-valued sums: 80 bands per block, and the half sum: seven digits, 32
+# bands per block over aqsn's and aqsm's bands, rows that end at their igp.
+@pytest.mark.parametrize("case", [
+    (80, 2, 4096, 43), (81, 1, 2017, 128), (159, 0, 513, 87), (5, 5, 16384, 63),
+], ids=lambda c: "x".join(map(str, c)))
+def test_real_band_sums_edges(sigma_lib, case):
+    assert 3 * case[0] * case[2] * case[3] >= 1 << 22
+    p = W.gpp_real_random(*case, seed=200 + case[0])
+    o, g = O.gpp_real(p), sigma_lib.gpp_real_host(p)
+    assert np.all(np.abs(g[0] - o[0]) <= 1e-12 * np.abs(o[0]))
+    assert np.all(np.abs(g[1] - o[1]) <= 1e-12 * np.abs(o[1]).max())
+    assert np.abs(g[2] - o[2]).max() <= 1e-12 * np.abs(o[2]).max()
+
+
+@pytest.mark.parametrize("case", [
+    (64, 2, 2048, 32, False), (31, 0, 4100, 96, True), (33, 3, 1025, 97, False), (129, 1, 3000, 43, True),
+    (16, 16, 5121, 65, False),
+], ids=lambda c: "x".join(map(str, c[:4])) + ("s" if c[4] else ""))
+@pytest.mark.parametrize("static", [True, False], ids=["static", "nostatic"])
+def test_halfsum_edges(sigma_lib, case, static):
+    nb, nvb, nc, ng, stress = case
+    assert 3 * nb * nc * ng >= 1 << 22
+    p = W.gpp_random(nb, nvb, nc, ng, 300 + nb, stress=stress)
+    o, g = O.gpp_halfsum(p), sigma_lib.gpp_halfsum_host(p, want_static=static)
+    assert np.all(np.abs(g[0] - o[0]) <= 1e-12 * np.abs(o[0]))
+    assert np.all(np.abs(g[1] - o[1]) <= 1e-12 * np.abs(o[1]))
+    assert np.abs(g[2] - o[2]).max() <= 1e-12 * np.abs(o[2]).max()
+    if static:
+        assert abs(g[3] - o[3]) <= 1e-12 * abs(o[3])
