@@ -33,6 +33,7 @@
 #include "ff_plan.h"
 #include "ff_ozaki.cuh"
 #include "gpp_tensor.cuh"
+#include "gpp_exact.cuh"
 #include "runtime.h"
 
 namespace sigma {
@@ -59,6 +60,11 @@ struct sigma_gpp_batch_s {
   int* counters = nullptr;  // [0] main pass, [1] occupied-band pass, [2] status
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  // FP64 with one frequency set per instance: exact contractions in stream
+  // order over one shared workspace; the queue's main pass then takes only
+  // the instances without one or with a raised flag
+  std::vector<sigma::GppExact> exact;
+  void* exact_ws = nullptr;
   // tensor form
   std::vector<sigma_ff_plan> ff;   // per instance (3 slabs, GPP column map)
   void* tensor_ws = nullptr;       // slice images: one region per instance (grouped) or one shared
@@ -278,6 +284,38 @@ int build_tensor_group(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst,
   g.r_warps = rwarps;
   g.status = b->counters + 2;
   return SIGMA_OK;
+}
+
+// FP64 with shared frequencies: an exact contraction per instance that is
+// large enough, when the device has room for the largest one's workspace.
+void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std::vector<std::vector<int>>& igp,
+                 int sms) {
+  size_t ws = 0;
+  bool all = true;
+  auto fits = [](const sigma_gpp_instance& q) {
+    return (double)kNW * q.ngpown * q.number_bands * q.ncouls >= kExactMin;
+  };
+  for (int i = 0; i < b->n; ++i)
+    if (fits(inst[i]))
+      ws = std::max(ws, gpp_exact_work_bytes(kGxGpp, inst[i].number_bands, inst[i].ncouls, inst[i].ngpown, kNW, igp[i],
+                                             sms));
+  if (ws == 0) return;
+  if (cudaMalloc(&b->exact_ws, ws) != cudaSuccess) {
+    cudaGetLastError();
+    b->exact_ws = nullptr;
+    return;
+  }
+  b->exact.resize(b->n);
+  for (int i = 0; i < b->n; ++i)
+    all = (fits(inst[i]) && gpp_exact_create(b->exact[i], kGxGpp, inst[i].number_bands, inst[i].ncouls,
+                                             inst[i].ngpown, kNW, igp[i], sms, b->exact_ws)) && all;
+  for (int i = 0; i < b->n; ++i)
+    if (b->exact[i]) {
+      b->sch[i].run_if = b->exact[i].ex.flag;
+      b->exact[i].ex.any = b->counters + 3;
+    }
+  // no instance needs the queue's main pass unless some flag is raised
+  if (all) b->sch_view.run_if = b->counters + 3;
 }
 
 // The grouped reductions of every form: one job per instance.
@@ -518,6 +556,7 @@ extern "C" int sigma_gpp_batch_create_tuned(sigma_gpp_batch* out, int n_instance
   };
   for (int i = 0; i < n_instances; ++i) up(o_igp[i], igp[i].data(), sizeof(int) * igp[i].size());
   up(o_dev, b->dev.data(), sizeof(GppDev) * n_instances);
+  if (precision == SIGMA_PREC_FP64 && all_shared && rc == SIGMA_OK) build_exact(b, inst, igp, sms);
   up(o_wsch, b->sch.data(), sizeof(GppWork) * n_instances);
   up(o_wssx, b->ssx.data(), sizeof(GppWork) * n_instances);
   up(o_prep, b->prep.data(), sizeof(MixedPrep) * n_instances);
@@ -525,8 +564,7 @@ extern "C" int sigma_gpp_batch_create_tuned(sigma_gpp_batch* out, int n_instance
   up(o_ssxoff, b->ssx_off.data(), sizeof(int) * (n_instances + 1));
   up(o_tile, b->tile.data(), sizeof(int) * n_instances);
   if (rc != SIGMA_OK) {
-    cudaFree(b->block);
-    delete b;
+    sigma_gpp_batch_destroy(b);
     return rc;
   }
   GppBatchView& v = b->sch_view;
@@ -539,6 +577,7 @@ extern "C" int sigma_gpp_batch_create_tuned(sigma_gpp_batch* out, int n_instance
   v.total = b->sch_off[n_instances];
   v.counter = b->counters;
   b->ssx_view = v;
+  b->ssx_view.run_if = nullptr;
   b->ssx_view.work = reinterpret_cast<const GppWork*>(base + o_wssx);
   b->ssx_view.item_off = reinterpret_cast<const int*>(base + o_ssxoff);
   b->ssx_view.total = b->ssx_off[n_instances];
@@ -547,6 +586,7 @@ extern "C" int sigma_gpp_batch_create_tuned(sigma_gpp_batch* out, int n_instance
   if (b->ssx_grid > b->ssx_view.total) b->ssx_grid = std::max(1, b->ssx_view.total);
   // every form: the two fixed-order reductions for all instances
   b->launches = (mixed ? 2 * n_instances : 0) + 1 + (b->ssx_view.total > 0 ? 1 : 0) + 2;
+  for (const GppExact& x : b->exact) b->launches += x ? kGxLaunches : 0;
   if (tensor && grouped) {
     int st = build_tensor_group(b, inst, igp, sms);
     if (st != SIGMA_OK) {
@@ -642,7 +682,13 @@ extern "C" int sigma_gpp_batch_execute(sigma_gpp_batch b, void* stream) {
                                          true);
       if (st != SIGMA_OK) return st;
     }
-  } else if (b->sch_view.total > 0)
+  }
+  for (int i = 0; i < (int)b->exact.size(); ++i)
+    if (b->exact[i]) {
+      SIGMA_CUDA_TRY(launch_gpp_exact_operands(b->exact[i], gx_dev(b->dev[i]), s));
+      SIGMA_CUDA_TRY(launch_gpp_exact_sums(b->exact[i], gx_dev(b->dev[i]), b->counters + 2, b->acht_n1[i], s));
+    }
+  if (!tensor && b->sch_view.total > 0)
     SIGMA_CUDA_TRY(b->mixedy ? launch_sch_mixedy_batch(b->sch_view, b->sch_grid, s)
                    : mixed ? launch_sch_mixed_batch(b->sch_view, b->sch_grid, s)
                          : (b->all_shared_wx ? launch_sch_fp64y_batch(b->sch_view, b->sch_grid, b->fp64y_small, s)
@@ -707,6 +753,8 @@ extern "C" int sigma_gpp_batch_destroy(sigma_gpp_batch b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   for (sigma_ff_plan f : b->ff)
     if (f) sigma_ff_plan_destroy(f);
+  for (sigma::GppExact& x : b->exact) sigma::gpp_exact_destroy(x);
+  if (b->exact_ws) cudaFree(b->exact_ws);
   if (b->tensor_ws) cudaFree(b->tensor_ws);
   if (b->group_block) cudaFree(b->group_block);
   if (b->red_block) cudaFree(b->red_block);

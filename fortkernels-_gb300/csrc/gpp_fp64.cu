@@ -748,6 +748,7 @@ template <bool kSmall>
 __global__ void __launch_bounds__(kThreads, kSmall ? 2 : 1) sch_fp64y_batch_kernel(GppBatchView b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
+  if (b.run_if && !*b.run_if) return;
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -758,6 +759,7 @@ __global__ void __launch_bounds__(kThreads, kSmall ? 2 : 1) sch_fp64y_batch_kern
     const int inst = batch_owner(b.item_off, b.n_inst, g);
     const GppDev p = b.dev[inst];
     const GppWork w = b.work[inst];
+    if (w.run_if && !*w.run_if) continue;
     const int local = g - b.item_off[inst];
     sch_fp64y_batch_item<kSmall>(p, w, b.tile[inst], local, smem_raw, tid);
   }

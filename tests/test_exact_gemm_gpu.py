@@ -147,3 +147,33 @@ def test_halfsum_edges(sigma_lib, case, static):
     assert np.abs(g[2] - o[2]).max() <= 1e-12 * np.abs(o[2]).max()
     if static:
         assert abs(g[3] - o[3]) <= 1e-12 * abs(o[3])
+
+
+def test_batch_mixes_exact_flagged_and_small_instances(sigma_lib):
+    import torch
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.float64).copy()).cuda()
+    probs = [W.gpp_random(60, 2, 2048, 50, 1), W.gpp_random(9, 1, 300, 20, 2), W.gpp_random(70, 3, 3001, 33, 3)]
+    probs[2].aqsntemp[3, 5] *= 2.0 ** 35   # outside the split's range
+    outs, inst = [], []
+    for p in probs:
+        o = [torch.zeros(n, dtype=torch.float64, device="cuda") for n in (6, 6, 2 * p.number_bands)]
+        outs.append(o)
+        inst.append(dict(number_bands=p.number_bands, nvband=p.nvband, ncouls=p.ncouls, ngpown=p.ngpown,
+                         inv_igp_index=p.inv_igp_index, indinv=p.indinv, wx_array=dev(p.wx_array),
+                         aqsmtemp=dev(p.aqsmtemp), aqsntemp=dev(p.aqsntemp), I_eps_array=dev(p.I_eps_array),
+                         wtilde_array=dev(p.wtilde_array), vcoul=dev(p.vcoul), achtemp=o[0], asxtemp=o[1],
+                         acht_n1_loc=o[2]))
+    for k in ([0, 1, 2], [0], [0, 2]):   # with and without an instance that always takes the queue
+        for o in outs:
+            for t in o:
+                t.zero_()
+        b = sigma_lib.GppBatch([inst[i] for i in k], sigma_lib.PREC_FP64)
+        b.execute()
+        torch.cuda.synchronize()
+        assert b.status() == 0
+        b.close()
+        for i in k:
+            ref = O.gpp(probs[i])
+            got = [t.cpu().numpy().view(np.complex128) for t in outs[i]]
+            for x, y in zip(got, ref):
+                assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max()
