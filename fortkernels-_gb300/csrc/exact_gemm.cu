@@ -88,12 +88,15 @@ struct ExItem {
 // blocks of one K split, the splits slowest.
 __device__ __forceinline__ ExItem ex_decode(const ExactPrep& ex, int item) {
   ExItem t;
-  t.cb = item % ex.n_col_blocks;
-  const int4 e = ex.entries[item / ex.n_col_blocks];
+  const int main_items = ex.n_main_entries * ex.n_col_blocks;
+  const bool main = item < main_items;
+  const int i = main ? item : item - main_items, n = main ? ex.n_col_blocks : ex.n_col_blocks2;
+  t.cb = i % n;
+  const int4 e = ex.entries[(main ? 0 : ex.n_main_entries) + i / n];
   t.rb = e.x;
   t.t0 = e.z;
   t.nst = e.w;
-  t.pidx = ((size_t)t.rb * ex.n_col_blocks + t.cb) * ex.max_pieces + e.y;
+  t.pidx = ex_block_index(ex, t.rb, t.cb) * ex.max_pieces + e.y;
   return t;
 }
 
@@ -487,17 +490,19 @@ __device__ __forceinline__ double2 ex_weight(const FfDev& p, int n, int f, int i
 // frequency in a fixed order.
 constexpr int kFinRow = kExRows + 1;
 template <bool kReal>
-__global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex) {
+__global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex, int rb0) {
   const int kBands = ex.bands, kCols = ex.cols;
   extern __shared__ double2 s_prod[];  // [bands][129], complex or real
   double* s_real = reinterpret_cast<double*>(s_prod);
   if (*ex.flag) return;
+  // row block rb of the group whose row blocks start at rb0
   const int rb = blockIdx.x, cb = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rows = p.nf * p.ng, r = tid & (kExRows - 1), R = rb * kExRows + r;
+  const size_t block = ex_block_index(ex, rb0 + rb, cb);
   const int f = R / p.ng, igp = R < rows ? p.igp_of[R % p.ng] : -1;
   const double wgt = ff_column_weight(p, igp);
-  const int e_row = R < rows ? ex.ea[R] : 0, np = ex.pieces[rb];
-  const size_t base = ((size_t)rb * ex.n_col_blocks + cb) * ex.max_pieces * kCols * kExRows + r;
+  const int e_row = R < rows ? ex.ea[rb0 * kExRows + R] : 0, np = ex.pieces[rb0 + rb];
+  const size_t base = block * ex.max_pieces * kCols * kExRows + r;
   for (int b = tid >> 7; b < kBands; b += 2) {
     const int n = cb * kBands + b;
     double2 v = make_double2(0.0, 0.0);
@@ -555,7 +560,7 @@ __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex
       }
     }
     if (lane == 0) {
-      const size_t i = (((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (fo - f0)) * kBands + b;
+      const size_t i = (block * ex.max_seg + (fo - f0)) * kBands + b;
       ex.partial[i] = make_double2(sx, sy);
       if (p.vcoul2) ex.partial2[i] = make_double2(tx, ty);
     }
@@ -563,7 +568,7 @@ __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex
 }
 
 // out[n][f]: one warp per entry, fixed-order compensated sum over the row blocks.
-__global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, const double2* partial, double2* out) {
+__global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, int rb0, const double2* partial, double2* out) {
   if (*ex.flag) return;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= p.nb * p.nf) return;
@@ -571,7 +576,7 @@ __global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, const double2* partia
   const int lo = f * p.ng / kExRows, hi = ((f + 1) * p.ng - 1) / kExRows;
   Comp sx, sy;
   for (int rb = lo + lane; rb <= hi; rb += 32) {
-    const double2 v = partial[(((size_t)rb * ex.n_col_blocks + cb) * ex.max_seg + (f - rb * kExRows / p.ng)) * ex.bands + b];
+    const double2 v = partial[(ex_block_index(ex, rb0 + rb, cb) * ex.max_seg + (f - rb * kExRows / p.ng)) * ex.bands + b];
     sx.add(v.x);
     sy.add(v.y);
   }
@@ -588,7 +593,8 @@ struct ExSizes {
 ExSizes ex_sizes(const ExactPrep& ex) {
   ExSizes z;
   const size_t kts = (size_t)ex.halves * ex.kt;
-  const size_t slots = (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_pieces * ex.cols * kExRows;
+  const size_t blocks = ex_block_index(ex, ex.n_row_blocks, 0);
+  const size_t slots = blocks * ex.max_pieces * ex.cols * kExRows;
   z.a = up256((size_t)ex.n_row_blocks * kts * ex_a_bytes(ex.slices));
   z.b = up256((size_t)ex.n_col_blocks * kts * ex_b_bytes(ex.slices));
   z.ea = up256(sizeof(int) * (size_t)ex.n_row_blocks * kExRows);
@@ -596,7 +602,7 @@ ExSizes ex_sizes(const ExactPrep& ex) {
   z.seg = up256(sizeof(int) * 2 * (size_t)ex.n_kseg);
   z.hi = up256(sizeof(long long) * slots);
   z.lo = up256(sizeof(float) * slots);
-  z.part = up256(sizeof(double2) * (size_t)ex.n_row_blocks * ex.n_col_blocks * ex.max_seg * ex.bands);
+  z.part = up256(sizeof(double2) * blocks * ex.max_seg * ex.bands);
   z.flag = 256;
   z.ent = up256(sizeof(int4) * (size_t)std::max(ex.n_entries, 1));
   z.pcs = up256(sizeof(int) * (size_t)ex.n_row_blocks);
@@ -606,32 +612,30 @@ ExSizes ex_sizes(const ExactPrep& ex) {
 }  // namespace
 
 void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
-                ExactTables* tables) {
+                ExactTables* tables, int nf2, int nb2) {
   const int rows = nf * ng;
   ex.halves = cplx ? 2 : 1;
   ex.slices = slices;
   ex.cols = ex_cols(slices);
   ex.bands = cplx ? ex.cols / 2 : ex.cols;
   ex.kt = (nc + 31) / 32 * 2;
-  ex.n_row_blocks = (rows + kExRows - 1) / kExRows;
+  ex.n_main_blocks = (rows + kExRows - 1) / kExRows;
+  ex.n_row_blocks = ex.n_main_blocks + (nf2 * ng + kExRows - 1) / kExRows;
   ex.n_col_blocks = (nb + ex.bands - 1) / ex.bands;
+  ex.n_col_blocks2 = (nb2 + ex.bands - 1) / ex.bands;
   ex.max_seg = (kExRows + ng - 2) / ng + 1;
   ex.n_kseg = (nc + kExSeg - 1) / kExSeg;
   std::vector<int> kl(ex.n_row_blocks, ex.kt);
-  long long active = 0;
-  for (int rb = 0; rb < ex.n_row_blocks; ++rb) {
-    if (row_kend) {
-      int k = 0;
-      for (int r = rb * kExRows; r < std::min(rows, (rb + 1) * kExRows); ++r) k = std::max(k, std::min(row_kend[r], nc));
-      kl[rb] = (k + 31) / 32 * 2;
-    }
-    active += (long long)ex.halves * kl[rb];
+  for (int rb = 0; rb < ex.n_main_blocks && row_kend; ++rb) {
+    int k = 0;
+    for (int r = rb * kExRows; r < std::min(rows, (rb + 1) * kExRows); ++r) k = std::max(k, std::min(row_kend[r], nc));
+    kl[rb] = (k + 31) / 32 * 2;
   }
   // K splits: as few as fill the grid's waves well.  An item costs its tiles
   // plus about 6 tiles' time for its raw sums and the ring's refill.  Ragged
   // row limits (items of different lengths) take at least 10 items per CTA.
   const int all = ex.halves * ex.kt;
-  const long long blocks = (long long)ex.n_row_blocks * ex.n_col_blocks;
+  const long long blocks = (long long)ex_block_index(ex, ex.n_row_blocks, 0);
   long long best = LLONG_MAX;
   int splits = 1;
   for (int s = 1; s <= std::min(all / 2, 96); ++s) {
@@ -647,11 +651,16 @@ void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool 
   }
   ex.split_tiles = (all / 2 + splits - 1) / splits * 2;
   ex.n_splits = (all + ex.split_tiles - 1) / ex.split_tiles;
-  std::vector<int4> ent;
-  std::vector<int> pieces;
-  k_entries(ex.n_row_blocks, ex.halves, ex.kt, ex.split_tiles, ex.n_splits, kl, ent, pieces);
+  std::vector<int4> ent, ent2;
+  std::vector<int> pieces, pieces2;
+  k_entries(ex.n_main_blocks, ex.halves, ex.kt, ex.split_tiles, ex.n_splits, kl, ent, pieces);
+  k_entries(ex.n_row_blocks - ex.n_main_blocks, ex.halves, ex.kt, ex.split_tiles, ex.n_splits,
+            std::vector<int>(kl.begin() + ex.n_main_blocks, kl.end()), ent2, pieces2);
+  ex.n_main_entries = (int)ent.size();
+  for (int4 e : ent2) ent.push_back(make_int4(e.x + ex.n_main_blocks, e.y, e.z, e.w));
+  pieces.insert(pieces.end(), pieces2.begin(), pieces2.end());
   ex.n_entries = (int)ent.size();
-  ex.n_items = ex.n_entries * ex.n_col_blocks;
+  ex.n_items = ex.n_main_entries * ex.n_col_blocks + (ex.n_entries - ex.n_main_entries) * ex.n_col_blocks2;
   ex.max_pieces = std::max(1, *std::max_element(pieces.begin(), pieces.end()));
   if (tables) {
     tables->entries = std::move(ent);
@@ -712,6 +721,9 @@ cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t) {
 cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(ex.flag, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
+  return exact_begin_counts(ex, s);
+}
+cudaError_t exact_begin_counts(const ExactPrep& ex, cudaStream_t s) {
   return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * 2 * (size_t)ex.n_kseg, s);
 }
 
@@ -724,7 +736,9 @@ cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const v
     exact_stats_kernel<true, false><<<nb, 256, 0, s>>>(ex, b0, nb0, b1, nc);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (ex.halves == 1)
+  if (ex.halves == 1 && ex.slices == 7)
+    exact_slice_b_kernel<7, true><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
+  else if (ex.halves == 1)
     exact_slice_b_kernel<6, true><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
   else if (ex.slices == 7)
     exact_slice_b_kernel<7, false><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
@@ -750,19 +764,22 @@ cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaSt
   return cudaGetLastError();
 }
 
-cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s) {
+cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s,
+                                bool second_rows) {
+  const int rb0 = second_rows ? ex.n_main_blocks : 0;
+  const int nrb = (d.nf * d.ng + kExRows - 1) / kExRows, ncb = (d.nb + ex.bands - 1) / ex.bands;
   const int smem = ex.cols / 2 * kFinRow * (int)sizeof(double2);
   auto* kernel = ex.halves == 1 ? exact_finish_kernel<true> : exact_finish_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  kernel<<<dim3(ex.n_row_blocks, ex.n_col_blocks), 256, smem, s>>>(d, ex);
+  kernel<<<dim3(nrb, ncb), 256, smem, s>>>(d, ex, rb0);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int blocks = (d.nb * d.nf * 32 + 255) / 256;
-  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, ex.partial, out);
+  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, rb0, ex.partial, out);
   e = cudaGetLastError();
   if (e != cudaSuccess || !out2) return e;
-  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, ex.partial2, out2);
+  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, rb0, ex.partial2, out2);
   return cudaGetLastError();
 }
 

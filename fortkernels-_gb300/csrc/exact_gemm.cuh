@@ -67,8 +67,12 @@ struct ExactPrep {
   int halves, kt;           // K tiles per half (K padded to 32: an even count)
   int bands;                // bands per column block (cols / 2 complex, cols real)
   int n_row_blocks, n_col_blocks;
+  // Row blocks from n_main_blocks on (a second group of rows, from row
+  // n_main_blocks * 128: the occupied bands' factors) meet the first
+  // n_col_blocks2 band blocks only.
+  int n_main_blocks, n_col_blocks2;
   int n_splits, split_tiles;
-  int n_entries, n_items, max_pieces;
+  int n_entries, n_main_entries, n_items, max_pieces;
   const int4* entries;      // [n_entries]: row block, piece, first K' tile, tiles (even)
   const int* pieces;        // [n_row_blocks]
   const int* kt_lim;        // [n_row_blocks]: K tiles per half that can be nonzero (even)
@@ -91,10 +95,18 @@ struct ExactTables {
   std::vector<int> pieces, kt_lim;
 };
 
-// Shape of a contraction: rows = nf * ng A rows over K = nc.  row_kend as in
-// ozaki_size.
+// Index of a (row block, band block) pair in the raw sums and partials.
+__host__ __device__ __forceinline__ size_t ex_block_index(const ExactPrep& ex, int rb, int cb) {
+  return rb < ex.n_main_blocks
+             ? (size_t)rb * ex.n_col_blocks + cb
+             : (size_t)ex.n_main_blocks * ex.n_col_blocks + (size_t)(rb - ex.n_main_blocks) * ex.n_col_blocks2 + cb;
+}
+
+// Shape of a contraction: nf * ng A rows over K = nc with nb bands, and nf2 *
+// ng further rows with the first nb2 bands.  row_kend as in ozaki_size (rows
+// of the first group).
 void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
-                ExactTables* tables);
+                ExactTables* tables, int nf2 = 0, int nb2 = 0);
 // Buffers: `work` (digits, exponents, raw sums) may be shared by contractions
 // that run one after another on one stream; `own` (flag and tables) may not.
 size_t exact_work_bytes(const ExactPrep& ex);
@@ -114,15 +126,18 @@ constexpr double kExactMin = 1 << 22;
 //   launch_exact_a    row exponents, overlap check and the A digits of
 //                     complex rows (or the caller's own producer of both)
 //   launch_exact_gemm the digit products
-//   launch_exact_finish  FP64 sums of the rows per band, into out[n][f]
+//   launch_exact_finish  FP64 sums of a row group per band, into out[n][f]
 //                     (complex; halves = 1: FfDev::aqsm holds real values and
-//                     the imaginary parts are zero)
+//                     the imaginary parts are zero); FfDev::nf and nb are the
+//                     group's
 cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s);
+cudaError_t exact_begin_counts(const ExactPrep& ex, cudaStream_t s);  // the flag kept (shared with an earlier one)
 cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const void* b1, int nb1, int nc,
                            cudaStream_t s);
 cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int nc, cudaStream_t s);
 cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s);
-cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s);
+cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s,
+                                bool second_rows = false);
 
 // ---------------------------------------------------------------- device helpers
 // Byte offset of element (row r, k) inside a K-major 32-byte-swizzled tile of
@@ -202,6 +217,42 @@ __device__ __forceinline__ void ex_put(unsigned char* tile, uint32_t slice_bytes
 #pragma unroll
   for (int j = 0; j < 8; ++j) x[j] = v[j];
   ex_store<S>(tile, slice_bytes, r, ch, ex_chunk<S>(x, e));
+}
+
+// The six digits of hi + lo (|lo| at most half an ulp of hi) in units of
+// 2^(7 - e), for |hi| < 2^(e - 1): FP32 operations only.  Every step is exact
+// but the last addition, which rounds at 2^-60 of 2^e (lo joins the third
+// remainder by TwoSum; its rounding error, 2^-51, joins the fourth).
+__device__ __forceinline__ void ex_ff_digits(float2 x, float scale, float (&d)[6]) {
+  constexpr float kM = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer
+  const float u = x.x * scale, w = x.y * (scale * 262144.f);
+  d[0] = (u + kM) - kM;
+  float r = u - d[0];
+  d[1] = fmaf(r, 512.f, kM) - kM;
+  r = fmaf(r, 512.f, -d[1]);
+  d[2] = (fmaf(r, 512.f, w) + kM) - kM;
+  float e;
+  two_sum_f(fmaf(r, 512.f, -d[2]), w, r, e);
+  d[3] = fmaf(r, 512.f, kM) - kM;
+  r = fmaf(e, 512.f, fmaf(r, 512.f, -d[3]));
+  d[4] = fmaf(r, 512.f, kM) - kM;
+  r = fmaf(r, 512.f, -d[4]);
+  d[5] = fmaf(r, 512.f, kM) - kM;
+}
+__device__ __forceinline__ void ex_put_ff(unsigned char* tile, int r, int ch, const float2* v, float scale) {
+  unsigned char* p = tile + sw32_offset(r, ch);
+  uint32_t w[6][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a[6], b[6];
+    ex_ff_digits(v[2 * j], scale, a);
+    ex_ff_digits(v[2 * j + 1], scale, b);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) w[i][j] = __byte_perm(__float_as_uint(a[i]), __float_as_uint(b[i]), 0x7632);
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+    *reinterpret_cast<uint4*>(p + i * kExASlice) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
 }
 
 }  // namespace sigma

@@ -36,8 +36,8 @@ struct sigma_gpp_plan_s {
   sigma::FactorJob fac{};
   int fac_grid = 0;
 
-  // FP64 with one frequency set: the band sums on the tensor cores (when
-  // set); schy then runs only when its flag is raised
+  // FP64 with one frequency set: the band sums and the occupied bands' sums on
+  // the tensor cores (when set); schy and ssx then run only when its flag is raised
   sigma::GppExact exact{};
   sigma::MixedPrep prep{};    // FP32 operands of the mixed path (unused for FP64)
   void* block = nullptr;      // one device allocation for everything below
@@ -266,7 +266,10 @@ extern "C" int sigma_gpp_plan_create(sigma_gpp_plan* plan_out, int number_bands,
     delete p;
     return SIGMA_ERR_CUDA;
   }
-  if (!mixed) gpp_exact_create(p->exact, kGxGpp, number_bands, ncouls, ngpown, kNW, igp_of, sms);
+  if (!mixed) {
+    const GxShape q{kGxGpp, number_bands, nvband, ncouls, ngpown, false};
+    if (gpp_exact_fits(q)) gpp_exact_create(p->exact, q, igp_of, sms);
+  }
   p->host_inv.assign(inv_igp_index, inv_igp_index + ngpown);
   p->host_indinv.assign(indinv, indinv + ncouls);
   *plan_out = p;
@@ -406,8 +409,9 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
   GppWork main = ypath ? plan->schy : (mypath ? plan->schmy : plan->sch);
   if (tensor) main.partial = nullptr;  // band sums land in acht_n1 directly
   const bool exact = ypath && plan->exact;
+  GppWork ssx = plan->fused ? plan->fac.ssx : plan->ssx;
   if (exact) {
-    main.run_if = plan->exact.ex.flag;  // unless it is raised, acht_n1 too
+    main.run_if = ssx.run_if = plan->exact.ex.flag;  // unless it is raised, acht_n1 too
     SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, gx_dev(p), s));
   }
   if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
@@ -436,7 +440,8 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
                                        true);
     if (st != SIGMA_OK) return st;
   } else if (ypath) {
-    if (exact) SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, gx_dev(p), plan->prep.status, plan->acht_n1, s));
+    if (exact) SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, gx_dev(p), plan->prep.status, plan->acht_n1,
+                                                    plan->acht_n1 + (size_t)plan->nb * kNW, s));
     SIGMA_CUDA_TRY(launch_sch_fp64y(p, main, plan->schy_grid, s));
   }
   else if (mypath)
@@ -447,9 +452,9 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
   if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[1], s));
   if (plan->ssx.n_items > 0 && !plan->fused)
     SIGMA_CUDA_TRY((mixed || tensor) ? launch_ssx_mixed(p, plan->ssx, plan->prep, plan->ssx_grid, s)
-                                     : launch_ssx_fp64(p, plan->ssx, plan->ssx_grid, s));
+                                     : launch_ssx_fp64(p, ssx, plan->ssx_grid, s));
   if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[2], s));
-  SIGMA_CUDA_TRY(launch_gpp_reduce(main, plan->fused ? plan->fac.ssx : plan->ssx, plan->nb, plan->acht_n1,
+  SIGMA_CUDA_TRY(launch_gpp_reduce(main, ssx, plan->nb, plan->acht_n1,
                                    reinterpret_cast<double2*>(achtemp),
                                    reinterpret_cast<double2*>(asxtemp),
                                    reinterpret_cast<double2*>(acht_n1_loc), s));

@@ -61,8 +61,8 @@ struct sigma_gpp_batch_s {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   // FP64 with one frequency set per instance: exact contractions in stream
-  // order over one shared workspace; the queue's main pass then takes only
-  // the instances without one or with a raised flag
+  // order over one shared workspace; the queue's passes then take only the
+  // instances without one or with a raised flag
   std::vector<sigma::GppExact> exact;
   void* exact_ws = nullptr;
   // tensor form
@@ -290,15 +290,12 @@ int build_tensor_group(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst,
 // large enough, when the device has room for the largest one's workspace.
 void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std::vector<std::vector<int>>& igp,
                  int sms) {
-  size_t ws = 0;
-  bool all = true;
-  auto fits = [](const sigma_gpp_instance& q) {
-    return (double)kNW * q.ngpown * q.number_bands * q.ncouls >= kExactMin;
+  auto shape = [&](int i) {
+    return GxShape{kGxGpp, inst[i].number_bands, inst[i].nvband, inst[i].ncouls, inst[i].ngpown, false};
   };
+  size_t ws = 0;
   for (int i = 0; i < b->n; ++i)
-    if (fits(inst[i]))
-      ws = std::max(ws, gpp_exact_work_bytes(kGxGpp, inst[i].number_bands, inst[i].ncouls, inst[i].ngpown, kNW, igp[i],
-                                             sms));
+    if (gpp_exact_fits(shape(i))) ws = std::max(ws, gpp_exact_work_bytes(shape(i), igp[i], sms));
   if (ws == 0) return;
   if (cudaMalloc(&b->exact_ws, ws) != cudaSuccess) {
     cudaGetLastError();
@@ -306,15 +303,16 @@ void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std
     return;
   }
   b->exact.resize(b->n);
-  for (int i = 0; i < b->n; ++i)
-    all = (fits(inst[i]) && gpp_exact_create(b->exact[i], kGxGpp, inst[i].number_bands, inst[i].ncouls,
-                                             inst[i].ngpown, kNW, igp[i], sms, b->exact_ws)) && all;
-  for (int i = 0; i < b->n; ++i)
-    if (b->exact[i]) {
-      b->sch[i].run_if = b->exact[i].ex.flag;
-      b->exact[i].ex.any = b->counters + 3;
+  bool all = true;
+  for (int i = 0; i < b->n; ++i) {
+    if (!gpp_exact_fits(shape(i)) || !gpp_exact_create(b->exact[i], shape(i), igp[i], sms, b->exact_ws)) {
+      all = false;
+      continue;
     }
-  // no instance needs the queue's main pass unless some flag is raised
+    b->sch[i].run_if = b->ssx[i].run_if = b->exact[i].ex.flag;
+    b->exact[i].ex.any = b->counters + 3;
+  }
+  // no instance needs the queue's passes unless some flag is raised
   if (all) b->sch_view.run_if = b->counters + 3;
 }
 
@@ -577,7 +575,6 @@ extern "C" int sigma_gpp_batch_create_tuned(sigma_gpp_batch* out, int n_instance
   v.total = b->sch_off[n_instances];
   v.counter = b->counters;
   b->ssx_view = v;
-  b->ssx_view.run_if = nullptr;
   b->ssx_view.work = reinterpret_cast<const GppWork*>(base + o_wssx);
   b->ssx_view.item_off = reinterpret_cast<const int*>(base + o_ssxoff);
   b->ssx_view.total = b->ssx_off[n_instances];
@@ -586,7 +583,7 @@ extern "C" int sigma_gpp_batch_create_tuned(sigma_gpp_batch* out, int n_instance
   if (b->ssx_grid > b->ssx_view.total) b->ssx_grid = std::max(1, b->ssx_view.total);
   // every form: the two fixed-order reductions for all instances
   b->launches = (mixed ? 2 * n_instances : 0) + 1 + (b->ssx_view.total > 0 ? 1 : 0) + 2;
-  for (const GppExact& x : b->exact) b->launches += x ? kGxLaunches : 0;
+  for (const GppExact& x : b->exact) b->launches += gpp_exact_launches(x);
   if (tensor && grouped) {
     int st = build_tensor_group(b, inst, igp, sms);
     if (st != SIGMA_OK) {
@@ -686,7 +683,8 @@ extern "C" int sigma_gpp_batch_execute(sigma_gpp_batch b, void* stream) {
   for (int i = 0; i < (int)b->exact.size(); ++i)
     if (b->exact[i]) {
       SIGMA_CUDA_TRY(launch_gpp_exact_operands(b->exact[i], gx_dev(b->dev[i]), s));
-      SIGMA_CUDA_TRY(launch_gpp_exact_sums(b->exact[i], gx_dev(b->dev[i]), b->counters + 2, b->acht_n1[i], s));
+      SIGMA_CUDA_TRY(launch_gpp_exact_sums(b->exact[i], gx_dev(b->dev[i]), b->counters + 2, b->acht_n1[i],
+                                           b->acht_n1[i] + (size_t)b->dev[i].nb * kNW, s));
     }
   if (!tensor && b->sch_view.total > 0)
     SIGMA_CUDA_TRY(b->mixedy ? launch_sch_mixedy_batch(b->sch_view, b->sch_grid, s)

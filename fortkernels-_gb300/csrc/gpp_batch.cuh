@@ -33,7 +33,7 @@ struct GppBatchView {
   int n_inst;
   int total;
   int* counter;
-  const int* run_if = nullptr;  // FP64 main pass: run only when this word is nonzero (null: always)
+  const int* run_if = nullptr;  // FP64 passes: run only when this word is nonzero (null: always)
 };
 
 // The instance that owns global item g: the last one whose offset is <= g.

@@ -5,14 +5,20 @@
 // (BGW-Kernels/gppKer.cpp:394-404, conj(aqsm) and vcoul moved to the
 // epilogue); the half sum keeps the terms the guard drops
 // (gppKerSeq.cpp:206-242).  Row iw * ng + g of the contraction is one
-// frequency of one column.
+// frequency of one column; the occupied bands' ssx factors (gppKer.cpp:38-58)
+// are a second group of rows.
 //
-// gx_max_kernel bounds |Y| per row (the digits' exponent) from FP32 factors,
-// one pass over the inputs at memory speed.
-// gx_factor_kernel forms Y in FP64 (34 FP64 operations per column and
-// g-vector for the three frequencies, bound by the FP64 pipe's 2 per clock per
-// SM; the digits run on the integer pipe beside them), stages 16 columns x 64
-// g-vectors in shared memory and writes each row's digits as 16-byte chunks.
+// gx_max_kernel bounds the factors per row (the digits' exponent) from FP32
+// values, one pass over the inputs at memory speed.
+// gx_ff_kernel forms them from FP64 numerators in float-float arithmetic (FP32
+// pairs: ~2^-48 rms, below the float-float terms it replaces), cuts them into
+// digits with FP32 operations and writes each row's digits as 16-byte
+// chunks: 16 columns x 32 g-vectors staged in shared memory, four CTAs per SM.
+// (The factors in FP64, 34 operations per column and g-vector, ran at the FP64
+// pipe's 2 per clock per SM: 3.54 ms at 1638 x 32768, with the occupied bands'
+// own pass another 3.86 ms.)  The half sum's factors, FP64 before, stay in FP64
+// (gx_f64_kernel): poles inside the guard, and occupied bands' sums that
+// cancel (2.3e-14 with float-float factors, 2e-15 so).
 #include <algorithm>
 
 #include "gpp_exact.cuh"
@@ -23,8 +29,6 @@ namespace {
 
 constexpr int kGxThreads = 256;
 constexpr int kGxCols = 16;  // columns per CTA
-constexpr int kGxK = 64;     // g-vectors per staged tile
-constexpr int kGxPad = 1;    // conflict-free planes: lanes run along g-vectors, then along columns
 constexpr int kIgBlk = 512;  // g-vector block of the half sum's reference loop
 // Half sum: poles inside the guard make a few factors of a row much larger
 // than the rest, so a count of large ones says little, and the row's exponent
@@ -37,13 +41,10 @@ constexpr float kHalfPower = 1.f / 1073741824.f;
 
 template <int kForm>
 struct Form {
-  static constexpr bool kReal = kForm == kGxReal, kHalf = kForm == kGxHalf;
-  static constexpr int kSlabs = kHalf ? 4 : kNW, kParts = kReal ? 1 : 2;
-  static constexpr int kSlices = kHalf ? 7 : 6;
-};
-template <int kForm>
-struct FactorPlanes {
-  double v[Form<kForm>::kParts][Form<kForm>::kSlabs][kGxCols][kGxK + kGxPad];
+  static constexpr bool kReal = kForm == kGxReal || kForm == kGxRealOcc, kRealOcc = kForm == kGxRealOcc;
+  static constexpr bool kHalf = kForm == kGxHalf, kHalfOcc = kForm == kGxHalfOcc;
+  static constexpr bool kF64 = kRealOcc || kHalf || kHalfOcc;  // factors in FP64, seven digits
+  static constexpr int kSlabs = kHalf ? 4 : kReal ? kNW : 2 * kNW, kParts = kReal ? 1 : 2;  // the most slabs
 };
 
 template <int kForm>
@@ -51,52 +52,84 @@ __device__ __forceinline__ double2 gx_load(const double* a, size_t off) {
   if (Form<kForm>::kReal) return make_double2(a[off], 0.0);
   return reinterpret_cast<const double2*>(a)[off];
 }
-// End of a slab's g-vectors in column igp.
+// End of a slab's g-vectors in column g.
 template <int kForm>
-__device__ __forceinline__ int gx_limit(int igp, int slab, int nc) {
-  if (!Form<kForm>::kHalf) return nc;
-  return igp < 0 ? 0 : (slab < kNW ? max(igp - 1, 0) : igp);
+__device__ __forceinline__ int gx_limit(const GxDev& p, int g, int slab) {
+  if (!Form<kForm>::kHalf && !Form<kForm>::kHalfOcc) return p.nc;
+  const int igp = p.igp_of[g];
+  if (igp < 0) return 0;
+  if (Form<kForm>::kHalfOcc) return min(igp, p.brk[g]);
+  return slab < kNW ? max(igp - 1, 0) : igp;
+}
+// Row of a slab's column, and the end of its group's row blocks.
+__device__ __forceinline__ int gx_row(const ExactPrep& ex, int ng, int nf, int slab, int g) {
+  return slab < nf ? slab * ng + g : ex.n_main_blocks * kExRows + (slab - nf) * ng + g;
+}
+__device__ __forceinline__ int gx_rows_end(const ExactPrep& ex, int nf, int slab) {
+  return (slab < nf ? ex.n_main_blocks : ex.n_row_blocks) * kExRows;
 }
 
-// One CTA per column: exponents of its rows.  |Y| from FP32 values (c from
-// exact FP32 halves), the guard taken somewhat wide, with a 2^-8 margin;
-// what FP32 cannot bound raises the flag.
+// One CTA per column: exponents of its rows.  Magnitudes from FP32 values (c
+// from exact FP32 halves), the guard taken somewhat wide on both sides, with
+// a 2^-8 margin; what FP32 cannot bound raises the flag.
 template <int kForm>
-__global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep ex, int nf) {
+__global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep ex, int nf, int nf2) {
   using F = Form<kForm>;
   __shared__ unsigned s_m[F::kSlabs][kGxThreads / 32];
   const int g = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int igp = p.igp_of[g];
+  const bool occ = F::kHalfOcc || F::kRealOcc || nf2 > 0;
   FF wx[kNW];
+  float iwx2[kNW];
 #pragma unroll
-  for (int iw = 0; iw < kNW; ++iw) wx[iw] = ff_of(p.wx[iw]);
-  unsigned m[F::kSlabs];  // bits of non-negative floats; NaN is the largest
+  for (int iw = 0; iw < kNW; ++iw) {
+    wx[iw] = ff_of(p.wx[iw]);
+    iwx2[iw] = __frcp_rn(wx[iw].hi * wx[iw].hi);
+  }
+  unsigned m[F::kSlabs];  // bits of non-negative floats; NaN counts as infinite
 #pragma unroll
   for (int i = 0; i < F::kSlabs; ++i) m[i] = 0u;
+  auto top = [](unsigned& v, float y) { v = max(v, __float_as_uint(y != y ? INFINITY : y)); };
   bool bad = false;
-  const int k_end = gx_limit<kForm>(igp, F::kSlabs - 1, p.nc), k_freq = gx_limit<kForm>(igp, 0, p.nc);
+  const int k_end = gx_limit<kForm>(p, g, F::kSlabs - 1), k_freq = gx_limit<kForm>(p, g, 0);
 #pragma unroll 4
   for (int k = tid; k < k_end; k += kGxThreads) {
     const double2 w = gx_load<kForm>(p.wt, (size_t)g * p.nc + k), e = gx_load<kForm>(p.ieps, (size_t)g * p.nc + k);
     const FF a = ff_of(w.x);
     const float b = __double2float_rn(w.y), er = __double2float_rn(e.x), ei = __double2float_rn(e.y);
     if (F::kHalf) {
-      m[F::kSlabs - 1] = max(m[F::kSlabs - 1], __float_as_uint(fmaxf(fabsf(er), fabsf(ei))));
+      top(m[F::kSlabs - 1], fmaxf(fabsf(er), fabsf(ei)));
       if (er != er || ei != ei) m[F::kSlabs - 1] = 0x7F800000u;
       if (k >= k_freq || k % kIgBlk == kIgBlk - 1) continue;
     }
     const float gx = er * a.hi - ei * b, gy = er * b + ei * a.hi;
-    const float lim = F::kHalf ? fmaxf(0.2501f, fmaf(a.hi, a.hi, b * b) * 4.001e-6f) : 0.f;
+    const float s2 = fmaf(a.hi, a.hi, b * b);
+    const float om = fmaxf(fabsf(gx * a.hi - gy * b), fabsf(gx * b + gy * a.hi));
+    // the guard's threshold, somewhat above and below
+    const float up = fmaxf(0.2501f, s2 * 4.001e-6f), low = 0.2499f;
     const bool any = (e.x != 0.0 || e.y != 0.0) && (w.x != 0.0 || w.y != 0.0);
 #pragma unroll
     for (int iw = 0; iw < kNW; ++iw) {
       const float c = (wx[iw].hi - a.hi) + (wx[iw].lo - a.lo);
       const float w2 = fmaf(c, c, b * b);
-      if (F::kHalf ? !(w2 > lim) : !(w2 <= 0.2499f)) {  // also NaN
-        const float r = __frcp_rn(w2);
-        const float y = fmaxf(fabsf(gx * c - gy * b), fabsf(gy * c + gx * b)) * r;
-        m[iw] = max(m[iw], __float_as_uint(y != y ? INFINITY : y));
-        if (w2 > 1e30f) m[iw] = 0x7F800000u;  // the FP32 reciprocal may be 0: flagged below
+      if (w2 > 1e30f) m[iw] = 0x7F800000u;  // the FP32 reciprocal may be 0: flagged below
+      if (!F::kRealOcc && (F::kHalf ? !(w2 > up) : !(w2 <= low))) {  // also NaN
+        const float y = fmaxf(fabsf(gx * c - gy * b), fabsf(gy * c + gx * b)) * __frcp_rn(w2);
+        top(m[iw], y);
+        bad = bad || (any && !(y > 1e-18f));
+      }
+      if (!F::kHalf && (!F::kReal || F::kRealOcc) && occ) {
+        const float z = (wx[iw].hi + a.hi) + (wx[iw].lo + a.lo);
+        const float rz = __frcp_rn(fmaf(z, z, b * b));
+        float y = 0.f;
+        if (!(w2 > up)) y = 0.5f * fmaxf(fabsf(gx * z + gy * b), fabsf(gy * z - gx * b)) * rz;
+        if (!(w2 <= low)) {
+          if (F::kHalfOcc) {  // Omega2 / ((wx - wtilde) (wx + wtilde)): within sqrt(2) of its larger part
+            y = fmaxf(y, 1.5f * om * sqrtf(__frcp_rn(w2) * rz));
+          } else {
+            y = fmaxf(y, om * iwx2[iw]);
+          }
+        }
+        top(m[F::kSlabs > kNW ? kNW + iw < F::kSlabs ? kNW + iw : 0 : iw], y);
         bad = bad || (any && !(y > 1e-18f));
       }
     }
@@ -108,134 +141,379 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
     if (lane == 0) s_m[i][warp] = v;
   }
   __syncthreads();
-  if (tid < nf) {
+  if (tid < nf + nf2) {
     unsigned v = 0;
     for (int q = 0; q < kGxThreads / 32; ++q) v = max(v, s_m[tid][q]);
     const float f = __uint_as_float(v) * (1.f + 1.f / 256.f);
     // a factor too small for FP32 may only be ignored beside large ones
     if (!(f < 1e18f) || (bad && !(f > 1e-6f)) || (v && f < 1e-18f)) ex_raise(ex);
-    ex.ea[tid * p.ng + g] = v ? (int)(__float_as_uint(f) >> 23) - 126 : kExZeroRow;
+    // float-float digits need a bit of room (ex_ff_digits)
+    ex.ea[gx_row(ex, p.ng, nf, tid, g)] =
+        v ? (int)(__float_as_uint(f) >> 23) - 126 + (F::kF64 ? 0 : 1) : kExZeroRow;
   }
 }
 
-// Items (column block, 512-g-vector segment).  Column blocks run past ng to
-// cover the padding rows of the last row block (zero digits).
-template <int kForm>
-__global__ void __launch_bounds__(kGxThreads, Form<kForm>::kHalf ? 3 : 4)
-    gx_factor_kernel(GxDev p, ExactPrep ex, float* stat, int nf) {
+// ---------------------------------------------------------------- float-float factors
+// Decisions in the FP64 path's expressions: bit 0 the guard keeps the term,
+// bit 1 the second occupied-band branch.
+static __device__ __noinline__ unsigned gx_decide(double wx, double a, double b) {
+  const double b2 = guard_b2(b), wv = guard_w(wx, a, b2);
+  if (keep_nonneg(wv, guard_thr(a, b2))) return 1u;
+  return gt_nonneg(wv, 0.0) && gt_nonneg(guard_thr2(a, b2), wv) ? 2u : 0u;
+}
+
+__device__ __forceinline__ FF gx_norm(FF x) { return ff_norm(x.hi, x.lo); }
+
+struct Factors {
+  double2 y, s;  // Y and ssx
+};
+// One frequency's factors in FP64, for elements or frequencies outside the
+// float-float range.
+static __device__ __noinline__ Factors gx_wide(double wx, double2 wt, double2 ie) {
+  const double a = wt.x, b = wt.y, b2 = guard_b2(b), c = __dsub_rn(wx, a), dr = wx + a;
+  const double gx = fma(ie.x, a, -(ie.y * b)), gy = fma(ie.x, b, ie.y * a);
+  const unsigned mask = gx_decide(wx, a, b);
+  Factors f{make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+  if (mask & 1u) {
+    const double r = rcp_f64(fma(c, c, b2)), i2 = rcp_f64(wx * wx);
+    f.y = make_double2(fma(gx, c, -(gy * b)) * r, fma(gy, c, gx * b) * r);
+    f.s = make_double2(fma(a, gx, -(b * gy)) * i2, fma(a, gy, b * gx) * i2);  // Omega2 / wx^2
+  } else if (mask & 2u) {
+    const double q = -0.5 * rcp_f64(fma(dr, dr, b2));
+    f.s = make_double2(fma(gx, dr, gy * b) * q, fma(gy, dr, -(gx * b)) * q);
+  }
+  return f;
+}
+
+// The three frequencies' factors of one element: put(slab, re, im) takes Y in
+// slabs 0-2 and ssx in 3-5 as normalised pairs.
+template <int kForm, bool kOcc, class Put>
+__device__ __forceinline__ void gx_factors(const FF (&wx)[kNW], const FF (&iwx2)[kNW], const double* wxd,
+                                           bool wx_wide, double2 wt, double2 ie, Put put) {
   using F = Form<kForm>;
+  if (wx_wide || !ff_range(wt.x, wt.y) || !ff_range(ie.x, ie.y)) {
+#pragma unroll
+    for (int iw = 0; iw < kNW; ++iw) {
+      const Factors f = gx_wide(wxd[iw], wt, ie);
+      put(iw, ff_of_rn(f.y.x), ff_of_rn(f.y.y));
+      if (kOcc) put(kNW + iw, ff_of_rn(f.s.x), ff_of_rn(f.s.y));
+    }
+    return;
+  }
+  // G, c and |wdiff|^2 in FP64 (11 operations, 5.5 clocks per SM, beside ~10
+  // clocks of FP32 work): exact decisions, and the factor's error is that of
+  // the float-float reciprocal and products alone (G and c in float-float put
+  // a strongly cancelling band sum at 2.3e-12)
+  const FF zero{0.f, 0.f};
+  const double b2d = guard_b2(wt.y);
+  FF gx, gy = zero, b = zero, b2 = zero, a = zero, ox = zero, oy = zero;
+  if (F::kReal) {
+    gx = ff_of_rn(__dmul_rn(ie.x, wt.x));
+  } else {
+    gx = ff_of_rn(fma(ie.x, wt.x, -__dmul_rn(ie.y, wt.y)));
+    gy = ff_of_rn(fma(ie.x, wt.y, __dmul_rn(ie.y, wt.x)));
+    b = ff_of_rn(wt.y);
+  }
+  if (kOcc) {
+    a = ff_of_rn(wt.x);
+    b2 = ff_mul(b, b);
+    ox = gx_norm(ff_dot2_raw(a, gx, b, gy));  // Omega2 = wtilde G
+    oy = gx_norm(ff_dot2_raw(a, gy, ff_neg(b), gx));
+  }
+  // the guard's second condition binds from |wtilde|^2 = 62500 on; dropped
+  // terms with |wtilde|^2 well above the second branch's bound take it
+  const float af = __double2float_rn(wt.x), bf = __double2float_rn(wt.y), s2 = fmaf(af, af, bf * bf);
+  const bool binds = s2 >= 62000.f, big = s2 > 1.01e-6f;
+#pragma unroll
+  for (int iw = 0; iw < kNW; ++iw) {
+    const double cd = __dsub_rn(wxd[iw], wt.x), wv = fma(cd, cd, b2d);
+    bool keep = keep_nonneg(wv, kLimitTwo), second = !keep && gt_nonneg(wv, 0.0);
+    if (binds || (kOcc && !keep && !big)) {
+      const unsigned mask = gx_decide(wxd[iw], wt.x, wt.y);
+      keep = mask & 1u;
+      second = mask & 2u;
+    }
+    const FF c = ff_of_rn(cd);
+    if (F::kReal) {
+      const FF y = ff_mul(gx, gx_norm(ff_rcp_raw(c)));
+      put(iw, keep ? y : zero, zero);
+    } else {
+      const FF r = gx_norm(ff_rcp_raw(ff_of_rn(wv)));
+      const FF yx = ff_mul(gx_norm(ff_dot2_raw(gx, c, gy, b)), r);
+      const FF yy = ff_mul(gx_norm(ff_dot2_raw(gy, c, ff_neg(gx), b)), r);
+      put(iw, keep ? yx : zero, keep ? yy : zero);
+      if (kOcc) {
+        // Omega2 / wx^2 or -G conj(z) / (2 |z|^2), z = wx + wtilde
+        const FF z = ff_add(wx[iw], a);
+        const FF rz = gx_norm(ff_rcp_raw(ff_sq_add(z, b2)));
+        const FF tx = gx_norm(ff_dot2_raw(gx, z, gy, ff_neg(b))), ty = gx_norm(ff_dot2_raw(gy, z, gx, b));
+        const FF m = keep ? iwx2[iw] : FF{-0.5f * rz.hi, -0.5f * rz.lo};
+        const FF sx = ff_mul(keep ? ox : tx, m), sy = ff_mul(keep ? oy : ty, m);
+        const bool on = keep || second;
+        put(kNW + iw, on ? sx : zero, on ? sy : zero);
+      }
+    }
+  }
+}
+
+constexpr int kFfK = 32;  // g-vectors per staged tile
+template <int kForm, bool kOcc>
+struct FfPlanes {
+  static constexpr int kSlabs = kOcc ? 6 : 3;
+  float2 v[Form<kForm>::kParts][kSlabs][kGxCols][kFfK + 1];  // conflict-free along g-vectors and along columns
+};
+
+// Items (column block, 512-g-vector segment).  Column blocks run past ng to
+// cover the padding rows of each group's last row block (zero digits).
+template <int kForm, bool kOcc>
+__global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep ex, float* stat, int nf) {
+  using F = Form<kForm>;
+  constexpr int kSlabs = FfPlanes<kForm, kOcc>::kSlabs;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  FactorPlanes<kForm>& sm = *reinterpret_cast<FactorPlanes<kForm>*>(smem_raw);
-  __shared__ int s_e[F::kSlabs][kGxCols], s_igp[kGxCols];
+  FfPlanes<kForm, kOcc>& sm = *reinterpret_cast<FfPlanes<kForm, kOcc>*>(smem_raw);
+  __shared__ float s_scale[kSlabs][kGxCols], s_thr[kSlabs][kGxCols];
+  __shared__ int s_lim[kGxCols], s_need;
+  __shared__ FF s_wx[kNW], s_iwx2[kNW];
+  __shared__ bool s_wide;
   if (*ex.flag) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int p0 = blockIdx.x * kGxCols, seg = blockIdx.y;
-  const int rows_pad = ex.n_row_blocks * kExRows;
-  const double wx[kNW] = {p.wx[0], p.wx[1], p.wx[2]};
-  // K tiles of the item's rows that the contraction reads
-  int need = 0;
-  if (tid < nf * kGxCols) {
-    const int iw = tid / kGxCols, g = p0 + tid % kGxCols, R = iw * p.ng + g;
-    s_e[iw][tid % kGxCols] = g < p.ng ? ex.ea[R] : kExZeroRow;
-    if (iw == 0) s_igp[tid % kGxCols] = g < p.ng ? p.igp_of[g] : -1;
-    if (R < rows_pad && (g < p.ng || iw == nf - 1)) need = ex.kt_lim[R / kExRows] * kExKTile;
+  if (tid == 0) {
+    s_need = 0;
+    bool wide = false;
+    for (int iw = 0; iw < kNW; ++iw) {
+      const double w = p.wx[iw];
+      wide = wide || !ff_freq_range(w);
+      s_wx[iw] = ff_of_rn(w);
+      s_iwx2[iw] = ff_of_rn(rcp_f64(w * w));
+    }
+    s_wide = wide;
   }
-  const int k_begin = seg * kExSeg;
-  int k_end = min(ex.kt * kExKTile, k_begin + kExSeg);
-  if (F::kHalf) {
-    __shared__ int s_need;
-    if (tid == 0) s_need = 0;
-    __syncthreads();
-    if (need) atomicMax(&s_need, need);
-    __syncthreads();
-    k_end = min(k_end, s_need);
+  __syncthreads();
+  if (tid < kSlabs * kGxCols) {
+    const int i = tid / kGxCols, pl = tid % kGxCols, g = p0 + pl, R = gx_row(ex, p.ng, nf, i, g);
+    const int e = g < p.ng ? ex.ea[R] : kExZeroRow;
+    // 2^(7 - e) and 2^(e - 2 - slack) (|e| < 64 unless flagged; a zero row's values are zero)
+    s_scale[i][pl] = e == kExZeroRow ? 0.f : __uint_as_float((unsigned)(134 - e) << 23);
+    s_thr[i][pl] = e == kExZeroRow ? INFINITY : __uint_as_float((unsigned)(125 - kExSlackA + e) << 23);
+    if (i == 0) s_lim[pl] = g < p.ng ? gx_limit<kForm>(p, g, 0) : 0;
+    const bool last = i == nf - 1 || i == kSlabs - 1;
+    if ((g < p.ng || last) && R < gx_rows_end(ex, nf, i)) atomicMax(&s_need, ex.kt_lim[R / kExRows] * kExKTile);
   }
-  float acc[2][F::kSlabs];  // large factors, or sums of squares, per column of this warp
+  __syncthreads();
+  const int k_begin = seg * kExSeg, k_end = min(s_need, k_begin + kExSeg);  // tiles the contraction reads
+  float acc[2][kSlabs];  // large factors per column of this warp
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int i = 0; i < F::kSlabs; ++i) acc[j][i] = 0.f;
-  for (int k0 = k_begin; k0 < k_end; k0 += kGxK) {
-    __syncthreads();
+    for (int i = 0; i < kSlabs; ++i) acc[j][i] = 0.f;
+  for (int k0 = k_begin; k0 < k_end; k0 += kFfK) {
+    const FF wx[kNW] = {s_wx[0], s_wx[1], s_wx[2]}, iwx2[kNW] = {s_iwx2[0], s_iwx2[1], s_iwx2[2]};
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const int pl = warp + 8 * j, g = p0 + pl;
-#pragma unroll
-      for (int h = 0; h < kGxK / 32; ++h) {
-        const int k = h * 32 + lane, ig = k0 + k;
-        double2 y[F::kSlabs];
-#pragma unroll
-        for (int i = 0; i < F::kSlabs; ++i) y[i] = make_double2(0.0, 0.0);
-        const int igp = F::kHalf ? s_igp[pl] : 0;
-        if (g < p.ng && ig < gx_limit<kForm>(igp, F::kSlabs - 1, p.nc)) {
-          const double2 wt = gx_load<kForm>(p.wt, (size_t)g * p.nc + ig);
-          const double2 ie = gx_load<kForm>(p.ieps, (size_t)g * p.nc + ig);
-          if (F::kHalf) y[F::kSlabs - 1] = make_double2(-ie.x, -ie.y);
-          // the guard's second condition binds only for |wtilde|^2 >= 62500
-          const bool plain =
-              fabsf(__double2float_rn(wt.x)) < 170.f && fabsf(__double2float_rn(wt.y)) < 170.f;
-          if (F::kReal) {
-            const double gr = __dmul_rn(ie.x, wt.x);
-            const double thr = plain ? kLimitTwo : guard_thr(wt.x, 0.0);
-#pragma unroll
-            for (int iw = 0; iw < kNW; ++iw) {
-              const double c = __dsub_rn(wx[iw], wt.x);
-              const double wv = __dmul_rn(c, c);
-              const double v = __dmul_rn(gr, __dmul_rn(c, rcp_f64(wv)));
-              y[iw].x = keep_nonneg(wv, thr) ? v : 0.0;
-            }
-          } else if (!F::kHalf || (ig < gx_limit<kForm>(igp, 0, p.nc) && ig % kIgBlk != kIgBlk - 1)) {
-            const double gx = fma(ie.x, wt.x, -__dmul_rn(ie.y, wt.y)), gy = fma(ie.x, wt.y, __dmul_rn(ie.y, wt.x));
-            const double gbx = __dmul_rn(gx, wt.y), gby = __dmul_rn(gy, wt.y);
-            const double b2 = guard_b2(wt.y);
-            const double thr = plain ? kLimitTwo : guard_thr(wt.x, b2);
-#pragma unroll
-            for (int iw = 0; iw < kNW; ++iw) {
-              const double c = __dsub_rn(wx[iw], wt.x);
-              const double wv = fma(c, c, b2);
-              const double r = rcp_f64(wv);
-              const double yx = __dmul_rn(fma(gx, c, -gby), r), yy = __dmul_rn(fma(gy, c, gbx), r);
-              const bool keep = F::kHalf ? gt_nonneg(thr, wv) : keep_nonneg(wv, thr);
-              y[iw] = make_double2(keep ? yx : 0.0, keep ? yy : 0.0);
-            }
+      const int pl = warp + 8 * j, g = p0 + pl, ig = k0 + lane;
+      if (ig < s_lim[pl]) {
+        const double2 wt = gx_load<kForm>(p.wt, (size_t)g * p.nc + ig);
+        const double2 ie = gx_load<kForm>(p.ieps, (size_t)g * p.nc + ig);
+        auto put = [&](int i, FF re, FF im) {
+          sm.v[0][i][pl][lane] = make_float2(re.hi, re.lo);
+          float big = fabsf(re.hi);
+          if (!F::kReal) {
+            sm.v[F::kParts - 1][i][pl][lane] = make_float2(im.hi, im.lo);
+            big = fmaxf(big, fabsf(im.hi));
           }
-        }
+          acc[j][i] += big >= s_thr[i][pl] ? 1.f : 0.f;
+        };
+        gx_factors<kForm, kOcc>(wx, iwx2, p.wx, s_wide, wt, ie, put);
+      } else {
 #pragma unroll
-        for (int i = 0; i < F::kSlabs; ++i) {
-          sm.v[0][i][pl][k] = y[i].x;
-          if (!F::kReal) sm.v[F::kParts - 1][i][pl][k] = y[i].y;
-          const int e = min(s_e[min(i, nf - 1)][pl], 1000);
-          if (F::kHalf) {
-            const float u = __uint_as_float((unsigned)(127 - e) << 23);  // 2^-e, |e| < 61 unless flagged
-            const float a = __double2float_rn(y[i].x) * u, b = __double2float_rn(y[i].y) * u;
-            acc[j][i] = fmaf(a, a, fmaf(b, b, acc[j][i]));
-          } else {
-            const int big = max(__double2hiint(y[i].x) & 0x7FFFFFFF, __double2hiint(y[i].y) & 0x7FFFFFFF);
-            acc[j][i] += big >= (e + 1022 - kExSlackA) << 20 ? 1.f : 0.f;
-          }
-        }
+        for (int i = 0; i < kSlabs; ++i)
+#pragma unroll
+          for (int q = 0; q < F::kParts; ++q) sm.v[q][i][pl][lane] = make_float2(0.f, 0.f);
       }
     }
     __syncthreads();
     // digits: a warp takes one (slab, part, K tile), its lanes the 16
     // columns x 2 chunks (512 contiguous bytes per slice)
-    constexpr int kTiles = kGxK / kExKTile;
 #pragma unroll 1
-    for (int t = warp; t < nf * F::kParts * kTiles; t += kGxThreads / 32) {
-      const int q = t % kTiles, part = t / kTiles % F::kParts, iw = t / (kTiles * F::kParts);
-      const int pl = lane & 15, ch = lane >> 4, g = p0 + pl, R = iw * p.ng + g;
+    for (int t = warp; t < kSlabs * F::kParts * 2; t += kGxThreads / 32) {
+      const int q = t & 1, part = (t >> 1) % F::kParts, i = (t >> 1) / F::kParts;
+      const int pl = lane & 15, ch = lane >> 4, g = p0 + pl, R = gx_row(ex, p.ng, nf, i, g);
       const int tile = k0 / kExKTile + q;
-      // padding rows follow the last slab's columns
-      if ((g >= p.ng && iw < nf - 1) || R >= rows_pad || tile >= ex.kt_lim[R / kExRows]) continue;
+      // padding rows follow the group's last slab's columns
+      if (g >= p.ng && i != nf - 1 && i != kSlabs - 1) continue;
+      if (R >= gx_rows_end(ex, nf, i) || tile >= ex.kt_lim[R / kExRows]) continue;
       unsigned char* dst =
-          ex.a_tiles + ((size_t)(R / kExRows) * F::kParts * ex.kt + part * ex.kt + tile) * ex_a_bytes(F::kSlices);
-      ex_put<F::kSlices>(dst, kExASlice, R % kExRows, ch, &sm.v[part][iw][pl][q * kExKTile + ch * 8], s_e[iw][pl]);
+          ex.a_tiles + ((size_t)(R / kExRows) * F::kParts * ex.kt + part * ex.kt + tile) * ex_a_bytes(6);
+      ex_put_ff(dst, R % kExRows, ch, &sm.v[part][i][pl][q * kExKTile + ch * 8], s_scale[i][pl]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < kSlabs; ++i) {
+      float a = acc[j][i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      const int g = p0 + warp + 8 * j;
+      if (lane == 0 && g < p.ng) stat[(size_t)gx_row(ex, p.ng, nf, i, g) * ex.n_kseg + seg] = a;
+    }
+}
+
+// ---------------------------------------------------------------- half-sum factors
+// kGxHalf: sums of squares per segment; kGxHalfOcc (sch and ssx,
+// gppKerSeq.cpp:96-139) and kGxRealOcc (gppKer_real.cpp:20-60): large factors
+// per segment.
+template <int kForm>
+struct F64 {
+  static constexpr bool kOcc = kForm != kGxHalf, kReal = kForm == kGxRealOcc;
+  static constexpr int S = 7, kSlabs = Form<kForm>::kSlabs, kParts = Form<kForm>::kParts;
+  static constexpr int kK = kForm == kGxHalfOcc ? 32 : 64;  // g-vectors per staged tile
+  struct Planes {
+    double v[kParts][kSlabs][kGxCols][kK + 1];
+  };
+};
+// 1 / x for either sign.
+__device__ __forceinline__ double rcp_signed(double x) {
+  const double r = rcp_f64(fabs(x));
+  return __hiloint2double(__double2hiint(r) | (__double2hiint(x) & 0x80000000), __double2loint(r));
+}
+
+// The factors of one element, FP64; in_freq: within the frequencies' range.
+template <int kForm>
+__device__ __forceinline__ void gx_f64_factors(const double (&wx)[kNW], const double (&iwx2)[kNW], double2 wt, double2 ie, bool in_freq,
+                                               double2 (&y)[Form<kForm>::kSlabs]) {
+  constexpr bool kOcc = F64<kForm>::kOcc;
+  if (!kOcc) y[F64<kForm>::kSlabs - 1] = make_double2(-ie.x, -ie.y);
+  if (!in_freq) return;
+  const double a = wt.x, b = wt.y;
+  if (F64<kForm>::kReal) {
+    // kept: Omega2 / wx^2, second branch: -G / (2 (wx + wtilde)): 20 FP64
+    // operations (for |wtilde| in the usual range the guard is |c| > 1/2)
+    const double g = __dmul_rn(ie.x, a), om = __dmul_rn(g, a);
+    const float af = fabsf(__double2float_rn(a));
+    const bool plain = af < 240.f && af > 1.01e-3f;
+#pragma unroll
+    for (int iw = 0; iw < kNW; ++iw) {
+      const double c = __dsub_rn(wx[iw], a);
+      bool keep = gt_nonneg(fabs(c), 0.5), second = !keep && gt_nonneg(fabs(c), 0.0);
+      if (!plain) {
+        const unsigned mask = gx_decide(wx[iw], a, 0.0);
+        keep = mask & 1u;
+        second = mask & 2u;
+      }
+      const double r = rcp_signed(__dadd_rn(wx[iw], a));
+      // -r / 2 (r normal: |wx + wtilde| is far from the overflow threshold here)
+      const double h = __hiloint2double((__double2hiint(r) - 0x100000) ^ 0x80000000, __double2loint(r));
+      const double v = __dmul_rn(keep ? om : g, keep ? iwx2[iw] : h);
+      y[iw].x = keep || second ? v : 0.0;
+    }
+    return;
+  }
+  const double gx = fma(ie.x, a, -__dmul_rn(ie.y, b)), gy = fma(ie.x, b, __dmul_rn(ie.y, a));
+  const double gbx = __dmul_rn(gx, b), gby = __dmul_rn(gy, b);
+  const double b2 = guard_b2(b);
+  // the guard's second condition binds only for |wtilde|^2 >= 62500
+  const float af = fabsf(__double2float_rn(a)), bf = fabsf(__double2float_rn(b));
+  const double thr = af < 170.f && bf < 170.f ? kLimitTwo : guard_thr(a, b2);
+  const bool some = !kOcc || fmaxf(af, bf) > 1.1e-6f || fma(a, a, b2) > kTo1 * kTo1;
+#pragma unroll
+  for (int iw = 0; iw < kNW; ++iw) {
+    const double c = __dsub_rn(wx[iw], a);
+    const double wv = fma(c, c, b2);
+    const double r = rcp_f64(wv);
+    const double yx = __dmul_rn(fma(gx, c, -gby), r), yy = __dmul_rn(fma(gy, c, gbx), r);
+    const bool low = gt_nonneg(thr, wv);
+    if (low != kOcc) y[iw] = make_double2(yx, yy);
+    if (kForm == kGxHalfOcc) {
+      // kept: Omega2 / (wx^2 - wtilde^2) = sch wtilde / z, else -G / (2 z), z = wx + wtilde
+      const double z = __dadd_rn(wx[iw], a), rz = rcp_f64(fma(z, z, b2));
+      const double qx = low ? __dmul_rn(gx, -0.5) : fma(yx, a, -__dmul_rn(yy, b));
+      const double qy = low ? __dmul_rn(gy, -0.5) : fma(yx, b, __dmul_rn(yy, a));
+      const double sx = __dmul_rn(fma(qx, z, __dmul_rn(qy, b)), rz), sy = __dmul_rn(fma(qy, z, -__dmul_rn(qx, b)), rz);
+      if (!low || some) y[(kNW + iw) % F64<kForm>::kSlabs] = make_double2(sx, sy);
+    }
+  }
+}
+
+template <int kForm>
+__global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm>::kReal ? 3 : 4)
+    gx_f64_kernel(GxDev p, ExactPrep ex, float* stat, int nf) {
+  using H = F64<kForm>;
+  constexpr int kSlabs = H::kSlabs, kK = H::kK;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typename H::Planes& sm = *reinterpret_cast<typename H::Planes*>(smem_raw);
+  __shared__ int s_e[kSlabs][kGxCols], s_lim[2][kGxCols], s_need;
+  if (*ex.flag) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int p0 = blockIdx.x * kGxCols, seg = blockIdx.y;
+  const int rows_pad = ex.n_row_blocks * kExRows;
+  const double wx[kNW] = {p.wx[0], p.wx[1], p.wx[2]};
+  double iwx2[kNW];
+#pragma unroll
+  for (int iw = 0; iw < kNW; ++iw) iwx2[iw] = H::kReal ? rcp_f64(__dmul_rn(wx[iw], wx[iw])) : 0.0;
+  if (tid == 0) s_need = 0;
+  __syncthreads();
+  if (tid < nf * kGxCols) {
+    const int i = tid / kGxCols, pl = tid % kGxCols, g = p0 + pl, R = i * p.ng + g;
+    s_e[i][pl] = g < p.ng ? ex.ea[R] : kExZeroRow;
+    if (i < 2) s_lim[i][pl] = g < p.ng ? gx_limit<kForm>(p, g, i ? kSlabs - 1 : 0) : 0;
+    if (R < rows_pad && (g < p.ng || i == nf - 1)) atomicMax(&s_need, ex.kt_lim[R / kExRows] * kExKTile);
+  }
+  __syncthreads();
+  const int k_begin = seg * kExSeg, k_end = min(s_need, k_begin + kExSeg);  // tiles the contraction reads
+  float acc[2][kSlabs] = {};  // per column of this warp
+  for (int k0 = k_begin; k0 < k_end; k0 += kK) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int pl = warp + 8 * j, g = p0 + pl;
+#pragma unroll
+      for (int h = 0; h < kK / 32; ++h) {
+        const int k = h * 32 + lane, ig = k0 + k;
+        double2 y[kSlabs];
+#pragma unroll
+        for (int i = 0; i < kSlabs; ++i) y[i] = make_double2(0.0, 0.0);
+        if (ig < s_lim[1][pl]) {
+          const double2 wt = gx_load<kForm>(p.wt, (size_t)g * p.nc + ig);
+          const double2 ie = gx_load<kForm>(p.ieps, (size_t)g * p.nc + ig);
+          const bool in_freq = ig < s_lim[0][pl] && (H::kOcc || ig % kIgBlk != kIgBlk - 1);
+          gx_f64_factors<kForm>(wx, iwx2, wt, ie, in_freq, y);
+        }
+#pragma unroll
+        for (int i = 0; i < kSlabs; ++i) {
+          sm.v[0][i][pl][k] = y[i].x;
+          if (!H::kReal) sm.v[H::kParts - 1][i][pl][k] = y[i].y;
+          const int e = s_e[min(i, nf - 1)][pl];  // |e| < 64 unless flagged; a zero row is not checked
+          if (H::kOcc) {
+            const int big = max(__double2hiint(y[i].x) & 0x7FFFFFFF, __double2hiint(y[i].y) & 0x7FFFFFFF);
+            acc[j][i] += big >= (min(e, 1000) + 1022 - kExSlackA) << 20 ? 1.f : 0.f;
+          } else {
+            const float u = __uint_as_float((unsigned)(127 - e) << 23);  // 2^-e
+            const float a = __double2float_rn(y[i].x) * u, b = __double2float_rn(y[i].y) * u;
+            acc[j][i] = fmaf(a, a, fmaf(b, b, acc[j][i]));
+          }
+        }
+      }
+    }
+    __syncthreads();
+    constexpr int kTiles = kK / kExKTile;
+#pragma unroll 1
+    for (int t = warp; t < nf * H::kParts * kTiles; t += kGxThreads / 32) {
+      const int q = t % kTiles, part = t / kTiles % H::kParts, i = t / (kTiles * H::kParts);
+      const int pl = lane & 15, ch = lane >> 4, g = p0 + pl, R = i * p.ng + g;
+      const int tile = k0 / kExKTile + q;
+      if ((g >= p.ng && i < nf - 1) || R >= rows_pad || tile >= ex.kt_lim[R / kExRows]) continue;
+      unsigned char* dst =
+          ex.a_tiles + ((size_t)(R / kExRows) * H::kParts * ex.kt + part * ex.kt + tile) * ex_a_bytes(H::S);
+      ex_put<H::S>(dst, kExASlice, R % kExRows, ch, &sm.v[part][i][pl][q * kExKTile + ch * 8], s_e[i][pl]);
     }
   }
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int i = 0; i < F::kSlabs; ++i) {
+    for (int i = 0; i < kSlabs; ++i) {
       float a = acc[j][i];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -248,84 +526,116 @@ __global__ void __launch_bounds__(kGxThreads, Form<kForm>::kHalf ? 3 : 4)
 // of every band (see exact_stats_kernel); half sum: the power shared with the
 // least band (kHalfPower).
 template <int kForm>
-__global__ void gx_check_kernel(ExactPrep ex, const float* stat, const int* kend, int rows, int nc) {
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (row >= rows || ex.ea[row] == kExZeroRow) return;
+__global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const int* kend, int nf, int slabs) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= slabs * p.ng) return;
+  const int g = i % p.ng, row = gx_row(ex, p.ng, nf, i / p.ng, g);
+  if (ex.ea[row] == kExZeroRow) return;
   const float* st = stat + (size_t)row * ex.n_kseg;
   if (Form<kForm>::kHalf) {
     const int k = kend[row];
     float sum = 0.f;
     for (int s = lane; s * kExSeg < k; s += 32)
-      sum += st[s] * fminf(__int_as_float(ex.seg_pow[s]), (float)kExSeg) / (float)min(kExSeg, nc - s * kExSeg);
+      sum += st[s] * fminf(__int_as_float(ex.seg_pow[s]), (float)kExSeg) / (float)min(kExSeg, p.nc - s * kExSeg);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0 && !(sum >= (float)k * kHalfPower)) ex_raise(ex);
   } else {
+    const int k = gx_limit<kForm>(p, g, 0);
+    // rows shorter than a segment (half sum, its first columns): the
+    // segment's counts say nothing of their few elements
+    if (k < min(kExSeg, p.nc)) return;
     int sum = 0;
-    for (int s = lane; s < ex.n_kseg; s += 32)
-      sum += max(0, (int)st[s] + min(ex.seg_min[s], kExSeg) - min(kExSeg, nc - s * kExSeg));
+    for (int s = lane; s * kExSeg < k; s += 32)
+      sum += max(0, (int)st[s] + min(ex.seg_min[s], kExSeg) - min(kExSeg, p.nc - s * kExSeg));
     sum = __reduce_add_sync(0xffffffffu, sum);
-    if (lane == 0 && (long long)sum * kExOverlap < nc) ex_raise(ex);
+    if (lane == 0 && (long long)sum * kExOverlap < k) ex_raise(ex);
   }
 }
 
 // Row limits of the half sum and the contraction's shape.
-void gx_size(ExactPrep& ex, GxForm form, int nb, int nc, int ng, int nf, const std::vector<int>& igp_of, int sms,
+void gx_size(ExactPrep& ex, const GxShape& q, const std::vector<int>& igp_of, int sms, int& nf, int& nf2,
              std::vector<int>& kend, ExactTables* t) {
+  const bool half = q.form == kGxHalf, half_occ = q.form == kGxHalfOcc;
+  nf = half_occ ? 2 * kNW : half && q.with_static ? kNW + 1 : kNW;
+  nf2 = q.form == kGxGpp && q.nvband > 0 ? kNW : 0;
   kend.clear();
-  if (form == kGxHalf) {
-    kend.resize((size_t)nf * ng);
+  if (half || half_occ) {
+    kend.resize((size_t)nf * q.ng);
     for (int f = 0; f < nf; ++f)
-      for (int g = 0; g < ng; ++g)
-        kend[(size_t)f * ng + g] = igp_of[g] < 0 ? 0 : std::max(igp_of[g] - (f < kNW ? 1 : 0), 0);
+      for (int g = 0; g < q.ng; ++g)
+        kend[(size_t)f * q.ng + g] = igp_of[g] < 0 ? 0 : std::max(igp_of[g] - (half && f < kNW ? 1 : 0), 0);
   }
-  exact_size(ex, form == kGxHalf ? 7 : 6, form == kGxHalf ? 2 * nb : nb, nc, ng, nf, form != kGxReal, sms,
-             form == kGxHalf ? kend.data() : nullptr, t);
+  const bool real = q.form == kGxReal || q.form == kGxRealOcc;
+  exact_size(ex, q.form == kGxGpp || q.form == kGxReal ? 6 : 7, half || half_occ ? 2 * q.nb : q.nb, q.nc, q.ng, nf, !real, sms,
+             kend.empty() ? nullptr : kend.data(), t, nf2, nf2 ? q.nvband : 0);
 }
-size_t gx_stat_bytes(const ExactPrep& ex, int ng, int nf) { return sizeof(float) * (size_t)nf * ng * ex.n_kseg; }
+size_t gx_stat_bytes(const ExactPrep& ex) {
+  return sizeof(float) * (size_t)ex.n_row_blocks * kExRows * ex.n_kseg;
+}
+
+template <int kForm, bool kOcc>
+cudaError_t launch_ff(const GppExact& g, const GxDev& p, dim3 grid, cudaStream_t s) {
+  constexpr int smem = sizeof(FfPlanes<kForm, kOcc>);
+  cudaError_t e =
+      cudaFuncSetAttribute(gx_ff_kernel<kForm, kOcc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  gx_ff_kernel<kForm, kOcc><<<grid, kGxThreads, smem, s>>>(p, g.ex, g.stat, g.nf);
+  return cudaGetLastError();
+}
 
 template <int kForm>
-cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s) {
+cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, bool begin) {
+  using F = Form<kForm>;
   const ExactPrep& ex = g.ex;
-  cudaError_t e = exact_begin(ex, s);
+  cudaError_t e = begin ? exact_begin(ex, s) : exact_begin_counts(ex, s);
   if (e != cudaSuccess) return e;
-  e = launch_exact_b(ex, p.aqsn, p.nb, p.aqsm, Form<kForm>::kHalf ? p.nb : 0, p.nc, s);
+  const int nb = F::kHalfOcc || F::kRealOcc ? p.nvband : p.nb;
+  e = launch_exact_b(ex, p.aqsn, nb, p.aqsm, F::kHalf || F::kHalfOcc ? nb : 0, p.nc, s);
   if (e != cudaSuccess) return e;
-  gx_max_kernel<kForm><<<p.ng, kGxThreads, 0, s>>>(p, ex, g.nf);
+  const int slabs = g.nf + g.nf2;
+  gx_max_kernel<kForm><<<p.ng, kGxThreads, 0, s>>>(p, ex, g.nf, g.nf2);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  constexpr int smem = sizeof(FactorPlanes<kForm>);
-  e = cudaFuncSetAttribute(gx_factor_kernel<kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int pad = std::max(ex.n_main_blocks * kExRows - g.nf * p.ng,
+                           (ex.n_row_blocks - ex.n_main_blocks) * kExRows - g.nf2 * p.ng);
+  const dim3 grid((p.ng + pad + kGxCols - 1) / kGxCols, ex.n_kseg);
+  if constexpr (F::kF64) {
+    constexpr int smem = sizeof(typename F64<kForm>::Planes);
+    e = cudaFuncSetAttribute(gx_f64_kernel<kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    gx_f64_kernel<kForm><<<grid, kGxThreads, smem, s>>>(p, ex, g.stat, g.nf);
+    e = cudaGetLastError();
+  } else if (kForm == kGxGpp && g.nf2) {
+    e = launch_ff<kGxGpp, true>(g, p, grid, s);
+  } else {
+    e = launch_ff<kForm, false>(g, p, grid, s);
+  }
   if (e != cudaSuccess) return e;
-  const int cols = p.ng + ex.n_row_blocks * kExRows - g.nf * p.ng;
-  gx_factor_kernel<kForm>
-      <<<dim3((cols + kGxCols - 1) / kGxCols, ex.n_kseg), kGxThreads, smem, s>>>(p, ex, g.stat, g.nf);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const int rows = g.nf * p.ng;
-  gx_check_kernel<kForm><<<(rows * 32 + 255) / 256, 256, 0, s>>>(ex, g.stat, g.kend, rows, p.nc);
+  gx_check_kernel<kForm><<<(slabs * p.ng * 32 + 255) / 256, 256, 0, s>>>(p, ex, g.stat, g.kend, g.nf, slabs);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t gpp_exact_work_bytes(GxForm form, int nb, int nc, int ng, int nf, const std::vector<int>& igp_of, int sms) {
+bool gpp_exact_fits(const GxShape& q) { return (double)kNW * q.ng * q.nb * q.nc >= kExactMin; }
+
+size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms) {
   ExactPrep ex{};
   std::vector<int> kend;
-  gx_size(ex, form, nb, nc, ng, nf, igp_of, sms, kend, nullptr);
-  return exact_work_bytes(ex) + gx_stat_bytes(ex, ng, nf);
+  int nf, nf2;
+  gx_size(ex, q, igp_of, sms, nf, nf2, kend, nullptr);
+  return exact_work_bytes(ex) + gx_stat_bytes(ex);
 }
 
-bool gpp_exact_create(GppExact& g, GxForm form, int nb, int nc, int ng, int nf, const std::vector<int>& igp_of,
-                      int sms, void* shared_work) {
+bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, void* shared_work) {
   g = GppExact();
-  if ((double)nf * ng * nb * nc < kExactMin) return false;
   ExactTables t;
   std::vector<int> kend;
-  gx_size(g.ex, form, nb, nc, ng, nf, igp_of, sms, kend, &t);
+  gx_size(g.ex, q, igp_of, sms, g.nf, g.nf2, kend, &t);
   const size_t work = exact_work_bytes(g.ex), own = exact_own_bytes(g.ex);
   if (cudaMalloc(&g.own, own + sizeof(int) * kend.size()) != cudaSuccess) g.own = nullptr;
-  if (g.own && !shared_work && cudaMalloc(&g.work, work + gx_stat_bytes(g.ex, ng, nf)) != cudaSuccess) {
+  if (g.own && !shared_work && cudaMalloc(&g.work, work + gx_stat_bytes(g.ex)) != cudaSuccess) {
     cudaFree(g.own);
     g.own = g.work = nullptr;
   }
@@ -336,8 +646,7 @@ bool gpp_exact_create(GppExact& g, GxForm form, int nb, int nc, int ng, int nf, 
   }
   void* w = shared_work ? shared_work : g.work;
   exact_bind(g.ex, w, g.own);
-  g.form = form;
-  g.nf = nf;
+  g.form = q.form;
   g.stat = reinterpret_cast<float*>(static_cast<char*>(w) + work);
   g.grid = sms;
   cudaError_t e = exact_upload_tables(g.ex, t);
@@ -359,17 +668,24 @@ void gpp_exact_destroy(GppExact& g) {
   g = GppExact();
 }
 
-cudaError_t launch_gpp_exact_operands(const GppExact& g, const GxDev& p, cudaStream_t s) {
-  if (g.form == kGxHalf) return launch_operands<kGxHalf>(g, p, s);
-  if (g.form == kGxReal) return launch_operands<kGxReal>(g, p, s);
-  return launch_operands<kGxGpp>(g, p, s);
+cudaError_t launch_gpp_exact_operands(const GppExact& g, const GxDev& p, cudaStream_t s, bool begin) {
+  switch (g.form) {
+    case kGxReal: return launch_operands<kGxReal>(g, p, s, begin);
+    case kGxRealOcc: return launch_operands<kGxRealOcc>(g, p, s, begin);
+    case kGxHalf: return launch_operands<kGxHalf>(g, p, s, begin);
+    case kGxHalfOcc: return launch_operands<kGxHalfOcc>(g, p, s, begin);
+    default: return launch_operands<kGxGpp>(g, p, s, begin);
+  }
 }
 
-cudaError_t launch_gpp_exact_sums(const GppExact& g, const GxDev& p, int* status, double2* out, cudaStream_t s) {
+cudaError_t launch_gpp_exact_sums(const GppExact& g, const GxDev& p, int* status, double2* out, double2* occ_out,
+                                  cudaStream_t s) {
   cudaError_t e = launch_exact_gemm(g.ex, g.grid, status, s);
   if (e != cudaSuccess) return e;
+  const int nb = g.form == kGxHalfOcc || g.form == kGxRealOcc ? p.nvband : p.nb;
+  const bool pair = g.form == kGxHalf || g.form == kGxHalfOcc;
   FfDev d{};
-  d.nb = g.form == kGxHalf ? 2 * p.nb : p.nb;
+  d.nb = pair ? 2 * nb : nb;
   d.nc = p.nc;
   d.ng = p.ng;
   d.nf = g.nf;
@@ -377,10 +693,15 @@ cudaError_t launch_gpp_exact_sums(const GppExact& g, const GxDev& p, int* status
   d.aqsn = reinterpret_cast<const double2*>(p.aqsn);
   d.igp_of = p.igp_of;
   d.vcoul = p.vcoul;
-  d.vfac = 0.5;
-  d.pair_bands = g.form == kGxHalf ? p.nb : 0;
-  d.pair_static = g.nf > kNW;
-  return launch_exact_finish(d, g.ex, out, nullptr, s);
+  d.vfac = g.form == kGxRealOcc ? p.occ : 0.5;
+  d.pair_bands = pair ? nb : 0;
+  d.pair_static = g.form == kGxHalf && g.nf > kNW;
+  e = launch_exact_finish(d, g.ex, out, nullptr, s);
+  if (e != cudaSuccess || g.nf2 == 0) return e;
+  d.nb = p.nvband;
+  d.nf = g.nf2;
+  d.vfac = p.occ;
+  return launch_exact_finish(d, g.ex, occ_out, nullptr, s, true);
 }
 
 }  // namespace sigma

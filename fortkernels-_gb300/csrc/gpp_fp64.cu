@@ -1064,6 +1064,7 @@ __global__ void __launch_bounds__(kThreads) ssx_fp64_kernel(GppDev p, GppWork w)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
   __shared__ SsxShared sh;
+  if (w.run_if && !*w.run_if) return;
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -1106,6 +1107,7 @@ __global__ void __launch_bounds__(kThreads) ssx_fp64_batch_kernel(GppBatchView b
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
   __shared__ SsxShared sh;
+  if (b.run_if && !*b.run_if) return;
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -1114,6 +1116,7 @@ __global__ void __launch_bounds__(kThreads) ssx_fp64_batch_kernel(GppBatchView b
     const int g = s_item;
     if (g >= b.total) break;
     const int inst = batch_owner(b.item_off, b.n_inst, g);
+    if (b.work[inst].run_if && !*b.work[inst].run_if) continue;
     ssx_fp64_item(b.dev[inst], b.work[inst], g - b.item_off[inst], smem_raw, sh, tid);
   }
 }

@@ -476,10 +476,39 @@ __device__ __forceinline__ void occ_finish(const HalfDev& p, const double (&acc)
   __syncthreads();
 }
 
+// sch and ssx of an occupied band at one (column, g-vector), in FP64.
+__device__ __forceinline__ void half_occ_factor(double2 wt, double2 ie, double wx, double2& sch, double2& ssx) {
+  const double a = wt.x, b = wt.y;
+  const double b2 = guard_b2(b);
+  const double2 g = cmul(ie, wt);
+  const double c = __dsub_rn(wx, a);
+  const double wv = fma(c, c, b2);
+  sch = ssx = make_double2(0.0, 0.0);
+  if (gt_nonneg(guard_thr(a, b2), wv)) {
+    // |wx - wtilde| < gamma or |delw|^2 < to1: sch = 0
+    if (fma(a, a, b2) > kTo1 * kTo1) {
+      const double dr = wx + a;
+      const double r = rcp_f64(fma(dr, dr, b2));
+      // -G / (2 (wx + wtilde)) = -0.5 G conj(d) / |d|^2, d = (wx + a, b)
+      ssx = make_double2(-0.5 * r * fma(g.x, dr, g.y * b), -0.5 * r * fma(g.y, dr, -g.x * b));
+    }
+  } else {
+    const double r = rcp_f64(wv);
+    sch = make_double2(fma(g.x, c, -g.y * b) * r, fma(g.x, b, g.y * c) * r);
+    // Omega2 / (wx^2 - wtilde^2), Omega2 = wtilde^2 I_eps
+    const double2 w2 = make_double2(fma(a, a, -b2), 2.0 * a * b);
+    const double2 om = cmul(w2, ie);
+    const double2 d = make_double2(fma(wx, wx, -w2.x), -w2.y);
+    const double rd = rcp_f64(fma(d.x, d.x, d.y * d.y));
+    ssx = make_double2(fma(om.x, d.x, om.y * d.y) * rd, fma(om.y, d.x, -om.x * d.y) * rd);
+  }
+}
+
 // Occupied bands: one CTA per (column, frequency), threads over g-vectors,
 // kOccBands bands per pass.
 __global__ void __launch_bounds__(kThreads) half_occ_kernel(HalfDev p, double2* occ_ach,
-                                                            double2* occ_asx) {
+                                                            double2* occ_asx, const int* run_if) {
+  if (run_if && !*run_if) return;
   constexpr int kVals = kOccBands * 8;  // per band: T_sch, U_sch, T_ssx, U_ssx (complex)
   __shared__ double red[kThreads / 32][kVals];
   __shared__ double tot[kVals];
@@ -496,30 +525,8 @@ __global__ void __launch_bounds__(kThreads) half_occ_kernel(HalfDev p, double2* 
     for (int ig = tid; ig < kend; ig += kThreads) {
       const size_t off = (size_t)col * p.nc + ig;
       const double2 wt = p.wt[off], ie = p.ieps[off];
-      const double a = wt.x, b = wt.y;
-      const double b2 = guard_b2(b);
-      const double2 g = cmul(ie, wt);
-      const double c = __dsub_rn(wx, a);
-      const double wv = fma(c, c, b2);
-      double2 sch = make_double2(0.0, 0.0), ssx = make_double2(0.0, 0.0);
-      if (gt_nonneg(guard_thr(a, b2), wv)) {
-        // |wx - wtilde| < gamma or |delw|^2 < to1: sch = 0
-        if (fma(a, a, b2) > kTo1 * kTo1) {
-          const double dr = wx + a;
-          const double r = rcp_f64(fma(dr, dr, b2));
-          // -G / (2 (wx + wtilde)) = -0.5 G conj(d) / |d|^2, d = (wx + a, b)
-          ssx = make_double2(-0.5 * r * fma(g.x, dr, g.y * b), -0.5 * r * fma(g.y, dr, -g.x * b));
-        }
-      } else {
-        const double r = rcp_f64(wv);
-        sch = make_double2(fma(g.x, c, -g.y * b) * r, fma(g.x, b, g.y * c) * r);
-        // Omega2 / (wx^2 - wtilde^2), Omega2 = wtilde^2 I_eps
-        const double2 w2 = make_double2(fma(a, a, -b2), 2.0 * a * b);
-        const double2 om = cmul(w2, ie);
-        const double2 d = make_double2(fma(wx, wx, -w2.x), -w2.y);
-        const double rd = rcp_f64(fma(d.x, d.x, d.y * d.y));
-        ssx = make_double2(fma(om.x, d.x, om.y * d.y) * rd, fma(om.y, d.x, -om.x * d.y) * rd);
-      }
+      double2 sch, ssx;
+      half_occ_factor(wt, ie, wx, sch, ssx);
       const bool pair = ig != igp - 1;
 #pragma unroll
       for (int q = 0; q < kOccBands; ++q)
@@ -944,7 +951,7 @@ __global__ void __launch_bounds__(256) half_zs_slices_kernel(HalfDev p, OzakiPre
 constexpr int kRowWarps = 8;
 __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
     HalfDev p, const double2* t3, const double2* u3, const double2* ts, const double2* us, int stride3, int stride1,
-    const int* skip_if, const double2* occ_ach, const double2* occ_asx, double2* acht_n1, double2* asx_n1, double2* stat_n1) {
+    const int* skip_if, const double2* tu_occ, const double2* occ_ach, const double2* occ_asx, double2* acht_n1, double2* asx_n1, double2* stat_n1) {
   constexpr int kVals = 4 * kNW + 2;  // ax, ay, sx, sy per frequency; qx, qy
   __shared__ double part[kRowWarps][kVals];
   if (skip_if && *skip_if) return;
@@ -969,7 +976,24 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
         qy.add(w * v.y);
       }
     }
-    if (occ) {
+    if (occ && tu_occ) {
+      // the partner's sum leaves g-vector igp - 1 out: its term, which the
+      // contraction holds, taken off again
+      if (igp > 0 && igp <= p.brk[col]) {
+        const size_t og = (size_t)col * p.nc + igp - 1;
+        const double2 ag = p.aqsm[(size_t)n1 * p.nc + igp - 1];
+#pragma unroll
+        for (int iw = 0; iw < kNW; ++iw) {
+          double2 sch, ssx;
+          half_occ_factor(p.wt[og], p.ieps[og], wx[iw], sch, ssx);
+          const double2 vs = cmul(am, cconj(cmul(ag, sch))), vx = cmul(am, cconj(cmul(ag, ssx)));
+          ax[iw].add(-w * vs.x);
+          ay[iw].add(-w * vs.y);
+          sx[iw].add(-2.0 * w * p.occ * vx.x);
+          sy[iw].add(-2.0 * w * p.occ * vx.y);
+        }
+      }
+    } else if (occ) {
 #pragma unroll
       for (int iw = 0; iw < kNW; ++iw) {
         const double2 a = occ_ach[((size_t)n1 * p.ng + col) * kNW + iw];
@@ -1018,8 +1042,16 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
   for (int iw = 0; iw < kNW; ++iw) {
     const double rx = tot[4 * iw], ry = tot[4 * iw + 1], ux = tot[4 * iw + 2], uy = tot[4 * iw + 3];
     if (occ) {
-      acht_n1[n1 * kNW + iw] = make_double2(rx, ry);
-      asx_n1[n1 * kNW + iw] = make_double2(ux, uy);
+      double2 a = make_double2(0.0, 0.0), x = a;
+      if (tu_occ) {  // T + conj(U) of sch and ssx, both weighted 0.5 vcoul
+        const double2* t = tu_occ + (size_t)n1 * 2 * kNW;
+        const double2* u = t + (size_t)p.nvband * 2 * kNW;
+        a = make_double2(t[iw].x + u[iw].x, t[iw].y - u[iw].y);
+        const double q = 2.0 * p.occ;
+        x = make_double2(q * (t[kNW + iw].x + u[kNW + iw].x), q * (t[kNW + iw].y - u[kNW + iw].y));
+      }
+      acht_n1[n1 * kNW + iw] = make_double2(rx + a.x, ry + a.y);
+      asx_n1[n1 * kNW + iw] = make_double2(ux + x.x, uy + x.y);
     } else {
       const double2 a = t3[(size_t)n1 * stride3 + iw], b = u3[(size_t)n1 * stride3 + iw];
       acht_n1[n1 * kNW + iw] = make_double2(rx + a.x + b.x, ry + a.y - b.y);
@@ -1066,7 +1098,9 @@ struct sigma_gpp_halfsum_plan_s {
   // exact contraction over the bands of aqsn and aqsm; the FP64 passes then
   // run only when its flag is raised
   sigma::GppExact exact{};
-  double2* tu = nullptr;  // [2 nb][3 or 4]
+  sigma::GppExact exact_occ{};  // the occupied bands' sch and ssx, one flag with exact
+  double2* tu = nullptr;        // [2 nb][3 or 4]
+  double2* tu_occ = nullptr;    // [2 nvband][6]
   double2 *t3 = nullptr, *u3 = nullptr, *ts = nullptr, *us = nullptr;  // [nb][3], [nb][1]
 };
 
@@ -1205,15 +1239,19 @@ extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int nu
       return st;
     }
   }
-  if (!tensor) {
-    const int nf = (flags & SIGMA_HALFSUM_STATIC) ? kNW + 1 : kNW;
-    if (gpp_exact_create(p->exact, kGxHalf, number_bands, ncouls, ngpown, nf, igp_of, sms) &&
-        cudaMalloc(&p->tblock, sizeof(double2) * 2 * (size_t)number_bands * nf) != cudaSuccess) {
+  const GxShape q{kGxHalf, number_bands, nvband, ncouls, ngpown, (flags & SIGMA_HALFSUM_STATIC) != 0};
+  if (!tensor && gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms)) {
+    const size_t n = 2 * (size_t)number_bands * p->exact.nf, n_occ = 2 * (size_t)nvband * 2 * kNW;
+    if (cudaMalloc(&p->tblock, sizeof(double2) * (n + n_occ)) != cudaSuccess) {
       cudaGetLastError();
       p->tblock = nullptr;
       gpp_exact_destroy(p->exact);
+    } else {
+      p->tu = static_cast<double2*>(p->tblock);
+      p->tu_occ = p->tu + n;
+      const GxShape qo{kGxHalfOcc, nvband, nvband, ncouls, ngpown, false};
+      if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->exact.ex.flag;
     }
-    p->tu = static_cast<double2*>(p->tblock);
   }
   *out = p;
   return SIGMA_OK;
@@ -1229,6 +1267,7 @@ extern "C" int sigma_gpp_halfsum_plan_destroy(sigma_gpp_halfsum_plan p) {
   if (p->ff1) sigma_ff_plan_destroy(p->ff1);
   if (p->tblock) cudaFree(p->tblock);
   sigma::gpp_exact_destroy(p->exact);
+  sigma::gpp_exact_destroy(p->exact_occ);
   cudaSetDevice(cur);
   delete p;
   return SIGMA_OK;
@@ -1278,10 +1317,8 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
       SIGMA_CUDA_TRY(cudaGetLastError());
       half_occ_ff_kernel<<<dim3(kNW, plan->ng), kThreads, 0, s>>>(p, plan->m32, plan->n32,
                                                                   plan->occ_ach, plan->occ_asx);
-    } else {
-      half_occ_kernel<<<dim3(plan->ng, kNW), kThreads, 0, s>>>(p, plan->occ_ach, plan->occ_asx);
+      SIGMA_CUDA_TRY(cudaGetLastError());
     }
-    SIGMA_CUDA_TRY(cudaGetLastError());
   }
   if (plan->ff3) {
     const bool stat = plan->ff1 && achstemp;
@@ -1311,7 +1348,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
     }
     if (st != SIGMA_OK) return st;
     half_tensor_rows_kernel<<<plan->nb, kRowWarps * 32, 0, s>>>(
-        p, plan->t3, plan->u3, stat ? plan->ts : nullptr, plan->us, kNW, 1, nullptr, plan->occ_ach, plan->occ_asx,
+        p, plan->t3, plan->u3, stat ? plan->ts : nullptr, plan->us, kNW, 1, nullptr, nullptr, plan->occ_ach, plan->occ_asx,
         plan->acht_n1, plan->asx_n1, plan->stat_n1);
     SIGMA_CUDA_TRY(cudaGetLastError());
     half_reduce_total_kernel<<<1, 256, 0, s>>>(plan->acht_n1, plan->asx_n1, plan->stat_n1, plan->nb,
@@ -1327,15 +1364,28 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
   const int* flag = nullptr;
   if (plan->exact) {
     auto D = [](const double2* x) { return reinterpret_cast<const double*>(x); };
-    const GxDev x{plan->nb, plan->nc, plan->ng, D(aqsm), D(aqsn), D(ieps), D(wt), vcoul, wx_array, plan->igp_of};
+    const GxDev x{plan->nb, plan->nvband, plan->nc, plan->ng, occ,      D(aqsm),       D(aqsn),
+                  D(ieps),  D(wt),        vcoul,    wx_array, plan->igp_of, plan->brk};
+    // one flag for both contractions
     SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s));
-    SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->tu, s));
+    if (plan->exact_occ) SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact_occ, x, s, false));
+    SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->tu, nullptr, s));
+    if (plan->exact_occ)
+      SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact_occ, x, plan->counters + 2, plan->tu_occ, nullptr, s));
+    wm.run_if = ws.run_if = flag = plan->exact.ex.flag;
+  }
+  if (plan->nvband > 0) {
+    half_occ_kernel<<<dim3(plan->ng, kNW), kThreads, 0, s>>>(p, plan->occ_ach, plan->occ_asx,
+                                                             plan->exact_occ ? flag : nullptr);
+    SIGMA_CUDA_TRY(cudaGetLastError());
+  }
+  if (plan->exact) {
     const int nf = plan->exact.nf;
     const double2* u = plan->tu + (size_t)plan->nb * nf;
-    wm.run_if = ws.run_if = flag = plan->exact.ex.flag;
     half_tensor_rows_kernel<<<plan->nb, kRowWarps * 32, 0, s>>>(
-        p, plan->tu, u, stat ? plan->tu + kNW : nullptr, u + kNW, nf, nf, flag, plan->occ_ach, plan->occ_asx,
-        plan->acht_n1, plan->asx_n1, plan->stat_n1);
+        p, plan->tu, u, stat ? plan->tu + kNW : nullptr, u + kNW, nf, nf, flag,
+        plan->exact_occ ? plan->tu_occ : nullptr, plan->occ_ach, plan->occ_asx, plan->acht_n1, plan->asx_n1,
+        plan->stat_n1);
     SIGMA_CUDA_TRY(cudaGetLastError());
   }
   if (plan->wm.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<3>(p, wm, plan->main_grid, s));

@@ -257,6 +257,7 @@ __global__ void __launch_bounds__(kThreads, 2) sch_real_kernel(GppRealDev p, Gpp
 __global__ void __launch_bounds__(kThreads) ssx_real_kernel(GppRealDev p, GppWork w) {
   __shared__ int s_item;
   __shared__ double red[kSsxBN][kNW][kThreads / 32];
+  if (w.run_if && !*w.run_if) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double iwx2[kNW];
 #pragma unroll
@@ -343,7 +344,9 @@ struct sigma_gpp_real_plan_s {
   int device = 0, nb = 0, nvband = 0, nc = 0, ng = 0;
   int sch_grid = 0, ssx_grid = 0;
   sigma::GppWork sch{}, ssx{};
-  sigma::GppExact exact{};  // when set, sch runs only when its flag is raised
+  // the band sums and (one flag) the occupied bands' on the tensor cores; sch and
+  // ssx run only without them or when the flag is raised
+  sigma::GppExact exact{}, exact_occ{};
   void* block = nullptr;
   int* igp_of = nullptr;
   int* counters = nullptr;
@@ -412,7 +415,11 @@ extern "C" int sigma_gpp_real_plan_create(sigma_gpp_real_plan* out, int number_b
     delete p;
     return SIGMA_ERR_CUDA;
   }
-  gpp_exact_create(p->exact, kGxReal, number_bands, ncouls, ngpown, kNW, igp_of, sms);
+  const GxShape q{kGxReal, number_bands, nvband, ncouls, ngpown, false};
+  if (gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms) && nvband > 0) {
+    const GxShape qo{kGxRealOcc, nvband, nvband, ncouls, ngpown, false};
+    if (gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->exact.ex.flag;
+  }
   *out = p;
   return SIGMA_OK;
 }
@@ -424,6 +431,7 @@ extern "C" int sigma_gpp_real_plan_destroy(sigma_gpp_real_plan p) {
   cudaSetDevice(p->device);
   if (p->block) cudaFree(p->block);
   sigma::gpp_exact_destroy(p->exact);
+  sigma::gpp_exact_destroy(p->exact_occ);
   cudaSetDevice(cur);
   delete p;
   return SIGMA_OK;
@@ -446,12 +454,18 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
   GppRealDev p{plan->nb, plan->nvband, plan->nc, plan->ng, occ, aqsmtemp, aqsntemp, I_eps_array,
                wtilde_array, vcoul, wx_array, plan->igp_of};
   SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 3 * sizeof(int), s));
-  GppWork sch = plan->sch;
+  GppWork sch = plan->sch, ssx = plan->ssx;
   if (plan->exact) {
-    const GxDev x{p.nb, p.nc, p.ng, p.aqsm, p.aqsn, p.ieps, p.wt, p.vcoul, p.wx, p.igp_of};
+    const GxDev x{p.nb, p.nvband, p.nc, p.ng, p.occ, p.aqsm, p.aqsn, p.ieps, p.wt, p.vcoul, p.wx, p.igp_of};
     SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s));
-    SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->acht_n1, s));
+    if (plan->exact_occ) SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact_occ, x, s, false));
+    SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->acht_n1, nullptr, s));
     sch.run_if = plan->exact.ex.flag;
+    if (plan->exact_occ) {
+      SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact_occ, x, plan->counters + 2,
+                                           plan->acht_n1 + (size_t)plan->nb * kNW, nullptr, s));
+      ssx.run_if = plan->exact.ex.flag;
+    }
   }
   if (plan->sch.n_items > 0) {
     SIGMA_CUDA_TRY(cudaFuncSetAttribute(sch_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -463,13 +477,13 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
     SIGMA_CUDA_TRY(cudaGetLastError());
   }
   if (plan->ssx.n_items > 0) {
-    ssx_real_kernel<<<plan->ssx_grid, kThreads, 0, s>>>(p, plan->ssx);
+    ssx_real_kernel<<<plan->ssx_grid, kThreads, 0, s>>>(p, ssx);
     SIGMA_CUDA_TRY(cudaGetLastError());
   }
   double2* ach_c = plan->outc;
   double2* asx_c = plan->outc + kNW;
   double2* n1_c = plan->outc + 2 * kNW;
-  SIGMA_CUDA_TRY(launch_gpp_reduce(sch, plan->ssx, plan->nb, plan->acht_n1, ach_c, asx_c,
+  SIGMA_CUDA_TRY(launch_gpp_reduce(sch, ssx, plan->nb, plan->acht_n1, ach_c, asx_c,
                                    acht_n1_loc ? n1_c : nullptr, s));
   const int nthreads = 256, n = std::max(plan->nb, kNW);
   real_parts_kernel<<<(n + nthreads - 1) / nthreads, nthreads, 0, s>>>(ach_c, asx_c, n1_c, plan->nb,

@@ -22,7 +22,8 @@ __device__ __forceinline__ void reduce_bands_row(const ReduceArgs& a, int row) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_sch = a.sch_rows * kNW;
   const bool is_sch = row < n_sch;
-  if (is_sch && a.sch_run_if && !*a.sch_run_if) return;
+  const int* run_if = is_sch ? a.sch_run_if : a.ssx_run_if;
+  if (run_if && !*run_if) return;
   const int e = is_sch ? row : row - n_sch;
   const int n1 = e / kNW, iw = e % kNW;
   const int bn = is_sch ? a.sch_bn : kSsxBN;
@@ -115,6 +116,7 @@ ReduceJob gpp_reduce_job(const GppWork& sch, const GppWork& ssx, int nb, double2
   a.sch_rows = sch.partial ? nb : 0;
   a.sch_partial = sch.partial;
   a.sch_run_if = sch.run_if;
+  a.ssx_run_if = ssx.run_if;
   a.sch_ncb = sch.n_col_blocks;
   a.sch_splits = sch.n_splits;
   a.sch_bn = sch.bn;
@@ -152,6 +154,7 @@ cudaError_t launch_gpp_reduce(const GppWork& sch, const GppWork& ssx, int nb, do
   a.sch_rows = sch.partial ? nb : 0;
   a.sch_partial = sch.partial;
   a.sch_run_if = sch.run_if;
+  a.ssx_run_if = ssx.run_if;
   a.sch_ncb = sch.n_col_blocks;
   a.sch_splits = sch.n_splits;
   a.sch_bn = sch.bn;

@@ -192,7 +192,8 @@ cudaError_t launch_tensor_factors(const GppDev& p, const GppWork& w, const Mixed
 struct ReduceArgs {
   int sch_rows;       // bands whose sums come from sch partials (0: acht_n1 already holds them)
   const double2* sch_partial;
-  const int* sch_run_if;  // nonnull: acht_n1 already holds the band sums unless this word is nonzero
+  // nonnull: acht_n1 (asx_n1) already holds the band sums unless this word is nonzero
+  const int *sch_run_if, *ssx_run_if;
   int sch_ncb, sch_splits, sch_bn;
   const double2* ssx_partial;
   int ssx_ncb, ssx_splits;
