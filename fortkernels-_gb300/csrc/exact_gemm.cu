@@ -485,13 +485,14 @@ __device__ __forceinline__ double2 ex_weight(const FfDev& p, int n, int f, int i
   return m[(size_t)(second ? n - p.pair_bands : n) * p.nc + igp];
 }
 
-// One CTA per (row block, band block): tempz of 128 rows x the block's bands from the pieces' raw sums (added as integers, so their order does not
+// One CTA per (row block, band block, eighth of its B' rows): tempz of 128 rows x
+// 8 to 10 bands from the pieces' raw sums (added as integers, so their order does not
 // matter), times weight * conj(aqsm[n1][igp]), summed over the rows of each
 // frequency in a fixed order.
-constexpr int kFinRow = kExRows + 1;
+constexpr int kFinRow = kExRows + 1, kFinThreads = 256;
 template <bool kReal>
-__global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex, int rb0) {
-  const int kBands = ex.bands, kCols = ex.cols;
+__global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, ExactPrep ex, int rb0) {
+  const int kCols = ex.cols, kBands = kCols / 8, b0 = blockIdx.z * kBands;  // bands b0 .. of the block
   extern __shared__ double2 s_prod[];  // [bands][129], complex or real
   double* s_real = reinterpret_cast<double*>(s_prod);
   if (*ex.flag) return;
@@ -503,14 +504,15 @@ __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex
   const double wgt = ff_column_weight(p, igp);
   const int e_row = R < rows ? ex.ea[rb0 * kExRows + R] : 0, np = ex.pieces[rb0 + rb];
   const size_t base = block * ex.max_pieces * kCols * kExRows + r;
-  for (int b = tid >> 7; b < kBands; b += 2) {
-    const int n = cb * kBands + b;
+  for (int b = tid >> 7; b < kBands; b += kFinThreads / kExRows) {
+    const int n = cb * ex.bands + b0 + b;
     double2 v = make_double2(0.0, 0.0);
     if (igp >= 0 && n < p.nb) {
       long long hr = 0, hi = 0;
       double lr = 0.0, li = 0.0;
+#pragma unroll 4
       for (int q = 0; q < np; ++q) {
-        const size_t o = base + ((size_t)q * kCols + (kReal ? b : 2 * b)) * kExRows;
+        const size_t o = base + ((size_t)q * kCols + (kReal ? b0 + b : 2 * (b0 + b))) * kExRows;
         hr += ex.raw_hi[o];
         lr += ex.raw_lo[o];
         if (!kReal) {
@@ -535,7 +537,7 @@ __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex
   }
   __syncthreads();
   const int f0 = rb * kExRows / p.ng, f1 = (min((rb + 1) * kExRows, rows) - 1) / p.ng;
-  for (int o = warp; o < kBands * (f1 - f0 + 1); o += 8) {
+  for (int o = warp; o < kBands * (f1 - f0 + 1); o += kFinThreads / 32) {
     const int b = o % kBands, fo = f0 + o / kBands;
     const int lo = max(fo * p.ng - rb * kExRows, 0), hi = min((fo + 1) * p.ng - rb * kExRows, kExRows);
     double sx = 0.0, sy = 0.0, tx = 0.0, ty = 0.0;
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(256) exact_finish_kernel(FfDev p, ExactPrep ex
       }
     }
     if (lane == 0) {
-      const size_t i = (block * ex.max_seg + (fo - f0)) * kBands + b;
+      const size_t i = (block * ex.max_seg + (fo - f0)) * ex.bands + b0 + b;
       ex.partial[i] = make_double2(sx, sy);
       if (p.vcoul2) ex.partial2[i] = make_double2(tx, ty);
     }
@@ -632,7 +634,8 @@ void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool 
     kl[rb] = (k + 31) / 32 * 2;
   }
   // K splits: as few as fill the grid's waves well.  An item costs its tiles
-  // plus about 6 tiles' time for its raw sums and the ring's refill.  Ragged
+  // plus about 6 tiles' time for its raw sums and the ring's refill, a piece
+  // about one tile's time in the epilogue.  Ragged
   // row limits (items of different lengths) take at least 10 items per CTA.
   const int all = ex.halves * ex.kt;
   const long long blocks = (long long)ex_block_index(ex, ex.n_row_blocks, 0);
@@ -642,7 +645,7 @@ void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool 
     const long long items = blocks * s;
     if (row_kend && items < 10LL * grid && s < std::min(all / 2, 96)) continue;
     const int len = (all / 2 + s - 1) / s * 2;
-    const long long cost = (items + grid - 1) / grid * (len + 6LL);
+    const long long cost = (items + grid - 1) / grid * (len + 6LL) + s;
     if (cost < best) {
       best = cost;
       splits = s;
@@ -768,12 +771,10 @@ cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* ou
                                 bool second_rows) {
   const int rb0 = second_rows ? ex.n_main_blocks : 0;
   const int nrb = (d.nf * d.ng + kExRows - 1) / kExRows, ncb = (d.nb + ex.bands - 1) / ex.bands;
-  const int smem = ex.cols / 2 * kFinRow * (int)sizeof(double2);
+  const int smem = ex.cols / 8 * kFinRow * (int)(ex.halves == 1 ? sizeof(double) : sizeof(double2));
   auto* kernel = ex.halves == 1 ? exact_finish_kernel<true> : exact_finish_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  kernel<<<dim3(nrb, ncb), 256, smem, s>>>(d, ex, rb0);
-  e = cudaGetLastError();
+  kernel<<<dim3(nrb, ncb, ex.bands / (ex.cols / 8)), kFinThreads, smem, s>>>(d, ex, rb0);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int blocks = (d.nb * d.nf * 32 + 255) / 256;
   exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, rb0, ex.partial, out);

@@ -69,9 +69,22 @@ __device__ __forceinline__ int gx_rows_end(const ExactPrep& ex, int nf, int slab
   return (slab < nf ? ex.n_main_blocks : ex.n_row_blocks) * kExRows;
 }
 
-// One CTA per column: exponents of its rows.  Magnitudes from FP32 values (c
-// from exact FP32 halves), the guard taken somewhat wide on both sides, with
-// a 2^-8 margin; what FP32 cannot bound raises the flag.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The leading 24 bits of a double as FP32 (integer pipe).
+__device__ __forceinline__ float f32_lead(double x) { return ff_of(x).hi; }
+__device__ __forceinline__ bool any_bits(double2 v) {
+  return ((unsigned)__double2hiint(v.x) << 1 | (unsigned)__double2loint(v.x) | (unsigned)__double2hiint(v.y) << 1 |
+          (unsigned)__double2loint(v.y)) != 0;
+}
+
+// One CTA per column: exponents of its rows.  Squared magnitudes from FP32
+// values (c from exact FP32 halves), the guard taken somewhat wide on both
+// sides, with a 2^-8 margin; what FP32 cannot bound raises the flag.
 template <int kForm>
 __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep ex, int nf, int nf2) {
   using F = Form<kForm>;
@@ -79,62 +92,70 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
   const int g = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool occ = F::kHalfOcc || F::kRealOcc || nf2 > 0;
   FF wx[kNW];
-  float iwx2[kNW];
+  float iwx4[kNW];
+  bool huge = false;  // |wx| or |wtilde| above 1e15: reciprocals may flush to 0
 #pragma unroll
   for (int iw = 0; iw < kNW; ++iw) {
     wx[iw] = ff_of(p.wx[iw]);
-    iwx2[iw] = __frcp_rn(wx[iw].hi * wx[iw].hi);
+    huge = huge || !(fabsf(wx[iw].hi) < 1e15f);
+    const float i2 = rcp_approx(wx[iw].hi * wx[iw].hi);
+    iwx4[iw] = i2 * i2;
   }
-  unsigned m[F::kSlabs];  // bits of non-negative floats; NaN counts as infinite
+  unsigned m[F::kSlabs];  // bits of non-negative floats; infinite and NaN are the largest
 #pragma unroll
   for (int i = 0; i < F::kSlabs; ++i) m[i] = 0u;
-  auto top = [](unsigned& v, float y) { v = max(v, __float_as_uint(y != y ? INFINITY : y)); };
+  auto top = [](unsigned& v, float y) { v = max(v, __float_as_uint(y)); };
   bool bad = false;
   const int k_end = gx_limit<kForm>(p, g, F::kSlabs - 1), k_freq = gx_limit<kForm>(p, g, 0);
-#pragma unroll 4
-  for (int k = tid; k < k_end; k += kGxThreads) {
-    const double2 w = gx_load<kForm>(p.wt, (size_t)g * p.nc + k), e = gx_load<kForm>(p.ieps, (size_t)g * p.nc + k);
-    const FF a = ff_of(w.x);
-    const float b = __double2float_rn(w.y), er = __double2float_rn(e.x), ei = __double2float_rn(e.y);
+  auto element = [&](int k, double2 w, double2 e) {
+    const float er = f32_lead(e.x), ei = F::kReal ? 0.f : f32_lead(e.y);
+    const float e2 = fmaf(er, er, ei * ei);
     if (F::kHalf) {
-      top(m[F::kSlabs - 1], fmaxf(fabsf(er), fabsf(ei)));
-      if (er != er || ei != ei) m[F::kSlabs - 1] = 0x7F800000u;
-      if (k >= k_freq || k % kIgBlk == kIgBlk - 1) continue;
+      top(m[F::kSlabs - 1], e2);
+      if (k >= k_freq || k % kIgBlk == kIgBlk - 1) return;
     }
-    const float gx = er * a.hi - ei * b, gy = er * b + ei * a.hi;
-    const float s2 = fmaf(a.hi, a.hi, b * b);
-    const float om = fmaxf(fabsf(gx * a.hi - gy * b), fabsf(gx * b + gy * a.hi));
+    const FF a = ff_of(w.x);
+    const float b = F::kReal ? 0.f : f32_lead(w.y), b2 = b * b;
+    const float s2 = fmaf(a.hi, a.hi, b2), g2 = s2 * e2;  // |wtilde|^2, |G|^2
+    huge = huge || !(s2 < 1e30f);
+    const bool any = any_bits(w) && any_bits(e);
     // the guard's threshold, somewhat above and below
     const float up = fmaxf(0.2501f, s2 * 4.001e-6f), low = 0.2499f;
-    const bool any = (e.x != 0.0 || e.y != 0.0) && (w.x != 0.0 || w.y != 0.0);
 #pragma unroll
     for (int iw = 0; iw < kNW; ++iw) {
       const float c = (wx[iw].hi - a.hi) + (wx[iw].lo - a.lo);
-      const float w2 = fmaf(c, c, b * b);
-      if (w2 > 1e30f) m[iw] = 0x7F800000u;  // the FP32 reciprocal may be 0: flagged below
+      const float w2 = fmaf(c, c, b2), r = rcp_approx(w2);
       if (!F::kRealOcc && (F::kHalf ? !(w2 > up) : !(w2 <= low))) {  // also NaN
-        const float y = fmaxf(fabsf(gx * c - gy * b), fabsf(gy * c + gx * b)) * __frcp_rn(w2);
+        const float y = g2 * r;
         top(m[iw], y);
-        bad = bad || (any && !(y > 1e-18f));
+        bad = bad || (any && !(y > 1e-36f));
       }
       if (!F::kHalf && (!F::kReal || F::kRealOcc) && occ) {
         const float z = (wx[iw].hi + a.hi) + (wx[iw].lo + a.lo);
-        const float rz = __frcp_rn(fmaf(z, z, b * b));
-        float y = 0.f;
-        if (!(w2 > up)) y = 0.5f * fmaxf(fabsf(gx * z + gy * b), fabsf(gy * z - gx * b)) * rz;
-        if (!(w2 <= low)) {
-          if (F::kHalfOcc) {  // Omega2 / ((wx - wtilde) (wx + wtilde)): within sqrt(2) of its larger part
-            y = fmaxf(y, 1.5f * om * sqrtf(__frcp_rn(w2) * rz));
-          } else {
-            y = fmaxf(y, om * iwx2[iw]);
-          }
-        }
+        const float rz = rcp_approx(fmaf(z, z, b2));
+        float y = w2 > up ? 0.f : 0.25f * g2 * rz;  // |G / (2 (wx + wtilde))|^2
+        // |Omega2 / (wx^2 - wtilde^2)|^2, |Omega2 / wx^2|^2
+        if (!(w2 <= low)) y = fmaxf(y, s2 * g2 * (F::kHalfOcc ? r * rz : iwx4[iw]));
         top(m[F::kSlabs > kNW ? kNW + iw < F::kSlabs ? kNW + iw : 0 : iw], y);
-        bad = bad || (any && !(y > 1e-18f));
+        bad = bad || (any && !(y > 1e-36f));
       }
     }
+  };
+  // four elements' loads in flight per thread
+  for (int k0 = tid; k0 < k_end; k0 += 4 * kGxThreads) {
+    double2 w[4], e[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = min(k0 + q * kGxThreads, k_end - 1);
+      w[q] = gx_load<kForm>(p.wt, (size_t)g * p.nc + k);
+      e[q] = gx_load<kForm>(p.ieps, (size_t)g * p.nc + k);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (k0 + q * kGxThreads < k_end) element(k0 + q * kGxThreads, w[q], e[q]);
   }
   bad = __syncthreads_or(bad);
+  huge = __syncthreads_or(huge);
 #pragma unroll
   for (int i = 0; i < F::kSlabs; ++i) {
     const unsigned v = __reduce_max_sync(0xffffffffu, m[i]);
@@ -144,9 +165,9 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
   if (tid < nf + nf2) {
     unsigned v = 0;
     for (int q = 0; q < kGxThreads / 32; ++q) v = max(v, s_m[tid][q]);
-    const float f = __uint_as_float(v) * (1.f + 1.f / 256.f);
+    const float f = sqrtf(__uint_as_float(v)) * (1.f + 1.f / 256.f);
     // a factor too small for FP32 may only be ignored beside large ones
-    if (!(f < 1e18f) || (bad && !(f > 1e-6f)) || (v && f < 1e-18f)) ex_raise(ex);
+    if (huge || !(f < 1e18f) || (bad && !(f > 1e-6f)) || (v && f < 1e-18f)) ex_raise(ex);
     // float-float digits need a bit of room (ex_ff_digits)
     ex.ea[gx_row(ex, p.ng, nf, tid, g)] =
         v ? (int)(__float_as_uint(f) >> 23) - 126 + (F::kF64 ? 0 : 1) : kExZeroRow;
@@ -263,10 +284,10 @@ struct FfPlanes {
   float2 v[Form<kForm>::kParts][kSlabs][kGxCols][kFfK + 1];  // conflict-free along g-vectors and along columns
 };
 
-// Items (column block, 512-g-vector segment).  Column blocks run past ng to
+// Items (column block, run of `run` g-vectors).  Column blocks run past ng to
 // cover the padding rows of each group's last row block (zero digits).
 template <int kForm, bool kOcc>
-__global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep ex, float* stat, int nf) {
+__global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep ex, float* stat, int nf, int run) {
   using F = Form<kForm>;
   constexpr int kSlabs = FfPlanes<kForm, kOcc>::kSlabs;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -277,7 +298,7 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
   __shared__ bool s_wide;
   if (*ex.flag) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int p0 = blockIdx.x * kGxCols, seg = blockIdx.y;
+  const int p0 = blockIdx.x * kGxCols;
   if (tid == 0) {
     s_need = 0;
     bool wide = false;
@@ -301,7 +322,7 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
     if ((g < p.ng || last) && R < gx_rows_end(ex, nf, i)) atomicMax(&s_need, ex.kt_lim[R / kExRows] * kExKTile);
   }
   __syncthreads();
-  const int k_begin = seg * kExSeg, k_end = min(s_need, k_begin + kExSeg);  // tiles the contraction reads
+  const int k_begin = blockIdx.y * run, k_end = min(s_need, k_begin + run);  // tiles the contraction reads
   float acc[2][kSlabs];  // large factors per column of this warp
 #pragma unroll
   for (int j = 0; j < 2; ++j)
@@ -357,7 +378,7 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       const int g = p0 + warp + 8 * j;
-      if (lane == 0 && g < p.ng) stat[(size_t)gx_row(ex, p.ng, nf, i, g) * ex.n_kseg + seg] = a;
+      if (lane == 0 && g < p.ng) stat[(size_t)gx_row(ex, p.ng, nf, i, g) * gridDim.y + blockIdx.y] = a;
     }
 }
 
@@ -439,7 +460,7 @@ __device__ __forceinline__ void gx_f64_factors(const double (&wx)[kNW], const do
 
 template <int kForm>
 __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm>::kReal ? 3 : 4)
-    gx_f64_kernel(GxDev p, ExactPrep ex, float* stat, int nf) {
+    gx_f64_kernel(GxDev p, ExactPrep ex, float* stat, int nf, int run) {
   using H = F64<kForm>;
   constexpr int kSlabs = H::kSlabs, kK = H::kK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -447,7 +468,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
   __shared__ int s_e[kSlabs][kGxCols], s_lim[2][kGxCols], s_need;
   if (*ex.flag) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int p0 = blockIdx.x * kGxCols, seg = blockIdx.y;
+  const int p0 = blockIdx.x * kGxCols;
   const int rows_pad = ex.n_row_blocks * kExRows;
   const double wx[kNW] = {p.wx[0], p.wx[1], p.wx[2]};
   double iwx2[kNW];
@@ -462,7 +483,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
     if (R < rows_pad && (g < p.ng || i == nf - 1)) atomicMax(&s_need, ex.kt_lim[R / kExRows] * kExKTile);
   }
   __syncthreads();
-  const int k_begin = seg * kExSeg, k_end = min(s_need, k_begin + kExSeg);  // tiles the contraction reads
+  const int k_begin = blockIdx.y * run, k_end = min(s_need, k_begin + run);  // tiles the contraction reads
   float acc[2][kSlabs] = {};  // per column of this warp
   for (int k0 = k_begin; k0 < k_end; k0 += kK) {
     __syncthreads();
@@ -518,7 +539,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       const int g = p0 + warp + 8 * j;
-      if (lane == 0 && i < nf && g < p.ng) stat[(size_t)(i * p.ng + g) * ex.n_kseg + seg] = a;
+      if (lane == 0 && i < nf && g < p.ng) stat[(size_t)(i * p.ng + g) * gridDim.y + blockIdx.y] = a;
     }
 }
 
@@ -526,17 +547,23 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
 // of every band (see exact_stats_kernel); half sum: the power shared with the
 // least band (kHalfPower).
 template <int kForm>
-__global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const int* kend, int nf, int slabs) {
+__global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const int* kend, int nf, int slabs, int per_seg) {
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= slabs * p.ng) return;
   const int g = i % p.ng, row = gx_row(ex, p.ng, nf, i / p.ng, g);
   if (ex.ea[row] == kExZeroRow) return;
-  const float* st = stat + (size_t)row * ex.n_kseg;
+  // a segment's value: the sum of its runs'
+  auto st = [&](int s) {
+    const float* v = stat + ((size_t)row * ex.n_kseg + s) * per_seg;
+    float sum = 0.f;
+    for (int q = 0; q < per_seg; ++q) sum += v[q];
+    return sum;
+  };
   if (Form<kForm>::kHalf) {
     const int k = kend[row];
     float sum = 0.f;
     for (int s = lane; s * kExSeg < k; s += 32)
-      sum += st[s] * fminf(__int_as_float(ex.seg_pow[s]), (float)kExSeg) / (float)min(kExSeg, p.nc - s * kExSeg);
+      sum += st(s) * fminf(__int_as_float(ex.seg_pow[s]), (float)kExSeg) / (float)min(kExSeg, p.nc - s * kExSeg);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0 && !(sum >= (float)k * kHalfPower)) ex_raise(ex);
@@ -547,7 +574,7 @@ __global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const 
     if (k < min(kExSeg, p.nc)) return;
     int sum = 0;
     for (int s = lane; s * kExSeg < k; s += 32)
-      sum += max(0, (int)st[s] + min(ex.seg_min[s], kExSeg) - min(kExSeg, p.nc - s * kExSeg));
+      sum += max(0, (int)st(s) + min(ex.seg_min[s], kExSeg) - min(kExSeg, p.nc - s * kExSeg));
     sum = __reduce_add_sync(0xffffffffu, sum);
     if (lane == 0 && (long long)sum * kExOverlap < k) ex_raise(ex);
   }
@@ -570,8 +597,15 @@ void gx_size(ExactPrep& ex, const GxShape& q, const std::vector<int>& igp_of, in
   exact_size(ex, q.form == kGxGpp || q.form == kGxReal ? 6 : 7, half || half_occ ? 2 * q.nb : q.nb, q.nc, q.ng, nf, !real, sms,
              kend.empty() ? nullptr : kend.data(), t, nf2, nf2 ? q.nvband : 0);
 }
-size_t gx_stat_bytes(const ExactPrep& ex) {
-  return sizeof(float) * (size_t)ex.n_row_blocks * kExRows * ex.n_kseg;
+// g-vectors per factor item: a segment, or less where the columns are too few
+// to give every SM its four CTAs twice (409 x 8192: 64 or 512 ... at 128).
+int gx_run(const ExactPrep& ex, int ng, int sms) {
+  int run = kExSeg;
+  while (run > 64 && (long long)((ng + kGxCols - 1) / kGxCols) * ex.n_kseg * (kExSeg / run) < 8LL * sms) run /= 2;
+  return run;
+}
+size_t gx_stat_bytes(const ExactPrep& ex, int run) {
+  return sizeof(float) * (size_t)ex.n_row_blocks * kExRows * ex.n_kseg * (kExSeg / run);
 }
 
 template <int kForm, bool kOcc>
@@ -580,7 +614,7 @@ cudaError_t launch_ff(const GppExact& g, const GxDev& p, dim3 grid, cudaStream_t
   cudaError_t e =
       cudaFuncSetAttribute(gx_ff_kernel<kForm, kOcc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  gx_ff_kernel<kForm, kOcc><<<grid, kGxThreads, smem, s>>>(p, g.ex, g.stat, g.nf);
+  gx_ff_kernel<kForm, kOcc><<<grid, kGxThreads, smem, s>>>(p, g.ex, g.stat, g.nf, g.run);
   return cudaGetLastError();
 }
 
@@ -599,12 +633,12 @@ cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, b
   if (e != cudaSuccess) return e;
   const int pad = std::max(ex.n_main_blocks * kExRows - g.nf * p.ng,
                            (ex.n_row_blocks - ex.n_main_blocks) * kExRows - g.nf2 * p.ng);
-  const dim3 grid((p.ng + pad + kGxCols - 1) / kGxCols, ex.n_kseg);
+  const dim3 grid((p.ng + pad + kGxCols - 1) / kGxCols, ex.n_kseg * (kExSeg / g.run));
   if constexpr (F::kF64) {
     constexpr int smem = sizeof(typename F64<kForm>::Planes);
     e = cudaFuncSetAttribute(gx_f64_kernel<kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    gx_f64_kernel<kForm><<<grid, kGxThreads, smem, s>>>(p, ex, g.stat, g.nf);
+    gx_f64_kernel<kForm><<<grid, kGxThreads, smem, s>>>(p, ex, g.stat, g.nf, g.run);
     e = cudaGetLastError();
   } else if (kForm == kGxGpp && g.nf2) {
     e = launch_ff<kGxGpp, true>(g, p, grid, s);
@@ -612,7 +646,8 @@ cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, b
     e = launch_ff<kForm, false>(g, p, grid, s);
   }
   if (e != cudaSuccess) return e;
-  gx_check_kernel<kForm><<<(slabs * p.ng * 32 + 255) / 256, 256, 0, s>>>(p, ex, g.stat, g.kend, g.nf, slabs);
+  gx_check_kernel<kForm><<<(slabs * p.ng * 32 + 255) / 256, 256, 0, s>>>(p, ex, g.stat, g.kend, g.nf, slabs,
+                                                                           kExSeg / g.run);
   return cudaGetLastError();
 }
 
@@ -625,7 +660,7 @@ size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, in
   std::vector<int> kend;
   int nf, nf2;
   gx_size(ex, q, igp_of, sms, nf, nf2, kend, nullptr);
-  return exact_work_bytes(ex) + gx_stat_bytes(ex);
+  return exact_work_bytes(ex) + gx_stat_bytes(ex, gx_run(ex, q.ng, sms));
 }
 
 bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, void* shared_work) {
@@ -633,9 +668,10 @@ bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp
   ExactTables t;
   std::vector<int> kend;
   gx_size(g.ex, q, igp_of, sms, g.nf, g.nf2, kend, &t);
+  g.run = gx_run(g.ex, q.ng, sms);
   const size_t work = exact_work_bytes(g.ex), own = exact_own_bytes(g.ex);
   if (cudaMalloc(&g.own, own + sizeof(int) * kend.size()) != cudaSuccess) g.own = nullptr;
-  if (g.own && !shared_work && cudaMalloc(&g.work, work + gx_stat_bytes(g.ex)) != cudaSuccess) {
+  if (g.own && !shared_work && cudaMalloc(&g.work, work + gx_stat_bytes(g.ex, g.run)) != cudaSuccess) {
     cudaFree(g.own);
     g.own = g.work = nullptr;
   }
