@@ -485,15 +485,15 @@ __device__ __forceinline__ double2 ex_weight(const FfDev& p, int n, int f, int i
   return m[(size_t)(second ? n - p.pair_bands : n) * p.nc + igp];
 }
 
-// One CTA per (row block, band block, eighth of its B' rows): tempz of 128 rows x
-// 8 to 10 bands from the pieces' raw sums (added as integers, so their order does not
+// One CTA per (row block, pair of bands): tempz of 128 rows x 2 bands from the pieces' raw sums (added as integers, so their order does not
 // matter), times weight * conj(aqsm[n1][igp]), summed over the rows of each
 // frequency in a fixed order.
-constexpr int kFinRow = kExRows + 1, kFinThreads = 256;
+constexpr int kFinRow = kExRows + 1, kFinThreads = 256, kFinBands = 2;
 template <bool kReal>
 __global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, ExactPrep ex, int rb0) {
-  const int kCols = ex.cols, kBands = kCols / 8, b0 = blockIdx.z * kBands;  // bands b0 .. of the block
-  extern __shared__ double2 s_prod[];  // [bands][129], complex or real
+  constexpr int kBands = kFinBands;
+  const int kCols = ex.cols, b0 = blockIdx.z * kBands;  // bands b0 and b0 + 1 of the block
+  __shared__ double2 s_prod[kBands * kFinRow];  // complex, or real
   double* s_real = reinterpret_cast<double*>(s_prod);
   if (*ex.flag) return;
   // row block rb of the group whose row blocks start at rb0
@@ -504,7 +504,9 @@ __global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, Exac
   const double wgt = ff_column_weight(p, igp);
   const int e_row = R < rows ? ex.ea[rb0 * kExRows + R] : 0, np = ex.pieces[rb0 + rb];
   const size_t base = block * ex.max_pieces * kCols * kExRows + r;
-  for (int b = tid >> 7; b < kBands; b += kFinThreads / kExRows) {
+  static_assert(kFinThreads == kBands * kExRows, "one thread per row and band");
+  {
+    const int b = tid >> 7;
     const int n = cb * ex.bands + b0 + b;
     double2 v = make_double2(0.0, 0.0);
     if (igp >= 0 && n < p.nb) {
@@ -633,24 +635,34 @@ void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool 
     for (int r = rb * kExRows; r < std::min(rows, (rb + 1) * kExRows); ++r) k = std::max(k, std::min(row_kend[r], nc));
     kl[rb] = (k + 31) / 32 * 2;
   }
-  // K splits: as few as fill the grid's waves well.  An item costs its tiles
-  // plus about 6 tiles' time for its raw sums and the ring's refill, a piece
-  // about one tile's time in the epilogue.  Ragged
-  // row limits (items of different lengths) take at least 10 items per CTA.
+  // K splits: the count whose slowest CTA is done first.  An item costs its
+  // tiles plus about 6 tiles' time for its raw sums and the ring's refill, a
+  // piece about one tile's time in the epilogue.  Items of one length take
+  // ceil(items / grid) turns; ragged ones (row limits) are dealt out as the
+  // kernel's static schedule does.
   const int all = ex.halves * ex.kt;
   const long long blocks = (long long)ex_block_index(ex, ex.n_row_blocks, 0);
   long long best = LLONG_MAX;
   int splits = 1;
-  for (int s = 1; s <= std::min(all / 2, 96); ++s) {
-    const long long items = blocks * s;
-    if (row_kend && items < 10LL * grid && s < std::min(all / 2, 96)) continue;
+  for (int s = 1; s <= std::min(all / 2, 96); s += row_kend && s >= 8 ? s / 4 : 1) {
     const int len = (all / 2 + s - 1) / s * 2;
-    const long long cost = (items + grid - 1) / grid * (len + 6LL) + s;
+    long long cost = 0;
+    if (!row_kend) {
+      cost = (blocks * s + grid - 1) / grid * (len + 6LL) + s;
+    } else {
+      std::vector<int4> ent;
+      std::vector<int> pieces;
+      k_entries(ex.n_main_blocks, ex.halves, ex.kt, len, (all + len - 1) / len, kl, ent, pieces);
+      std::vector<long long> load(grid, 0);
+      long long i = 0;
+      for (const int4& e : ent)
+        for (int c = 0; c < ex.n_col_blocks; ++c, ++i) load[i % grid] += e.w + 6;
+      cost = *std::max_element(load.begin(), load.end()) + *std::max_element(pieces.begin(), pieces.end());
+    }
     if (cost < best) {
       best = cost;
       splits = s;
     }
-    if (row_kend) break;
   }
   ex.split_tiles = (all / 2 + splits - 1) / splits * 2;
   ex.n_splits = (all + ex.split_tiles - 1) / ex.split_tiles;
@@ -771,9 +783,8 @@ cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* ou
                                 bool second_rows) {
   const int rb0 = second_rows ? ex.n_main_blocks : 0;
   const int nrb = (d.nf * d.ng + kExRows - 1) / kExRows, ncb = (d.nb + ex.bands - 1) / ex.bands;
-  const int smem = ex.cols / 8 * kFinRow * (int)(ex.halves == 1 ? sizeof(double) : sizeof(double2));
   auto* kernel = ex.halves == 1 ? exact_finish_kernel<true> : exact_finish_kernel<false>;
-  kernel<<<dim3(nrb, ncb, ex.bands / (ex.cols / 8)), kFinThreads, smem, s>>>(d, ex, rb0);
+  kernel<<<dim3(nrb, ncb, ex.bands / kFinBands), kFinThreads, 0, s>>>(d, ex, rb0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int blocks = (d.nb * d.nf * 32 + 255) / 256;

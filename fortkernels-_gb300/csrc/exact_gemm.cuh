@@ -114,9 +114,10 @@ size_t exact_own_bytes(const ExactPrep& ex);
 void exact_bind(ExactPrep& ex, void* work, void* own);
 cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t);
 
-// Plans take the exact form from this many products on (rows x bands x K): below it
-// its ten launches cost more than the FP64 kernel.
-constexpr double kExactMin = 1 << 22;
+// FF plans take the exact form from this many products on (rows x bands x K):
+// 16 x (5 x 20) x 512 = 0.8 M takes 75 us, 119 us on the FP64 pipe, but the
+// exact form's nine launches never take less than ~65 us.
+constexpr double kExactMin = 1 << 19;
 
 // One contraction, in order:
 //   exact_begin       clears the flag and the overlap counts

@@ -653,7 +653,19 @@ cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, b
 
 }  // namespace
 
-bool gpp_exact_fits(const GxShape& q) { return (double)kNW * q.ng * q.nb * q.nc >= kExactMin; }
+// From these products on (3 x columns x bands x g-vectors) the contraction beats
+// the float-float passes, whose time stays flat below (one CTA's latency):
+// measured us, contraction against passes, at 16 x 20 x 512 (0.5 M) 105 / 165
+// with occupied bands and 80 / 75 without, real 24 x 40 x 1024 (2.9 M) 140 / 149,
+// half sum 60 x 60 x 2048 (22 M) 303 / 372.
+bool gpp_exact_fits(const GxShape& q) {
+  const double products = (double)kNW * q.ng * q.nb * q.nc;
+  switch (q.form) {
+    case kGxReal: return products >= 1 << 22;
+    case kGxHalf: return products >= 1 << 23;
+    default: return products >= (q.nvband > 0 ? 1 << 18 : 1 << 20);
+  }
+}
 
 size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms) {
   ExactPrep ex{};

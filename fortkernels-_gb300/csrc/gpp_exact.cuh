@@ -60,8 +60,8 @@ struct GxShape {
 };
 
 // Sizes, allocates and fills the contraction of one instance; false (with
-// nothing allocated) when the problem is below kExactMin products or the
-// device has no room: the FP64 kernels keep the work.  With shared_work set
+// nothing allocated) when the device has no room: the FP64 kernels keep the
+// work, as for problems too small for it (gpp_exact_fits).  With shared_work set
 // (at least gpp_exact_work_bytes) the instance has no workspace of its own.
 bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms,
                       void* shared_work = nullptr);

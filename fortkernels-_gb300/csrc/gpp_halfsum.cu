@@ -948,7 +948,8 @@ __global__ void __launch_bounds__(256) half_zs_slices_kernel(HalfDev p, OzakiPre
 //                   = sum_col occ_ach                (n1 <  nvband)
 //   asx_n1[n1][iw]  = sum_col occ_asx                (n1 <  nvband)
 //   stat_n1[n1]     = Ts + conj(Us) + unpaired       (static remainder)
-constexpr int kRowWarps = 8;
+constexpr int kRowWarps = 8;  // at most; no more than the columns fill
+inline int row_threads(int ng) { return 32 * std::min(kRowWarps, (ng + 31) / 32); }
 __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
     HalfDev p, const double2* t3, const double2* u3, const double2* ts, const double2* us, int stride3, int stride1,
     const int* skip_if, const double2* tu_occ, const double2* occ_ach, const double2* occ_asx, double2* acht_n1, double2* asx_n1, double2* stat_n1) {
@@ -960,7 +961,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
   const bool occ = n1 < p.nvband;
   const double wx[3] = {p.wx[0], p.wx[1], p.wx[2]};
   Comp ax[3], ay[3], sx[3], sy[3], qx, qy;
-  for (int col = warp * 32 + lane; col < p.ng; col += kRowWarps * 32) {
+  for (int col = warp * 32 + lane; col < p.ng; col += blockDim.x) {
     const int igp = p.igp_of[col];
     if (igp < 0) continue;
     const size_t off = (size_t)col * p.nc + igp;
@@ -1035,7 +1036,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
   double tot[kVals];
   for (int v = 0; v < kVals; ++v) {
     Comp c;
-    for (int q = 0; q < kRowWarps; ++q) c.add(part[q][v]);
+    for (int q = 0; q < (int)blockDim.x / 32; ++q) c.add(part[q][v]);
     tot[v] = c.value();
   }
 #pragma unroll
@@ -1347,7 +1348,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
                                  nullptr, true);
     }
     if (st != SIGMA_OK) return st;
-    half_tensor_rows_kernel<<<plan->nb, kRowWarps * 32, 0, s>>>(
+    half_tensor_rows_kernel<<<plan->nb, row_threads(plan->ng), 0, s>>>(
         p, plan->t3, plan->u3, stat ? plan->ts : nullptr, plan->us, kNW, 1, nullptr, nullptr, plan->occ_ach, plan->occ_asx,
         plan->acht_n1, plan->asx_n1, plan->stat_n1);
     SIGMA_CUDA_TRY(cudaGetLastError());
@@ -1382,7 +1383,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
   if (plan->exact) {
     const int nf = plan->exact.nf;
     const double2* u = plan->tu + (size_t)plan->nb * nf;
-    half_tensor_rows_kernel<<<plan->nb, kRowWarps * 32, 0, s>>>(
+    half_tensor_rows_kernel<<<plan->nb, row_threads(plan->ng), 0, s>>>(
         p, plan->tu, u, stat ? plan->tu + kNW : nullptr, u + kNW, nf, nf, flag,
         plan->exact_occ ? plan->tu_occ : nullptr, plan->occ_ach, plan->occ_asx, plan->acht_n1, plan->asx_n1,
         plan->stat_n1);
