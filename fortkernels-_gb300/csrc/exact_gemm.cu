@@ -325,8 +325,9 @@ __device__ __forceinline__ unsigned ex_mag(const int2* v, size_t k, unsigned& lo
 }
 
 // One CTA per row of values: its exponent (largest part below 2^e) and, per
-// 512-value segment, how many elements are large.  Bands (kB) lower seg_min
-// to their counts and seg_pow to their sums of squares (of the larger parts);
+// 512-value segment, how many of its first 128 elements are large.  Bands (kB)
+// lower seg_min to their counts and seg_pow to their sums of squares (of the
+// larger parts);
 // A rows add up how many large elements must coincide with large elements of
 // every band and raise the flag when they are too few.  Zero rows are exact
 // and pass.
@@ -361,11 +362,12 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const vo
   for (int s = warp; s < ex.n_kseg; s += 8) {
     int c = 0;
     float q = 0.f;
-    const int k1 = min(nc, (s + 1) * kExSeg);
+    const int kc = s * kExSeg + kExCount;  // the counted part; bands' powers take the whole segment
+    const int k1 = min(nc, kB ? (s + 1) * kExSeg : kc);
     for (int k = s * kExSeg + lane; k < k1; k += 32) {
       unsigned low;
       const unsigned d = ex_mag<kReal>(v, k, low);
-      c += d >= thr ? 1 : 0;
+      c += k < kc && d >= thr ? 1 : 0;
       if (kB) {
         // the larger part over 2^e to 20 bits: exponent d >> 20 against exm + 1
         const int sh = exm + 1 - (int)(d >> 20);
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const vo
         atomicMin(&ex.seg_min[s], c);
         atomicMin(&ex.seg_pow[s], __float_as_int(q));
       } else {
-        sum += max(0, c + min(ex.seg_min[s], kExSeg) - min(kExSeg, nc - s * kExSeg));
+        sum += max(0, c + min(ex.seg_min[s], kExCount) - min(kExCount, nc - s * kExSeg));
       }
     }
   }

@@ -40,7 +40,8 @@ namespace sigma {
 
 constexpr int kExKTile = 16;     // K elements per staged tile (one 32-byte swizzle row)
 constexpr int kExRows = 128;     // A rows per tile
-constexpr int kExSeg = 512;      // K values per segment of the overlap check
+constexpr int kExSeg = 512;      // K values per segment of the overlap check,
+constexpr int kExCount = 128;    // of which the first are counted (a lower bound, at a quarter of the work)
 constexpr uint32_t kExASlice = kExRows * kExKTile * 2;  // 4 KB
 // S slices (digits) per value and B' rows per slice, such that the S
 // accumulators fit tensor memory's 512 columns: 6 x 80 (40 complex bands, Re
@@ -220,36 +221,43 @@ __device__ __forceinline__ void ex_put(unsigned char* tile, uint32_t slice_bytes
   ex_store<S>(tile, slice_bytes, r, ch, ex_chunk<S>(x, e));
 }
 
-// The six digits of hi + lo (|lo| at most half an ulp of hi) in units of
-// 2^(7 - e), for |hi| < 2^(e - 1): FP32 operations only.  Every step is exact
-// but the last addition, which rounds at 2^-60 of 2^e (lo joins the third
-// remainder by TwoSum; its rounding error, 2^-51, joins the fourth).
-__device__ __forceinline__ void ex_ff_digits(float2 x, float scale, float (&d)[6]) {
-  constexpr float kM = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer
-  const float u = x.x * scale, w = x.y * (scale * 262144.f);
-  d[0] = (u + kM) - kM;
-  float r = u - d[0];
-  d[1] = fmaf(r, 512.f, kM) - kM;
-  r = fmaf(r, 512.f, -d[1]);
-  d[2] = (fmaf(r, 512.f, w) + kM) - kM;
-  float e;
-  two_sum_f(fmaf(r, 512.f, -d[2]), w, r, e);
-  d[3] = fmaf(r, 512.f, kM) - kM;
-  r = fmaf(e, 512.f, fmaf(r, 512.f, -d[3]));
-  d[4] = fmaf(r, 512.f, kM) - kM;
-  r = fmaf(r, 512.f, -d[4]);
-  d[5] = fmaf(r, 512.f, kM) - kM;
+// The six digits of two values hi + lo (|lo| at most half an ulp of hi) in
+// units of 2^(7 - e), for |hi| < 2^(e - 1): FP32 operations on both lanes of
+// paired instructions.  Every step is exact but the last addition, which
+// rounds at 2^-60 of 2^e (lo joins the third remainder by TwoSum; its
+// rounding error, 2^-51, joins the fourth).  neg_scale = -2^(7 - e): the
+// digits of the negated value come out negated, kM - (x + kM), without an
+// instruction of their own.
+__device__ __forceinline__ void ex_ff_digits(float2 hi, float2 lo, float neg_scale, float2 (&d)[6]) {
+  const float2 kM = make_float2(12582912.f, 12582912.f);  // 1.5 * 2^23: adding it rounds to an integer
+  const float2 k512 = make_float2(512.f, 512.f), m1 = make_float2(-1.f, -1.f);
+  const float w0 = neg_scale * 262144.f;
+  const float2 u = __fmul2_rn(hi, make_float2(neg_scale, neg_scale)), w = __fmul2_rn(lo, make_float2(w0, w0));
+  d[0] = __ffma2_rn(__fadd2_rn(u, kM), m1, kM);
+  float2 r = __fadd2_rn(u, d[0]);
+  d[1] = __ffma2_rn(__ffma2_rn(r, k512, kM), m1, kM);
+  r = __ffma2_rn(r, k512, d[1]);
+  d[2] = __ffma2_rn(__fadd2_rn(__ffma2_rn(r, k512, w), kM), m1, kM);
+  r = __ffma2_rn(r, k512, d[2]);
+  const float2 s = __fadd2_rn(r, w);
+  const float2 bv = __ffma2_rn(r, m1, s), av = __ffma2_rn(bv, m1, s);
+  const float2 e = __fadd2_rn(__ffma2_rn(av, m1, r), __ffma2_rn(bv, m1, w));
+  d[3] = __ffma2_rn(__ffma2_rn(s, k512, kM), m1, kM);
+  r = __ffma2_rn(e, k512, __ffma2_rn(s, k512, d[3]));
+  d[4] = __ffma2_rn(__ffma2_rn(r, k512, kM), m1, kM);
+  r = __ffma2_rn(r, k512, d[4]);
+  d[5] = __ffma2_rn(__ffma2_rn(r, k512, kM), m1, kM);
 }
-__device__ __forceinline__ void ex_put_ff(unsigned char* tile, int r, int ch, const float2* v, float scale) {
+__device__ __forceinline__ void ex_put_ff(unsigned char* tile, int r, int ch, const float2* hi, const float2* lo,
+                                          float neg_scale) {
   unsigned char* p = tile + sw32_offset(r, ch);
   uint32_t w[6][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    float a[6], b[6];
-    ex_ff_digits(v[2 * j], scale, a);
-    ex_ff_digits(v[2 * j + 1], scale, b);
+    float2 d[6];
+    ex_ff_digits(hi[j], lo[j], neg_scale, d);
 #pragma unroll
-    for (int i = 0; i < 6; ++i) w[i][j] = __byte_perm(__float_as_uint(a[i]), __float_as_uint(b[i]), 0x7632);
+    for (int i = 0; i < 6; ++i) w[i][j] = __byte_perm(__float_as_uint(d[i].x), __float_as_uint(d[i].y), 0x7632);
   }
 #pragma unroll
   for (int i = 0; i < 6; ++i)

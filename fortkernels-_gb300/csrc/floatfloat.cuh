@@ -209,6 +209,24 @@ __device__ __forceinline__ double f32_widen(float f) {
   const unsigned hi = (u & 0x80000000u) | (mag >= 0x00800000u ? (mag >> 3) + 0x38000000u : 0u);
   return __hiloint2double((int)hi, mag >= 0x00800000u ? (int)(mag << 29) : 0);
 }
+// split_round for |x| < 2^127 without its branch, two thirds of its
+// instructions: hi = x rounded to the nearest FP32 value (ties away from
+// zero), lo the signed rest; lo = 0 below 2^-74 and both 0 below 2^-126.
+__device__ __forceinline__ FF ff_split_in_range(double x) {
+  const unsigned whi = (unsigned)__double2hiint(x), wlo = (unsigned)__double2loint(x);
+  const unsigned long long r = (((unsigned long long)whi << 32) | wlo) + 0x10000000ull;
+  const unsigned f = __funnelshift_l((unsigned)r, (unsigned)(r >> 32), 3);
+  const int m = (int)((unsigned)r & 0x1FFFFFFFu) - 0x10000000;  // x - hi in units of 2^(ex - 1075)
+  const unsigned sign = whi & 0x80000000u;
+  const unsigned ex = whi & 0x7FF00000u;
+  const unsigned scale = (max(ex, 948u << 20) - (948u << 20)) << 3 | sign;  // 2^(ex - 1075) with x's sign
+  const bool zero = ex < (897u << 20);
+  FF v;
+  v.hi = zero ? 0.f : __uint_as_float(((f + 0x40000000u) & 0x7FFFFFFFu) | sign);
+  v.lo = __int2float_rn(m) * __uint_as_float(scale);
+  return v;
+}
+
 // A float-float value as the nearest double: both halves widened exactly,
 // one FP64 addition.
 __device__ __forceinline__ double ff_widen(FF x) { return f32_widen(x.hi) + f32_widen(x.lo); }

@@ -12,8 +12,13 @@
 // values, one pass over the inputs at memory speed.
 // gx_ff_kernel forms them from FP64 numerators in float-float arithmetic (FP32
 // pairs: ~2^-48 rms, below the float-float terms it replaces), cuts them into
-// digits with FP32 operations and writes each row's digits as 16-byte
+// digits with paired FP32 operations and writes each row's digits as 16-byte
 // chunks: 16 columns x 32 g-vectors staged in shared memory, four CTAs per SM.
+// Bound by issue slots (69 % issuing, FP64 pipe 52 %, FMA 48 %): 2.43 ms at
+// 1638 x 32768 with the occupied bands' factors, 2.74 ms with digits of one
+// value per instruction, the general FP64 split and all large factors counted.
+// Factors of two elements per instruction need 80 registers or spill at two
+// or three CTAs per SM: 3.13 and 3.35 ms.
 // (The factors in FP64, 34 operations per column and g-vector, ran at the FP64
 // pipe's 2 per clock per SM: 3.54 ms at 1638 x 32768, with the occupied bands'
 // own pass another 3.86 ms.)  The half sum's factors, FP64 before, stay in FP64
@@ -229,14 +234,14 @@ __device__ __forceinline__ void gx_factors(const FF (&wx)[kNW], const FF (&iwx2)
   const double b2d = guard_b2(wt.y);
   FF gx, gy = zero, b = zero, b2 = zero, a = zero, ox = zero, oy = zero;
   if (F::kReal) {
-    gx = ff_of_rn(__dmul_rn(ie.x, wt.x));
+    gx = ff_split_in_range(__dmul_rn(ie.x, wt.x));
   } else {
-    gx = ff_of_rn(fma(ie.x, wt.x, -__dmul_rn(ie.y, wt.y)));
-    gy = ff_of_rn(fma(ie.x, wt.y, __dmul_rn(ie.y, wt.x)));
-    b = ff_of_rn(wt.y);
+    gx = ff_split_in_range(fma(ie.x, wt.x, -__dmul_rn(ie.y, wt.y)));
+    gy = ff_split_in_range(fma(ie.x, wt.y, __dmul_rn(ie.y, wt.x)));
+    b = ff_split_in_range(wt.y);
   }
   if (kOcc) {
-    a = ff_of_rn(wt.x);
+    a = ff_split_in_range(wt.x);
     b2 = ff_mul(b, b);
     ox = gx_norm(ff_dot2_raw(a, gx, b, gy));  // Omega2 = wtilde G
     oy = gx_norm(ff_dot2_raw(a, gy, ff_neg(b), gx));
@@ -254,12 +259,12 @@ __device__ __forceinline__ void gx_factors(const FF (&wx)[kNW], const FF (&iwx2)
       keep = mask & 1u;
       second = mask & 2u;
     }
-    const FF c = ff_of_rn(cd);
+    const FF c = ff_split_in_range(cd);
     if (F::kReal) {
       const FF y = ff_mul(gx, gx_norm(ff_rcp_raw(c)));
       put(iw, keep ? y : zero, zero);
     } else {
-      const FF r = gx_norm(ff_rcp_raw(ff_of_rn(wv)));
+      const FF r = gx_norm(ff_rcp_raw(ff_split_in_range(wv)));
       const FF yx = ff_mul(gx_norm(ff_dot2_raw(gx, c, gy, b)), r);
       const FF yy = ff_mul(gx_norm(ff_dot2_raw(gy, c, ff_neg(gx), b)), r);
       put(iw, keep ? yx : zero, keep ? yy : zero);
@@ -281,7 +286,8 @@ constexpr int kFfK = 32;  // g-vectors per staged tile
 template <int kForm, bool kOcc>
 struct FfPlanes {
   static constexpr int kSlabs = kOcc ? 6 : 3;
-  float2 v[Form<kForm>::kParts][kSlabs][kGxCols][kFfK + 1];  // conflict-free along g-vectors and along columns
+  // high and low halves; conflict-free along g-vectors, and for pairs of them along columns
+  float hi[Form<kForm>::kParts][kSlabs][kGxCols][kFfK + 2], lo[Form<kForm>::kParts][kSlabs][kGxCols][kFfK + 2];
 };
 
 // Items (column block, run of `run` g-vectors).  Column blocks run past ng to
@@ -314,8 +320,8 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
   if (tid < kSlabs * kGxCols) {
     const int i = tid / kGxCols, pl = tid % kGxCols, g = p0 + pl, R = gx_row(ex, p.ng, nf, i, g);
     const int e = g < p.ng ? ex.ea[R] : kExZeroRow;
-    // 2^(7 - e) and 2^(e - 2 - slack) (|e| < 64 unless flagged; a zero row's values are zero)
-    s_scale[i][pl] = e == kExZeroRow ? 0.f : __uint_as_float((unsigned)(134 - e) << 23);
+    // -2^(7 - e) and 2^(e - 2 - slack) (|e| < 64 unless flagged; a zero row's values are zero)
+    s_scale[i][pl] = e == kExZeroRow ? 0.f : -__uint_as_float((unsigned)(134 - e) << 23);
     s_thr[i][pl] = e == kExZeroRow ? INFINITY : __uint_as_float((unsigned)(125 - kExSlackA + e) << 23);
     if (i == 0) s_lim[pl] = g < p.ng ? gx_limit<kForm>(p, g, 0) : 0;
     const bool last = i == nf - 1 || i == kSlabs - 1;
@@ -330,28 +336,32 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
     for (int i = 0; i < kSlabs; ++i) acc[j][i] = 0.f;
   for (int k0 = k_begin; k0 < k_end; k0 += kFfK) {
     const FF wx[kNW] = {s_wx[0], s_wx[1], s_wx[2]}, iwx2[kNW] = {s_iwx2[0], s_iwx2[1], s_iwx2[2]};
+    const bool counted = k0 % kExSeg < kExCount;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int pl = warp + 8 * j, g = p0 + pl, ig = k0 + lane;
       if (ig < s_lim[pl]) {
         const double2 wt = gx_load<kForm>(p.wt, (size_t)g * p.nc + ig);
         const double2 ie = gx_load<kForm>(p.ieps, (size_t)g * p.nc + ig);
-        auto put = [&](int i, FF re, FF im) {
-          sm.v[0][i][pl][lane] = make_float2(re.hi, re.lo);
-          float big = fabsf(re.hi);
+        gx_factors<kForm, kOcc>(wx, iwx2, p.wx, s_wide, wt, ie, [&](int i, FF re, FF im) {
+          sm.hi[0][i][pl][lane] = re.hi;
+          sm.lo[0][i][pl][lane] = re.lo;
           if (!F::kReal) {
-            sm.v[F::kParts - 1][i][pl][lane] = make_float2(im.hi, im.lo);
-            big = fmaxf(big, fabsf(im.hi));
+            sm.hi[F::kParts - 1][i][pl][lane] = im.hi;
+            sm.lo[F::kParts - 1][i][pl][lane] = im.lo;
           }
-          acc[j][i] += big >= s_thr[i][pl] ? 1.f : 0.f;
-        };
-        gx_factors<kForm, kOcc>(wx, iwx2, p.wx, s_wide, wt, ie, put);
+        });
       } else {
 #pragma unroll
         for (int i = 0; i < kSlabs; ++i)
 #pragma unroll
-          for (int q = 0; q < F::kParts; ++q) sm.v[q][i][pl][lane] = make_float2(0.f, 0.f);
+          for (int q = 0; q < F::kParts; ++q) sm.hi[q][i][pl][lane] = sm.lo[q][i][pl][lane] = 0.f;
       }
+      if (counted)
+#pragma unroll
+        for (int i = 0; i < kSlabs; ++i)
+          acc[j][i] += fmaxf(fabsf(sm.hi[0][i][pl][lane]), fabsf(sm.hi[F::kParts - 1][i][pl][lane])) >= s_thr[i][pl]
+                           ? 1.f : 0.f;
     }
     __syncthreads();
     // digits: a warp takes one (slab, part, K tile), its lanes the 16
@@ -366,7 +376,9 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
       if (R >= gx_rows_end(ex, nf, i) || tile >= ex.kt_lim[R / kExRows]) continue;
       unsigned char* dst =
           ex.a_tiles + ((size_t)(R / kExRows) * F::kParts * ex.kt + part * ex.kt + tile) * ex_a_bytes(6);
-      ex_put_ff(dst, R % kExRows, ch, &sm.v[part][i][pl][q * kExKTile + ch * 8], s_scale[i][pl]);
+      const int k = q * kExKTile + ch * 8;
+      ex_put_ff(dst, R % kExRows, ch, reinterpret_cast<const float2*>(&sm.hi[part][i][pl][k]),
+                reinterpret_cast<const float2*>(&sm.lo[part][i][pl][k]), s_scale[i][pl]);
     }
     __syncthreads();
   }
@@ -509,7 +521,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
           const int e = s_e[min(i, nf - 1)][pl];  // |e| < 64 unless flagged; a zero row is not checked
           if (H::kOcc) {
             const int big = max(__double2hiint(y[i].x) & 0x7FFFFFFF, __double2hiint(y[i].y) & 0x7FFFFFFF);
-            acc[j][i] += big >= (min(e, 1000) + 1022 - kExSlackA) << 20 ? 1.f : 0.f;
+            acc[j][i] += ig % kExSeg < kExCount && big >= (min(e, 1000) + 1022 - kExSlackA) << 20 ? 1.f : 0.f;
           } else {
             const float u = __uint_as_float((unsigned)(127 - e) << 23);  // 2^-e
             const float a = __double2float_rn(y[i].x) * u, b = __double2float_rn(y[i].y) * u;
@@ -574,7 +586,7 @@ __global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const 
     if (k < min(kExSeg, p.nc)) return;
     int sum = 0;
     for (int s = lane; s * kExSeg < k; s += 32)
-      sum += max(0, (int)st(s) + min(ex.seg_min[s], kExSeg) - min(kExSeg, p.nc - s * kExSeg));
+      sum += max(0, (int)st(s) + min(ex.seg_min[s], kExCount) - min(kExCount, p.nc - s * kExSeg));
     sum = __reduce_add_sync(0xffffffffu, sum);
     if (lane == 0 && (long long)sum * kExOverlap < k) ex_raise(ex);
   }
