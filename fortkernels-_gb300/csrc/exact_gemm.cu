@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
   // full[5], empty[5], lo full, hi full, lo empty, hi empty, done
   __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
   __shared__ uint32_t tmem_slot;
+  chain_begin();
   if (*ex.flag) return;  // operands outside the split's range: the FP64 kernel runs instead
 
   const uint32_t raw = smem_u32(smem_raw);
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const vo
                                                           int nc) {
   __shared__ unsigned s_max[8];
   __shared__ int s_sum[8];
+  chain_begin();
   const int row = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int2* v = static_cast<const int2*>(row < n0 ? x0 : x1) + (size_t)(row < n0 ? row : row - n0) * nc * (kReal ? 1 : 2);
   unsigned m = 0, any = 0;
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const vo
 // Element t: (row block, K tile pair, row, 8-value chunk of the 32 K values).
 __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const double2* a, int rows, int nc) {
   constexpr int S = 6;
+  chain_begin();
   if (*ex.flag) return;
   const int pairs = ex.kt / 2;
   const long long total = (long long)ex.n_row_blocks * pairs * kExRows * 4;
@@ -429,6 +432,7 @@ __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const 
 template <int S, bool kReal>
 __global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const void* b0, int nb0, const void* b1,
                                                             int nb, int nc) {
+  chain_begin();
   if (*ex.flag) return;
   constexpr int kW = kReal ? 1 : 2, kBands = kReal ? ex_cols(S) : ex_cols(S) / 2;
   constexpr uint32_t kSlice = ex_b_slice(S), kBytes = ex_b_bytes(S);
@@ -492,15 +496,20 @@ __device__ __forceinline__ double2 ex_weight(const FfDev& p, int n, int f, int i
 // frequency in a fixed order.
 constexpr int kFinRow = kExRows + 1, kFinThreads = 256, kFinBands = 2;
 template <bool kReal>
-__global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, ExactPrep ex, int rb0) {
+__global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, ExactPrep ex, ExSecond p2) {
   constexpr int kBands = kFinBands;
   const int kCols = ex.cols, b0 = blockIdx.z * kBands;  // bands b0 and b0 + 1 of the block
   __shared__ double2 s_prod[kBands * kFinRow];  // complex, or real
   double* s_real = reinterpret_cast<double*>(s_prod);
+  chain_begin();
   if (*ex.flag) return;
   // row block rb of the group whose row blocks start at rb0
-  const int rb = blockIdx.x, cb = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rows = p.nf * p.ng, r = tid & (kExRows - 1), R = rb * kExRows + r;
+  const bool first = (int)blockIdx.x < ex.n_main_blocks;
+  const int rb0 = first ? 0 : ex.n_main_blocks, nf = first ? p.nf : p2.nf, nb = first ? p.nb : p2.nb;
+  const int rb = (int)blockIdx.x - rb0, cb = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (!first && cb >= ex.n_col_blocks2) return;
+  if (!first) p.vfac = p2.vfac;
+  const int rows = nf * p.ng, r = tid & (kExRows - 1), R = rb * kExRows + r;
   const size_t block = ex_block_index(ex, rb0 + rb, cb);
   const int f = R / p.ng, igp = R < rows ? p.igp_of[R % p.ng] : -1;
   const double wgt = ff_column_weight(p, igp);
@@ -511,10 +520,10 @@ __global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, Exac
     const int b = tid >> 7;
     const int n = cb * ex.bands + b0 + b;
     double2 v = make_double2(0.0, 0.0);
-    if (igp >= 0 && n < p.nb) {
+    if (igp >= 0 && n < nb) {
       long long hr = 0, hi = 0;
       double lr = 0.0, li = 0.0;
-#pragma unroll 4
+#pragma unroll 8
       for (int q = 0; q < np; ++q) {
         const size_t o = base + ((size_t)q * kCols + (kReal ? b0 + b : 2 * (b0 + b))) * kExRows;
         hr += ex.raw_hi[o];
@@ -573,21 +582,30 @@ __global__ void __launch_bounds__(kFinThreads) exact_finish_kernel(FfDev p, Exac
   }
 }
 
-// out[n][f]: one warp per entry, fixed-order compensated sum over the row blocks.
-__global__ void exact_reduce_kernel(FfDev p, ExactPrep ex, int rb0, const double2* partial, double2* out) {
+// out[n][f], then out2, then the second group's: eight lanes per entry,
+// fixed-order compensated sum over the row blocks (a warp per entry took 8 us
+// even for a few hundred entries: 80 FP64 operations a warp, at two lanes per
+// clock).
+constexpr int kRedThreads = 64, kRedLanes = 8;
+__global__ void __launch_bounds__(kRedThreads) exact_reduce_kernel(FfDev p, ExactPrep ex, ExSecond p2, double2* out,
+                                                                   double2* out2) {
+  chain_begin();
   if (*ex.flag) return;
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= p.nb * p.nf) return;
-  const int n = w / p.nf, f = w % p.nf, cb = n / ex.bands, b = n % ex.bands;
-  const int lo = f * p.ng / kExRows, hi = ((f + 1) * p.ng - 1) / kExRows;
+  const int lane = threadIdx.x % kRedLanes, w = (blockIdx.x * kRedThreads + threadIdx.x) / kRedLanes;
+  const int n1 = p.nb * p.nf, n2 = out2 ? n1 : 0, n3 = p2.out ? p2.nb * p2.nf : 0;
+  const bool second = w >= n1 + n2, extra = !second && w >= n1;
+  const int e = second ? w - n1 - n2 : extra ? w - n1 : w, nf = second ? p2.nf : p.nf;
+  const int n = e / nf, f = e % nf, cb = n / ex.bands, b = n % ex.bands, rb0 = second ? ex.n_main_blocks : 0;
+  const int lo = f * p.ng / kExRows, hi = w < n1 + n2 + n3 ? ((f + 1) * p.ng - 1) / kExRows : -1;
+  const double2* partial = extra ? ex.partial2 : ex.partial;
   Comp sx, sy;
-  for (int rb = lo + lane; rb <= hi; rb += 32) {
+  for (int rb = lo + lane; rb <= hi; rb += kRedLanes) {
     const double2 v = partial[(ex_block_index(ex, rb0 + rb, cb) * ex.max_seg + (f - rb * kExRows / p.ng)) * ex.bands + b];
     sx.add(v.x);
     sy.add(v.y);
   }
-  const double x = warp_sum_comp(sx), y = warp_sum_comp(sy);
-  if (lane == 0) out[(size_t)n * p.nf + f] = make_double2(x, y);
+  const double x = lanes_sum_comp<kRedLanes>(sx), y = lanes_sum_comp<kRedLanes>(sy);
+  if (lane == 0 && hi >= 0) (second ? p2.out : extra ? out2 : out)[(size_t)n * nf + f] = make_double2(x, y);
 }
 
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
@@ -735,41 +753,31 @@ cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t) {
   return e;
 }
 
-cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(ex.flag, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  return exact_begin_counts(ex, s);
+cudaError_t exact_begin_flag(const ExactPrep& ex, cudaStream_t s) {
+  return cudaMemsetAsync(ex.flag, 0, sizeof(int), s);
 }
-cudaError_t exact_begin_counts(const ExactPrep& ex, cudaStream_t s) {
+cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s) {
+  cudaError_t e = exact_begin_flag(ex, s);
+  if (e != cudaSuccess) return e;
   return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * 2 * (size_t)ex.n_kseg, s);
 }
 
 cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const void* b1, int nb1, int nc,
                            cudaStream_t s) {
   const int nb = nb0 + nb1;
-  if (ex.halves == 1)
-    exact_stats_kernel<true, true><<<nb, 256, 0, s>>>(ex, b0, nb0, b1, nc);
-  else
-    exact_stats_kernel<true, false><<<nb, 256, 0, s>>>(ex, b0, nb0, b1, nc);
-  cudaError_t e = cudaGetLastError();
+  const bool real = ex.halves == 1;
+  auto* stats = real ? exact_stats_kernel<true, true> : exact_stats_kernel<true, false>;
+  cudaError_t e = launch_chained(stats, nb, 256, 0, s, true, ex, b0, nb0, b1, nc);
   if (e != cudaSuccess) return e;
-  if (ex.halves == 1 && ex.slices == 7)
-    exact_slice_b_kernel<7, true><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
-  else if (ex.halves == 1)
-    exact_slice_b_kernel<6, true><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
-  else if (ex.slices == 7)
-    exact_slice_b_kernel<7, false><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
-  else
-    exact_slice_b_kernel<6, false><<<152 * 8, 256, 0, s>>>(ex, b0, nb0, b1, nb, nc);
-  return cudaGetLastError();
+  auto* slice = ex.slices == 7 ? (real ? exact_slice_b_kernel<7, true> : exact_slice_b_kernel<7, false>)
+                               : (real ? exact_slice_b_kernel<6, true> : exact_slice_b_kernel<6, false>);
+  return launch_chained(slice, 152 * 8, 256, 0, s, true, ex, b0, nb0, b1, nb, nc);
 }
 
 cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int nc, cudaStream_t s) {
-  exact_stats_kernel<false, false><<<rows, 256, 0, s>>>(ex, a, rows, nullptr, nc);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(exact_stats_kernel<false, false>, rows, 256, 0, s, true, ex, a, rows, nullptr, nc);
   if (e != cudaSuccess) return e;
-  exact_slice_a_kernel<<<152 * 16, 256, 0, s>>>(ex, a, rows, nc);
-  return cudaGetLastError();
+  return launch_chained(exact_slice_a_kernel, 152 * 16, 256, 0, s, true, ex, a, rows, nc);
 }
 
 cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s) {
@@ -777,24 +785,18 @@ cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaSt
   const uint32_t smem = ex_smem(ex.slices);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  kernel<<<std::min(grid, ex.n_items), kThreadsEx, smem, s>>>(ex, status);
-  return cudaGetLastError();
+  return launch_chained(kernel, std::min(grid, ex.n_items), kThreadsEx, smem, s, true, ex, status);
 }
 
 cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s,
-                                bool second_rows) {
-  const int rb0 = second_rows ? ex.n_main_blocks : 0;
-  const int nrb = (d.nf * d.ng + kExRows - 1) / kExRows, ncb = (d.nb + ex.bands - 1) / ex.bands;
+                                const ExSecond& second) {
   auto* kernel = ex.halves == 1 ? exact_finish_kernel<true> : exact_finish_kernel<false>;
-  kernel<<<dim3(nrb, ncb, ex.bands / kFinBands), kFinThreads, 0, s>>>(d, ex, rb0);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(kernel, dim3(ex.n_row_blocks, ex.n_col_blocks, ex.bands / kFinBands), kFinThreads, 0,
+                                 s, true, d, ex, second);
   if (e != cudaSuccess) return e;
-  const int blocks = (d.nb * d.nf * 32 + 255) / 256;
-  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, rb0, ex.partial, out);
-  e = cudaGetLastError();
-  if (e != cudaSuccess || !out2) return e;
-  exact_reduce_kernel<<<blocks, 256, 0, s>>>(d, ex, rb0, ex.partial2, out2);
-  return cudaGetLastError();
+  const int entries = d.nb * d.nf * (out2 ? 2 : 1) + (second.out ? second.nb * second.nf : 0);
+  return launch_chained(exact_reduce_kernel, (entries * kRedLanes + kRedThreads - 1) / kRedThreads, kRedThreads, 0, s,
+                        true, d, ex, second, out, out2);
 }
 
 }  // namespace sigma

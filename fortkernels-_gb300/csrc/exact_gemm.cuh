@@ -116,9 +116,8 @@ void exact_bind(ExactPrep& ex, void* work, void* own);
 cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t);
 
 // FF plans take the exact form from this many products on (rows x bands x K):
-// 16 x (5 x 20) x 512 = 0.8 M takes 75 us, 119 us on the FP64 pipe, but the
-// exact form's nine launches never take less than ~65 us.
-constexpr double kExactMin = 1 << 19;
+// 8 x (5 x 12) x 256 = 0.12 M takes 42 us, 67 us on the FP64 pipe.
+constexpr double kExactMin = 1 << 16;
 
 // One contraction, in order:
 //   exact_begin       clears the flag and the overlap counts
@@ -128,18 +127,25 @@ constexpr double kExactMin = 1 << 19;
 //   launch_exact_a    row exponents, overlap check and the A digits of
 //                     complex rows (or the caller's own producer of both)
 //   launch_exact_gemm the digit products
-//   launch_exact_finish  FP64 sums of a row group per band, into out[n][f]
+//   launch_exact_finish  FP64 sums of the row groups per band, into out[n][f]
 //                     (complex; halves = 1: FfDev::aqsm holds real values and
-//                     the imaginary parts are zero); FfDev::nf and nb are the
-//                     group's
+//                     the imaginary parts are zero); FfDev::nf, nb and vfac
+//                     are the first group's
 cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s);
-cudaError_t exact_begin_counts(const ExactPrep& ex, cudaStream_t s);  // the flag kept (shared with an earlier one)
+cudaError_t exact_begin_flag(const ExactPrep& ex, cudaStream_t s);  // the flag alone (the caller's first kernel
+                                                                     // calls ex_begin_counts)
 cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const void* b1, int nb1, int nc,
                            cudaStream_t s);
 cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int nc, cudaStream_t s);
 cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s);
+// The second row group's epilogue, and its sums.
+struct ExSecond {
+  int nb, nf;
+  double vfac;
+  double2* out;  // [nb][nf]; null: no such group
+};
 cudaError_t launch_exact_finish(const FfDev& d, const ExactPrep& ex, double2* out, double2* out2, cudaStream_t s,
-                                bool second_rows = false);
+                                const ExSecond& second = ExSecond{0, 0, 0.0, nullptr});
 
 // ---------------------------------------------------------------- device helpers
 // Byte offset of element (row r, k) inside a K-major 32-byte-swizzled tile of
@@ -148,6 +154,12 @@ __host__ __device__ __forceinline__ uint32_t sw32_offset(int r, int ch) {
   return (uint32_t)(r * 32 + ((ch ^ ((r >> 2) & 1)) << 4));
 }
 
+// The overlap counts' start values, by the threads of a grid that precedes
+// launch_exact_b.
+__device__ __forceinline__ void ex_begin_counts(const ExactPrep& ex) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * ex.n_kseg; i += gridDim.x * blockDim.x)
+    ex.seg_min[i] = 0x7f7f7f7f;  // seg_pow follows it
+}
 __device__ __forceinline__ void ex_raise(const ExactPrep& ex) {
   *ex.flag = 1;
   if (ex.any) *ex.any = 1;

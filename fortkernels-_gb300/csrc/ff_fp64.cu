@@ -35,7 +35,10 @@ __global__ void __launch_bounds__(kFfThreads, 1) ff_fp64_kernel(FfDev p, FfWork 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FfSmem& sm = *reinterpret_cast<FfSmem*>(smem_raw);
   __shared__ int s_item;
-  if (w.run_if && !*w.run_if) return;
+  if (w.run_if) {  // launched in a chain
+    chain_begin();
+    if (!*w.run_if) return;
+  }
   const int tid = threadIdx.x, tc = tid & 15, tr = tid >> 4;
   const int blocks_per_freq = p.ngp / kFfRows;
 
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) ff_fp64_kernel(FfDev p, FfWork 
 // schDt[n1][ifreq]: one warp per entry sums its row blocks and K splits in a
 // fixed order with compensated FP64.
 __global__ void ff_reduce_kernel(FfDev p, FfWork w, double2* schdt) {
+  if (w.run_if) chain_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= p.nb * p.nf || (w.run_if && !*w.run_if)) return;
@@ -186,16 +190,14 @@ cudaError_t launch_ff_fp64(const FfDev& p, const FfWork& w, int grid, cudaStream
   cudaError_t e =
       cudaFuncSetAttribute(ff_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FfSmem));
   if (e != cudaSuccess) return e;
-  ff_fp64_kernel<<<grid, kFfThreads, sizeof(FfSmem), s>>>(p, w);
-  return cudaGetLastError();
+  return launch_chained(ff_fp64_kernel, grid, kFfThreads, sizeof(FfSmem), s, w.run_if != nullptr, p, w);
 }
 
 cudaError_t launch_ff_reduce(const FfDev& p, const FfWork& w, double2* schdt, cudaStream_t s) {
   const int warps = p.nb * p.nf;
   const int threads = 256;
   const int blocks = (warps * 32 + threads - 1) / threads;
-  ff_reduce_kernel<<<blocks, threads, 0, s>>>(p, w, schdt);
-  return cudaGetLastError();
+  return launch_chained(ff_reduce_kernel, blocks, threads, 0, s, w.run_if != nullptr, p, w, schdt);
 }
 
 }  // namespace sigma

@@ -76,7 +76,7 @@ struct sigma_gpp_batch_s {
   sigma::OzGroup grp{};
   // grouped reductions (every form)
   const sigma::ReduceJob* d_red = nullptr;
-  int red_warps = 0;
+  int red_warps = 0, red_count = 0;  // rows, partials of the longest
   void* red_block = nullptr;
   std::vector<sigma::GppWork> fssx;  // grouped tensor form: the factor pass's ssx partials per instance
 };
@@ -329,6 +329,7 @@ int build_reductions(sigma_gpp_batch_s* b) {
                           reinterpret_cast<double2*>(b->inst[i].asxtemp),
                           reinterpret_cast<double2*>(b->inst[i].acht_n1_loc), warps);
     warps += gpp_reduce_job_rows(r[i]);
+    b->red_count = std::max(b->red_count, gpp_reduce_job_count(r[i]));
   }
   cudaError_t e = cudaMalloc(&b->red_block, sizeof(ReduceJob) * b->n);
   if (e != cudaSuccess) {
@@ -658,7 +659,7 @@ extern "C" int sigma_gpp_batch_execute(sigma_gpp_batch b, void* stream) {
     SIGMA_CUDA_TRY(launch_factor_pass(b->d_fac, b->n, b->fac_total, b->fac_grid, b->fac_nvband, s));
     SIGMA_CUDA_TRY(launch_ozaki_group_gemm(b->grp, device_sm_count(), s));
     SIGMA_CUDA_TRY(launch_ozaki_group_reduce(b->grp, s));
-    SIGMA_CUDA_TRY(launch_gpp_reduce_group(b->d_red, b->n, b->red_warps, s));
+    SIGMA_CUDA_TRY(launch_gpp_reduce_group(b->d_red, b->n, b->red_warps, b->red_count, s));
     return SIGMA_OK;
   }
   if (mixed && !tensor)
@@ -694,7 +695,7 @@ extern "C" int sigma_gpp_batch_execute(sigma_gpp_batch b, void* stream) {
   if (b->ssx_view.total > 0)
     SIGMA_CUDA_TRY(mixed ? launch_ssx_mixed_batch(b->ssx_view, b->ssx_grid, b->all_shared_wx, s)
                          : launch_ssx_fp64_batch(b->ssx_view, b->ssx_grid, s));
-  SIGMA_CUDA_TRY(launch_gpp_reduce_group(b->d_red, b->n, b->red_warps, s));
+  SIGMA_CUDA_TRY(launch_gpp_reduce_group(b->d_red, b->n, b->red_warps, b->red_count, s));
   return SIGMA_OK;
 }
 

@@ -94,6 +94,8 @@ template <int kForm>
 __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep ex, int nf, int nf2) {
   using F = Form<kForm>;
   __shared__ unsigned s_m[F::kSlabs][kGxThreads / 32];
+  chain_begin();
+  ex_begin_counts(ex);  // the first kernel of an execution
   const int g = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool occ = F::kHalfOcc || F::kRealOcc || nf2 > 0;
   FF wx[kNW];
@@ -302,6 +304,7 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
   __shared__ int s_lim[kGxCols], s_need;
   __shared__ FF s_wx[kNW], s_iwx2[kNW];
   __shared__ bool s_wide;
+  chain_begin();
   if (*ex.flag) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int p0 = blockIdx.x * kGxCols;
@@ -478,6 +481,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename H::Planes& sm = *reinterpret_cast<typename H::Planes*>(smem_raw);
   __shared__ int s_e[kSlabs][kGxCols], s_lim[2][kGxCols], s_need;
+  chain_begin();
   if (*ex.flag) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int p0 = blockIdx.x * kGxCols;
@@ -560,6 +564,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
 // least band (kHalfPower).
 template <int kForm>
 __global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const int* kend, int nf, int slabs, int per_seg) {
+  chain_begin();
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= slabs * p.ng) return;
   const int g = i % p.ng, row = gx_row(ex, p.ng, nf, i / p.ng, g);
@@ -610,10 +615,11 @@ void gx_size(ExactPrep& ex, const GxShape& q, const std::vector<int>& igp_of, in
              kend.empty() ? nullptr : kend.data(), t, nf2, nf2 ? q.nvband : 0);
 }
 // g-vectors per factor item: a segment, or less where the columns are too few
-// to give every SM its four CTAs twice (409 x 8192: 64 or 512 ... at 128).
+// to give every SM its four CTAs twice (409 x 8192: 64 or 512 ... at 128); at
+// least one staged tile.
 int gx_run(const ExactPrep& ex, int ng, int sms) {
   int run = kExSeg;
-  while (run > 64 && (long long)((ng + kGxCols - 1) / kGxCols) * ex.n_kseg * (kExSeg / run) < 8LL * sms) run /= 2;
+  while (run > (ex.slices == 6 ? kFfK : 64) && (long long)((ng + kGxCols - 1) / kGxCols) * ex.n_kseg * (kExSeg / run) < 8LL * sms) run /= 2;
   return run;
 }
 size_t gx_stat_bytes(const ExactPrep& ex, int run) {
@@ -626,23 +632,21 @@ cudaError_t launch_ff(const GppExact& g, const GxDev& p, dim3 grid, cudaStream_t
   cudaError_t e =
       cudaFuncSetAttribute(gx_ff_kernel<kForm, kOcc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  gx_ff_kernel<kForm, kOcc><<<grid, kGxThreads, smem, s>>>(p, g.ex, g.stat, g.nf, g.run);
-  return cudaGetLastError();
+  return launch_chained(gx_ff_kernel<kForm, kOcc>, grid, kGxThreads, smem, s, true, p, g.ex, g.stat, g.nf, g.run);
 }
 
 template <int kForm>
 cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, bool begin) {
   using F = Form<kForm>;
   const ExactPrep& ex = g.ex;
-  cudaError_t e = begin ? exact_begin(ex, s) : exact_begin_counts(ex, s);
+  cudaError_t e = begin ? exact_begin_flag(ex, s) : cudaSuccess;
+  if (e != cudaSuccess) return e;
+  e = launch_chained(gx_max_kernel<kForm>, p.ng, kGxThreads, 0, s, true, p, ex, g.nf, g.nf2);
   if (e != cudaSuccess) return e;
   const int nb = F::kHalfOcc || F::kRealOcc ? p.nvband : p.nb;
   e = launch_exact_b(ex, p.aqsn, nb, p.aqsm, F::kHalf || F::kHalfOcc ? nb : 0, p.nc, s);
   if (e != cudaSuccess) return e;
   const int slabs = g.nf + g.nf2;
-  gx_max_kernel<kForm><<<p.ng, kGxThreads, 0, s>>>(p, ex, g.nf, g.nf2);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   const int pad = std::max(ex.n_main_blocks * kExRows - g.nf * p.ng,
                            (ex.n_row_blocks - ex.n_main_blocks) * kExRows - g.nf2 * p.ng);
   const dim3 grid((p.ng + pad + kGxCols - 1) / kGxCols, ex.n_kseg * (kExSeg / g.run));
@@ -650,32 +654,31 @@ cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, b
     constexpr int smem = sizeof(typename F64<kForm>::Planes);
     e = cudaFuncSetAttribute(gx_f64_kernel<kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    gx_f64_kernel<kForm><<<grid, kGxThreads, smem, s>>>(p, ex, g.stat, g.nf, g.run);
-    e = cudaGetLastError();
+    e = launch_chained(gx_f64_kernel<kForm>, grid, kGxThreads, smem, s, true, p, ex, g.stat, g.nf, g.run);
   } else if (kForm == kGxGpp && g.nf2) {
     e = launch_ff<kGxGpp, true>(g, p, grid, s);
   } else {
     e = launch_ff<kForm, false>(g, p, grid, s);
   }
   if (e != cudaSuccess) return e;
-  gx_check_kernel<kForm><<<(slabs * p.ng * 32 + 255) / 256, 256, 0, s>>>(p, ex, g.stat, g.kend, g.nf, slabs,
-                                                                           kExSeg / g.run);
-  return cudaGetLastError();
+  return launch_chained(gx_check_kernel<kForm>, (slabs * p.ng * 32 + 255) / 256, 256, 0, s, true, p, ex, g.stat, g.kend,
+                        g.nf, slabs, kExSeg / g.run);
 }
 
 }  // namespace
 
 // From these products on (3 x columns x bands x g-vectors) the contraction beats
 // the float-float passes, whose time stays flat below (one CTA's latency):
-// measured us, contraction against passes, at 16 x 20 x 512 (0.5 M) 105 / 165
-// with occupied bands and 80 / 75 without, real 24 x 40 x 1024 (2.9 M) 140 / 149,
-// half sum 60 x 60 x 2048 (22 M) 303 / 372.
+// measured us, contraction against passes, at 8 x 12 x 256 (74 k) 58 / 158 with
+// occupied bands and 50 / 66 without, real 16 x 20 x 512 (0.5 M) 105 / 138 and
+// 52 / 56; the half sum's two contractions 221 / 187 at 24 x 40 x 1024 (2.9 M),
+// 230 / 229 at 60 x 60 x 1024 (11 M), 315 / 372 at 60 x 60 x 2048.
 bool gpp_exact_fits(const GxShape& q) {
   const double products = (double)kNW * q.ng * q.nb * q.nc;
   switch (q.form) {
-    case kGxReal: return products >= 1 << 22;
+    case kGxReal: return products >= 1 << 18;
     case kGxHalf: return products >= 1 << 23;
-    default: return products >= (q.nvband > 0 ? 1 << 18 : 1 << 20);
+    default: return products >= 1 << 16;
   }
 }
 
@@ -756,12 +759,8 @@ cudaError_t launch_gpp_exact_sums(const GppExact& g, const GxDev& p, int* status
   d.vfac = g.form == kGxRealOcc ? p.occ : 0.5;
   d.pair_bands = pair ? nb : 0;
   d.pair_static = g.form == kGxHalf && g.nf > kNW;
-  e = launch_exact_finish(d, g.ex, out, nullptr, s);
-  if (e != cudaSuccess || g.nf2 == 0) return e;
-  d.nb = p.nvband;
-  d.nf = g.nf2;
-  d.vfac = p.occ;
-  return launch_exact_finish(d, g.ex, occ_out, nullptr, s, true);
+  return launch_exact_finish(d, g.ex, out, nullptr, s,
+                             ExSecond{p.nvband, g.nf2, p.occ, g.nf2 ? occ_out : nullptr});
 }
 
 }  // namespace sigma

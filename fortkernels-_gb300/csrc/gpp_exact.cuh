@@ -80,8 +80,8 @@ cudaError_t launch_gpp_exact_sums(const GppExact& g, const GxDev& p, int* status
                                   cudaStream_t s);
 
 // Kernels of one execution: two for the bands, three for the factors, the
-// contraction and two for each epilogue.
-inline int gpp_exact_launches(const GppExact& g) { return g ? 6 + (g.nf2 ? 4 : 2) : 0; }
+// contraction and two for the epilogue.
+inline int gpp_exact_launches(const GppExact& g) { return g ? 8 : 0; }
 
 inline GxDev gx_dev(const GppDev& p) {
   auto d = [](const double2* x) { return reinterpret_cast<const double*>(x); };

@@ -671,7 +671,10 @@ template <int BN, int BP>
 __global__ void __launch_bounds__(kThreads, 2) sch_fp64y_kernel(GppDev p, GppWork w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
-  if (w.run_if && !*w.run_if) return;
+  if (w.run_if) {  // launched in a chain
+    chain_begin();
+    if (!*w.run_if) return;
+  }
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -748,7 +751,10 @@ template <bool kSmall>
 __global__ void __launch_bounds__(kThreads, kSmall ? 2 : 1) sch_fp64y_batch_kernel(GppBatchView b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
-  if (b.run_if && !*b.run_if) return;
+  if (b.run_if) {  // launched in a chain
+    chain_begin();
+    if (!*b.run_if) return;
+  }
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -1064,7 +1070,10 @@ __global__ void __launch_bounds__(kThreads) ssx_fp64_kernel(GppDev p, GppWork w)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
   __shared__ SsxShared sh;
-  if (w.run_if && !*w.run_if) return;
+  if (w.run_if) {  // launched in a chain
+    chain_begin();
+    if (!*w.run_if) return;
+  }
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -1107,7 +1116,10 @@ __global__ void __launch_bounds__(kThreads) ssx_fp64_batch_kernel(GppBatchView b
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
   __shared__ SsxShared sh;
-  if (b.run_if && !*b.run_if) return;
+  if (b.run_if) {  // launched in a chain
+    chain_begin();
+    if (!*b.run_if) return;
+  }
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -1147,8 +1159,7 @@ cudaError_t launch_sch_fp64y(const GppDev& p, const GppWork& w, int grid, cudaSt
   e = cudaFuncSetAttribute(sch_fp64y_kernel<kBNY, kBPY>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  sch_fp64y_kernel<kBNY, kBPY><<<grid, kThreads, smem, s>>>(p, w);
-  return cudaGetLastError();
+  return launch_chained(sch_fp64y_kernel<kBNY, kBPY>, grid, kThreads, smem, s, w.run_if != nullptr, p, w);
 }
 int ssx_blocks_per_sm_fp64() { return blocks_per_sm(ssx_fp64_kernel, sizeof(SsxSmem)); }
 int sch_batch_blocks_per_sm_fp64() { return blocks_per_sm(sch_fp64_batch_kernel, kSchBatchSmem); }
@@ -1165,8 +1176,7 @@ cudaError_t launch_sch_fp64y_batch(const GppBatchView& b, int grid, bool small, 
     e = cudaFuncSetAttribute(sch_fp64y_batch_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    sch_fp64y_batch_kernel<true><<<grid, kThreads, kSchYBatchSmallSmem, s>>>(b);
-    return cudaGetLastError();
+    return launch_chained(sch_fp64y_batch_kernel<true>, grid, kThreads, kSchYBatchSmallSmem, s, b.run_if != nullptr, b);
   }
   cudaError_t e = cudaFuncSetAttribute(sch_fp64y_batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kSchYBatchSmem);
@@ -1174,8 +1184,7 @@ cudaError_t launch_sch_fp64y_batch(const GppBatchView& b, int grid, bool small, 
   e = cudaFuncSetAttribute(sch_fp64y_batch_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  sch_fp64y_batch_kernel<false><<<grid, kThreads, kSchYBatchSmem, s>>>(b);
-  return cudaGetLastError();
+  return launch_chained(sch_fp64y_batch_kernel<false>, grid, kThreads, kSchYBatchSmem, s, b.run_if != nullptr, b);
 }
 int ssx_batch_blocks_per_sm_fp64() { return blocks_per_sm(ssx_fp64_batch_kernel, sizeof(SsxSmem)); }
 
@@ -1195,8 +1204,7 @@ cudaError_t launch_ssx_fp64(const GppDev& p, const GppWork& w, int grid, cudaStr
   cudaError_t e = cudaFuncSetAttribute(ssx_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        sizeof(SsxSmem));
   if (e != cudaSuccess) return e;
-  ssx_fp64_kernel<<<grid, kThreads, sizeof(SsxSmem), s>>>(p, w);
-  return cudaGetLastError();
+  return launch_chained(ssx_fp64_kernel, grid, kThreads, sizeof(SsxSmem), s, w.run_if != nullptr, p, w);
 }
 
 cudaError_t launch_sch_fp64_batch(const GppBatchView& b, int grid, cudaStream_t s) {
@@ -1211,8 +1219,7 @@ cudaError_t launch_ssx_fp64_batch(const GppBatchView& b, int grid, cudaStream_t 
   cudaError_t e = cudaFuncSetAttribute(ssx_fp64_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        sizeof(SsxSmem));
   if (e != cudaSuccess) return e;
-  ssx_fp64_batch_kernel<<<grid, kThreads, sizeof(SsxSmem), s>>>(b);
-  return cudaGetLastError();
+  return launch_chained(ssx_fp64_batch_kernel, grid, kThreads, sizeof(SsxSmem), s, b.run_if != nullptr, b);
 }
 
 }  // namespace sigma

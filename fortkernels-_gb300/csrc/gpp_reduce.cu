@@ -8,17 +8,28 @@
 // a fixed strided subset, then a fixed butterfly per warp and the warps in
 // order), then one warp per frequency sums the bands.  Results are
 // identical run to run.
+#include <algorithm>
+
 #include "sigma_internal.cuh"
 
 namespace sigma {
 namespace {
 
 
-constexpr int kRowThreads = 256;
+// Threads per row: two warps where the rows fill the chip and are short (eight
+// spend most of the time in their butterflies, 80 FP64 operations each at two
+// lanes per clock per SM: 100 -> 41 us at the FP32 form's 1542 rows), else
+// eight, whose loads overlap (the tensor form's six long rows: 43 us, 73 us
+// with two).
+constexpr int kRowWarps = 8;
+int row_threads(int rows, int count) { return rows >= 304 && count <= 1024 ? 64 : 32 * kRowWarps; }
+int row_count(const ReduceArgs& a) {
+  return std::max(a.sch_rows > 0 ? a.sch_ncb * a.sch_splits : 0, a.nvband > 0 ? a.ssx_ncb * a.ssx_splits : 0);
+}
 
 // Row `row` of the band-sum stage (one block).
 __device__ __forceinline__ void reduce_bands_row(const ReduceArgs& a, int row) {
-  __shared__ double s_x[kRowThreads / 32], s_y[kRowThreads / 32];
+  __shared__ double s_x[kRowWarps], s_y[kRowWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_sch = a.sch_rows * kNW;
   const bool is_sch = row < n_sch;
@@ -33,7 +44,8 @@ __device__ __forceinline__ void reduce_bands_row(const ReduceArgs& a, int row) {
   const int bb = n1 / bn, bl = n1 % bn;
   Comp sx, sy;
   const int count = ncb * ns;
-  for (int q = threadIdx.x; q < count; q += kRowThreads) {
+#pragma unroll 4
+  for (int q = threadIdx.x; q < count; q += blockDim.x) {
     const size_t item = (size_t)bb * count + q;  // (bb * ncb + cb) * ns + s
     const double2 v = part[item * bn * kNW + bl * kNW + iw];
     sx.add(v.x);
@@ -47,7 +59,7 @@ __device__ __forceinline__ void reduce_bands_row(const ReduceArgs& a, int row) {
   __syncthreads();
   if (threadIdx.x == 0) {
     Comp tx, ty;
-    for (int w = 0; w < kRowThreads / 32; ++w) {
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) {
       tx.add(s_x[w]);
       ty.add(s_y[w]);
     }
@@ -58,41 +70,50 @@ __device__ __forceinline__ void reduce_bands_row(const ReduceArgs& a, int row) {
   }
 }
 
-__global__ void __launch_bounds__(kRowThreads) reduce_bands_kernel(ReduceArgs a) {
+__global__ void __launch_bounds__(32 * kRowWarps) reduce_bands_kernel(ReduceArgs a) {
+  chain_begin();
   reduce_bands_row(a, blockIdx.x);
 }
 
-__device__ __forceinline__ void reduce_total_block(const double2* acht_n1, const double2* asx_n1, int nb,
+// One warp per frequency and sum (blocks 0-5), each on an SM of its own: six
+// warps of one SM share its two FP64 lanes per clock (15.5 -> 13.4 us at
+// 512 bands).  Block 6: the band sums of the last frequency.
+constexpr int kTotalBlocks = 2 * kNW + 1;
+__device__ __forceinline__ void reduce_total_block(int block, const double2* acht_n1, const double2* asx_n1, int nb,
                                                    int nvband, double2* achtemp, double2* asxtemp,
                                                    double2* acht_n1_loc) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < 2 * kNW) {
-    const bool ach = warp < kNW;
-    const int iw = ach ? warp : warp - kNW;
-    const double2* src = ach ? acht_n1 : asx_n1;
-    const int n = ach ? nb : nvband;
-    Comp sx, sy;
-    for (int n1 = lane; n1 < n; n1 += 32) {
-      const double2 v = src[n1 * kNW + iw];
-      sx.add(v.x);
-      sy.add(v.y);
-    }
-    const double rx = warp_sum_comp(sx), ry = warp_sum_comp(sy);
-    if (lane == 0) (ach ? achtemp : asxtemp)[iw] = make_double2(rx, ry);
+  const int lane = threadIdx.x;
+  if (block == 2 * kNW) {
+    if (acht_n1_loc)
+      for (int n1 = lane; n1 < nb; n1 += 32) acht_n1_loc[n1] = acht_n1[n1 * kNW + 2];
+    return;
   }
-  if (acht_n1_loc)
-    for (int n1 = threadIdx.x; n1 < nb; n1 += blockDim.x) acht_n1_loc[n1] = acht_n1[n1 * kNW + 2];
+  const bool ach = block < kNW;
+  const int iw = ach ? block : block - kNW;
+  const double2* src = ach ? acht_n1 : asx_n1;
+  const int n = ach ? nb : nvband;
+  Comp sx, sy;
+#pragma unroll 8
+  for (int n1 = lane; n1 < n; n1 += 32) {
+    const double2 v = src[n1 * kNW + iw];
+    sx.add(v.x);
+    sy.add(v.y);
+  }
+  const double rx = warp_sum_comp(sx), ry = warp_sum_comp(sy);
+  if (lane == 0) (ach ? achtemp : asxtemp)[iw] = make_double2(rx, ry);
 }
 
 __global__ void reduce_total_kernel(const double2* acht_n1, const double2* asx_n1, int nb,
                                     int nvband, double2* achtemp, double2* asxtemp,
                                     double2* acht_n1_loc) {
-  reduce_total_block(acht_n1, asx_n1, nb, nvband, achtemp, asxtemp, acht_n1_loc);
+  chain_begin();
+  reduce_total_block(blockIdx.x, acht_n1, asx_n1, nb, nvband, achtemp, asxtemp, acht_n1_loc);
 }
 
 // Group forms over many instances: blocks row_off .. + (sch_rows + nvband) * 3
 // of each job, then one block per job.
-__global__ void __launch_bounds__(kRowThreads) reduce_bands_group_kernel(const ReduceJob* jobs, int n) {
+__global__ void __launch_bounds__(32 * kRowWarps) reduce_bands_group_kernel(const ReduceJob* jobs, int n) {
+  chain_begin();
   const int row = blockIdx.x;
   int lo = 0, hi = n - 1;
   while (lo < hi) {
@@ -103,8 +124,9 @@ __global__ void __launch_bounds__(kRowThreads) reduce_bands_group_kernel(const R
 }
 
 __global__ void reduce_total_group_kernel(const ReduceJob* jobs) {
-  const ReduceJob& j = jobs[blockIdx.x];
-  reduce_total_block(j.a.acht_n1, j.a.asx_n1, j.a.nb, j.a.nvband, j.achtemp, j.asxtemp, j.acht_n1_loc);
+  chain_begin();
+  const ReduceJob& j = jobs[blockIdx.x / kTotalBlocks];
+  reduce_total_block(blockIdx.x % kTotalBlocks, j.a.acht_n1, j.a.asx_n1, j.a.nb, j.a.nvband, j.achtemp, j.asxtemp, j.acht_n1_loc);
 }
 
 }  // namespace
@@ -134,17 +156,16 @@ ReduceJob gpp_reduce_job(const GppWork& sch, const GppWork& ssx, int nb, double2
   return j;
 }
 
+int gpp_reduce_job_count(const ReduceJob& j) { return row_count(j.a); }
 int gpp_reduce_job_rows(const ReduceJob& j) { return (j.a.sch_rows + j.a.nvband) * kNW; }
 
-cudaError_t launch_gpp_reduce_group(const ReduceJob* jobs, int n, int total_rows, cudaStream_t s) {
+cudaError_t launch_gpp_reduce_group(const ReduceJob* jobs, int n, int total_rows, int max_count, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (total_rows > 0) {
-    reduce_bands_group_kernel<<<total_rows, kRowThreads, 0, s>>>(jobs, n);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(reduce_bands_group_kernel, total_rows, row_threads(total_rows, max_count), 0, s, true, jobs, n);
     if (e != cudaSuccess) return e;
   }
-  reduce_total_group_kernel<<<n, 256, 0, s>>>(jobs);
-  return cudaGetLastError();
+  return launch_chained(reduce_total_group_kernel, n * kTotalBlocks, 32, 0, s, true, jobs);
 }
 
 cudaError_t launch_gpp_reduce(const GppWork& sch, const GppWork& ssx, int nb, double2* acht_n1,
@@ -167,13 +188,11 @@ cudaError_t launch_gpp_reduce(const GppWork& sch, const GppWork& ssx, int nb, do
   a.asx_n1 = acht_n1 + (size_t)nb * kNW;
   const int rows = (a.sch_rows + a.nvband) * kNW;
   if (rows > 0) {
-    reduce_bands_kernel<<<rows, kRowThreads, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(reduce_bands_kernel, rows, row_threads(rows, row_count(a)), 0, s, true, a);
     if (e != cudaSuccess) return e;
   }
-  reduce_total_kernel<<<1, 256, 0, s>>>(acht_n1, a.asx_n1, nb, a.nvband, achtemp, asxtemp,
-                                        acht_n1_loc);
-  return cudaGetLastError();
+  return launch_chained(reduce_total_kernel, kTotalBlocks, 32, 0, s, true, acht_n1, a.asx_n1, nb, a.nvband, achtemp, asxtemp,
+                        acht_n1_loc);
 }
 
 }  // namespace sigma

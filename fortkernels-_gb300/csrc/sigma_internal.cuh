@@ -210,8 +210,9 @@ struct ReduceJob {
 ReduceJob gpp_reduce_job(const GppWork& sch, const GppWork& ssx, int nb, double2* acht_n1, double2* achtemp,
                          double2* asxtemp, double2* acht_n1_loc, int row_off);
 int gpp_reduce_job_rows(const ReduceJob& j);
+int gpp_reduce_job_count(const ReduceJob& j);  // partials of its longest row
 // The reductions of jobs[0 .. n) (device array): two launches for all.
-cudaError_t launch_gpp_reduce_group(const ReduceJob* jobs, int n, int total_rows, cudaStream_t s);
+cudaError_t launch_gpp_reduce_group(const ReduceJob* jobs, int n, int total_rows, int max_count, cudaStream_t s);
 
 // Sums the partials of the sch and ssx passes in a fixed order into
 // acht_n1[nb][3] (workspace), achtemp[3], asxtemp[3] and acht_n1_loc[nb].
@@ -332,9 +333,10 @@ struct Comp {
 
 // Butterfly combine of compensated pairs; every lane ends with the same value
 // (TwoSum's error term is exact, so a+b and b+a agree bit for bit).
-__device__ __forceinline__ double warp_sum_comp(Comp c) {
+template <int kLanes>
+__device__ __forceinline__ double lanes_sum_comp(Comp c) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = kLanes / 2; o > 0; o >>= 1) {
     const double s2 = __shfl_xor_sync(0xffffffffu, c.s, o);
     const double c2 = __shfl_xor_sync(0xffffffffu, c.c, o);
     double t, e;
@@ -343,6 +345,37 @@ __device__ __forceinline__ double warp_sum_comp(Comp c) {
     c.c = __dadd_rn(__dadd_rn(c.c, c2), e);
   }
   return c.value();
+}
+__device__ __forceinline__ double warp_sum_comp(Comp c) { return lanes_sum_comp<32>(c); }
+
+// ---------------------------------------------------------------- chained launches
+// A chain of short kernels costs its launch latencies: at 24 bands x 40
+// columns x 1024 g-vectors the kernels of an execution do a few microseconds'
+// work each.  A kernel that begins with chain_begin() may be launched by
+// launch_chained: its CTAs are then placed while the kernel before it still
+// runs, and wait there until that one has ended and its writes are visible
+// (fourteen launches 118 us, twelve chained ones 68 us).  Every thread calls it
+// before anything else, so that the end of each kernel of a chain implies the
+// end of all before it.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// chained = false: an ordinary launch.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool chained,
+                           A... args) {
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &a;
+  c.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
 }  // namespace sigma
