@@ -763,40 +763,34 @@ __global__ void half_reduce_bands_kernel(HalfReduceArgs a) {
   if (lane == 0) *dst = make_double2(rx, ry);
 }
 
+// One warp per sum (blocks 0-5 the frequencies' achtemp and asxtemp, 6 the
+// static remainder), block 7 the last frequency's band sums: six warps of one
+// SM share its two FP64 lanes per clock (17.6 -> 13.9 us at 512 bands).
+constexpr int kHalfTotalBlocks = 2 * kNW + 2;
 __global__ void half_reduce_total_kernel(const double2* acht_n1, const double2* asx_n1,
                                          const double2* stat_n1, int nb, int nvband,
                                          double2* achtemp, double2* asxtemp, double2* achstemp,
                                          double2* acht_n1_loc) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < 2 * kNW + 1) {
-    Comp sx, sy;
-    if (warp < 2 * kNW) {
-      const bool ach = warp < kNW;
-      const int iw = ach ? warp : warp - kNW;
-      const double2* src = ach ? acht_n1 : asx_n1;
-      const int n = ach ? nb : nvband;
-      for (int n1 = lane; n1 < n; n1 += 32) {
-        sx.add(src[n1 * kNW + iw].x);
-        sy.add(src[n1 * kNW + iw].y);
-      }
-    } else if (achstemp) {
-      for (int n1 = lane; n1 < nb; n1 += 32) {
-        sx.add(stat_n1[n1].x);
-        sy.add(stat_n1[n1].y);
-      }
-    }
-    const double rx = warp_sum_comp(sx), ry = warp_sum_comp(sy);
-    if (lane == 0) {
-      if (warp < kNW)
-        achtemp[warp] = make_double2(rx, ry);
-      else if (warp < 2 * kNW)
-        asxtemp[warp - kNW] = make_double2(rx, ry);
-      else if (achstemp)
-        achstemp[0] = make_double2(rx, ry);
-    }
+  chain_begin();
+  const int block = blockIdx.x, lane = threadIdx.x;
+  if (block == 2 * kNW + 1) {
+    if (acht_n1_loc)
+      for (int n1 = lane; n1 < nb; n1 += 32) acht_n1_loc[n1] = acht_n1[n1 * kNW + 2];
+    return;
   }
-  if (acht_n1_loc)
-    for (int n1 = threadIdx.x; n1 < nb; n1 += blockDim.x) acht_n1_loc[n1] = acht_n1[n1 * kNW + 2];
+  const bool ach = block < kNW, stat = block == 2 * kNW;
+  if (stat && !achstemp) return;
+  const double2* src = stat ? stat_n1 : ach ? acht_n1 + block : asx_n1 + (block - kNW);
+  const int n = stat || ach ? nb : nvband, stride = stat ? 1 : kNW;
+  Comp sx, sy;
+#pragma unroll 8
+  for (int n1 = lane; n1 < n; n1 += 32) {
+    const double2 v = src[(size_t)n1 * stride];
+    sx.add(v.x);
+    sy.add(v.y);
+  }
+  const double rx = warp_sum_comp(sx), ry = warp_sum_comp(sy);
+  if (lane == 0) (stat ? achstemp : ach ? achtemp + block : asxtemp + (block - kNW))[0] = make_double2(rx, ry);
 }
 
 // [rows][cols] complex -> [cols][rows], 32 x 32 tiles through shared memory.
@@ -941,26 +935,65 @@ __global__ void __launch_bounds__(256) half_zs_slices_kernel(HalfDev p, OzakiPre
   }
 }
 
-// Band rows of the tensor form: one CTA per band, its 8 warps over the
+// Occupied bands of the exact form: the partner's sum leaves g-vector igp - 1
+// out, so its term, which the contraction holds, goes into the column
+// partials with the opposite sign.  One thread per (column, frequency): the
+// factor serves every band (inside the rows' kernel, per band, the occupied
+// bands' CTAs ran 0.3 ms behind the others at 1638 columns).
+__global__ void __launch_bounds__(64) half_occ_last_kernel(HalfDev p, const int* skip_if, double2* occ_ach,
+                                                           double2* occ_asx) {
+  chain_begin();
+  if (skip_if && *skip_if) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= p.ng * kNW) return;
+  const int col = t / kNW, iw = t % kNW, igp = p.igp_of[col];
+  const bool on = igp > 0 && igp <= p.brk[col];
+  double2 sch = make_double2(0.0, 0.0), ssx = sch;
+  if (on) {
+    const size_t og = (size_t)col * p.nc + igp - 1;
+    half_occ_factor(p.wt[og], p.ieps[og], p.wx[iw], sch, ssx);
+  }
+  for (int n1 = 0; n1 < p.nvband; ++n1) {
+    double2 a = make_double2(0.0, 0.0), x = a;
+    if (on) {
+      const double w = -0.5 * p.vcoul[igp], wx2 = 2.0 * w * p.occ;
+      const double2 am = p.aqsm[(size_t)n1 * p.nc + igp], ag = p.aqsm[(size_t)n1 * p.nc + igp - 1];
+      const double2 vs = cmul(am, cconj(cmul(ag, sch))), vx = cmul(am, cconj(cmul(ag, ssx)));
+      a = make_double2(w * vs.x, w * vs.y);
+      x = make_double2(wx2 * vx.x, wx2 * vx.y);
+    }
+    const size_t o = ((size_t)n1 * p.ng + col) * kNW + iw;
+    occ_ach[o] = a;
+    occ_asx[o] = x;
+  }
+}
+
+// Band rows of the tensor form: one CTA per band, its warps over the
 // columns, compensated sums of the unpaired igp terms (and of the
 // occupied-band partials) combined in a fixed order, then
 //   acht_n1[n1][iw] = T + conj(U) + unpaired       (n1 >= nvband)
 //                   = sum_col occ_ach                (n1 <  nvband)
 //   asx_n1[n1][iw]  = sum_col occ_asx                (n1 <  nvband)
+// (with tu_occ the occupied bands' T + conj(U) on top)
 //   stat_n1[n1]     = Ts + conj(Us) + unpaired       (static remainder)
-constexpr int kRowWarps = 8;  // at most; no more than the columns fill
+// At most two warps, no more than the columns fill: a warp's butterflies are 40
+// FP64 operations a value, so eight of them took most of the time (two lanes
+// per clock per SM): 300 -> 193 us at 512 bands x 1638 columns.
+constexpr int kRowWarps = 2;
 inline int row_threads(int ng) { return 32 * std::min(kRowWarps, (ng + 31) / 32); }
 __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
     HalfDev p, const double2* t3, const double2* u3, const double2* ts, const double2* us, int stride3, int stride1,
     const int* skip_if, const double2* tu_occ, const double2* occ_ach, const double2* occ_asx, double2* acht_n1, double2* asx_n1, double2* stat_n1) {
   constexpr int kVals = 4 * kNW + 2;  // ax, ay, sx, sy per frequency; qx, qy
   __shared__ double part[kRowWarps][kVals];
+  chain_begin();
   if (skip_if && *skip_if) return;
   const int n1 = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool occ = n1 < p.nvband;
   const double wx[3] = {p.wx[0], p.wx[1], p.wx[2]};
   Comp ax[3], ay[3], sx[3], sy[3], qx, qy;
+#pragma unroll 4
   for (int col = warp * 32 + lane; col < p.ng; col += blockDim.x) {
     const int igp = p.igp_of[col];
     if (igp < 0) continue;
@@ -977,24 +1010,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
         qy.add(w * v.y);
       }
     }
-    if (occ && tu_occ) {
-      // the partner's sum leaves g-vector igp - 1 out: its term, which the
-      // contraction holds, taken off again
-      if (igp > 0 && igp <= p.brk[col]) {
-        const size_t og = (size_t)col * p.nc + igp - 1;
-        const double2 ag = p.aqsm[(size_t)n1 * p.nc + igp - 1];
-#pragma unroll
-        for (int iw = 0; iw < kNW; ++iw) {
-          double2 sch, ssx;
-          half_occ_factor(p.wt[og], p.ieps[og], wx[iw], sch, ssx);
-          const double2 vs = cmul(am, cconj(cmul(ag, sch))), vx = cmul(am, cconj(cmul(ag, ssx)));
-          ax[iw].add(-w * vs.x);
-          ay[iw].add(-w * vs.y);
-          sx[iw].add(-2.0 * w * p.occ * vx.x);
-          sy[iw].add(-2.0 * w * p.occ * vx.y);
-        }
-      }
-    } else if (occ) {
+    if (occ) {
 #pragma unroll
       for (int iw = 0; iw < kNW; ++iw) {
         const double2 a = occ_ach[((size_t)n1 * p.ng + col) * kNW + iw];
@@ -1018,7 +1034,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
 #pragma unroll
   for (int iw = 0; iw < kNW; ++iw) {
     const double v0 = warp_sum_comp(ax[iw]), v1 = warp_sum_comp(ay[iw]);
-    const double v2 = warp_sum_comp(sx[iw]), v3 = warp_sum_comp(sy[iw]);
+    const double v2 = occ ? warp_sum_comp(sx[iw]) : 0.0, v3 = occ ? warp_sum_comp(sy[iw]) : 0.0;
     if (lane == 0) {
       part[warp][4 * iw + 0] = v0;
       part[warp][4 * iw + 1] = v1;
@@ -1026,7 +1042,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
       part[warp][4 * iw + 3] = v3;
     }
   }
-  const double q0 = warp_sum_comp(qx), q1 = warp_sum_comp(qy);
+  const double q0 = ts ? warp_sum_comp(qx) : 0.0, q1 = ts ? warp_sum_comp(qy) : 0.0;
   if (lane == 0) {
     part[warp][4 * kNW] = q0;
     part[warp][4 * kNW + 1] = q1;
@@ -1034,11 +1050,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) half_tensor_rows_kernel(
   __syncthreads();
   if (threadIdx.x != 0) return;
   double tot[kVals];
-  for (int v = 0; v < kVals; ++v) {
-    Comp c;
-    for (int q = 0; q < (int)blockDim.x / 32; ++q) c.add(part[q][v]);
-    tot[v] = c.value();
-  }
+#pragma unroll
+  for (int v = 0; v < kVals; ++v) tot[v] = blockDim.x > 32 ? part[0][v] + part[1][v] : part[0][v];
 #pragma unroll
   for (int iw = 0; iw < kNW; ++iw) {
     const double rx = tot[4 * iw], ry = tot[4 * iw + 1], ux = tot[4 * iw + 2], uy = tot[4 * iw + 3];
@@ -1348,16 +1361,14 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
                                  nullptr, true);
     }
     if (st != SIGMA_OK) return st;
-    half_tensor_rows_kernel<<<plan->nb, row_threads(plan->ng), 0, s>>>(
-        p, plan->t3, plan->u3, stat ? plan->ts : nullptr, plan->us, kNW, 1, nullptr, nullptr, plan->occ_ach, plan->occ_asx,
-        plan->acht_n1, plan->asx_n1, plan->stat_n1);
-    SIGMA_CUDA_TRY(cudaGetLastError());
-    half_reduce_total_kernel<<<1, 256, 0, s>>>(plan->acht_n1, plan->asx_n1, plan->stat_n1, plan->nb,
-                                               plan->nvband, reinterpret_cast<double2*>(achtemp),
-                                               reinterpret_cast<double2*>(asxtemp),
-                                               stat ? reinterpret_cast<double2*>(achstemp) : nullptr,
-                                               reinterpret_cast<double2*>(acht_n1_loc));
-    SIGMA_CUDA_TRY(cudaGetLastError());
+    SIGMA_CUDA_TRY(launch_chained(half_tensor_rows_kernel, plan->nb, row_threads(plan->ng), 0, s, true, p, plan->t3,
+                                  plan->u3, stat ? plan->ts : nullptr, plan->us, kNW, 1, nullptr, nullptr,
+                                  plan->occ_ach, plan->occ_asx, plan->acht_n1, plan->asx_n1, plan->stat_n1));
+    SIGMA_CUDA_TRY(launch_chained(half_reduce_total_kernel, kHalfTotalBlocks, 32, 0, s, true, plan->acht_n1,
+                                  plan->asx_n1, plan->stat_n1, plan->nb, plan->nvband,
+                                  reinterpret_cast<double2*>(achtemp), reinterpret_cast<double2*>(asxtemp),
+                                  stat ? reinterpret_cast<double2*>(achstemp) : nullptr,
+                                  reinterpret_cast<double2*>(acht_n1_loc)));
     return SIGMA_OK;
   }
   const bool stat = plan->ws.partial && achstemp;
@@ -1375,6 +1386,9 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
       SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact_occ, x, plan->counters + 2, plan->tu_occ, nullptr, s));
     wm.run_if = ws.run_if = flag = plan->exact.ex.flag;
   }
+  if (plan->exact_occ)
+    SIGMA_CUDA_TRY(launch_chained(half_occ_last_kernel, (plan->ng * kNW + 63) / 64, 64, 0, s, true, p, flag,
+                                  plan->occ_ach, plan->occ_asx));
   if (plan->nvband > 0) {
     half_occ_kernel<<<dim3(plan->ng, kNW), kThreads, 0, s>>>(p, plan->occ_ach, plan->occ_asx,
                                                              plan->exact_occ ? flag : nullptr);
@@ -1383,11 +1397,10 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
   if (plan->exact) {
     const int nf = plan->exact.nf;
     const double2* u = plan->tu + (size_t)plan->nb * nf;
-    half_tensor_rows_kernel<<<plan->nb, row_threads(plan->ng), 0, s>>>(
-        p, plan->tu, u, stat ? plan->tu + kNW : nullptr, u + kNW, nf, nf, flag,
-        plan->exact_occ ? plan->tu_occ : nullptr, plan->occ_ach, plan->occ_asx, plan->acht_n1, plan->asx_n1,
-        plan->stat_n1);
-    SIGMA_CUDA_TRY(cudaGetLastError());
+    SIGMA_CUDA_TRY(launch_chained(half_tensor_rows_kernel, plan->nb, row_threads(plan->ng), 0, s, true, p, plan->tu, u,
+                                  stat ? plan->tu + kNW : nullptr, u + kNW, nf, nf, flag,
+                                  plan->exact_occ ? plan->tu_occ : nullptr, plan->occ_ach, plan->occ_asx,
+                                  plan->acht_n1, plan->asx_n1, plan->stat_n1));
   }
   if (plan->wm.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<3>(p, wm, plan->main_grid, s));
   if (stat && plan->ws.n_items > 0) SIGMA_CUDA_TRY(launch_half_main<1>(p, ws, plan->stat_grid, s));
@@ -1408,12 +1421,11 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
   const int warps = plan->nb * kNW + plan->nvband * kNW + (stat ? plan->nb : 0);
   half_reduce_bands_kernel<<<(warps * 32 + 255) / 256, 256, 0, s>>>(a);
   SIGMA_CUDA_TRY(cudaGetLastError());
-  half_reduce_total_kernel<<<1, 256, 0, s>>>(plan->acht_n1, plan->asx_n1, plan->stat_n1, plan->nb,
-                                             plan->nvband, reinterpret_cast<double2*>(achtemp),
-                                             reinterpret_cast<double2*>(asxtemp),
-                                             stat ? reinterpret_cast<double2*>(achstemp) : nullptr,
-                                             reinterpret_cast<double2*>(acht_n1_loc));
-  SIGMA_CUDA_TRY(cudaGetLastError());
+  SIGMA_CUDA_TRY(launch_chained(half_reduce_total_kernel, kHalfTotalBlocks, 32, 0, s, true, plan->acht_n1,
+                                plan->asx_n1, plan->stat_n1, plan->nb, plan->nvband,
+                                reinterpret_cast<double2*>(achtemp), reinterpret_cast<double2*>(asxtemp),
+                                stat ? reinterpret_cast<double2*>(achstemp) : nullptr,
+                                reinterpret_cast<double2*>(acht_n1_loc)));
   return SIGMA_OK;
 }
 
