@@ -59,7 +59,7 @@ constexpr int kMaxTimedExecutions = 256;
 namespace sigma {
 
 void gpp_size_work(GppWork& w, int band_begin, int band_count, int bn, int bp, int nc, int ng,
-               int grid, int items_per_slot) {
+               int grid, int items_per_slot, int granule) {
   w.band_begin = band_begin;
   w.band_count = band_count;
   w.bn = bn;
@@ -76,8 +76,7 @@ void gpp_size_work(GppWork& w, int band_begin, int band_count, int bn, int bp, i
   long long s = (want + base - 1) / base;
   if (s < 1) s = 1;
   int len = (int)((nc + s - 1) / s);
-  len = (len + kCK - 1) / kCK * kCK;
-  if (len < kCK) len = kCK;
+  len = std::max(granule, (len + granule - 1) / granule * granule);
   w.split_len = len;
   w.n_splits = (nc + len - 1) / len;
   w.n_items = (int)(base * w.n_splits);
@@ -169,7 +168,10 @@ extern "C" int sigma_gpp_plan_create(sigma_gpp_plan* plan_out, int number_bands,
   p->ssx_grid = sms * (mixed ? ssx_blocks_per_sm_mixed() : ssx_blocks_per_sm_fp64());
   gpp_size_work(p->sch, 0, number_bands, kBN, mixed ? kBPM : kBP, ncouls, ngpown, p->sch_grid,
             mixed ? kItemsPerSlotMixed : kItemsPerSlot);
-  gpp_size_work(p->ssx, 0, nvband, kSsxBN, kSsxBP, ncouls, ngpown, p->ssx_grid, 2);
+  // FP64: short items, four per CTA (blocks of four bands and a remainder take
+  // very different times: 5 bands x 167 columns x 5003 in items of 64
+  // g-vectors 0.48 ms, 0.30 ms so)
+  gpp_size_work(p->ssx, 0, nvband, kSsxBN, kSsxBP, ncouls, ngpown, p->ssx_grid, mixed ? 2 : 4, mixed ? kCK : kSsxGran);
   if (p->sch.n_items < p->sch_grid) p->sch_grid = p->sch.n_items;
   if (p->ssx.n_items < p->ssx_grid) p->ssx_grid = p->ssx.n_items;
   if (!mixed) {

@@ -74,12 +74,6 @@ __device__ __forceinline__ int gx_rows_end(const ExactPrep& ex, int nf, int slab
   return (slab < nf ? ex.n_main_blocks : ex.n_row_blocks) * kExRows;
 }
 
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // The leading 24 bits of a double as FP32 (integer pipe).
 __device__ __forceinline__ float f32_lead(double x) { return ff_of(x).hi; }
 __device__ __forceinline__ bool any_bits(double2 v) {

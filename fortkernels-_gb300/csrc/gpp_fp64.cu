@@ -17,9 +17,8 @@
 // With per-band frequencies (this first pass) every term is formed in
 // float-float arithmetic (FP32 pairs on the FP32 pipe: G in FP64 per column
 // and g-vector, c = wx - Re wtilde in FP64 per term, the rest from exact
-// splits), its FP32 high half widened and added to an FP64 sum and its low
-// half to an FP32 sum of one staged chunk, added to the FP64 sum at the
-// chunk's end: ~3 FP64 operations per term instead of 10 (the FP64
+// splits) and added to a float-float sum of one staged chunk, added to an FP64
+// sum at the chunk's end: ~1 FP64 operation per term instead of 10 (the FP64
 // form had 8 per term plus 6 per band, column and g-vector).  A term's error
 // is about twice the FP64 form's, whose reciprocal is itself an FP32 seed
 // refined once (rcp_f64_seed32, within 2^-44.8).  conj(aqsm[n1][igp]), 0.5
@@ -36,29 +35,52 @@ namespace {
 
 constexpr int kPad = 1;
 
-// Staging of the per-band-frequency pass: per (g-vector, column) wtilde's
-// parts in FP64 (c = wx - Re wtilde is formed in FP64, and the rare FP64
-// decisions read them), Im wtilde and its square and G = I_eps wtilde as
-// float-float values, and flags (bit 0: the guard's second condition can
-// bind, bit 1: outside the float-float range, bit 2: no term); per
-// (g-vector, band) aqsn as a float-float pair and its range flag.
-// Each thread's FP64 sums (its 2 x 2 tile x 3 frequencies) live in shared
-// memory, one slot row per output; 16-g-vector chunks keep two CTAs' staging
-// and sums within an SM.
+// Staging of the per-band-frequency pass: per (g-vector, column) Re wtilde in
+// FP64 (c = wx - Re wtilde is formed in FP64), Im wtilde and its square and
+// G = I_eps wtilde as float-float values, and flags (bit 0: the guard's second
+// condition can bind, bit 1: outside the float-float range); per (g-vector,
+// pair of bands) aqsn as float-float values, the two bands' side by side, and
+// their range flags.  Each thread's FP64 sums (its 2 x 2 tile x 3 frequencies) live
+// in shared memory, one slot row per output; 16-g-vector chunks keep two CTAs'
+// staging and sums within an SM.
 constexpr int kCKB = 16;
 static_assert(kCK % kCKB == 0, "split lengths are multiples of the chunk");
 template <int BN, int BP>
 struct SchSmem {
   double2 acc[2 * 2 * kNW][kThreads];
   double a[kCKB][BP + kPad];
-  double b[kCKB][BP + kPad];
   float4 fb[kCKB][BP + kPad];  // (b.hi, b.lo, b^2.hi, b^2.lo)
   float4 fg[kCKB][BP + kPad];  // (G.x hi, lo, G.y hi, lo)
   unsigned flag[kCKB][BP + kPad];
-  float4 fn[kCKB][BN + kPad];  // (aqsn.x hi, lo, aqsn.y hi, lo)
-  unsigned nflag[kCKB][BN + kPad];
+  float4 nh[kCKB][BN / 2 + kPad], nl[kCKB][BN / 2 + kPad];  // aqsn.x of two bands, aqsn.y: high and low halves
+  unsigned nflag[kCKB][BN / 2 + kPad];                      // bit i: band i of the pair
 };
-constexpr unsigned kFlagBinds = 1u, kFlagWide = 2u, kFlagDead = 4u;
+constexpr unsigned kFlagBinds = 1u, kFlagWide = 2u;
+
+// Two values per instruction, differences as fma(b, -1, a).
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+__device__ __forceinline__ float2 f2_neg(float2 a) { return __fmul2_rn(a, f2(-1.f)); }
+__device__ __forceinline__ void two_sum_f2(float2 a, float2 b, float2& s, float2& e) {
+  s = __fadd2_rn(a, b);
+  const float2 bv = f2_sub(s, a), av = f2_sub(s, bv);
+  e = __fadd2_rn(f2_sub(a, av), f2_sub(b, bv));
+}
+__device__ __forceinline__ void two_diff_f2(float2 a, float2 b, float2& s, float2& e) {  // a - b
+  s = f2_sub(a, b);
+  const float2 bv = f2_sub(s, a), av = f2_sub(s, bv);
+  e = f2_sub(f2_sub(a, av), __fadd2_rn(b, bv));
+}
+// x y = -(hi) + lo: the rounded product negated, so that the exact error
+// takes one FMA; xm = -x.hi.
+struct NProd {
+  float2 nhi, lo;
+};
+__device__ __forceinline__ NProd nprod(float2 xh, float2 xl, float2 xm, float2 yh, float2 yl) {
+  const float2 n = __fmul2_rn(xm, yh);
+  return NProd{n, __ffma2_rn(xh, yl, __ffma2_rn(xl, yh, __ffma2_rn(xh, yh, n)))};
+}
+
 
 __device__ __forceinline__ double2 cmul(double2 x, double2 y) {
   return make_double2(fma(x.x, y.x, -__dmul_rn(x.y, y.y)), fma(x.x, y.y, __dmul_rn(x.y, y.x)));
@@ -78,8 +100,32 @@ static __device__ __noinline__ double2 sch_term_fp64(const double2* aqsn, const 
   return make_double2(fma(R.x, c, -__dmul_rn(b, R.y)) * r, fma(R.y, c, __dmul_rn(b, R.x)) * r);
 }
 
+// One term of the per-band-frequency pass in float-float arithmetic, scalar, for
+// chunks that hold elements outside the float-float range or with the guard's second
+// condition in reach.
+__device__ __forceinline__ void sch_term_ff(FF nx, FF ny, FF gx, FF gy, FF b, FF b2, double wx, double a, FF& sx,
+                                            FF& sy, bool& near, bool& keep) {
+  const FF rx = ff_dot2_raw(nx, gx, ny, gy), ry = ff_dot2_raw(nx, gy, ff_neg(ny), gx);
+  const FF c = ff_split_in_range(__dsub_rn(wx, a));
+  const FF wv = ff_sq_add(c, b2);
+  keep = ff_gt_quarter(wv, near);
+  const FF r = ff_rcp_raw(wv);
+  sx = ff_mul_raw(ff_dot2_raw(rx, c, ry, b), r);
+  sy = ff_mul_raw(ff_dot2_raw(rx, b, ff_neg(ry), c), r);
+}
+
 // One work item of the main pass.  Leaves the item's partial sums in
 // w.partial[pidx * BN * 3 + bl * 3 + iw].
+//
+// A thread's tile is two adjacent bands x two columns; the two bands' terms go
+// through each paired FP32 instruction together (no operand is rearranged for
+// it), R = aqsn G and R b once for the three frequencies.  About 85 FP32 lane
+// operations, 1 FP64 operation and ~15 integer ones a term; bound by latency
+// and the FP64 and FP32 pipes at 16 warps per SM (57 % and 51 %).  Warps without a band and
+// column halves without a column skip their terms.  133 x 167 x 5003: 1.66 ms, 2.46 ms
+// with scalar instructions, every padded term formed and the range tested per
+// term.  (|wdiff|^2 unnormalised under the reciprocal's seed: 1.58 ms, but errors 12 %
+// above the scalar form's, 1.1e-14.)
 template <int BN, int BP>
 __device__ __forceinline__ void sch_fp64_item(const GppDev& p, const GppWork& w, int item,
                                               unsigned char* smem_raw, int tid) {
@@ -94,54 +140,53 @@ __device__ __forceinline__ void sch_fp64_item(const GppDev& p, const GppWork& w,
   const int p0 = ic.cb * BP;
   const int ig_begin = ic.s * w.split_len;
   const int ig_end = min(ig_begin + w.split_len, p.nc);
+  const bool warp_on = n1_0 + 2 * ((tid & ~31) / TXN) < band_end;  // a band of this warp's exists
+  const int nj = p0 + TXN < p.ng ? 2 : 1;                          // column halves
 
   double wxr[2][kNW];
-  bool wx_wide[2];
+  bool wx_wide = false;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const int n1 = n1_0 + ty + TYN * i;
-    wx_wide[i] = false;
+    const int n1 = n1_0 + 2 * ty + i;
 #pragma unroll
     for (int iw = 0; iw < kNW; ++iw) {
       wxr[i][iw] = n1 < band_end ? p.wx[(size_t)n1 * p.wx_stride + iw] : 1.0;
-      wx_wide[i] = wx_wide[i] || !ff_freq_range(wxr[i][iw]);
+      wx_wide = wx_wide || !ff_freq_range(wxr[i][iw]);
     }
   }
-  // float-float sums in registers (lanes: real and imaginary parts): each
-  // term's high pair added exactly (TwoSum) to the high pair, the errors and
-  // low halves to the low pair; after each chunk the pair renormalised
-  // (Fast2Sum), its high pair added to the FP64 sums in shared memory and
-  // its low pair carried on (an FP32 sum over a whole item's thousands of
+  const bool item_wide = __syncthreads_or(wx_wide);
+  // negated float-float sums in registers (lanes: the two bands): each
+  // term's high half added exactly (TwoSum) to the high part, the errors and
+  // low halves to the low part; after each chunk the pair renormalised
+  // (Fast2Sum), its high part added to the FP64 sums in shared memory and
+  // its low part carried on (an FP32 sum over a whole item's thousands of
   // terms would lose ~n 2^-47 of the output)
-  const float2 m1 = make_float2(-1.f, -1.f);
-  float2 ach[2][2][kNW], acl[2][2][kNW];
+  float2 ach[2][kNW][2], acl[2][kNW][2];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int iw = 0; iw < kNW; ++iw) {
-        sm.acc[(i * 2 + j) * kNW + iw][tid] = make_double2(0.0, 0.0);
-        ach[i][j][iw] = make_float2(0.f, 0.f);
-        acl[i][j][iw] = make_float2(0.f, 0.f);
-      }
+    for (int iw = 0; iw < kNW; ++iw) {
+      sm.acc[j * kNW + iw][tid] = sm.acc[(2 + j) * kNW + iw][tid] = make_double2(0.0, 0.0);
+      ach[j][iw][0] = ach[j][iw][1] = f2(0.f);
+      acl[j][iw][0] = acl[j][iw][1] = f2(0.f);
+    }
 
   for (int ig0 = ig_begin; ig0 < ig_end; ig0 += kCKB) {
     __syncthreads();
+    bool special = item_wide;  // a value of this chunk outside the fast terms' range
     for (int e = tid; e < kCKB * BP; e += kThreads) {
       const int k = e % kCKB, pl = e / kCKB;
       const int ig = ig0 + k, my_igp = p0 + pl;
-      double a = 0.0, b = 0.0;
+      double a = 0.0;
       float4 fb = make_float4(0.f, 0.f, 0.f, 0.f), fg = fb;
-      unsigned flag = kFlagDead;
+      unsigned flag = 0u;  // elements past the end: G = 0
       if (ig < ig_end && my_igp < p.ng) {
         const size_t off = (size_t)my_igp * p.nc + ig;
         const double2 wt = p.wt[off];
         const double2 ie = p.ieps[off];
         const double2 g = cmul(ie, wt);
         a = wt.x;
-        b = wt.y;
-        const FF f = ff_of_rn(b), f2 = ff_mul_raw(f, f), gx = ff_of_rn(g.x), gy = ff_of_rn(g.y);
+        const FF f = ff_of_rn(wt.y), f2 = ff_mul_raw(f, f), gx = ff_of_rn(g.x), gy = ff_of_rn(g.y);
         fb = make_float4(f.hi, f.lo, f2.hi, f2.lo);
         fg = make_float4(gx.hi, gx.lo, gy.hi, gy.lo);
         const float ah = ff_of_rn(a).hi;
@@ -150,114 +195,186 @@ __device__ __forceinline__ void sch_fp64_item(const GppDev& p, const GppWork& w,
                (ff_range(wt.x, wt.y) && ff_range(ie.x, ie.y) ? 0u : kFlagWide);
       }
       sm.a[k][pl] = a;
-      sm.b[k][pl] = b;
       sm.fb[k][pl] = fb;
       sm.fg[k][pl] = fg;
       sm.flag[k][pl] = flag;
+      special = special || flag;
     }
-    for (int e = tid; e < kCKB * BN; e += kThreads) {
-      const int k = e % kCKB, bl = e / kCKB;
-      const int ig = ig0 + k, n1 = n1_0 + bl;
-      double2 v = make_double2(0.0, 0.0);
-      if (ig < ig_end && n1 < band_end) v = p.aqsn[(size_t)n1 * p.nc + ig];
-      const FF nx = ff_of_rn(v.x), ny = ff_of_rn(v.y);
-      sm.fn[k][bl] = make_float4(nx.hi, nx.lo, ny.hi, ny.lo);
-      sm.nflag[k][bl] = ff_range(v.x, v.y) ? 0u : kFlagWide;
-    }
-    __syncthreads();
-
-#pragma unroll 1
-    for (int k = 0; k < kCKB; ++k) {
-      double a[2], b[2];
-      FF fb[2], fb2[2], gx[2], gy[2], nx[2], ny[2];
-      unsigned flag[2], nflag[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int pl = tx + TXN * j;
-        a[j] = sm.a[k][pl];
-        b[j] = sm.b[k][pl];
-        const float4 v = sm.fb[k][pl], g = sm.fg[k][pl];
-        fb[j] = FF{v.x, v.y};
-        fb2[j] = FF{v.z, v.w};
-        gx[j] = FF{g.x, g.y};
-        gy[j] = FF{g.z, g.w};
-        flag[j] = sm.flag[k][pl];
-      }
+    for (int e = tid; e < kCKB * TYN; e += kThreads) {
+      const int k = e % kCKB, bp = e / kCKB;
+      const int ig = ig0 + k, n1 = n1_0 + 2 * bp;
+      double2 v[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+      unsigned flag = 0u;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float4 v = sm.fn[k][ty + TYN * i];
-        nx[i] = FF{v.x, v.y};
-        ny[i] = FF{v.z, v.w};
-        nflag[i] = sm.nflag[k][ty + TYN * i];
+        if (ig < ig_end && n1 + i < band_end) v[i] = p.aqsn[(size_t)(n1 + i) * p.nc + ig];
+        flag |= ff_range(v[i].x, v[i].y) ? 0u : 1u << i;
       }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
+      const FF x0 = ff_of_rn(v[0].x), x1 = ff_of_rn(v[1].x), y0 = ff_of_rn(v[0].y), y1 = ff_of_rn(v[1].y);
+      sm.nh[k][bp] = make_float4(x0.hi, x1.hi, y0.hi, y1.hi);
+      sm.nl[k][bp] = make_float4(x0.lo, x1.lo, y0.lo, y1.lo);
+      sm.nflag[k][bp] = flag;
+      special = special || flag;
+    }
+    special = __syncthreads_or(special);
+    if (!warp_on) continue;
+
+    if (!special) {
+#pragma unroll 1
+      for (int k = 0; k < kCKB; ++k) {
+        const float4 nh = sm.nh[k][ty], nl = sm.nl[k][ty];
+        const float2 nxh = f4_lo(nh), nyh = f4_hi(nh), nxl = f4_lo(nl), nyl = f4_hi(nl);
+        const float2 nxm = f2_neg(nxh), nym = f2_neg(nyh);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          // R = aqsn G, then per frequency (R (c + i b)) / |wdiff|^2
-          const FF rx = ff_dot2_raw(nx[i], gx[j], ny[i], gy[j]);
-          const FF ry = ff_dot2_raw(nx[i], gy[j], ff_neg(ny[i]), gx[j]);
-          const bool wide = (flag[j] & kFlagWide) || nflag[i] || wx_wide[i];
-          const bool any_wide = __any_sync(0xffffffffu, wide);
+          if (j >= nj) continue;
+          const int pl = tx + TXN * j;
+          const double a = sm.a[k][pl];
+          const float4 vb = sm.fb[k][pl], vg = sm.fg[k][pl];
+          const float2 gxh = f2(vg.x), gxl = f2(vg.y), gyh = f2(vg.z), gyl = f2(vg.w);
+          const float2 bh = f2(vb.x), bl = f2(vb.y), b2h = f2(vb.z), b2l = f2(vb.w);
+          // N = -R, R = aqsn G
+          float2 nrxh, nrxl, nryh, nryl;
+          {
+            const NProd u = nprod(nxh, nxl, nxm, gxh, gxl), v = nprod(nyh, nyl, nym, gyh, gyl);
+            two_diff_f2(u.nhi, v.nhi, nrxh, nrxl);
+            nrxl = __fadd2_rn(f2_sub(nrxl, u.lo), v.lo);
+          }
+          {
+            const NProd u = nprod(nxh, nxl, nxm, gyh, gyl), v = nprod(nyh, nyl, nym, gxh, gxl);
+            two_sum_f2(u.nhi, v.nhi, nryh, nryl);
+            nryl = f2_sub(nryl, __fadd2_rn(u.lo, v.lo));
+          }
+          const float2 bm = f2(-vb.x);
+          const NProd rxb = nprod(bh, bl, bm, nrxh, nrxl);  // b N.x: R.x b = nhi - lo
+          const NProd ryb = nprod(bh, bl, bm, nryh, nryl);
 #pragma unroll
           for (int iw = 0; iw < kNW; ++iw) {
-            const FF c = ff_of_rn(__dsub_rn(wxr[i][iw], a[j]));  // wx - Re wtilde in FP64
-            const FF wv = ff_sq_add(c, fb2[j]);               // |wdiff|^2
-            bool near;
-            bool keep = ff_gt_quarter(wv, near);
-            if (near || (flag[j] & kFlagBinds)) keep = keep_fp64(wxr[i][iw], a[j], b[j]);
-            keep = keep && !(flag[j] & kFlagDead);
-            const FF r = ff_rcp_raw(wv);
-            const FF ux = ff_dot2_raw(rx, c, ry, fb[j]), uy = ff_dot2_raw(rx, fb[j], ff_neg(ry), c);
-            const FF sx = ff_mul_raw(ux, r), sy = ff_mul_raw(uy, r);
-            if (any_wide && wide) {
-              if (!(flag[j] & kFlagDead)) {
-                const int n1 = n1_0 + ty + TYN * i, ig = ig0 + k, my_igp = p0 + tx + TXN * j;
-                const double2 s = sch_term_fp64(p.aqsn, p.wt, p.ieps,
-                                                n1 < band_end ? (size_t)n1 * p.nc + ig : ~size_t(0),
-                                                (size_t)my_igp * p.nc + ig, wxr[i][iw]);
-                double2& a = sm.acc[(i * 2 + j) * kNW + iw][tid];
-                a.x += s.x;
-                a.y += s.y;
-              }
-            } else {
-              const float2 hv = keep ? make_float2(sx.hi, sy.hi) : make_float2(0.f, 0.f);
-              const float2 lv = keep ? make_float2(sx.lo, sy.lo) : make_float2(0.f, 0.f);
-              float2& h = ach[i][j][iw];
-              const float2 hs = __fadd2_rn(h, hv);
-              const float2 hb = __ffma2_rn(h, m1, hs);
-              const float2 ha = __ffma2_rn(hb, m1, hs);
-              const float2 he = __fadd2_rn(__ffma2_rn(ha, m1, h), __ffma2_rn(hb, m1, hv));
-              h = hs;
-              acl[i][j][iw] = __fadd2_rn(acl[i][j][iw], __fadd2_rn(he, lv));
+            const FF c0 = ff_split_in_range(__dsub_rn(wxr[0][iw], a));  // wx - Re wtilde in FP64
+            const FF c1 = ff_split_in_range(__dsub_rn(wxr[1][iw], a));
+            const float2 ch = make_float2(c0.hi, c1.hi), cl = make_float2(c0.lo, c1.lo), cm = f2_neg(ch);
+            // |wdiff|^2 = c^2 + b^2
+            const float2 q = __fmul2_rn(ch, cm);  // -c^2
+            float2 wh, wl;
+            two_diff_f2(b2h, q, wh, wl);
+            wl = __fadd2_rn(__fadd2_rn(wl, b2l), __ffma2_rn(__fadd2_rn(ch, ch), cl, __ffma2_rn(ch, ch, q)));
+            {
+              const float2 h = __fadd2_rn(wh, wl);
+              wl = __fadd2_rn(f2_sub(wh, h), wl);
+              wh = h;
+            }
+            const float2 full = __fadd2_rn(__fadd2_rn(wh, f2(-0.25f)), wl);  // against the guard's 0.25
+            bool k0 = full.x > 0.f, k1 = full.y > 0.f;
+            if (fminf(fabsf(full.x), fabsf(full.y)) <= 2.3283064e-10f) {  // 2^-32: decided in FP64
+              const bool in = p0 + pl < p.ng && ig0 + k < ig_end;
+              const double b = in ? p.wt[(size_t)(p0 + pl) * p.nc + ig0 + k].y : 0.0;
+              k0 = keep_fp64(wxr[0][iw], a, b);
+              k1 = keep_fp64(wxr[1][iw], a, b);
+            }
+            // 1 / |wdiff|^2 (0 for a dropped term): the rounded FP32 reciprocal
+            // and one float-float correction
+            const float2 r0 = make_float2(k0 ? rcp_f32(wh.x) : 0.f, k1 ? rcp_f32(wh.y) : 0.f), rn = f2_neg(r0);
+            const float2 t = __ffma2_rn(wl, r0, __ffma2_rn(wh, r0, f2(-1.f)));  // w r0 - 1
+            const float2 rl = __fmul2_rn(rn, t);
+            // u = R (c + i b)
+            float2 uh[2], ul[2];
+            {
+              const NProd x = nprod(ch, cl, cm, nrxh, nrxl);  // R.x c = nhi - lo
+              two_diff_f2(x.nhi, ryb.nhi, uh[0], ul[0]);
+              ul[0] = f2_sub(__fadd2_rn(ul[0], ryb.lo), x.lo);
+            }
+            {
+              const NProd x = nprod(ch, cl, cm, nryh, nryl);  // R.y c
+              two_sum_f2(x.nhi, rxb.nhi, uh[1], ul[1]);
+              ul[1] = f2_sub(ul[1], __fadd2_rn(x.lo, rxb.lo));
+            }
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+              const float2 n = __fmul2_rn(uh[d], rn);
+              const float2 lo = __ffma2_rn(uh[d], rl, __ffma2_rn(ul[d], r0, __ffma2_rn(uh[d], r0, n)));
+              float2 s, e;
+              two_sum_f2(ach[j][iw][d], n, s, e);
+              ach[j][iw][d] = s;
+              acl[j][iw][d] = __fadd2_rn(acl[j][iw][d], f2_sub(e, lo));
             }
           }
         }
-    }
+      }
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < kCKB; ++k) {
+        const float4 nh = sm.nh[k][ty], nl = sm.nl[k][ty];
+        const unsigned nflag = sm.nflag[k][ty];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j) {
+          const int pl = tx + TXN * j, my_igp = p0 + pl, ig = ig0 + k;
+          const bool dead = ig >= ig_end || my_igp >= p.ng;
+          const double a = sm.a[k][pl];
+          const float4 vb = sm.fb[k][pl], vg = sm.fg[k][pl];
+          const unsigned flag = sm.flag[k][pl];
+          const size_t off = (size_t)my_igp * p.nc + ig;
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+          for (int i = 0; i < 2; ++i) {
+            const int n1 = n1_0 + 2 * ty + i;
+            const bool wide = item_wide || (flag & kFlagWide) || ((nflag >> i) & 1u);
+            const FF nx = i ? FF{nh.y, nl.y} : FF{nh.x, nl.x}, ny = i ? FF{nh.w, nl.w} : FF{nh.z, nl.z};
 #pragma unroll
-        for (int iw = 0; iw < kNW; ++iw) {
-          const float2 s = __fadd2_rn(ach[i][j][iw], acl[i][j][iw]);
-          acl[i][j][iw] = __ffma2_rn(__ffma2_rn(ach[i][j][iw], m1, s), m1, acl[i][j][iw]);
-          ach[i][j][iw] = make_float2(0.f, 0.f);
-          double2& a = sm.acc[(i * 2 + j) * kNW + iw][tid];
-          a.x += f32_widen(s.x);
-          a.y += f32_widen(s.y);
+            for (int iw = 0; iw < kNW; ++iw) {
+              if (dead) continue;
+              if (wide) {
+                const double2 s = sch_term_fp64(p.aqsn, p.wt, p.ieps, n1 < band_end ? (size_t)n1 * p.nc + ig : ~size_t(0),
+                                                off, wxr[i][iw]);
+                double2& d = sm.acc[(i * 2 + j) * kNW + iw][tid];
+                d.x += s.x;
+                d.y += s.y;
+                continue;
+              }
+              FF s[2];
+              bool near, keep;
+              sch_term_ff(nx, ny, FF{vg.x, vg.y}, FF{vg.z, vg.w}, FF{vb.x, vb.y}, FF{vb.z, vb.w}, wxr[i][iw], a, s[0],
+                          s[1], near, keep);
+              if (near || (flag & kFlagBinds)) keep = keep_fp64(wxr[i][iw], a, p.wt[off].y);
+#pragma unroll
+              for (int d = 0; d < 2; ++d) {
+                float& h = i ? ach[j][iw][d].y : ach[j][iw][d].x;
+                float& l = i ? acl[j][iw][d].y : acl[j][iw][d].x;
+                float t, e;
+                two_sum_f(h, keep ? -s[d].hi : 0.f, t, e);
+                h = t;
+                l += e - (keep ? s[d].lo : 0.f);
+              }
+            }
+          }
         }
-  }
-  double2 acc[2][2][kNW];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int iw = 0; iw < kNW; ++iw) {
-        const double2 a = sm.acc[(i * 2 + j) * kNW + iw][tid];
-        acc[i][j][iw] = make_double2(a.x + f32_widen(acl[i][j][iw].x), a.y + f32_widen(acl[i][j][iw].y));
+        float2 s[2];
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          s[d] = __fadd2_rn(ach[j][iw][d], acl[j][iw][d]);
+          acl[j][iw][d] = __fadd2_rn(f2_sub(ach[j][iw][d], s[d]), acl[j][iw][d]);
+          ach[j][iw][d] = f2(0.f);
+        }
+        double2 &x = sm.acc[j * kNW + iw][tid], &y = sm.acc[(2 + j) * kNW + iw][tid];
+        x.x -= f32_widen(s[0].x);
+        x.y -= f32_widen(s[1].x);
+        y.x -= f32_widen(s[0].y);
+        y.y -= f32_widen(s[1].y);
       }
+  }
+  double2 acc[2][2][kNW];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int iw = 0; iw < kNW; ++iw) {
+      const double2 x = sm.acc[j * kNW + iw][tid], y = sm.acc[(2 + j) * kNW + iw][tid];
+      acc[0][j][iw] = make_double2(x.x - f32_widen(acl[j][iw][0].x), x.y - f32_widen(acl[j][iw][1].x));
+      acc[1][j][iw] = make_double2(y.x - f32_widen(acl[j][iw][0].y), y.y - f32_widen(acl[j][iw][1].y));
+    }
 
   // epilogue: x conj(aqsm[n1][igp]) * 0.5 * vcoul[igp], then a fixed-order
   // sum over the tile's columns
@@ -267,7 +384,7 @@ __device__ __forceinline__ void sch_fp64_item(const GppDev& p, const GppWork& w,
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const int bl = ty + TYN * i, pl = tx + TXN * j;
+      const int bl = 2 * ty + i, pl = tx + TXN * j;
       const int n1 = n1_0 + bl, my_igp = p0 + pl;
       const int igp = my_igp < p.ng ? p.igp_of[my_igp] : -1;
       if (n1 < band_end && igp >= 0) {
@@ -792,7 +909,7 @@ __global__ void __launch_bounds__(kThreads, kSmall ? 2 : 1) sch_fp64y_batch_kern
 // and each term's high halves are added in FP64 one at a time.  Chunks
 // holding a value outside the float-float range take FP64 factors and FP64
 // multiply-adds.
-constexpr int kSsxCK = 8;      // g-vectors per staged chunk
+constexpr int kSsxCK = kSsxGran;  // g-vectors per staged chunk
 
 struct SsxSmem {  // column rows padded by one element (see SchYSmem)
   double a[kSsxCK][kSsxBP + 1];
@@ -909,10 +1026,11 @@ __device__ __forceinline__ void ssx_fp64_item(const GppDev& p, const GppWork& w,
     }
     chunk_wide = __syncthreads_or(chunk_wide);
 
+    const bool no_column = p0 + (tid & ~31) >= p.ng;  // the whole warp's
     if (!chunk_wide && p.wx_stride != 0) {
       // per-band frequencies: each band's float-float factor and term; the
       // term's high halves added in FP64
-      for (int k = 0; k < kSsxCK; ++k) {
+      for (int k = no_column ? kSsxCK : 0; k < kSsxCK; ++k) {
         const double a = sm.a[k][tid], b = sm.b[k][tid];
         const double2 ie = sm.ie[k][tid];
         const double b2 = guard_b2(b);
@@ -954,7 +1072,7 @@ __device__ __forceinline__ void ssx_fp64_item(const GppDev& p, const GppWork& w,
       // by the item's bands; each term a float-float product, the high
       // halves of two g-vectors' terms added exactly and then in FP64
       static_assert(kSsxCK % 2 == 0, "g-vector pairs");
-      for (int k = 0; k < kSsxCK; k += 2) {
+      for (int k = no_column ? kSsxCK : 0; k < kSsxCK; k += 2) {
         float4 sv[2][kNW];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

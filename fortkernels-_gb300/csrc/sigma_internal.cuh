@@ -94,6 +94,7 @@ constexpr int kThreads = 256;
 constexpr int kBNY = 64;   // bands per FP64 item when the frequencies are shared
 constexpr int kBPY = 16;   // columns per FP64 item when the frequencies are shared
 constexpr int kSsxBN = 4;   // bands per occupied-band item
+constexpr int kSsxGran = 8; // g-vectors per staged chunk of the FP64 occupied-band pass
 constexpr int kSsxBP = 256; // columns per occupied-band item, one per thread
 
 // The pre-pass work of the tensor form: only the occupied bands' FP32 rows
@@ -148,7 +149,7 @@ struct MixedPrep {
 // Sizes a pass: band blocks of bn, column blocks of bp, g-vector splits so
 // that the grid gets about items_per_slot items per resident CTA.
 void gpp_size_work(GppWork& w, int band_begin, int band_count, int bn, int bp, int nc, int ng,
-                   int grid, int items_per_slot);
+                   int grid, int items_per_slot, int granule = kCK);
 // Column map of BGW-Kernels/gppKer.cpp:322-328 (-1 marks a skipped column);
 // SIGMA_ERR_INDEX_RANGE where the reference would read out of bounds.
 int gpp_map_columns(int nc, int ng, const int* inv, const int* indinv, int indinv_len,
@@ -255,6 +256,12 @@ __device__ __forceinline__ double rcp_f64_seed32(double w) {
   return fma(r0, eps, r0);
 }
 
+// The FP32 reciprocal's seed (relative error about 2^-23).
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ float rcp_f32(float w) {
   // rcp.approx.f32 plus one Newton-Raphson step r = r0 (2 - w r0).
   float r0;
