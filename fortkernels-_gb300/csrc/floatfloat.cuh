@@ -200,6 +200,64 @@ __device__ __forceinline__ void ff_add2(float2& hi, float2& lo, float2 x, float2
   lo = __ffma2_rn(__ffma2_rn(s, m1, hi), m1, e);  // e - (hi - s)
 }
 
+// Two values per instruction, differences as fma(b, -1, a).
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+__device__ __forceinline__ float2 f2_neg(float2 a) { return __fmul2_rn(a, f2(-1.f)); }
+__device__ __forceinline__ void two_sum_f2(float2 a, float2 b, float2& s, float2& e) {
+  s = __fadd2_rn(a, b);
+  const float2 bv = f2_sub(s, a), av = f2_sub(s, bv);
+  e = __fadd2_rn(f2_sub(a, av), f2_sub(b, bv));
+}
+__device__ __forceinline__ void two_diff_f2(float2 a, float2 b, float2& s, float2& e) {  // a - b
+  s = f2_sub(a, b);
+  const float2 bv = f2_sub(s, a), av = f2_sub(s, bv);
+  e = f2_sub(f2_sub(a, av), __fadd2_rn(b, bv));
+}
+// Float-float values of two elements, with the roundings of the scalar
+// functions of the same name (a product's error takes the negated product as
+// its FMA's addend, one more product instead of a negation per lane).
+struct FF2 {
+  float2 hi, lo;
+};
+__device__ __forceinline__ FF2 ff2(FF a, FF b) { return FF2{make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)}; }
+__device__ __forceinline__ FF2 ff2_neg(FF2 x) { return FF2{f2_neg(x.hi), f2_neg(x.lo)}; }
+__device__ __forceinline__ FF2 ff2_norm(float2 s, float2 e) {
+  const float2 h = __fadd2_rn(s, e);
+  return FF2{h, f2_sub(e, f2_sub(h, s))};
+}
+__device__ __forceinline__ FF2 ff2_sub_raw(FF2 x, FF2 y) {
+  float2 s, e;
+  two_diff_f2(x.hi, y.hi, s, e);
+  return FF2{s, __fadd2_rn(e, f2_sub(x.lo, y.lo))};
+}
+__device__ __forceinline__ FF2 ff2_sq_add(FF2 c, FF2 b2) {
+  const float2 n = __fmul2_rn(c.hi, f2_neg(c.hi));
+  const float2 e = __ffma2_rn(__fadd2_rn(c.hi, c.hi), c.lo, __ffma2_rn(c.hi, c.hi, n));
+  float2 s, t;
+  two_diff_f2(b2.hi, n, s, t);
+  return ff2_norm(s, __fadd2_rn(t, __fadd2_rn(e, b2.lo)));
+}
+__device__ __forceinline__ FF2 ff2_mul_raw(FF2 x, FF2 y) {
+  const float2 n = __fmul2_rn(f2_neg(x.hi), y.hi);
+  return FF2{f2_neg(n), __ffma2_rn(x.hi, y.lo, __ffma2_rn(x.lo, y.hi, __ffma2_rn(x.hi, y.hi, n)))};
+}
+// a g - b h; am, bm the negated high halves of a and b
+__device__ __forceinline__ FF2 ff2_dot2_raw(FF2 a, float2 am, FF2 g, FF2 b, float2 bm, FF2 h) {
+  const float2 n1 = __fmul2_rn(am, g.hi), n2 = __fmul2_rn(bm, h.hi);
+  const float2 e1 = __ffma2_rn(a.hi, g.hi, n1), e2 = __ffma2_rn(b.hi, h.hi, n2);
+  const float2 t = f2_sub(__ffma2_rn(a.hi, g.lo, __ffma2_rn(a.lo, g.hi, e1)),
+                          __ffma2_rn(b.hi, h.lo, __ffma2_rn(b.lo, h.hi, e2)));
+  float2 s, e;
+  two_diff_f2(n2, n1, s, e);
+  return FF2{s, __fadd2_rn(e, t)};
+}
+__device__ __forceinline__ FF2 ff2_rcp_raw(FF2 x) {
+  const float2 r = make_float2(rcp_f32(x.hi.x), rcp_f32(x.hi.y));
+  const float2 t = __ffma2_rn(x.lo, r, __ffma2_rn(x.hi, r, f2(-1.f)));
+  return FF2{r, __fmul2_rn(f2_neg(r), t)};
+}
+
 // An FP32 value as a double, on the integer pipe (exponent rebiased,
 // mantissa shifted): exact for normal values and zero; FP32 subnormals (below
 // 1.2e-38) give zero.  cvt.f64.f32 would take the FP64 pipe, GB300's

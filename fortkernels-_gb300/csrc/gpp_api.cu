@@ -426,7 +426,7 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
     j.d.aqsm = p.aqsm;
     j.d.vcoul = vcoul;
     j.d.vfac = 0.5;
-    SIGMA_CUDA_TRY(launch_factor_pass(j, plan->fac_grid, s));
+    SIGMA_CUDA_TRY(launch_factor_pass(j, plan->fac_grid, plan->counters, s));
     const int st = ff_execute_weighted(plan->ff, nullptr, aqsntemp, aqsmtemp, vcoul, 0.5,
                                        reinterpret_cast<sigma_complex128*>(plan->acht_n1), stream, nullptr,
                                        true, nullptr, 1.0, nullptr, true);

@@ -656,7 +656,7 @@ extern "C" int sigma_gpp_batch_execute(sigma_gpp_batch b, void* stream) {
     // B slices and epilogue factors, the GEMM over the group's item table,
     // its reduction
     // the factor pass writes every operand of the contractions
-    SIGMA_CUDA_TRY(launch_factor_pass(b->d_fac, b->n, b->fac_total, b->fac_grid, b->fac_nvband, s));
+    SIGMA_CUDA_TRY(launch_factor_pass(b->d_fac, b->n, b->fac_total, b->fac_grid, b->fac_nvband, b->counters, s));
     SIGMA_CUDA_TRY(launch_ozaki_group_gemm(b->grp, device_sm_count(), s));
     SIGMA_CUDA_TRY(launch_ozaki_group_reduce(b->grp, s));
     SIGMA_CUDA_TRY(launch_gpp_reduce_group(b->d_red, b->n, b->red_warps, b->red_count, s));

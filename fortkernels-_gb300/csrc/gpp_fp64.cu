@@ -57,20 +57,6 @@ struct SchSmem {
 };
 constexpr unsigned kFlagBinds = 1u, kFlagWide = 2u;
 
-// Two values per instruction, differences as fma(b, -1, a).
-__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
-__device__ __forceinline__ float2 f2_neg(float2 a) { return __fmul2_rn(a, f2(-1.f)); }
-__device__ __forceinline__ void two_sum_f2(float2 a, float2 b, float2& s, float2& e) {
-  s = __fadd2_rn(a, b);
-  const float2 bv = f2_sub(s, a), av = f2_sub(s, bv);
-  e = __fadd2_rn(f2_sub(a, av), f2_sub(b, bv));
-}
-__device__ __forceinline__ void two_diff_f2(float2 a, float2 b, float2& s, float2& e) {  // a - b
-  s = f2_sub(a, b);
-  const float2 bv = f2_sub(s, a), av = f2_sub(s, bv);
-  e = f2_sub(f2_sub(a, av), __fadd2_rn(b, bv));
-}
 // x y = -(hi) + lo: the rounded product negated, so that the exact error
 // takes one FMA; xm = -x.hi.
 struct NProd {

@@ -28,10 +28,18 @@
 // and summed over the item's columns in a fixed order.  The inputs are read
 // once for both, and no intermediate operand is written.
 //
-// Items are (g-vector segment, column block of 16 columns), plus, per
+// Items are (g-vector segment, column block of 8 columns), plus, per
 // instance, a few items that zero the A slices' padding rows; a batch
-// concatenates the items of every instance (one static schedule).
+// concatenates the items of every instance; the CTAs take them from a counter.
+//
+// A warp's two columns share each paired FP32 instruction (same roundings as
+// one at a time).  Bound by latency between the tile's barriers at five CTAs of
+// 128 threads (53 % of issue slots, FMA and integer pipes 40 and 37 %): 1.43 ms
+// at 1638 columns x 32768 with two occupied bands and 6.48 ms for a batch of
+// twelve, 1.54 and 7.76 ms with one column per instruction, 256 threads over 16 columns,
+// fixed items and no prefetch.  Four CTAs without spills 1.56 ms, six 1.52 ms.
 #include <algorithm>
+#include <cmath>
 
 #include "gpp_tensor.cuh"
 #include "floatfloat.cuh"
@@ -39,7 +47,9 @@
 namespace sigma {
 namespace {
 
-constexpr int kFacThreads = 256;
+constexpr int kFacThreads = 128;
+constexpr int kFacWarps = kFacThreads / 32, kFacPerSm = 5;
+static_assert(kFacCols == 2 * kFacWarps, "two columns per warp");
 constexpr int kZeroTiles = 64;  // K tiles per padding-row item
 
 // Slot of g-vector k in the ssx planes: the middle two of every four are
@@ -78,7 +88,7 @@ __host__ __device__ constexpr size_t factor_acc_bytes(int nvband) {
 // ssx sums: output o = r * 64 + 8 * warp + lane / 4 is computed by the four
 // lanes 4 (lane / 4) + q (q = 0..3, 8 g-vectors each) in round r, so every
 // warp takes part; each lane owns the accumulator acc[4 o + q]
-constexpr int kSsxRounds = (kFusedBands * kNW * kFacCols * 4 + 255) / 256;
+constexpr int kSsxRounds = (kFusedBands * kNW * kFacCols * 4 + kFacThreads - 1) / kFacThreads;
 
 __device__ __forceinline__ int find_job(const FactorJob* jobs, int n, int item) {
   int lo = 0, hi = n - 1;
@@ -104,29 +114,26 @@ __device__ __forceinline__ void put_a(unsigned char* a_tiles, int kt, int R, int
   oz_put_row_chunk(base + (size_t)(kt + t) * kOzOperandBytes, r, ch, im);
 }
 
-// (w g - se) r rounded once to FP32, for an FP32-exact w (w.lo == 0): w g
-// as an exact product pair, the difference by TwoSum, no normalisation
-// before the final rounding (same accuracy as the general form).
-__device__ __forceinline__ float ff_factor_round(float w, FF g, FF se, FF r) {
-  const float p = w * g.hi;
-  const float e = fmaf(w, g.lo, fmaf(w, g.hi, -p));
-  float s, t;
-  two_sum_f(p, -se.hi, s, t);
-  t += e - se.lo;
-  return fmaf(s, r.hi, fmaf(s, r.lo, t * r.hi));
-}
-
-// a g - b h of float-float values rounded once to FP32: the products' exact
-// errors by FMA, the difference of the hi products by TwoSum, so the result
-// is within 1/2 ulp plus ~2^-46 of the products' magnitude (lo * lo terms
-// dropped).
-__device__ __forceinline__ float ff_dot2_round(FF a, FF g, FF b, FF h) {
-  const float p1 = a.hi * g.hi, p2 = b.hi * h.hi;
-  const float e1 = fmaf(a.hi, g.hi, -p1), e2 = fmaf(b.hi, h.hi, -p2);
-  const float t = fmaf(a.hi, g.lo, fmaf(a.lo, g.hi, e1)) - fmaf(b.hi, h.lo, fmaf(b.lo, h.hi, e2));
-  float s, es;
-  two_sum_f(p1, -p2, s, es);  // the difference exact: one rounding at the end
-  return s + (es + t);
+// (w g - se) r of two elements, rounded once to FP32.  For an FP32-exact w
+// (w.lo == 0) w g is an exact product pair, the difference by TwoSum, with no
+// normalisation before the final rounding (same accuracy as the general form).
+__device__ __forceinline__ float2 factor_round(bool w32, FF w, FF2 g, FF2 se, FF2 r) {
+  const float2 wh = f2(w.hi), n = __fmul2_rn(f2(-w.hi), g.hi);
+  float2 s, t;
+  if (w32) {
+    const float2 e = __ffma2_rn(wh, g.lo, __ffma2_rn(wh, g.hi, n));
+    two_sum_f2(n, se.hi, s, t);  // -(w g - se)
+    t = f2_sub(t, f2_sub(e, se.lo));
+  } else {
+    float2 e = __ffma2_rn(wh, g.hi, n);
+    e = __ffma2_rn(wh, g.lo, __ffma2_rn(f2(w.lo), g.hi, e));
+    const FF2 p = ff2_norm(f2_neg(n), e);
+    two_diff_f2(se.hi, p.hi, s, t);
+    const FF2 d = ff2_norm(s, __fadd2_rn(t, f2_sub(se.lo, p.lo)));
+    s = d.hi;
+    t = d.lo;
+  }
+  return f2_neg(__ffma2_rn(s, r.hi, __ffma2_rn(s, r.lo, __fmul2_rn(t, r.hi))));
 }
 
 // Decisions of one element that the fast path leaves open, out of line so
@@ -171,20 +178,23 @@ static __device__ __noinline__ unsigned factor_rare(unsigned mask, unsigned rare
 // kGroup: the jobs of a batch from a device array; else the one job `single`
 // (a kernel parameter, so that an execution can be captured in a graph).
 template <bool kGroup>
-__global__ void __launch_bounds__(kFacThreads, 4) factor_kernel(const FactorJob single,
+__global__ void __launch_bounds__(kFacThreads, kFacPerSm) factor_kernel(const FactorJob single,
                                                                  const FactorJob* __restrict__ jobs, int n_jobs,
-                                                                 int total) {
+                                                                 int total, int* next) {
   __shared__ FactorSmem sm;
+  __shared__ int s_item;
   extern __shared__ float4 acc_dyn[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int cached = -1;  // job whose frequency constants sm.wxc holds
-  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+  // items, of unequal length in a batch, are taken from a counter
+  for (int item = blockIdx.x; item < total; item = s_item) {
     const int ji = kGroup ? find_job(jobs, n_jobs, item) : 0;
     const FactorJob& J = kGroup ? jobs[ji] : single;
     const GppDev& p = J.p;
     const int local = item - J.item_off;
     const int main_items = J.ncb * J.n_seg;
     __syncthreads();  // the previous item is done with shared memory
+    if (tid == 0) s_item = gridDim.x + atomicAdd(next, 1);
     if (local >= main_items) {
       // zero the A slices of the padding rows for kZeroTiles K tiles
       const int rows = kNW * p.ng, pad = padding_rows(J);
@@ -194,6 +204,7 @@ __global__ void __launch_bounds__(kFacThreads, 4) factor_kernel(const FactorJob 
         const int ch = e % 4, r = (e / 4) % pad, t = t0 + e / (4 * pad);
         put_a(J.a_tiles, J.kt, rows + r, t * kOzKTile + ch * 8, z, z);
       }
+      __syncthreads();  // s_item
       continue;
     }
     {  // this item's share of the B slices and epilogue factors
@@ -221,17 +232,9 @@ __global__ void __launch_bounds__(kFacThreads, 4) factor_kernel(const FactorJob 
       __syncthreads();
       cached = ji;
     }
-    FF wx[kNW];
-    float wxh[kNW], wxl[kNW], iwx2[kNW];
     bool wx32 = true;  // every frequency exact in FP32 (the mini-app's 3, 4, 5)
 #pragma unroll
-    for (int iw = 0; iw < kNW; ++iw) {
-      wx[iw] = FF{sm.wxc[iw][0], sm.wxc[iw][1]};
-      wx32 = wx32 && wx[iw].lo == 0.f;
-      wxh[iw] = sm.wxc[iw][2];
-      wxl[iw] = sm.wxc[iw][3];
-      iwx2[iw] = sm.wxc[iw][4];
-    }
+    for (int iw = 0; iw < kNW; ++iw) wx32 = wx32 && sm.wxc[iw][1] == 0.f;
     // float-float accumulators of the ssx sums this thread owns
     for (int r = 0; r < kSsxRounds; ++r) {
       const int o = r * (kFacThreads / 4) + warp * 8 + (lane >> 2);
@@ -252,77 +255,104 @@ __global__ void __launch_bounds__(kFacThreads, 4) factor_kernel(const FactorJob 
         sm.ani[n1][ks] = v.y;
         sm.anm[n1][ks] = -v.y;
       }
-#pragma unroll 1
-      for (int j = 0; j < 2; ++j) {
-        const int pl = warp + 8 * j, my_igp = cb * kFacCols + pl, ig = ig0 + lane;
-        float2 yt[kNW] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        float2 sv[kNW] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        if (my_igp < p.ng && ig < p.nc) {
-          const size_t off = (size_t)my_igp * p.nc + ig;
-          const double2 wt = p.wt[off];
-          const double2 ie = p.ieps[off];
-          const FF a = ff_of(wt.x), b = ff_of(wt.y), er = ff_of(ie.x), ei = ff_of(ie.y);
-          const FF gx = ff_dot2_raw(er, a, ei, b);           // G = I_eps wtilde
-          const FF gy = ff_dot2_raw(er, b, ff_neg(ei), a);
-          const FF b2 = ff_mul_raw(b, b);
-          const FF s2 = ff_dot2_raw(a, a, b, ff_neg(b));     // |wtilde|^2
-          // G (c + i b) = wx G - G conj(wtilde) = wx G - |wtilde|^2 I_eps
-          const FF sex = ff_mul_raw(s2, er), sey = ff_mul_raw(s2, ei);
-          // |wtilde|^2 * 4e-6 >= 0.25 only for |wtilde|^2 >= 62500; below,
-          // |wdiff|^2 > 0.25 implies the guard's second condition
-          const bool thr2_binds = s2.hi >= 62000.f;
-          // |wtilde|^2 / to1 > 1 >= |wdiff|^2 of a dropped term: its second
-          // occupied-band branch is then the exact-pole test alone
-          const bool big_s = s2.hi > 1.01e-6f;
-          unsigned mask = 0u, rare = thr2_binds ? 7u : 0u;
-          float2 yv[kNW];
+      {
+        // the warp's two columns, both elements in each paired instruction;
+        // elements past the ends are zero inputs without decisions
+        const int pl = warp, ig = ig0 + lane;
+        double2 wt[2], ie[2];
+        bool in[2];
 #pragma unroll
-          for (int iw = 0; iw < kNW; ++iw) {
-            const FF wv = ff_sq_add(ff_sub_raw(wx[iw], a), b2);  // |wdiff|^2
-            // keep: |wdiff|^2 > max(0.25, |wtilde|^2 * 4e-6), i.e. both
-            // wv > 0.25 and wv * 250000 > |wtilde|^2 (250000 exact in FP32);
-            // the second condition only binds for thr2_binds (rare path)
+        for (int j = 0; j < 2; ++j) {
+          const int my_igp = cb * kFacCols + pl + kFacWarps * j;
+          in[j] = my_igp < p.ng && ig < p.nc;
+          const size_t off = (size_t)my_igp * p.nc + ig;
+          wt[j] = in[j] ? p.wt[off] : make_double2(0.0, 0.0);
+          ie[j] = in[j] ? p.ieps[off] : make_double2(0.0, 0.0);
+          if (my_igp < p.ng && ig + kFacK < p.nc) {
+            prefetch_l2(&p.wt[off + kFacK]);
+            prefetch_l2(&p.ieps[off + kFacK]);
+          }
+        }
+        const FF2 a = ff2(ff_of(wt[0].x), ff_of(wt[1].x)), b = ff2(ff_of(wt[0].y), ff_of(wt[1].y));
+        FF2 gx, gy, sex, sey;
+        float2 s2h;
+        const float2 am = f2_neg(a.hi), bm = f2_neg(b.hi);
+        {
+          const FF2 er = ff2(ff_of(ie[0].x), ff_of(ie[1].x)), ei = ff2(ff_of(ie[0].y), ff_of(ie[1].y));
+          const float2 erm = f2_neg(er.hi);
+          const FF2 eim = ff2_neg(ei);
+          gx = ff2_dot2_raw(er, erm, a, ei, eim.hi, b);  // G = I_eps wtilde
+          gy = ff2_dot2_raw(er, erm, b, eim, ei.hi, a);
+          const FF2 s2 = ff2_dot2_raw(a, am, a, FF2{bm, f2_neg(b.lo)}, b.hi, b);  // |wtilde|^2
+          // G (c + i b) = wx G - G conj(wtilde) = wx G - |wtilde|^2 I_eps
+          sex = ff2_mul_raw(s2, er);
+          sey = ff2_mul_raw(s2, ei);
+          s2h = s2.hi;
+        }
+        const FF2 b2 = ff2_mul_raw(b, b);
+        // |wtilde|^2 * 4e-6 >= 0.25 only for |wtilde|^2 >= 62500; below,
+        // |wdiff|^2 > 0.25 implies the guard's second condition
+        const bool binds[2] = {s2h.x >= 62000.f, s2h.y >= 62000.f};
+        // |wtilde|^2 / to1 > 1 >= |wdiff|^2 of a dropped term: its second
+        // occupied-band branch is then the exact-pole test alone
+        const bool big[2] = {s2h.x > 1.01e-6f, s2h.y > 1.01e-6f};
+        unsigned mask[2] = {0u, 0u}, rare[2] = {binds[0] ? 7u : 0u, binds[1] ? 7u : 0u};
+        FF2 wv[kNW];
+#pragma unroll
+        for (int iw = 0; iw < kNW; ++iw) {
+          wv[iw] = ff2_sq_add(ff2_sub_raw(FF2{f2(sm.wxc[iw][0]), f2(sm.wxc[iw][1])}, a), b2);  // |wdiff|^2
+          // keep: |wdiff|^2 > max(0.25, |wtilde|^2 * 4e-6), i.e. both
+          // wv > 0.25 and wv * 250000 > |wtilde|^2 (250000 exact in FP32);
+          // the second condition only binds for `binds` (rare path)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const FF v = j ? FF{wv[iw].hi.y, wv[iw].lo.y} : FF{wv[iw].hi.x, wv[iw].lo.x};
             bool near;
-            const bool keep = ff_gt_quarter(wv, near);
-            // the factor of every term (the warp's lanes almost always
-            // disagree on keep), selected by the final keep bit below
-            const FF r = ff_rcp_raw(wv);
-            if (wx32) {
-              yv[iw] = make_float2(ff_factor_round(wx[iw].hi, gx, sex, r), ff_factor_round(wx[iw].hi, gy, sey, r));
-            } else {
-              yv[iw] = make_float2(ff_mul_round(ff_add(ff_mul(wx[iw], gx), ff_neg(sex)), r),
-                                   ff_mul_round(ff_add(ff_mul(wx[iw], gy), ff_neg(sey)), r));
-            }
+            const bool keep = ff_gt_quarter(v, near);
             // second occupied-band branch: 0 < |wdiff|^2 < |wtilde|^2 / to1,
             // which for |wtilde|^2 > 1e-6 and a dropped term is |wdiff|^2 > 0
-            const bool plain = big_s && wv.hi >= 1e-30f;
-            mask |= (keep ? (1u << iw) : 0u) | ((!keep && plain) ? (8u << iw) : 0u);
-            rare |= (near ? (1u << iw) : 0u) | ((nvb > 0 && !keep && !plain) ? (8u << iw) : 0u);
-          }
-          if (rare) mask = factor_rare(mask, rare, p.wx, wt.x, wt.y, thr2_binds, big_s);
-          if (nvb == 0) mask &= 7u;
-#pragma unroll
-          for (int iw = 0; iw < kNW; ++iw) yt[iw] = (mask & (1u << iw)) ? yv[iw] : make_float2(0.f, 0.f);
-          if (nvb > 0) {
-            const float2 g32 = make_float2(ff_round(gx), ff_round(gy));
-            const float bb = ff_round(b);
-            // Omega2 = wtilde G
-            const float2 om = make_float2(ff_dot2_round(a, gx, b, gy), ff_dot2_round(a, gy, ff_neg(b), gx));
-#pragma unroll
-            for (int iw = 0; iw < kNW; ++iw) {
-              const float zr = (wxh[iw] + a.hi) + (wxl[iw] + a.lo);
-              const float q = -0.5f * rcp_f32(fmaf(zr, zr, bb * bb));
-              const float2 s1 = make_float2(om.x * iwx2[iw], om.y * iwx2[iw]);
-              const float2 s2v = make_float2(fmaf(g32.x, zr, g32.y * bb) * q, fmaf(g32.y, zr, -g32.x * bb) * q);
-              sv[iw] = (mask & (1u << iw)) ? s1 : ((mask & (8u << iw)) ? s2v : make_float2(0.f, 0.f));
-            }
+            const bool plain = big[j] && v.hi >= 1e-30f;
+            mask[j] |= (keep ? (1u << iw) : 0u) | ((!keep && plain) ? (8u << iw) : 0u);
+            rare[j] |= (near ? (1u << iw) : 0u) | ((nvb > 0 && !keep && !plain) ? (8u << iw) : 0u);
           }
         }
 #pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (rare[j] && in[j]) mask[j] = factor_rare(mask[j], rare[j], p.wx, wt[j].x, wt[j].y, binds[j], big[j]);
+        float2 omx, omy, g32x, g32y, bb;
+        if (nvb > 0) {
+          // Omega2 = wtilde G
+          const FF2 ox = ff2_dot2_raw(a, am, gx, b, bm, gy), oy = ff2_dot2_raw(a, am, gy, FF2{bm, f2_neg(b.lo)}, b.hi, gx);
+          omx = __fadd2_rn(ox.hi, ox.lo);
+          omy = __fadd2_rn(oy.hi, oy.lo);
+          g32x = __fadd2_rn(gx.hi, gx.lo);
+          g32y = __fadd2_rn(gy.hi, gy.lo);
+          bb = __fadd2_rn(b.hi, b.lo);
+        }
+#pragma unroll
         for (int iw = 0; iw < kNW; ++iw) {
-          sm.y[iw][pl][lane] = yt[iw];
-          sm.x.r[pl][iw][ssx_slot(lane)] = sv[iw].x;
-          sm.x.i[pl][iw][ssx_slot(lane)] = sv[iw].y;
+          // the factor of every term (the warp's lanes almost always
+          // disagree on keep), selected by the final keep bit
+          const bool k0 = mask[0] & (1u << iw), k1 = mask[1] & (1u << iw);
+          const FF2 r = ff2_rcp_raw(wv[iw]);
+          const FF w{sm.wxc[iw][0], sm.wxc[iw][1]};
+          const float2 yx = factor_round(wx32, w, gx, sex, r), yy = factor_round(wx32, w, gy, sey, r);
+          sm.y[iw][pl][lane] = k0 ? make_float2(yx.x, yy.x) : make_float2(0.f, 0.f);
+          sm.y[iw][pl + kFacWarps][lane] = k1 ? make_float2(yx.y, yy.y) : make_float2(0.f, 0.f);
+          if (nvb > 0) {
+            const float2 zr = __fadd2_rn(__fadd2_rn(f2(sm.wxc[iw][2]), a.hi), __fadd2_rn(f2(sm.wxc[iw][3]), a.lo));
+            const float2 d = __ffma2_rn(zr, zr, __fmul2_rn(bb, bb));
+            const float2 q = __fmul2_rn(f2(-0.5f), make_float2(rcp_f32(d.x), rcp_f32(d.y)));
+            const float2 i2 = f2(sm.wxc[iw][4]), s1x = __fmul2_rn(omx, i2), s1y = __fmul2_rn(omy, i2);
+            const float2 s2x = __fmul2_rn(__ffma2_rn(g32x, zr, __fmul2_rn(g32y, bb)), q);
+            const float2 s2y = __fmul2_rn(__ffma2_rn(g32y, zr, __fmul2_rn(f2_neg(g32x), bb)), q);
+            const bool n0 = mask[0] & (8u << iw), n1 = mask[1] & (8u << iw);
+            const int ks = ssx_slot(lane);
+            sm.x.r[pl][iw][ks] = k0 ? s1x.x : n0 ? s2x.x : 0.f;
+            sm.x.i[pl][iw][ks] = k0 ? s1y.x : n0 ? s2y.x : 0.f;
+            sm.x.r[pl + kFacWarps][iw][ks] = k1 ? s1x.y : n1 ? s2x.y : 0.f;
+            sm.x.i[pl + kFacWarps][iw][ks] = k1 ? s1y.y : n1 ? s2y.y : 0.f;
+          }
         }
       }
       __syncthreads();
@@ -430,10 +460,26 @@ void factor_job_size(FactorJob& j, const GppDev& p, int kt, int grid, double sha
   j.p = p;
   j.kt = kt;
   j.ncb = (p.ng + kFacCols - 1) / kFacCols;
-  // about 12 items per CTA over this instance's share of the launch
+  // about 12 items per CTA over this instance's share of the launch; an
+  // instance alone takes the tiles per item that finish first, an item costing half
+  // a tile beside its tiles and a partial its share of the reduction (a tile
+  // takes ~5 us; 77 bands, 8 of them occupied, x 406 x 4067: the whole sum 419 us
+  // in one-tile items, 250 us so)
   const double want = std::max(1.0, 12.0 * grid * share);
   int seg = (int)std::max(1.0, std::min((double)kt, want / j.ncb + 0.5));
   j.seg_tiles = (kt + seg - 1) / seg;
+  if (share >= 1.0) {
+    double best = 0.0;
+    for (int len = j.seg_tiles; len <= kt; ++len) {
+      const double items = (double)j.ncb * ((kt + len - 1) / len), cost = std::ceil(items / grid) * (len + 0.5) + 1.5e-4 * items;
+      if (len == j.seg_tiles || cost < best) {
+        best = cost;
+        seg = len;
+      }
+      if (items <= grid) break;  // longer items only take longer
+    }
+    j.seg_tiles = seg;
+  }
   j.n_seg = (kt + j.seg_tiles - 1) / j.seg_tiles;
   GppWork& w = j.ssx;
   w = GppWork{};
@@ -484,22 +530,22 @@ int factor_blocks_per_sm(int max_nvband) {
 }
 
 cudaError_t launch_factor_pass(const FactorJob* jobs, int n_jobs, int total, int grid, int max_nvband,
-                               cudaStream_t s) {
+                               int* next, cudaStream_t s) {
   if (total <= 0) return cudaSuccess;
   cudaError_t e = factor_smem_attr<true>();
   if (e != cudaSuccess) return e;
   factor_kernel<true><<<std::min(grid, total), kFacThreads, factor_acc_bytes(max_nvband), s>>>(
-      FactorJob{}, jobs, n_jobs, total);
+      FactorJob{}, jobs, n_jobs, total, next);
   return cudaGetLastError();
 }
 
-cudaError_t launch_factor_pass(const FactorJob& job, int grid, cudaStream_t s) {
+cudaError_t launch_factor_pass(const FactorJob& job, int grid, int* next, cudaStream_t s) {
   const int total = factor_job_items(job);
   if (total <= 0) return cudaSuccess;
   cudaError_t e = factor_smem_attr<false>();
   if (e != cudaSuccess) return e;
   factor_kernel<false><<<std::min(grid, total), kFacThreads, factor_acc_bytes(job.p.nvband), s>>>(
-      job, nullptr, 1, total);
+      job, nullptr, 1, total, next);
   return cudaGetLastError();
 }
 

@@ -7,7 +7,7 @@
 
 namespace sigma {
 
-constexpr int kFacCols = 16;        // columns (my_igp) per factor tile
+constexpr int kFacCols = 8;         // columns (my_igp) per factor tile
 constexpr int kFacK = 32;           // g-vectors per factor tile (one K tile of the contraction)
 constexpr int kFusedBands = 8;      // occupied bands whose ssx sums the factor pass takes
 
@@ -50,10 +50,10 @@ int factor_blocks_per_sm(int max_nvband);
 inline bool factor_fuses_ssx(int nvband) { return nvband <= kFusedBands; }
 
 // The factor pass over jobs[0 .. n_jobs) (device array; job i's items are
-// [item_off, item_off + factor_job_items)), `total` items in all.
+// [item_off, item_off + factor_job_items)), `total` items in all; *next is 0.
 cudaError_t launch_factor_pass(const FactorJob* jobs, int n_jobs, int total, int grid, int max_nvband,
-                               cudaStream_t s);
+                               int* next, cudaStream_t s);
 // One instance, the job passed by value (item_off 0).
-cudaError_t launch_factor_pass(const FactorJob& job, int grid, cudaStream_t s);
+cudaError_t launch_factor_pass(const FactorJob& job, int grid, int* next, cudaStream_t s);
 
 }  // namespace sigma

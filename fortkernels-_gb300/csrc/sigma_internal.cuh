@@ -256,6 +256,10 @@ __device__ __forceinline__ double rcp_f64_seed32(double w) {
   return fma(r0, eps, r0);
 }
 
+// Brings a line of global memory into L2 ahead of its load.
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 // The FP32 reciprocal's seed (relative error about 2^-23).
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
