@@ -15,7 +15,8 @@
 // digits with paired FP32 operations and writes each row's digits as 16-byte
 // chunks: 16 columns x 32 g-vectors staged in shared memory, four CTAs per SM.
 // Bound by issue slots (69 % issuing, FP64 pipe 52 %, FMA 48 %): 2.43 ms at
-// 1638 x 32768 with the occupied bands' factors, 2.74 ms with digits of one
+// 1638 x 32768 with the occupied bands' factors (2.38 ms with the next tile
+// prefetched to L2), 2.74 ms with digits of one
 // value per instruction, the general FP64 split and all large factors counted.
 // Factors of two elements per instruction need 80 registers or spill at two
 // or three CTAs per SM: 3.13 and 3.35 ms.
@@ -340,6 +341,11 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
       if (ig < s_lim[pl]) {
         const double2 wt = gx_load<kForm>(p.wt, (size_t)g * p.nc + ig);
         const double2 ie = gx_load<kForm>(p.ieps, (size_t)g * p.nc + ig);
+        if (ig + kFfK < s_lim[pl]) {
+          const size_t next = ((size_t)g * p.nc + ig + kFfK) * (F::kReal ? 1 : 2);
+          prefetch_l2(p.wt + next);
+          prefetch_l2(p.ieps + next);
+        }
         gx_factors<kForm, kOcc>(wx, iwx2, p.wx, s_wide, wt, ie, [&](int i, FF re, FF im) {
           sm.hi[0][i][pl][lane] = re.hi;
           sm.lo[0][i][pl][lane] = re.lo;
