@@ -93,59 +93,65 @@ __global__ void __launch_bounds__(256) ozaki_weights_kernel(FfDev p, OzakiPrep o
     oz_weights_elem(p, oz, t);
 }
 
-// schDt[n1][ifreq]: one warp per entry, fixed-order compensated sum over the
-// row blocks that hold frequency ifreq and over their work entries.
+// schDt[n1][ifreq]: eight lanes per entry, fixed-order compensated sum over
+// the row blocks that hold frequency ifreq and over their work entries, four
+// partials in flight per lane.  (A warp per entry spent its time in FP64
+// butterflies and in one load after another: 100 -> 28 us at 512 x 15 entries,
+// 45 -> 28 us at 512 x 3.)
+constexpr int kRedThreads = 64, kRedLanes = 8;
 __device__ __forceinline__ void reduce_entry(const FfDev& p, const OzakiPrep& oz, const double2* partial,
-                                             double2* schdt, int warp, int lane) {
-  const int n = warp / p.nf, f = warp % p.nf;
+                                             double2* schdt, int entry, bool on) {
+  const int lane = threadIdx.x % kRedLanes;
+  const int n = entry / p.nf, f = entry % p.nf;
   const int cb = n / kOzCols, c = n % kOzCols;
-  const int rb_lo = (f * p.ng) / kOzRows, rb_hi = ((f + 1) * p.ng - 1) / kOzRows;
+  const int rb_hi = on ? ((f + 1) * p.ng - 1) / kOzRows : -1;
   Comp sx, sy;
-  int q0 = 0;  // entries of the row blocks before rb, lanes take every 32nd
-  for (int rb = rb_lo; rb <= rb_hi; ++rb) {
-    const int np = oz.pieces[rb];
-    const int seg = f - (rb * kOzRows) / p.ng;
-    for (int j = (lane - q0 % 32 + 32) % 32; j < np; j += 32) {
-      const size_t pidx = ((size_t)rb * oz.n_col_blocks + cb) * oz.max_pieces + j;
-      const double2 v = partial[(pidx * oz.max_seg + seg) * kOzCols + c];
-      sx.add(v.x);
-      sy.add(v.y);
-    }
-    q0 += np;
-  }
+  // the entries' work pieces in row-block order, every eighth one this lane's
+  int rb = (f * p.ng) / kOzRows, j = lane, np = rb <= rb_hi ? oz.pieces[rb] : 0;
+  while (rb <= rb_hi) {
+    double2 v[4];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double a = __shfl_xor_sync(0xffffffffu, sx.s, o), b = __shfl_xor_sync(0xffffffffu, sx.c, o);
-    const double c2 = __shfl_xor_sync(0xffffffffu, sy.s, o), d = __shfl_xor_sync(0xffffffffu, sy.c, o);
-    double t, e;
-    two_sum_d(sx.s, a, t, e);
-    sx.s = t;
-    sx.c = __dadd_rn(__dadd_rn(sx.c, b), e);
-    two_sum_d(sy.s, c2, t, e);
-    sy.s = t;
-    sy.c = __dadd_rn(__dadd_rn(sy.c, d), e);
+    for (int q = 0; q < 4; ++q) {
+      while (rb <= rb_hi && j >= np) {
+        j -= np;
+        if (++rb <= rb_hi) np = oz.pieces[rb];
+      }
+      v[q] = make_double2(0.0, 0.0);
+      if (rb <= rb_hi) {
+        const int seg = f - (rb * kOzRows) / p.ng;
+        const size_t pidx = ((size_t)rb * oz.n_col_blocks + cb) * oz.max_pieces + j;
+        v[q] = partial[(pidx * oz.max_seg + seg) * kOzCols + c];
+      }
+      j += kRedLanes;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      sx.add(v[q].x);
+      sy.add(v[q].y);
+    }
   }
-  if (lane == 0) schdt[(size_t)n * p.nf + f] = make_double2(sx.value(), sy.value());
+  const double x = lanes_sum_comp<kRedLanes>(sx), y = lanes_sum_comp<kRedLanes>(sy);
+  if (on && lane == 0) schdt[(size_t)n * p.nf + f] = make_double2(x, y);
 }
 
-__global__ void ozaki_reduce_kernel(FfDev p, OzakiPrep oz, const double2* partial, double2* schdt) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= p.nb * p.nf) return;
-  reduce_entry(p, oz, partial, schdt, warp, threadIdx.x & 31);
+__global__ void __launch_bounds__(kRedThreads) ozaki_reduce_kernel(FfDev p, OzakiPrep oz, const double2* partial,
+                                                                   double2* schdt) {
+  const int entry = (blockIdx.x * kRedThreads + threadIdx.x) / kRedLanes;
+  reduce_entry(p, oz, partial, schdt, entry, entry < p.nb * p.nf);
 }
 
-// Group form: warps r_warp_off .. + nb * nf of each job reduce its entries.
-__global__ void ozaki_group_reduce_kernel(OzGroup g) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= g.r_warps) return;
+// Group form: entries r_warp_off .. + nb * nf of each job.
+__global__ void __launch_bounds__(kRedThreads) ozaki_group_reduce_kernel(OzGroup g) {
+  const int entry = (blockIdx.x * kRedThreads + threadIdx.x) / kRedLanes;
   int lo = 0, hi = g.n_jobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (g.jobs[mid].r_warp_off <= warp) lo = mid; else hi = mid - 1;
+    if (g.jobs[mid].r_warp_off <= entry) lo = mid; else hi = mid - 1;
   }
   const OzGroupJob& J = g.jobs[lo];
-  reduce_entry(J.d, J.oz, J.oz.partial, J.out, warp - J.r_warp_off, threadIdx.x & 31);
+  reduce_entry(J.d, J.oz, J.oz.partial, J.out, entry - J.r_warp_off, entry < g.r_warps);
 }
+constexpr int red_blocks(int entries) { return (entries * kRedLanes + kRedThreads - 1) / kRedThreads; }
 
 }  // namespace
 
@@ -351,18 +357,17 @@ cudaError_t launch_ozaki_group_gemm(const OzGroup& g, int grid, cudaStream_t s) 
 
 cudaError_t launch_ozaki_group_reduce(const OzGroup& g, cudaStream_t s) {
   if (g.r_warps <= 0) return cudaSuccess;
-  ozaki_group_reduce_kernel<<<(g.r_warps * 32 + 255) / 256, 256, 0, s>>>(g);
+  ozaki_group_reduce_kernel<<<red_blocks(g.r_warps), kRedThreads, 0, s>>>(g);
   return cudaGetLastError();
 }
 
 cudaError_t launch_ozaki_reduce(const FfDev& d, const OzakiPrep& oz, double2* schdt, cudaStream_t s,
                                 double2* schdt2) {
-  const int warps = d.nb * d.nf;
-  const int blocks = (warps * 32 + 255) / 256;
-  ozaki_reduce_kernel<<<blocks, 256, 0, s>>>(d, oz, oz.partial, schdt);
+  const int blocks = red_blocks(d.nb * d.nf);
+  ozaki_reduce_kernel<<<blocks, kRedThreads, 0, s>>>(d, oz, oz.partial, schdt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !schdt2) return e;
-  ozaki_reduce_kernel<<<blocks, 256, 0, s>>>(d, oz, oz.partial2, schdt2);
+  ozaki_reduce_kernel<<<blocks, kRedThreads, 0, s>>>(d, oz, oz.partial2, schdt2);
   return cudaGetLastError();
 }
 
