@@ -93,12 +93,15 @@ __global__ void __launch_bounds__(256) ozaki_weights_kernel(FfDev p, OzakiPrep o
     oz_weights_elem(p, oz, t);
 }
 
-// schDt[n1][ifreq]: eight lanes per entry, fixed-order compensated sum over
-// the row blocks that hold frequency ifreq and over their work entries, four
-// partials in flight per lane.  (A warp per entry spent its time in FP64
-// butterflies and in one load after another: 100 -> 28 us at 512 x 15 entries,
-// 45 -> 28 us at 512 x 3.)
-constexpr int kRedThreads = 64, kRedLanes = 8;
+// schDt[n1][ifreq]: fixed-order compensated sum over the row blocks that hold
+// frequency ifreq and over their work entries, four partials in flight per
+// lane.  Eight lanes per entry from kRedMany entries on (a warp's FP64
+// butterflies and its one load after another took 100 us at 512 x 15
+// entries, 28 us so); a warp per entry below, where an entry's partials are many
+// and the loads bound it (128 bands x 409 columns x 8192, tensor form: 277 us
+// in all, 307 us with eight lanes; 512 x 3 entries 45 -> 28 us).
+constexpr int kRedThreads = 64, kRedMany = 3072;
+template <int kRedLanes>
 __device__ __forceinline__ void reduce_entry(const FfDev& p, const OzakiPrep& oz, const double2* partial,
                                              double2* schdt, int entry, bool on) {
   const int lane = threadIdx.x % kRedLanes;
@@ -110,6 +113,7 @@ __device__ __forceinline__ void reduce_entry(const FfDev& p, const OzakiPrep& oz
   int rb = (f * p.ng) / kOzRows, j = lane, np = rb <= rb_hi ? oz.pieces[rb] : 0;
   while (rb <= rb_hi) {
     double2 v[4];
+    int n_in = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       while (rb <= rb_hi && j >= np) {
@@ -121,26 +125,30 @@ __device__ __forceinline__ void reduce_entry(const FfDev& p, const OzakiPrep& oz
         const int seg = f - (rb * kOzRows) / p.ng;
         const size_t pidx = ((size_t)rb * oz.n_col_blocks + cb) * oz.max_pieces + j;
         v[q] = partial[(pidx * oz.max_seg + seg) * kOzCols + c];
+        ++n_in;
       }
       j += kRedLanes;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      sx.add(v[q].x);
-      sy.add(v[q].y);
-    }
+    for (int q = 0; q < 4; ++q)
+      if (q < n_in) {
+        sx.add(v[q].x);
+        sy.add(v[q].y);
+      }
   }
   const double x = lanes_sum_comp<kRedLanes>(sx), y = lanes_sum_comp<kRedLanes>(sy);
   if (on && lane == 0) schdt[(size_t)n * p.nf + f] = make_double2(x, y);
 }
 
+template <int kRedLanes>
 __global__ void __launch_bounds__(kRedThreads) ozaki_reduce_kernel(FfDev p, OzakiPrep oz, const double2* partial,
                                                                    double2* schdt) {
   const int entry = (blockIdx.x * kRedThreads + threadIdx.x) / kRedLanes;
-  reduce_entry(p, oz, partial, schdt, entry, entry < p.nb * p.nf);
+  reduce_entry<kRedLanes>(p, oz, partial, schdt, entry, entry < p.nb * p.nf);
 }
 
 // Group form: entries r_warp_off .. + nb * nf of each job.
+template <int kRedLanes>
 __global__ void __launch_bounds__(kRedThreads) ozaki_group_reduce_kernel(OzGroup g) {
   const int entry = (blockIdx.x * kRedThreads + threadIdx.x) / kRedLanes;
   int lo = 0, hi = g.n_jobs - 1;
@@ -149,9 +157,11 @@ __global__ void __launch_bounds__(kRedThreads) ozaki_group_reduce_kernel(OzGroup
     if (g.jobs[mid].r_warp_off <= entry) lo = mid; else hi = mid - 1;
   }
   const OzGroupJob& J = g.jobs[lo];
-  reduce_entry(J.d, J.oz, J.oz.partial, J.out, entry - J.r_warp_off, entry < g.r_warps);
+  reduce_entry<kRedLanes>(J.d, J.oz, J.oz.partial, J.out, entry - J.r_warp_off, entry < g.r_warps);
 }
-constexpr int red_blocks(int entries) { return (entries * kRedLanes + kRedThreads - 1) / kRedThreads; }
+constexpr int red_blocks(int entries) {
+  return (entries * (entries >= kRedMany ? 8 : 32) + kRedThreads - 1) / kRedThreads;
+}
 
 }  // namespace
 
@@ -357,17 +367,19 @@ cudaError_t launch_ozaki_group_gemm(const OzGroup& g, int grid, cudaStream_t s) 
 
 cudaError_t launch_ozaki_group_reduce(const OzGroup& g, cudaStream_t s) {
   if (g.r_warps <= 0) return cudaSuccess;
-  ozaki_group_reduce_kernel<<<red_blocks(g.r_warps), kRedThreads, 0, s>>>(g);
+  auto* kernel = g.r_warps >= kRedMany ? ozaki_group_reduce_kernel<8> : ozaki_group_reduce_kernel<32>;
+  kernel<<<red_blocks(g.r_warps), kRedThreads, 0, s>>>(g);
   return cudaGetLastError();
 }
 
 cudaError_t launch_ozaki_reduce(const FfDev& d, const OzakiPrep& oz, double2* schdt, cudaStream_t s,
                                 double2* schdt2) {
   const int blocks = red_blocks(d.nb * d.nf);
-  ozaki_reduce_kernel<<<blocks, kRedThreads, 0, s>>>(d, oz, oz.partial, schdt);
+  auto* kernel = d.nb * d.nf >= kRedMany ? ozaki_reduce_kernel<8> : ozaki_reduce_kernel<32>;
+  kernel<<<blocks, kRedThreads, 0, s>>>(d, oz, oz.partial, schdt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !schdt2) return e;
-  ozaki_reduce_kernel<<<blocks, kRedThreads, 0, s>>>(d, oz, oz.partial2, schdt2);
+  kernel<<<blocks, kRedThreads, 0, s>>>(d, oz, oz.partial2, schdt2);
   return cudaGetLastError();
 }
 

@@ -108,6 +108,7 @@ static __device__ __noinline__ void real_wide_chunk(const GppRealDev& p, double 
 }
 
 __global__ void __launch_bounds__(kThreads, 2) sch_real_kernel(GppRealDev p, GppWork w) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RealSmem& sm = *reinterpret_cast<RealSmem*>(smem_raw);
   __shared__ int s_item;
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(kThreads, 2) sch_real_kernel(GppRealDev p, Gpp
 
 // Occupied bands: thread = column, kSsxBN bands per item.
 __global__ void __launch_bounds__(kThreads) ssx_real_kernel(GppRealDev p, GppWork w) {
+  chain_begin();
   __shared__ int s_item;
   __shared__ double red[kSsxBN][kNW][kThreads / 32];
   if (w.run_if && !*w.run_if) return;
@@ -327,6 +329,7 @@ __global__ void __launch_bounds__(kThreads) ssx_real_kernel(GppRealDev p, GppWor
 
 __global__ void real_parts_kernel(const double2* ach, const double2* asx, const double2* n1, int nb,
                                   double* ach_out, double* asx_out, double* n1_out) {
+  chain_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < kNW) {
     ach_out[t] = ach[t].x;
@@ -473,12 +476,10 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
     // two CTAs per SM hold ~180 KB of shared memory between them
     SIGMA_CUDA_TRY(cudaFuncSetAttribute(sch_real_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared));
-    sch_real_kernel<<<plan->sch_grid, kThreads, sizeof(RealSmem), s>>>(p, sch);
-    SIGMA_CUDA_TRY(cudaGetLastError());
+    SIGMA_CUDA_TRY(launch_chained(sch_real_kernel, plan->sch_grid, kThreads, sizeof(RealSmem), s, true, p, sch));
   }
   if (plan->ssx.n_items > 0) {
-    ssx_real_kernel<<<plan->ssx_grid, kThreads, 0, s>>>(p, ssx);
-    SIGMA_CUDA_TRY(cudaGetLastError());
+    SIGMA_CUDA_TRY(launch_chained(ssx_real_kernel, plan->ssx_grid, kThreads, 0, s, true, p, ssx));
   }
   double2* ach_c = plan->outc;
   double2* asx_c = plan->outc + kNW;
@@ -486,9 +487,8 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
   SIGMA_CUDA_TRY(launch_gpp_reduce(sch, ssx, plan->nb, plan->acht_n1, ach_c, asx_c,
                                    acht_n1_loc ? n1_c : nullptr, s));
   const int nthreads = 256, n = std::max(plan->nb, kNW);
-  real_parts_kernel<<<(n + nthreads - 1) / nthreads, nthreads, 0, s>>>(ach_c, asx_c, n1_c, plan->nb,
-                                                                       achtemp, asxtemp, acht_n1_loc);
-  SIGMA_CUDA_TRY(cudaGetLastError());
+  SIGMA_CUDA_TRY(launch_chained(real_parts_kernel, (n + nthreads - 1) / nthreads, nthreads, 0, s, true, ach_c, asx_c,
+                                n1_c, plan->nb, achtemp, asxtemp, acht_n1_loc));
   return SIGMA_OK;
 }
 
