@@ -1,8 +1,8 @@
 // Exact digit contraction (exact_gemm.cuh): operand checks and digits, the
 // tcgen05 kernel, and the FP64 epilogue.
 //
-// The contraction kernel.  A CTA takes one (128 rows x 80 B' rows x K range)
-// item at a time.  Per 16-K tile the 21 digit products run as nine MMAs: the
+// The contraction kernel.  A CTA takes one (128 rows x 80 B' rows x K range;
+// 64 or 48 B' rows where they pad the bands less) item at a time.  Per 16-K tile the 21 digit products run as nine MMAs: the
 // B slices are stacked along N, so A_i times [B_j .. B_k] fills the adjacent
 // accumulators s = i + j .. i + k in one instruction (N up to 240), which
 // reads A from shared memory once for up to three products (107 bytes per
@@ -15,7 +15,7 @@
 // no FP64 operation (2 per clock per SM on this part); an item ends with its
 // raw sums written out, and exact_finish_kernel forms the weighted FP64 sums.
 //
-// Measured: the FF contraction of 512 x (15 x 820) x 16384 in 13.8 ms, 555 ms
+// Measured: the FF contraction of 512 x (15 x 820) x 16384 in 13.2 ms, 555 ms
 // with FP64 multiply-adds (ff_fp64.cu); normwise error 2.8e-15 (5e-15).
 //
 // Roles (352 threads): warps 0-7 drain, warp 8 streams 39 KB tiles (one bulk
@@ -35,8 +35,8 @@ using namespace tma;
 constexpr int kThreadsEx = 352;
 constexpr int kCopyWarp = 8, kIssueWarp = 9, kGateWarpEx = 10;
 constexpr int kStagesEx = 5;
-constexpr uint32_t ex_stage(int S) { return ex_a_bytes(S) + ex_b_bytes(S); }  // 39 / 42 KB
-constexpr uint32_t ex_smem(int S) { return kStagesEx * ex_stage(S) + 1024; }
+constexpr uint32_t ex_stage(int S, int cols) { return ex_a_bytes(S) + ex_b_bytes(S, cols); }  // 33 to 42 KB
+constexpr uint32_t ex_smem(int S, int cols) { return kStagesEx * ex_stage(S, cols) + 1024; }
 constexpr int kBlockTiles = 8;  // K tiles per accumulator lifetime (128 K values)
 
 // 32-byte swizzle: rows of 16 elements (32 B), 8-row groups of 256 B (layout
@@ -102,11 +102,12 @@ __device__ __forceinline__ ExItem ex_decode(const ExactPrep& ex, int item) {
 
 constexpr uint32_t idesc_n(int n) { return idesc_bf16_f32(128, n); }
 
-template <int S>
+template <int S, int kCols>
 __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex, int* status) {
-  constexpr int kCols = ex_cols(S), kColsHalf = kCols / 2, kHi = S - 3;  // kHi accumulators from s = 3 on
-  constexpr uint32_t kStage = ex_stage(S), kABytes = ex_a_bytes(S), kBBytes = ex_b_bytes(S), kBSlice = ex_b_slice(S);
-  static_assert(S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
+  constexpr int kColsHalf = kCols / 2, kHi = S - 3;  // kHi accumulators from s = 3 on
+  constexpr uint32_t kStage = ex_stage(S, kCols), kABytes = ex_a_bytes(S), kBBytes = ex_b_bytes(S, kCols),
+                     kBSlice = ex_b_slice(kCols);
+  static_assert(kCols % 16 == 0 && S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
   extern __shared__ unsigned char smem_raw[];
   // full[5], empty[5], lo full, hi full, lo empty, hi empty, done
   __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
@@ -429,13 +430,13 @@ __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const 
   }
 }
 
-template <int S, bool kReal>
+template <int S, int kCols, bool kReal>
 __global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const void* b0, int nb0, const void* b1,
                                                             int nb, int nc) {
   chain_begin();
   if (*ex.flag) return;
-  constexpr int kW = kReal ? 1 : 2, kBands = kReal ? ex_cols(S) : ex_cols(S) / 2;
-  constexpr uint32_t kSlice = ex_b_slice(S), kBytes = ex_b_bytes(S);
+  constexpr int kW = kReal ? 1 : 2, kBands = kReal ? kCols : kCols / 2;
+  constexpr uint32_t kSlice = ex_b_slice(kCols), kBytes = ex_b_bytes(S, kCols);
   const int pairs = ex.kt / 2;
   const long long total = (long long)ex.n_col_blocks * pairs * kBands * 4;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -620,7 +621,7 @@ ExSizes ex_sizes(const ExactPrep& ex) {
   const size_t blocks = ex_block_index(ex, ex.n_row_blocks, 0);
   const size_t slots = blocks * ex.max_pieces * ex.cols * kExRows;
   z.a = up256((size_t)ex.n_row_blocks * kts * ex_a_bytes(ex.slices));
-  z.b = up256((size_t)ex.n_col_blocks * kts * ex_b_bytes(ex.slices));
+  z.b = up256((size_t)ex.n_col_blocks * kts * ex_b_bytes(ex.slices, ex.cols));
   z.ea = up256(sizeof(int) * (size_t)ex.n_row_blocks * kExRows);
   z.eb = up256(sizeof(int) * (size_t)ex.n_col_blocks * ex.bands);
   z.seg = up256(sizeof(int) * 2 * (size_t)ex.n_kseg);
@@ -635,12 +636,31 @@ ExSizes ex_sizes(const ExactPrep& ex) {
 
 }  // namespace
 
+// B' rows per column block.  A narrower block's MMAs take less time but read A
+// from shared memory as often: 680, 625 and 565 us per block of 80, 64 and
+// 48 rows at 4914 A rows x 65536 K' (DRAM-bound below).  The fewest padded rows win only
+// where the number of blocks stays: 128 bands take four blocks of 64, 2.51 ms
+// there, 2.72 in four of 80; 72 bands two of 80, 1.36 ms, 1.70 in three of 48.
+int ex_pick_cols(int S, int b_rows) {
+  if (S != 6) return ex_max_cols(S);
+  int best = 80;
+  long long cost = LLONG_MAX;
+  for (const int c : {80, 64, 48}) {
+    const long long t = (long long)((b_rows + c - 1) / c) * (c == 80 ? 680 : c == 64 ? 625 : 565);
+    if (t < cost) {
+      cost = t;
+      best = c;
+    }
+  }
+  return best;
+}
+
 void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
                 ExactTables* tables, int nf2, int nb2) {
   const int rows = nf * ng;
   ex.halves = cplx ? 2 : 1;
   ex.slices = slices;
-  ex.cols = ex_cols(slices);
+  ex.cols = ex_pick_cols(slices, (cplx ? 2 : 1) * nb);
   ex.bands = cplx ? ex.cols / 2 : ex.cols;
   ex.kt = (nc + 31) / 32 * 2;
   ex.n_main_blocks = (rows + kExRows - 1) / kExRows;
@@ -769,8 +789,15 @@ cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const v
   auto* stats = real ? exact_stats_kernel<true, true> : exact_stats_kernel<true, false>;
   cudaError_t e = launch_chained(stats, nb, 256, 0, s, true, ex, b0, nb0, b1, nc);
   if (e != cudaSuccess) return e;
-  auto* slice = ex.slices == 7 ? (real ? exact_slice_b_kernel<7, true> : exact_slice_b_kernel<7, false>)
-                               : (real ? exact_slice_b_kernel<6, true> : exact_slice_b_kernel<6, false>);
+  auto* slice = exact_slice_b_kernel<6, 80, false>;
+  if (ex.slices == 7)
+    slice = real ? exact_slice_b_kernel<7, 64, true> : exact_slice_b_kernel<7, 64, false>;
+  else if (ex.cols == 80)
+    slice = real ? exact_slice_b_kernel<6, 80, true> : exact_slice_b_kernel<6, 80, false>;
+  else if (ex.cols == 64)
+    slice = real ? exact_slice_b_kernel<6, 64, true> : exact_slice_b_kernel<6, 64, false>;
+  else
+    slice = real ? exact_slice_b_kernel<6, 48, true> : exact_slice_b_kernel<6, 48, false>;
   return launch_chained(slice, 152 * 8, 256, 0, s, true, ex, b0, nb0, b1, nb, nc);
 }
 
@@ -781,8 +808,11 @@ cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int 
 }
 
 cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s) {
-  auto* kernel = ex.slices == 7 ? exact_gemm_kernel<7> : exact_gemm_kernel<6>;
-  const uint32_t smem = ex_smem(ex.slices);
+  auto* kernel = ex.slices == 7    ? exact_gemm_kernel<7, 64>
+                 : ex.cols == 80 ? exact_gemm_kernel<6, 80>
+                 : ex.cols == 64 ? exact_gemm_kernel<6, 64>
+                                 : exact_gemm_kernel<6, 48>;
+  const uint32_t smem = ex_smem(ex.slices, ex.cols);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return launch_chained(kernel, std::min(grid, ex.n_items), kThreadsEx, smem, s, true, ex, status);

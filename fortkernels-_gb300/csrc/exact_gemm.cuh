@@ -43,13 +43,15 @@ constexpr int kExRows = 128;     // A rows per tile
 constexpr int kExSeg = 512;      // K values per segment of the overlap check,
 constexpr int kExCount = 128;    // of which the first are counted (a lower bound, at a quarter of the work)
 constexpr uint32_t kExASlice = kExRows * kExKTile * 2;  // 4 KB
-// S slices (digits) per value and B' rows per slice, such that the S
-// accumulators fit tensor memory's 512 columns: 6 x 80 (40 complex bands, Re
-// and Im interleaved, or 80 real ones) or 7 x 64.
-constexpr int ex_cols(int S) { return S == 6 ? 80 : 64; }
-constexpr uint32_t ex_a_bytes(int S) { return S * kExASlice; }                        // 24 / 28 KB
-constexpr uint32_t ex_b_slice(int S) { return (uint32_t)ex_cols(S) * kExKTile * 2; }  // 2.5 / 2 KB
-constexpr uint32_t ex_b_bytes(int S) { return S * ex_b_slice(S); }                    // 15 / 14 KB
+// S slices (digits) per value and at most so many B' rows per slice, such that
+// the S accumulators fit tensor memory's 512 columns: 6 x 80 (40 complex bands,
+// Re and Im interleaved, or 80 real ones) or 7 x 64.  ex_pick_cols takes fewer (48
+// or 64) where they pad the bands less.
+constexpr int ex_max_cols(int S) { return S == 6 ? 80 : 64; }
+int ex_pick_cols(int S, int b_rows);
+constexpr uint32_t ex_a_bytes(int S) { return S * kExASlice; }                                 // 24 / 28 KB
+constexpr uint32_t ex_b_slice(int cols) { return (uint32_t)cols * kExKTile * 2; }              // 1.5 to 2.5 KB
+constexpr uint32_t ex_b_bytes(int S, int cols) { return S * ex_b_slice(cols); }                // 9 to 15 KB
 // Exponent slack of the overlap check: an element counts as large when its
 // larger part is within 2^-slack of its row's maximum.
 constexpr int kExSlackA = 4, kExSlackB = 3;
@@ -64,7 +66,7 @@ constexpr int kExZeroRow = 4096; // exponent of a row without a nonzero value (i
 struct ExactPrep {
   unsigned char* a_tiles;   // [n_row_blocks][halves*kt][slices][128][16] bf16
   unsigned char* b_tiles;   // [n_col_blocks][halves*kt][slices][cols][16] bf16
-  int slices, cols;         // 6 and 80, or 7 and 64
+  int slices, cols;         // 6 and 48, 64 or 80, or 7 and 64
   int halves, kt;           // K tiles per half (K padded to 32: an even count)
   int bands;                // bands per column block (cols / 2 complex, cols real)
   int n_row_blocks, n_col_blocks;

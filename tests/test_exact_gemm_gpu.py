@@ -87,6 +87,8 @@ def test_out_of_range_operands_take_the_fp64_kernel(sigma_lib, kind):
     # number_bands, nvband, ncouls, ngpown, stress: 16-column tiles, 64- and 512-g-vector segments, padding rows
     (40, 1, 4096, 64, False), (39, 2, 1985, 43, True), (41, 0, 513, 129, False), (100, 3, 511, 85, False),
     (1, 1, 32767, 43, False), (81, 8, 2049, 17, True), (300, 2, 4000, 3, False), (512, 0, 63, 63, False),
+    (24, 2, 4097, 33, False), (25, 3, 4095, 31, False), (32, 0, 4100, 31, True), (64, 5, 1991, 40, False),
+    (128, 2, 1023, 41, True),
 ], ids=lambda c: "x".join(map(str, c[:4])) + ("s" if c[4] else ""))
 def test_gpp_band_sums_edges(sigma_lib, case):
     nb, nvb, nc, ng, stress = case
