@@ -42,7 +42,7 @@ struct sigma_gpp_plan_s {
   sigma::MixedPrep prep{};    // FP32 operands of the mixed path (unused for FP64)
   void* block = nullptr;      // one device allocation for everything below
   int* igp_of = nullptr;      // [ng]
-  int* counters = nullptr;    // [2] item counters, [2] device status word
+  int* counters = nullptr;    // [2] item counters, [2] device status word, [3] the contraction's flag
   double2* acht_n1 = nullptr; // [nb + nvband][3]
   std::vector<int> host_inv, host_indinv;  // kept for the host drop-in's plan cache
   // optional per-launch timing: events around the main pass, the occupied-band
@@ -270,7 +270,8 @@ extern "C" int sigma_gpp_plan_create(sigma_gpp_plan* plan_out, int number_bands,
   }
   if (!mixed) {
     const GxShape q{kGxGpp, number_bands, nvband, ncouls, ngpown, false};
-    if (gpp_exact_fits(q)) gpp_exact_create(p->exact, q, igp_of, sms);
+    if (gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms))
+      p->exact.ex.flag = p->counters + 3;  // cleared with them
   }
   p->host_inv.assign(inv_igp_index, inv_igp_index + ngpown);
   p->host_indinv.assign(indinv, indinv + ncouls);
@@ -414,7 +415,7 @@ extern "C" int sigma_gpp_execute(sigma_gpp_plan plan, const double* wx_array, in
   GppWork ssx = plan->fused ? plan->fac.ssx : plan->ssx;
   if (exact) {
     main.run_if = ssx.run_if = plan->exact.ex.flag;  // unless it is raised, acht_n1 too
-    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, gx_dev(p), s));
+    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, gx_dev(p), s, false));
   }
   if (ev) SIGMA_CUDA_TRY(cudaEventRecord(ev[0], s));
   if (tensor && plan->fused) {
@@ -630,7 +631,7 @@ int gpp_host(int precision, int nb, int nvband, int nc, int ng, int nstart, int 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // The gated pipeline below pays when the FP64 pass takes much longer than the
   // copies: large instances for whose contraction the device had no room.
-  // Small ones copy whole arrays and run the plan: 24 x 40 x 1024 takes 277 us
+  // Small ones copy whole arrays and run the plan: 24 x 40 x 1024 takes 183 us
   // so, 531 us in ~30 pieces.
   if (precision == SIGMA_PREC_FP64 && plan->schy.n_items > 0 && !plan->exact &&
       gpp_exact_fits(GxShape{kGxGpp, nb, nvband, nc, ng, false})) {

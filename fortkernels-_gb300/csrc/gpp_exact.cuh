@@ -70,7 +70,8 @@ size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, in
 void gpp_exact_destroy(GppExact& g);
 
 // launch_gpp_exact_operands forms the operands and raises g.ex.flag for
-// values outside the split's range (begin: clears the flag first); unless it
+// values outside the split's range (begin: clears the flag first, else the
+// caller has); unless it
 // is raised, launch_gpp_exact_sums leaves the sums in out: [nb][3] (kGxHalf:
 // [2 nb][nf], T then U; kGxHalfOcc: [2 nvband][6], sch then ssx, both
 // weighted 0.5 vcoul; kGxRealOcc: [nvband][3], weighted occ vcoul) and

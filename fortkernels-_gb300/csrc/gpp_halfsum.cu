@@ -1263,8 +1263,9 @@ extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int nu
     } else {
       p->tu = static_cast<double2*>(p->tblock);
       p->tu_occ = p->tu + n;
+      p->exact.ex.flag = p->counters + 3;  // cleared with the counters
       const GxShape qo{kGxHalfOcc, nvband, nvband, ncouls, ngpown, false};
-      if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->exact.ex.flag;
+      if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->counters + 3;
     }
   }
   *out = p;
@@ -1322,7 +1323,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
   }
   HalfDev p{plan->nb, plan->nvband, plan->nc, plan->ng, occ, aqsm, aqsn, ieps, wt,
             vcoul, wx_array, plan->igp_of, plan->brk};
-  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 3 * sizeof(int), s));
+  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 4 * sizeof(int), s));
   if (plan->nvband > 0) {
     half_brk_kernel<<<plan->ng, kThreads, 0, s>>>(p, plan->brk);
     SIGMA_CUDA_TRY(cudaGetLastError());
@@ -1379,7 +1380,7 @@ extern "C" int sigma_gpp_halfsum_execute(sigma_gpp_halfsum_plan plan, const doub
     const GxDev x{plan->nb, plan->nvband, plan->nc, plan->ng, occ,      D(aqsm),       D(aqsn),
                   D(ieps),  D(wt),        vcoul,    wx_array, plan->igp_of, plan->brk};
     // one flag for both contractions
-    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s));
+    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s, false));
     if (plan->exact_occ) SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact_occ, x, s, false));
     SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->tu, nullptr, s));
     if (plan->exact_occ)

@@ -419,9 +419,10 @@ extern "C" int sigma_gpp_real_plan_create(sigma_gpp_real_plan* out, int number_b
     return SIGMA_ERR_CUDA;
   }
   const GxShape q{kGxReal, number_bands, nvband, ncouls, ngpown, false};
-  if (gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms) && nvband > 0) {
+  if (gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms)) {
+    p->exact.ex.flag = p->counters + 3;  // cleared with the counters
     const GxShape qo{kGxRealOcc, nvband, nvband, ncouls, ngpown, false};
-    if (gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->exact.ex.flag;
+    if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->counters + 3;
   }
   *out = p;
   return SIGMA_OK;
@@ -456,11 +457,11 @@ extern "C" int sigma_gpp_real_execute(sigma_gpp_real_plan plan, const double* wx
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GppRealDev p{plan->nb, plan->nvband, plan->nc, plan->ng, occ, aqsmtemp, aqsntemp, I_eps_array,
                wtilde_array, vcoul, wx_array, plan->igp_of};
-  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 3 * sizeof(int), s));
+  SIGMA_CUDA_TRY(cudaMemsetAsync(plan->counters, 0, 4 * sizeof(int), s));
   GppWork sch = plan->sch, ssx = plan->ssx;
   if (plan->exact) {
     const GxDev x{p.nb, p.nvband, p.nc, p.ng, p.occ, p.aqsm, p.aqsn, p.ieps, p.wt, p.vcoul, p.wx, p.igp_of};
-    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s));
+    SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact, x, s, false));
     if (plan->exact_occ) SIGMA_CUDA_TRY(launch_gpp_exact_operands(plan->exact_occ, x, s, false));
     SIGMA_CUDA_TRY(launch_gpp_exact_sums(plan->exact, x, plan->counters + 2, plan->acht_n1, nullptr, s));
     sch.run_if = plan->exact.ex.flag;
