@@ -15,12 +15,11 @@ device.  One step = one full evaluation of achtemp / asxtemp / acht_n1_loc.
   mixed      the mixed-precision path on the same inputs, its Gterms/s and
              the relative error of every achtemp / asxtemp output against the
              FP64 path (and on the stress fill with 5% near-pole wtilde)
-  roofline   the main FP64 kernel (sch_fp64y_kernel): the FP64 pipe work its
-             algorithm issues per term (1.34 operations: the FP64 sums of the
-             float-float terms plus the shared frequency factor) over
-             its CUDA-event time, against the FP64 pipe peak (2 DFMA / clk / SM
-             at the SM clock sampled during the timed region); the reference's
-             27 flop per term is reported beside it as a rate
+  roofline   the FP64 band sums' contraction (exact_gemm_kernel with its
+             epilogue): the BF16 work of its 21 digit products per real
+             FP64 product over its CUDA-event time, against the measured dense
+             BF16 peak; the reference's 27 flop per term is reported beside it
+             as a rate
   rel_err_vs_oracle  every achtemp / asxtemp output (and acht_n1_loc) of each
              form against the CPU oracle's full outputs of the same seeded
              inputs (tests/golden/config_*.npz)
@@ -118,7 +117,7 @@ class ClockSampler:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--query-gpu={','.join(self.FIELDS)}", "--format=csv,noheader,nounits",
-                 "-i", str(self.index), "-lms", "200"],
+                 "-i", str(self.index), "-lms", "20"],
                 stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
         except (OSError, ValueError):
             self.proc = None
@@ -129,6 +128,14 @@ class ClockSampler:
     def _read(self):
         for line in self.proc.stdout:
             self.lines.append(line.strip())
+
+    def wait_live(self, run, limit=2.0):
+        """Runs untimed steps until the first sample arrives, then forgets the
+        samples so far: a timed region of a tenth of a second holds several."""
+        t0 = time.perf_counter()
+        while self.proc is not None and not self.lines and time.perf_counter() - t0 < limit:
+            run()
+        self.lines.clear()
 
     def stop(self):
         if self.proc is None:
@@ -298,28 +305,16 @@ def timed(torch, dist, world, fn, steps, stream):
     return ms
 
 
-# FMA-pipe (FP32) lane operations of sch_fp64y_kernel per term, counted from
-# its algorithm: 24 paired (f32x2) instructions per term (two products, six
-# FMAs of their exact errors and cross terms, one addition, a TwoSum of the
-# products, the low sum, a TwoSum into the chunk's float-float sum and two
-# additions of its low pair) = 48 lane operations, + the negated high pairs of
-# the frequency factors (2 paired per column, frequency and g-vector over 4
-# bands: 1 per term) + the chunk-end renormalisation (3 paired per output and
-# 16-g-vector chunk: 0.375 per term).
-FP64_FMA_LANE_OPS_PER_TERM = 48.0 + 1.0 + 6.0 / 16
-# FP64 pipe operations per term: the frequency factor in FP64 (~40 per column
-# and g-vector over 64 bands x 3 frequencies = 192 terms) + the chunk-end
-# addition of the float-float sums' high pairs (2 per output and 16-g-vector
-# chunk).
-FP64_PIPE_OPS_PER_TERM = 40.0 / 192 + 2.0 / 16
-# ncu, sch_fp64y_kernel, 128-band capture of the production instance
-# (--set full): dram__bytes_read.sum + dram__bytes_write.sum per term, and
-# sm__pipe_fma_cycles_active / sm__pipe_fp64_cycles_active over elapsed
-# cycles.  Traffic scales with the band blocks, so the per-term figure
-# carries to the 512-band launch.
-FP64_DRAM_BYTES_PER_TERM = 0.1975
-FP64_FMA_PIPE_ACTIVE_NCU = 0.713
-FP64_PIPE_ACTIVE_NCU = 0.297
+# BF16 work of exact_gemm_kernel per term (one complex product): 4 real
+# products of 21 digit products, 2 flop each.
+EXACT_BF16_FLOP_PER_TERM = 2.0 * 4 * 21
+# ncu, exact_gemm_kernel, 80 bands x 1638 columns x 16384 g-vectors with the two
+# occupied bands: DRAM bytes (read + write) per 128-row x 16-K' tile of A digits (24 KB),
+# and sm__pipe_tensor_cycles_active.  The band blocks running at one time share
+# A's tiles in L2, so the traffic of a launch is A's digits once per pass over
+# its bands.
+EXACT_DRAM_BYTES_PER_A_BYTE = 1.06
+EXACT_TENSOR_PIPE_ACTIVE_NCU = 0.673
 # FP32 pipe operations of sch_mixedy_kernel per term: 4 FFMA (complex
 # multiply-add) + the float-float fold of each accumulator every 8 g-vectors
 # (2 x 7 operations / 8) + the shared frequency factor (~10 per column,
@@ -806,6 +801,8 @@ def run_ours(args, rank, world, local_rank):
     plan.set_timing(True)
     clocks = ClockSampler(local_rank)
     clocks.start()
+    clocks.wait_live(lambda: (inst.run(plan, sptr), torch.cuda.synchronize()))
+    plan.timing()  # forgets the untimed executions
     ms = timed(torch, dist, world, lambda: inst.run(plan, sptr), args.steps, stream)
     clk = clocks.stop()
     kt = plan.timing()
@@ -815,8 +812,10 @@ def run_ours(args, rank, world, local_rank):
     value = terms * world / (ms_step * 1e-3) / 1e9
     main_s = kt["main_ms"] / max(1, kt["executions"]) * 1e-3
     algorithmic_tflops = FLOP_PER_TERM * terms / main_s / 1e12
-    pipe_tflops = 2 * FP64_FMA_LANE_OPS_PER_TERM * terms / main_s / 1e12
-    fp64_pipe_tflops = 2 * FP64_PIPE_OPS_PER_TERM * terms / main_s / 1e12
+    occupied_terms = terms // NB * NVB  # their factors are further rows of the contraction
+    exact_tflops = EXACT_BF16_FLOP_PER_TERM * (terms + occupied_terms) / main_s / 1e12
+    exact_peak, exact_peak_source = bf16_peak()
+    exact_a_bytes = 6.0 * NG * 2 * NC * 6 * 2  # six factors' digits
     production = (NB, NVB, NC, NPG) == PRODUCTION
     ref_prod = golden("config_gpp_production.npz") if production else None
     ref_stress = golden("config_gpp_stress.npz") if production else None
@@ -948,35 +947,24 @@ def run_ours(args, rank, world, local_rank):
         "e2e": {"value": (round(e2e_value, 4) if e2e_steps else None), "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps,
                 "path": "sigma_gpp_fp64 host C ABI, pinned buffers", "matches_device_path": e2e_match},
-        "roofline": {"bound": "fp32_pipe", "kernel": "sch_fp64y_kernel",
-                     "achieved": round(pipe_tflops, 4), "peak": round(fp32_pipe_peak, 4), "unit": "TFLOP/s",
-                     "frac": round(pipe_tflops / fp32_pipe_peak, 4),
-                     "traffic": round(FP64_DRAM_BYTES_PER_TERM * terms),
+        "roofline": {"bound": "tensor_pipe", "kernel": "exact_gemm_kernel",
+                     "achieved": round(exact_tflops, 4), "peak": exact_peak, "unit": "TFLOP/s",
+                     "frac": round(exact_tflops / exact_peak, 4),
+                     "traffic": round(EXACT_DRAM_BYTES_PER_A_BYTE * exact_a_bytes),
                      "kernel_ms_per_launch": round(main_s * 1e3, 3),
-                     "fma_lane_ops_per_term": round(FP64_FMA_LANE_OPS_PER_TERM, 4),
-                     "peak_source": f"FMA pipe 128 lanes/clk/SM x {sms} SMs x {clock_mhz:.0f} MHz, 2 flop "
-                                    "per lane operation (SM clock sampled during the timed region; the "
-                                    "measured-peaks file has no FP32 figure)",
-                     "ncu_fma_pipe_active": FP64_FMA_PIPE_ACTIVE_NCU,
-                     "fp64_pipe": {"achieved": round(fp64_pipe_tflops, 4), "peak": round(fp64_pipe_peak, 4),
-                                   "frac": round(fp64_pipe_tflops / fp64_pipe_peak, 4),
-                                   "ops_per_term": round(FP64_PIPE_OPS_PER_TERM, 4),
-                                   "ncu_active": FP64_PIPE_ACTIVE_NCU,
-                                   "peak_source": f"FP64 pipe 2 DFMA/clk/SM x {sms} SMs at the sampled clock; "
-                                                  f"dependent-FMA probe on this device: {fp64_peak:.3f} TFLOP/s"},
+                     "bf16_flop_per_term": EXACT_BF16_FLOP_PER_TERM,
+                     "peak_source": exact_peak_source,
+                     "ncu_tensor_pipe_active": EXACT_TENSOR_PIPE_ACTIVE_NCU,
                      "algorithmic": {"flop_per_term": FLOP_PER_TERM,
                                      "tflops": round(algorithmic_tflops, 4),
                                      "note": "the reference's 27 flop per term (its own formulation, which "
                                              "rebuilds the frequency factor for every band) at the measured "
                                              "term rate: a rate, not a pipe fraction"},
-                     "note": "achieved = FMA-pipe work of the kernel's own algorithm (each lane operation "
-                             "one FMA slot, 2 flop): with one frequency set for all bands the frequency "
-                             "factor is formed in FP64 once per column and g-vector and split to float-float; "
-                             "every term is a float-float product in paired FP32 instructions (real and "
-                             "imaginary parts as the two lanes), added exactly (TwoSum) to a per-chunk "
-                             "float-float sum whose high pair is added to the FP64 sums every 16 g-vectors; "
-                             "the FP64 pipe carries the factor and those additions (fp64_pipe); "
-                             "traffic = ncu DRAM bytes per term x terms"},
+                     "note": "achieved = BF16 work of the digit products (21 per real product, of 8 to 9 bits "
+                             "each, summed exactly) of the band sums and the occupied bands' sums over the "
+                             "time of the contraction and its epilogue; the factors and digits are formed "
+                             "before it (ms_per_step - kernel_ms_per_launch); traffic = ncu DRAM bytes per "
+                             "byte of A digits x A digits"},
         "rel_err_vs_oracle": oracle,
         "mixed": {"value": round(mixed_value, 4), "unit": UNIT,
                   "speedup_vs_fp64": round(mixed_value / value, 3),

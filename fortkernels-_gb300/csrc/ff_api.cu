@@ -226,7 +226,9 @@ extern "C" int sigma_ff_plan_timing(sigma_ff_plan plan, int* executions, double*
   if (executions) *executions = n;
   if (main_ms) *main_ms = tm;
   if (other_ms) *other_ms = to;
-  if (launches_per_execution) *launches_per_execution = plan->mode == SIGMA_FF_FP64 ? 2 : 4;
+  // FP64: two for each exact operand, the contraction, its epilogue (2), and the
+  // FP64 kernels it stands in for
+  if (launches_per_execution) *launches_per_execution = plan->mode == SIGMA_FF_FP64 ? (plan->ex_block ? 9 : 2) : 4;
   plan->recorded = 0;
   return SIGMA_OK;
 }

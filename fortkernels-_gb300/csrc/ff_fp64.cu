@@ -1,5 +1,6 @@
-// FF schDt contraction, FP64 form (sm_103a), and the fixed-order reduction
-// shared by both FF forms.
+// FF schDt contraction with FP64 multiply-adds (sm_103a), for sums too small for the
+// exact contraction (exact_gemm.cu) or outside its range, and its fixed-order
+// reduction.
 //
 // tempz[(ifreq, my_igp), n1] = sum_ig I_epsR[ifreq][my_igp][ig] * aqsn[n1][ig] is a
 // complex GEMM (M = nfreq*ngpown, N = number_bands, K = ncouls); the reference

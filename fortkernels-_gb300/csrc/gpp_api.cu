@@ -346,7 +346,7 @@ extern "C" int sigma_gpp_plan_timing(sigma_gpp_plan plan, int* executions, doubl
       // epilogue factors included), GEMM, its reduction, 2 reductions
       *launches_per_execution = plan->fused ? 1 + 2 + 2 : (occ ? 2 : 1) + pad + 2 + 2 + (occ ? 1 : 0) + 2;
     } else
-      *launches_per_execution = (plan->sch.n_items > 0 ? (mixed ? 3 : 1) : 0) +
+      *launches_per_execution = sigma::gpp_exact_launches(plan->exact) + (plan->sch.n_items > 0 ? (mixed ? 3 : 1) : 0) +
                                 (plan->ssx.n_items > 0 ? 1 : 0) + 2;
   }
   plan->recorded = 0;

@@ -20,6 +20,11 @@
 // bands take the earlier form instead: per-instance contractions in stream
 // order over one shared slice workspace, occupied bands in a separate pass.
 //
+// The FP64 form with one frequency set per instance runs each instance's exact
+// contraction (gpp_exact.cu) in turn over one shared workspace; the persistent
+// kernels then take only the instances whose contraction raised its flag or
+// has none.
+//
 // The FP64 and mixed forms reduce all instances with the grouped reduction
 // (two launches).
 #include <algorithm>

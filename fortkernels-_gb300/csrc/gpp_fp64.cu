@@ -1,4 +1,7 @@
-// GPP sigma sum, plain FP64 path (sm_103a).
+// GPP sigma sum, FP64 path (sm_103a): per-band frequencies; and, for one
+// frequency set, the passes that run where the exact contraction
+// (gpp_exact.cu) has no room, is not worth its launches or finds its operands
+// outside its range.
 //
 // Replaces the band / column / g-vector / frequency loop nest of
 // BGW-Kernels/gppKer.cpp:303-439.  Work is cut into items (BN bands x BP

@@ -34,7 +34,9 @@
 // Items past a column block's range write zero partials.  Occupied bands run
 // one CTA per (column, frequency).  All partials have fixed slots and are
 // summed in a fixed order with compensation: results are identical run to
-// run.
+// run.  From 2^23 products on the FP64 form takes T, U and the occupied bands'
+// sums from two exact contractions (gpp_exact.cu) instead, and these passes run
+// only where those find their operands outside their range.
 #include <algorithm>
 #include <cstring>
 #include <mutex>

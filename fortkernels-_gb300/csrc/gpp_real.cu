@@ -20,6 +20,9 @@
 // complex path's fixed slots and reduction (imaginary parts zero); the
 // outputs are their real parts.
 //
+// These passes run where the exact contractions (gpp_exact.cu) have no room, are
+// not worth their launches or find their operands outside their range.
+//
 // Where the reference's unoccupied loop adds a stale scha[ig] from an
 // earlier frequency or g-vector block for a dropped term
 // (gppKer_real.cpp:367-371 writes scha only when the guard passes), this

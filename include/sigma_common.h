@@ -40,7 +40,7 @@ enum sigma_status {
 
 /* Arithmetic forms. */
 enum sigma_precision {
-  SIGMA_PREC_FP64 = 0,  /* plain FP64: every term in double precision */
+  SIGMA_PREC_FP64 = 0,  /* FP64 results: exact digit contractions, float-float or FP64 terms */
   SIGMA_PREC_MIXED = 1, /* FP32 bulk, FP64 pole-guard decisions, compensated FP64 reductions */
   SIGMA_PREC_TENSOR = 2 /* one frequency set for all bands only: the band sum as a complex GEMM
                            on tcgen05 tensor cores (split-BF16 operands, FP32 accumulation
