@@ -23,7 +23,7 @@
 // into a four-stage shared ring, up to three tiles ahead of the tensor
 // cores; warp 6 waits for each tile's stage (and for the accumulator pair
 // to be drained) and releases warp 5 through a named barrier; warp 5 lane 0
-// issues 12 tcgen05.mma (M=128, N=128, K=16) per tile and releases each
+// issues 10 tcgen05.mma (M=128, N=128 or 256, K=16) per tile and releases each
 // stage with tcgen05.commit; warps 0-3 drain TMEM and run the epilogue,
 // which multiplies tempz by conj(aqsm[n1][igp(my_igp)]) and sums the tile's
 // rows per frequency (:408-418) with a reduce-scatter butterfly.  Items are
