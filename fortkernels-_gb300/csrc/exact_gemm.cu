@@ -1,27 +1,32 @@
 // Exact digit contraction (exact_gemm.cuh): operand checks and digits, the
 // tcgen05 kernel, and the FP64 epilogue.
 //
-// The contraction kernel.  A CTA takes one (128 rows x 80 B' rows x K range;
-// 64 or 48 B' rows where they pad the bands less) item at a time.  Per 16-K tile the 21 digit products run as nine MMAs: the
-// B slices are stacked along N, so A_i times [B_j .. B_k] fills the adjacent
-// accumulators s = i + j .. i + k in one instruction (N up to 240), which
-// reads A from shared memory once for up to three products (107 bytes per
-// clock of the 128 available; one MMA per product would need 166).  TMEM
-// holds the six accumulators (480 of 512 columns).  They live 128 K values;
-// the nine MMAs are issued as two groups (s = 0..2, then s = 3..5) over pairs
-// of tiles, so that one group's accumulators are read while the other
-// group's products run.  Eight drain warps convert the FP32 integers and add
-// them to 64-bit integer sums (s <= 3) and FP32 sums (s = 4, 5) in registers,
-// no FP64 operation (2 per clock per SM on this part); an item ends with its
-// raw sums written out, and exact_finish_kernel forms the weighted FP64 sums.
+// The contraction kernel.  A CTA takes one (128 rows x 80 B' rows x K range; 64
+// or 48 B' rows where they pad the bands less) item at a time.  Per 16-K tile
+// the 21 digit products run as nine MMAs: the B slices are stacked along N, so
+// A_i times [B_j .. B_k] fills the adjacent accumulators s = i + j .. i + k in
+// one instruction (N up to 240), which reads A from shared memory once for up
+// to three products (107 bytes per clock of the 128 available; one MMA per
+// product would need 166).  TMEM holds the six accumulators (480 of 512
+// columns).  They live 128 K values; the nine MMAs are issued as two groups (s
+// = 0..2, then s = 3..5) over three, two and three tiles, so that one group's
+// accumulators are read while the other group's products run: reading them
+// costs 18 % of the kernel with pairs of tiles and eight reading warps, whose
+// windows (the first group's products over two tiles) are too short, 15 % so.
+// Sixteen drain warps convert the FP32 integers and add them to 64-bit integer
+// sums (s <= 3) and FP32 sums (s = 4, 5) in registers, no FP64 operation (2 per
+// clock per SM on this part); an item ends with its raw sums written out, and
+// exact_finish_kernel forms the weighted FP64 sums.
 //
-// Measured: the FF contraction of 512 x (15 x 820) x 16384 in 13.2 ms, 555 ms
-// with FP64 multiply-adds (ff_fp64.cu); normwise error 2.8e-15 (5e-15).
+// Measured: the kernel at 512 bands x 4914 rows x 65536 K' with the occupied
+// rows 9.31 -> 8.93 ms with the longer windows; the FF contraction of 512 x (15
+// x 820) x 16384 in 12.8 ms, 555 ms with FP64 multiply-adds (ff_fp64.cu);
+// normwise error 2.8e-15 (5e-15).
 //
-// Roles (352 threads): warps 0-7 drain, warp 8 streams 39 KB tiles (one bulk
-// copy per operand) into a five-stage ring, warp 10 waits for the stages and
-// the accumulators and releases warp 9, which issues the MMAs (the issuing
-// thread polls no shared memory, which would stall the tensor pipe).
+// Roles (608 threads): warps 0-15 drain, warp 16 streams 39 KB tiles (one bulk
+// copy per operand) into a ring of five or six stages, warp 18 waits for the
+// stages and the accumulators and releases warp 17, which issues the MMAs (the
+// issuing thread polls no shared memory, which would stall the tensor pipe).
 #include <algorithm>
 #include <climits>
 
@@ -32,12 +37,21 @@ namespace {
 
 using namespace tma;
 
-constexpr int kThreadsEx = 352;
-constexpr int kCopyWarp = 8, kIssueWarp = 9, kGateWarpEx = 10;
-constexpr int kStagesEx = 5;
+constexpr int kDrainWarps = 16;
+constexpr int kCopyWarp = kDrainWarps, kIssueWarp = kDrainWarps + 1, kGateWarpEx = kDrainWarps + 2;
+constexpr int kThreadsEx = (kDrainWarps + 3) * 32;
 constexpr uint32_t ex_stage(int S, int cols) { return ex_a_bytes(S) + ex_b_bytes(S, cols); }  // 33 to 42 KB
-constexpr uint32_t ex_smem(int S, int cols) { return kStagesEx * ex_stage(S, cols) + 1024; }
-constexpr int kBlockTiles = 8;  // K tiles per accumulator lifetime (128 K values)
+// Stages of the ring: five, or six where they fit 227 KB (48 and 64 columns of six slices).
+constexpr int ex_stages(int S, int cols) { return 6 * ex_stage(S, cols) + 1024 <= 227 * 1024 ? 6 : 5; }
+constexpr uint32_t ex_smem(int S, int cols) { return ex_stages(S, cols) * ex_stage(S, cols) + 1024; }
+constexpr int kBlockTiles = 8;  // K tiles per accumulator lifetime (128 K values),
+// taken in groups of three, two and three tiles from tile s of an item on, or,
+// where the ring holds too few for that (seven slices), in pairs
+template <int S>
+__device__ __forceinline__ int ex_group(int s, int nst) {
+  const int n = S == 7 || s % kBlockTiles == 3 ? 2 : 3;
+  return min(n, nst - s);
+}
 
 // 32-byte swizzle: rows of 16 elements (32 B), 8-row groups of 256 B (layout
 // code 6 in bits 61-63).
@@ -68,15 +82,23 @@ __device__ __forceinline__ bool gate_sync(bool flag) {
   return r != 0;
 }
 
-// 8 consecutive TMEM columns of this warp's 32 lanes (no wait).
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-  uint32_t r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
+// W (8 or 4) consecutive TMEM columns of this warp's 32 lanes (no wait).
+template <int W>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[W]) {
+  static_assert(W == 8 || W == 4, "columns per load");
+  uint32_t r[W];
+  if constexpr (W == 8)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+  else
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < W; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -102,12 +124,46 @@ __device__ __forceinline__ ExItem ex_decode(const ExactPrep& ex, int item) {
 
 constexpr uint32_t idesc_n(int n) { return idesc_bf16_f32(128, n); }
 
+// Columns Q .. Q + W of a drain: the lo accumulators (s = 0 .. 2) into the 64-bit
+// sums, the hi ones (s = 3 on) into those and the FP32 sums.
+template <int kCols, int Q, int W, int N>
+__device__ __forceinline__ void drain_lo(uint32_t t, long long (&hi)[N]) {
+  float v0[W], v1[W], v2[W];
+  tmem_ld<W>(t + Q, v0);
+  tmem_ld<W>(t + kCols + Q, v1);
+  tmem_ld<W>(t + 2 * kCols + Q, v2);
+  tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    // |v0| <= 2^21: its integer from the bits of v0 + 1.5 * 2^23 (a conversion
+    // takes three to four issue slots' time)
+    const int i0 = __float_as_int(v0[i] + 12582912.f) - 0x4B400000;
+    const int u = i0 * 512 + __float2int_rn(v1[i]);  // below 2^31
+    hi[Q + i] += (long long)u * (1 << 18) + (long long)__float2int_rn(v2[i]) * 512;
+  }
+}
+template <int kHi, int kCols, int Q, int W, int N>
+__device__ __forceinline__ void drain_hi(uint32_t t, long long (&hi)[N], float (&lo)[N]) {
+  float v[kHi][W];
+#pragma unroll
+  for (int d = 0; d < kHi; ++d) tmem_ld<W>(t + (3 + d) * kCols + Q, v[d]);
+  tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    hi[Q + i] += __float2int_rn(v[0][i]);
+    float f = v[kHi - 1][i];
+#pragma unroll
+    for (int d = kHi - 2; d >= 1; --d) f = fmaf(f, 1.f / 512.f, v[d][i]);
+    lo[Q + i] = fmaf(f, 1.f / 512.f, lo[Q + i]);
+  }
+}
+
 template <int S, int kCols>
 __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex, int* status) {
-  constexpr int kColsHalf = kCols / 2, kHi = S - 3;  // kHi accumulators from s = 3 on
+  constexpr int kColsQ = kCols / 4, kStagesEx = ex_stages(S, kCols), kHi = S - 3;  // kHi accumulators from s = 3 on
   constexpr uint32_t kStage = ex_stage(S, kCols), kABytes = ex_a_bytes(S), kBBytes = ex_b_bytes(S, kCols),
                      kBSlice = ex_b_slice(kCols);
-  static_assert(kCols % 16 == 0 && S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
+  static_assert(kCols % 16 == 0 && kColsQ >= 8 && kColsQ <= 20 && S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
   extern __shared__ unsigned char smem_raw[];
   // full[5], empty[5], lo full, hi full, lo empty, hi empty, done
   __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
@@ -125,8 +181,8 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
   if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 512);
   if (tid == 0) {
     for (int i = 0; i < 2 * kStagesEx + 2; ++i) mbar_init(smem_u32(&bars[i]), 1);
-    mbar_init(acce, 8);
-    mbar_init(acce + 8u, 8);
+    mbar_init(acce, kDrainWarps);
+    mbar_init(acce + 8u, kDrainWarps);
     mbar_init(done0, 1);
     fence_mbar_init();
   }
@@ -163,17 +219,18 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
     }
     __syncwarp();
   } else if (warp == kGateWarpEx) {
-    // per pair of tiles: both stages full; at a block's first pair also the
+    // per group of tiles: its stages full; at a block's first group also the
     // lo accumulators drained, and (second meeting) the hi accumulators
     bool failed = false;
     uint32_t g = 0, blk = 0;  // tiles and accumulator lifetimes so far
     for (int item = blockIdx.x; item < ex.n_items; item += gridDim.x) {
       const int nst = ex_decode(ex, item).nst;
-      for (int s = 0; s < nst; s += 2, g += 2) {
+      for (int s = 0, n; s < nst; s += n, g += n) {
+        n = ex_group<S>(s, nst);
         const bool first = s % kBlockTiles == 0;
         if (lane == 0 && !failed) {
           if (first && blk > 0) failed = !mbar_wait(acce, (blk - 1) & 1u, status);
-          for (uint32_t t = g; t < g + 2 && !failed; ++t)
+          for (uint32_t t = g; t < g + n && !failed; ++t)
             failed = !mbar_wait(full0 + 8u * (t % kStagesEx), (t / kStagesEx) & 1u, status);
         }
         __syncwarp();
@@ -197,14 +254,14 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
     bool failed = false;
     for (int item = blockIdx.x; item < ex.n_items; item += gridDim.x) {
       const int nst = ex_decode(ex, item).nst;
-      for (int s = 0; s < nst; s += 2, g += 2) {
+      for (int s = 0, n; s < nst; s += n, g += n) {
+        n = ex_group<S>(s, nst);
         const bool first = s % kBlockTiles == 0;
-        const bool last = s % kBlockTiles == kBlockTiles - 2 || s + 2 >= nst;
+        const bool last = (s + n) % kBlockTiles == 0 || s + n >= nst;
         failed = gate_sync(false) || failed;
         if (lane == 0 && !failed) {
           tc_fence_after();
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
+          for (int q = 0; q < n; ++q) {
             const uint32_t a = sbase + ((g + q) % kStagesEx) * kStage, b = a + kABytes;
             const uint64_t b0 = sw32_desc(b);
             mma_f16(tmem, sw32_desc(a), b0, idesc_n(3 * kCols), first && q == 0 ? 0u : 1u);
@@ -218,8 +275,7 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         if (lane == 0 && !failed) {
           tc_fence_after();
           const uint32_t d = tmem + 3 * kCols;
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
+          for (int q = 0; q < n; ++q) {
             const uint32_t st = (g + q) % kStagesEx;
             const uint32_t a = sbase + st * kStage, b = a + kABytes;
             // A_i times the B slices j with 3 <= i + j < S
@@ -244,15 +300,15 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
     }
     __syncwarp();
   } else {
-    const int half = warp >> 2, row = (warp & 3) * 32 + lane;
-    const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + half * kColsHalf;
+    const int quarter = warp >> 2, row = (warp & 3) * 32 + lane;
+    const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + quarter * kColsQ;
     uint32_t blk = 0;
     for (int item = blockIdx.x; item < ex.n_items; item += gridDim.x) {
       const ExItem it = ex_decode(ex, item);
-      long long hi[kColsHalf];
-      float lo[kColsHalf];
+      long long hi[kColsQ];
+      float lo[kColsQ];
 #pragma unroll
-      for (int i = 0; i < kColsHalf; ++i) {
+      for (int i = 0; i < kColsQ; ++i) {
         hi[i] = 0;
         lo[i] = 0.f;
       }
@@ -261,46 +317,24 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
       for (int c = 0; c < nblk; ++c, ++blk) {
         mbar_wait(accf, blk & 1u, status);
         tc_fence_after();
-#pragma unroll
-        for (int q = 0; q < kColsHalf / 8; ++q) {
-          float v0[8], v1[8], v2[8];
-          tmem_ld8(tl + q * 8, v0);
-          tmem_ld8(tl + kCols + q * 8, v1);
-          tmem_ld8(tl + 2 * kCols + q * 8, v2);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int u = __float2int_rn(v0[i]) * 512 + __float2int_rn(v1[i]);  // below 2^31
-            hi[q * 8 + i] += (long long)u * (1 << 18) + (long long)__float2int_rn(v2[i]) * 512;
-          }
-        }
+        drain_lo<kCols, 0, 8>(tl, hi);
+        if constexpr (kColsQ >= 16) drain_lo<kCols, 8, 8>(tl, hi);
+        if constexpr (kColsQ % 8 == 4) drain_lo<kCols, kColsQ - 4, 4>(tl, hi);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive(acce);
         mbar_wait(accf + 8u, blk & 1u, status);
         tc_fence_after();
-#pragma unroll
-        for (int q = 0; q < kColsHalf / 8; ++q) {
-          float v[kHi][8];
-#pragma unroll
-          for (int d = 0; d < kHi; ++d) tmem_ld8(tl + (3 + d) * kCols + q * 8, v[d]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            hi[q * 8 + i] += __float2int_rn(v[0][i]);
-            float t = v[kHi - 1][i];
-#pragma unroll
-            for (int d = kHi - 2; d >= 1; --d) t = fmaf(t, 1.f / 512.f, v[d][i]);
-            lo[q * 8 + i] = fmaf(t, 1.f / 512.f, lo[q * 8 + i]);
-          }
-        }
+        drain_hi<kHi, kCols, 0, 8>(tl, hi, lo);
+        if constexpr (kColsQ >= 16) drain_hi<kHi, kCols, 8, 8>(tl, hi, lo);
+        if constexpr (kColsQ % 8 == 4) drain_hi<kHi, kCols, kColsQ - 4, 4>(tl, hi, lo);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive(acce + 8u);
       }
-      const size_t base = (it.pidx * kCols + half * kColsHalf) * kExRows + row;
+      const size_t base = (it.pidx * kCols + quarter * kColsQ) * kExRows + row;
 #pragma unroll
-      for (int i = 0; i < kColsHalf; ++i) {
+      for (int i = 0; i < kColsQ; ++i) {
         ex.raw_hi[base + (size_t)i * kExRows] = hi[i];
         ex.raw_lo[base + (size_t)i * kExRows] = lo[i];
       }
