@@ -160,7 +160,8 @@ __device__ __forceinline__ void drain_hi(uint32_t t, long long (&hi)[N], float (
 
 template <int S, int kCols>
 __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex, int* status) {
-  constexpr int kColsQ = kCols / 4, kStagesEx = ex_stages(S, kCols), kHi = S - 3;  // kHi accumulators from s = 3 on
+  constexpr int kColsQ = kCols / 4, kStagesEx = ex_stages(S, kCols), kHi = S - 3,
+                kGroup = S == 7 ? 2 : 3;  // most tiles of ex_group (seven slices: always two)  // kHi accumulators from s = 3 on
   constexpr uint32_t kStage = ex_stage(S, kCols), kABytes = ex_a_bytes(S), kBBytes = ex_b_bytes(S, kCols),
                      kBSlice = ex_b_slice(kCols);
   static_assert(kCols % 16 == 0 && kColsQ >= 8 && kColsQ <= 20 && S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
@@ -261,7 +262,9 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         failed = gate_sync(false) || failed;
         if (lane == 0 && !failed) {
           tc_fence_after();
-          for (int q = 0; q < n; ++q) {
+#pragma unroll
+          for (int q = 0; q < kGroup; ++q) {
+            if (kGroup > 2 && q >= n) break;
             const uint32_t a = sbase + ((g + q) % kStagesEx) * kStage, b = a + kABytes;
             const uint64_t b0 = sw32_desc(b);
             mma_f16(tmem, sw32_desc(a), b0, idesc_n(3 * kCols), first && q == 0 ? 0u : 1u);
@@ -275,7 +278,9 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         if (lane == 0 && !failed) {
           tc_fence_after();
           const uint32_t d = tmem + 3 * kCols;
-          for (int q = 0; q < n; ++q) {
+#pragma unroll
+          for (int q = 0; q < kGroup; ++q) {
+            if (kGroup > 2 && q >= n) break;
             const uint32_t st = (g + q) % kStagesEx;
             const uint32_t a = sbase + st * kStage, b = a + kABytes;
             // A_i times the B slices j with 3 <= i + j < S
