@@ -244,23 +244,22 @@ __global__ void __launch_bounds__(kOzThreads, 1) ozaki_gemm_kernel(FfDev p, FfWo
         const uint32_t tb = gc & 1u;
         // stages full, accumulator pair free (or the gate warp gave up)
         if (s % kGateTiles == 0) failed = mma_gate_sync(false) || failed;
+        // descriptors of the tile's first slices (further ones at constant
+        // distances in the address field), formed by the whole warp: inside the
+        // single lane's branch each instruction waits for its operands' moves
+        // (2.34 -> 2.24 ms at 4914 rows x 1024 x 65536)
+        const uint32_t b = g % kStages;
+        const uint64_t da = sw64_desc(sbase + b * kStageBytes), db = da + (kOperandBytes >> 4);
+        const uint32_t d_big = tmem + tb * 256u, d_small = d_big + 128u;
         if (lane == 0 && !failed) {
           tc_fence_after();
-          const uint32_t b = g % kStages;
-          const uint32_t a_addr = sbase + b * kStageBytes;
-          const uint32_t b_addr = a_addr + kOperandBytes;
-          const uint32_t d_big = tmem + tb * 256u, d_small = d_big + 128u;
 #pragma unroll
           for (int kk = 0; kk < kOzKTile / 16; ++kk) {
-            const uint64_t a1 = sw64_desc(a_addr + kk * 32);
-            const uint64_t a2 = sw64_desc(a_addr + kSliceBytes + kk * 32);
-            const uint64_t a3 = sw64_desc(a_addr + 2 * kSliceBytes + kk * 32);
-            const uint64_t b1 = sw64_desc(b_addr + kk * 32);
-            const uint64_t b2 = sw64_desc(b_addr + kSliceBytes + kk * 32);  // and rows 128 .. 255 of b1's
-            const uint64_t b3 = sw64_desc(b_addr + 2 * kSliceBytes + kk * 32);
+            const uint64_t a1 = da + 2 * kk, a2 = a1 + (kSliceBytes >> 4), a3 = a1 + (2 * kSliceBytes >> 4);
+            const uint64_t b1 = db + 2 * kk, b2 = b1 + (kSliceBytes >> 4), b3 = b1 + (2 * kSliceBytes >> 4);
             const uint32_t acc = (cs > 0 || kk > 0) ? 1u : 0u;
-            // A1 [B1 | B2] in one instruction of twice the width, into the two
-            // adjacent accumulators: A1 is read from shared memory once
+            // A1 [B1 | B2] in one instruction of twice the width (B2 follows
+            // B1), into the two adjacent accumulators: A1 is read from shared memory once
             // (44 instead of 48 KB per 384 tensor clocks, at 128 bytes a
             // clock: 2.45 -> 2.34 ms at 4914 rows x 1024 x 65536, the same
             // results)
