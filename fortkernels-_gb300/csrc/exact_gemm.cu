@@ -21,7 +21,7 @@
 // Measured: the kernel at 512 bands x 4914 rows x 65536 K' with the occupied
 // rows 9.31 -> 8.93 ms with the longer windows, 8.45 ms with a
 // leaner issue loop; the FF contraction of 512 x (15
-// x 820) x 16384 in 12.2 ms, 555 ms with FP64 multiply-adds (ff_fp64.cu);
+// x 820) x 16384 in 12.4 ms, 555 ms with FP64 multiply-adds (ff_fp64.cu);
 // normwise error 2.8e-15 (5e-15).
 //
 // Roles (608 threads): warps 0-15 drain, warp 16 streams 39 KB tiles (one bulk

@@ -12,8 +12,8 @@ namespace sigma {
 // The band sums are acht_n1[n][iw] = sum_g 0.5 vcoul conj(aqsm) sum_ig aqsn Y
 // with the band-independent factors Y[iw][g][ig], formed in FP64 once per
 // (column, g-vector) and written as the contraction's A digits.  512 bands x
-// 1638 columns x 32768 g-vectors: 12.2 ms with the occupied bands, 150 ms with
-// float-float terms (sch_fp64y_kernel); 128 x 409 x 8192: 0.48 ms, 3.40 ms.
+// 1638 columns x 32768 g-vectors: 11.8 ms with the occupied bands, 150 ms with
+// float-float terms (sch_fp64y_kernel); 128 x 409 x 8192: 0.46 ms, 3.40 ms.
 // The occupied bands' sums (asxtemp) are the same contraction with other
 // factors, of the first bands only: further rows of it, or, where the kernel
 // they replace was FP64 throughout, a contraction of their own with seven

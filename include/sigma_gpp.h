@@ -90,7 +90,7 @@ int sigma_gpp_mixed(int number_bands, int nvband, int ncouls, int ngpown, int ns
  *   rel_err_out[iw]     = |achtemp[iw] - achtemp_fp64[iw]| / |achtemp_fp64[iw]|
  *   rel_err_out[3 + iw] = the same for asxtemp (0 where both are 0),
  * the mixed outputs being the ones returned.  The check costs one FP64
- * evaluation (about as long as half a mixed one at the production shape), so it
+ * evaluation (about half a mixed one's time at the production shape), so it
  * is a validation mode.  sigma_gpp_mixed keeps the argument list of
  * sigma_gpp_fp64 (no extra argument) so that the two are interchangeable
  * where the reference's loop is replaced (BGW-Kernels/gppKer.cpp:303-439). */
