@@ -161,11 +161,13 @@ __device__ __forceinline__ void drain_hi(uint32_t t, long long (&hi)[N], float (
 
 template <int S, int kCols>
 __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex, int* status) {
-  constexpr int kColsQ = kCols / 4, kStagesEx = ex_stages(S, kCols), kHi = S - 3,
-                kGroup = S == 7 ? 2 : 3;  // most tiles of ex_group (seven slices: always two)  // kHi accumulators from s = 3 on
+  constexpr int kColsQ = kCols / 4, kStagesEx = ex_stages(S, kCols);
+  constexpr int kHi = S - 3;                // accumulators from s = 3 on
+  constexpr int kGroup = S == 7 ? 2 : 3;    // most tiles of ex_group (seven slices: always two)
   constexpr uint32_t kStage = ex_stage(S, kCols), kABytes = ex_a_bytes(S), kBBytes = ex_b_bytes(S, kCols),
                      kBSlice = ex_b_slice(kCols);
-  static_assert(kCols % 16 == 0 && kColsQ >= 8 && kColsQ <= 20 && S * kCols <= 512 && kHi * kCols <= 256, "tensor memory and one MMA's width");
+  static_assert(kCols % 16 == 0 && kColsQ >= 8 && kColsQ <= 20 && S * kCols <= 512 && kHi * kCols <= 256,
+                "tensor memory and one MMA's width");
   extern __shared__ unsigned char smem_raw[];
   // full[5], empty[5], lo full, hi full, lo empty, hi empty, done
   __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
@@ -543,8 +545,8 @@ __device__ __forceinline__ double2 ex_weight(const FfDev& p, int n, int f, int i
   return m[(size_t)(second ? n - p.pair_bands : n) * p.nc + igp];
 }
 
-// One CTA per (row block, pair of bands): tempz of 128 rows x 2 bands from the pieces' raw sums (added as integers, so their order does not
-// matter), times weight * conj(aqsm[n1][igp]), summed over the rows of each
+// One CTA per (row block, pair of bands): tempz of 128 rows x 2 bands from the
+// pieces' raw sums (added as integers, so their order does not matter), times weight * conj(aqsm[n1][igp]), summed over the rows of each
 // frequency in a fixed order.
 constexpr int kFinRow = kExRows + 1, kFinThreads = 256, kFinBands = 2;
 template <bool kReal>

@@ -418,7 +418,8 @@ __device__ __forceinline__ double rcp_signed(double x) {
 
 // The factors of one element, FP64; in_freq: within the frequencies' range.
 template <int kForm>
-__device__ __forceinline__ void gx_f64_factors(const double (&wx)[kNW], const double (&iwx2)[kNW], const FF (&wxf)[kNW], double2 wt, double2 ie, bool in_freq,
+__device__ __forceinline__ void gx_f64_factors(const double (&wx)[kNW], const double (&iwx2)[kNW],
+                                               const FF (&wxf)[kNW], double2 wt, double2 ie, bool in_freq,
                                                double2 (&y)[Form<kForm>::kSlabs]) {
   constexpr bool kOcc = F64<kForm>::kOcc;
   if (!kOcc) y[F64<kForm>::kSlabs - 1] = make_double2(-ie.x, -ie.y);
