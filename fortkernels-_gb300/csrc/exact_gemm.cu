@@ -690,16 +690,17 @@ ExSizes ex_sizes(const ExactPrep& ex) {
 }  // namespace
 
 // B' rows per column block.  A narrower block's MMAs take less time but read A
-// from shared memory as often: 680, 625 and 565 us per block of 80, 64 and
-// 48 rows at 4914 A rows x 65536 K' (DRAM-bound below).  The fewest padded rows win only
-// where the number of blocks stays: 128 bands take four blocks of 64, 2.51 ms
-// there, 2.72 in four of 80; 72 bands two of 80, 1.36 ms, 1.70 in three of 48.
+// from shared memory as often: 620, 530 and 480 us per block of 80, 64 and
+// 48 rows at 4914 A rows x 65536 K' (DRAM-bound below).  The fewest padded rows
+// win mostly where the number of blocks stays: 128 bands take four blocks of
+// 64, 2.11 ms there, 2.5 in four of 80; 72 bands two of 80, 1.24 ms, 1.44 in
+// three of 48.
 int ex_pick_cols(int S, int b_rows) {
   if (S != 6) return ex_max_cols(S);
   int best = 80;
   long long cost = LLONG_MAX;
   for (const int c : {80, 64, 48}) {
-    const long long t = (long long)((b_rows + c - 1) / c) * (c == 80 ? 680 : c == 64 ? 625 : 565);
+    const long long t = (long long)((b_rows + c - 1) / c) * (c == 80 ? 620 : c == 64 ? 530 : 480);
     if (t < cost) {
       cost = t;
       best = c;
