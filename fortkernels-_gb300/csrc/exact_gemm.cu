@@ -381,8 +381,7 @@ __device__ __forceinline__ unsigned ex_mag(const int2* v, size_t k, unsigned& lo
 
 // One CTA per row of values: its exponent (largest part below 2^e) and, per
 // 512-value segment, how many of its first 128 elements are large.  Bands (kB)
-// lower seg_min to their counts and seg_pow to their sums of squares (of the
-// larger parts);
+// lower seg_min to their counts;
 // A rows add up how many large elements must coincide with large elements of
 // every band and raise the flag when they are too few.  Zero rows are exact
 // and pass.
@@ -417,28 +416,15 @@ __global__ void __launch_bounds__(256) exact_stats_kernel(ExactPrep ex, const vo
   int sum = 0;
   for (int s = warp; s < ex.n_kseg; s += 8) {
     int c = 0;
-    float q = 0.f;
-    const int kc = s * kExSeg + kExCount;  // the counted part; bands' powers take the whole segment
-    const int k1 = min(nc, kB ? (s + 1) * kExSeg : kc);
+    const int k1 = min(nc, s * kExSeg + kExCount);  // the counted part
     for (int k = s * kExSeg + lane; k < k1; k += 32) {
       unsigned low;
-      const unsigned d = ex_mag<kReal>(v, k, low);
-      c += k < kc && d >= thr ? 1 : 0;
-      if (kB) {
-        // the larger part over 2^e to 20 bits: exponent d >> 20 against exm + 1
-        const int sh = exm + 1 - (int)(d >> 20);
-        const float f = sh < 100 ? __uint_as_float(((unsigned)(127 - sh) << 23) | ((d & 0xFFFFFu) << 3)) : 0.f;
-        q = fmaf(f, f, q);
-      }
+      c += ex_mag<kReal>(v, k, low) >= thr ? 1 : 0;
     }
     c = __reduce_add_sync(0xffffffffu, c);
-    if (kB)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
     if (lane == 0) {
       if (kB) {
         atomicMin(&ex.seg_min[s], c);
-        atomicMin(&ex.seg_pow[s], __float_as_int(q));
       } else {
         sum += max(0, c + min(ex.seg_min[s], kExCount) - min(kExCount, nc - s * kExSeg));
       }
@@ -483,6 +469,13 @@ __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const 
   }
 }
 
+// The larger part of (re, im) over 2^e, rounded towards zero to 20 bits (|x| < 2^e).
+__device__ __forceinline__ float ex_rel_mag(double re, double im, int e) {
+  const int d = max(__double2hiint(re) & 0x7FFFFFFF, __double2hiint(im) & 0x7FFFFFFF);
+  const int sh = 1023 + e - (d >> 20);
+  return sh < 100 ? __uint_as_float(((unsigned)(127 - sh) << 23) | ((unsigned)(d & 0xFFFFF) << 3)) : 0.f;
+}
+
 template <int S, int kCols, bool kReal>
 __global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const void* b0, int nb0, const void* b1,
                                                             int nb, int nc) {
@@ -515,6 +508,18 @@ __global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const 
       }
     }
     const int e = n < nb ? ex.eb[n] : kExZeroRow;
+    if constexpr (S == 7 && !kReal) {
+      // band_min: the warp's eight bands first (its lanes are 4 chunks x 8
+      // bands of one band block and K tile pair); a band of zeros is exact
+      static_assert(kBands % 8 == 0, "whole warps in a band block");
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float m = e == kExZeroRow ? INFINITY : ex_rel_mag(re[j], im[j], e);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((threadIdx.x & 31) < 4) atomicMin(reinterpret_cast<int*>(&ex.band_min[k0 + j]), __float_as_int(m));
+      }
+    }
     unsigned char* tile = ex.b_tiles + ((size_t)cb * ex.halves * ex.kt + 2 * kp + (ch >> 1)) * kBytes;
     const ExChunk<S> cr = ex_chunk<S>(re, e);
     if (kReal) {
@@ -677,7 +682,7 @@ ExSizes ex_sizes(const ExactPrep& ex) {
   z.b = up256((size_t)ex.n_col_blocks * kts * ex_b_bytes(ex.slices, ex.cols));
   z.ea = up256(sizeof(int) * (size_t)ex.n_row_blocks * kExRows);
   z.eb = up256(sizeof(int) * (size_t)ex.n_col_blocks * ex.bands);
-  z.seg = up256(sizeof(int) * 2 * (size_t)ex.n_kseg);
+  z.seg = up256(sizeof(int) * (size_t)ex_count_words(ex));
   z.hi = up256(sizeof(long long) * slots);
   z.lo = up256(sizeof(float) * slots);
   z.part = up256(sizeof(double2) * blocks * ex.max_seg * ex.bands);
@@ -804,7 +809,7 @@ void exact_bind(ExactPrep& ex, void* work, void* own) {
   ex.ea = reinterpret_cast<int*>(take(z.ea));
   ex.eb = reinterpret_cast<int*>(take(z.eb));
   ex.seg_min = reinterpret_cast<int*>(take(z.seg));
-  ex.seg_pow = ex.seg_min + ex.n_kseg;
+  ex.band_min = reinterpret_cast<float*>(ex.seg_min + ex.n_kseg);
   ex.raw_hi = reinterpret_cast<long long*>(take(z.hi));
   ex.raw_lo = reinterpret_cast<float*>(take(z.lo));
   ex.partial = reinterpret_cast<double2*>(take(z.part));
@@ -833,7 +838,7 @@ cudaError_t exact_begin_flag(const ExactPrep& ex, cudaStream_t s) {
 cudaError_t exact_begin(const ExactPrep& ex, cudaStream_t s) {
   cudaError_t e = exact_begin_flag(ex, s);
   if (e != cudaSuccess) return e;
-  return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * 2 * (size_t)ex.n_kseg, s);
+  return cudaMemsetAsync(ex.seg_min, 0x7f, sizeof(int) * (size_t)ex_count_words(ex), s);
 }
 
 cudaError_t launch_exact_b(const ExactPrep& ex, const void* b0, int nb0, const void* b1, int nb1, int nc,

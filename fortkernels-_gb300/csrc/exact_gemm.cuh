@@ -20,15 +20,21 @@
 // Dropped products (s >= 6) and the digits' own rounding are 2^-53 of the
 // product of the row maxima.
 //
-// Seven digits (28 products, 2^-62) serve operands whose rows hold a few
-// elements far above the rest: the half sum's factors near poles.
+// Seven digits (28 products) serve operands whose rows hold a few elements
+// far above the rest: the half sum's factors near poles.
 //
-// That error is relative to the rows' largest elements.  The statistics passes
-// check that elements within 2^-5 (A) and 2^-4 (B) of their rows' largest meet
-// in at least K / 128 places of every row pair, which bounds it by 2^-41 of
-// the sum's root mean square (2^-47 to 2^-51 on uniform inputs, as the
-// float-float terms or better).  Rows that fail, and values that are not
-// finite, raise ExactPrep::flag, and the callers' FP64 kernels run instead.
+// Over random digits a product's error is 2^-52 (six digits) or 2^-61 (seven)
+// rms of the product of its rows' largest elements, and that of a sum of K
+// products sqrt(K) times it, whatever the elements' own size.  So every row pair
+// is checked for a sum of squares that is large enough beside it.  The
+// statistics passes count that elements within 2^-5 (A) and 2^-4 (B) of their
+// rows' largest meet in at least K / 128 places of every row pair (if all
+// others were zero, the error would be 2^-39.5 of the sum's root mean square
+// with six digits, 2^-48 with seven; uniform inputs: 2^-51 with six).  Rows that fail, and values that are not finite, raise
+// ExactPrep::flag, and the callers' FP64 kernels run instead.  The half sum's
+// rows with factors near poles hold too few large elements for that count;
+// they are checked against band_min, the least element of any band at each K
+// value (gx_check_kernel).
 #pragma once
 
 #include <vector>
@@ -84,7 +90,7 @@ struct ExactPrep {
   int* ea;                  // [n_row_blocks * 128] exponents of the A rows
   int* eb;                  // [n_col_blocks * bands] exponents of the bands
   int* seg_min;             // [n_kseg] over the bands: large elements per segment
-  int* seg_pow;             // [n_kseg] over the bands: least sum of squares per segment, FP32 bits, unit 2^(2 eb)
+  float* band_min;          // [16 kt] least magnitude of the bands per K value, unit 2^eb (complex, seven slices)
   int* flag;                // nonzero: the operands are outside the split's range
   int* any;                 // nullable: raised with flag (one word for a batch)
   long long* raw_hi;        // [row block][col block][piece][cols][128] sums of s <= 3, unit 2^(ea+eb-41)
@@ -97,6 +103,14 @@ struct ExactTables {
   std::vector<int4> entries;
   std::vector<int> pieces, kt_lim;
 };
+
+// Complex contractions of seven digits keep band_min, after seg_min.
+__host__ __device__ __forceinline__ bool ex_has_band_min(const ExactPrep& ex) {
+  return ex.slices == 7 && ex.halves == 2;
+}
+__host__ __device__ __forceinline__ int ex_count_words(const ExactPrep& ex) {
+  return ex.n_kseg + (ex_has_band_min(ex) ? ex.kt * kExKTile : 0);
+}
 
 // Index of a (row block, band block) pair in the raw sums and partials.
 __host__ __device__ __forceinline__ size_t ex_block_index(const ExactPrep& ex, int rb, int cb) {
@@ -159,8 +173,8 @@ __host__ __device__ __forceinline__ uint32_t sw32_offset(int r, int ch) {
 // The overlap counts' start values, by the threads of a grid that precedes
 // launch_exact_b.
 __device__ __forceinline__ void ex_begin_counts(const ExactPrep& ex) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * ex.n_kseg; i += gridDim.x * blockDim.x)
-    ex.seg_min[i] = 0x7f7f7f7f;  // seg_pow follows it
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ex_count_words(ex); i += gridDim.x * blockDim.x)
+    ex.seg_min[i] = 0x7f7f7f7f;  // band_min follows it
 }
 __device__ __forceinline__ void ex_raise(const ExactPrep& ex) {
   *ex.flag = 1;

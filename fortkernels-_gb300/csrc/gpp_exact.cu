@@ -38,12 +38,15 @@ constexpr int kGxCols = 16;  // columns per CTA
 constexpr int kIgBlk = 512;  // g-vector block of the half sum's reference loop
 // Half sum: poles inside the guard make a few factors of a row much larger
 // than the rest, so a count of large ones says little, and the row's exponent
-// serves the rest badly: its operands take seven digits.  Its check compares
-// the sum of squares that each row and the least band share per segment with
-// K: at 2^-30 the estimated error is 2^-48 of the sum's root mean square
-// (taking elements within a segment as unrelated), below the float-float
-// terms', whose factors come from a 2^-45 reciprocal.
-constexpr float kHalfPower = 1.f / 1073741824.f;
+// serves the rest badly: its operands take seven digits.  Its check sums, over
+// the row's own range, the factors' squares times those of the least element
+// that any band has there (ExactPrep::band_min): no row pair's sum of squares
+// is below that.  From 2^-38 K on (units of the rows' largest elements) the
+// error of 2^-61 sqrt(K) is at most 2^-42 of the root mean square.  Uniform
+// inputs with the nearest of 5e7 poles at 7e-5 lie at 2^-32 or above.  (Segment
+// sums of squares of row and bands, multiplied as if unrelated, let a factor of
+// 2^30 through that met zeros: errors of 6e-10.)
+constexpr float kHalfPower = 1.f / 274877906944.f;
 
 template <int kForm>
 struct Form {
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
 }
 
 // ---------------------------------------------------------------- half-sum factors
-// kGxHalf: sums of squares per segment; kGxHalfOcc (sch and ssx,
+// kGxHalf: least sums of squares per run; kGxHalfOcc (sch and ssx,
 // gppKerSeq.cpp:96-139) and kGxRealOcc (gppKer_real.cpp:20-60): large factors
 // per segment.
 template <int kForm>
@@ -516,6 +519,8 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
 #pragma unroll
       for (int h = 0; h < kK / 32; ++h) {
         const int k = h * 32 + lane, ig = k0 + k;
+        float least = 0.f;  // of any band at this g-vector, relative to its largest
+        if (!H::kOcc && ig < s_lim[1][pl]) least = fminf(ex.band_min[ig], 1.f);
         double2 y[kSlabs];
 #pragma unroll
         for (int i = 0; i < kSlabs; ++i) y[i] = make_double2(0.0, 0.0);
@@ -539,7 +544,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
             const int big = max(__double2hiint(y[i].x) & 0x7FFFFFFF, __double2hiint(y[i].y) & 0x7FFFFFFF);
             acc[j][i] += ig % kExSeg < kExCount && big >= (min(e, 1000) + 1022 - kExSlackA) << 20 ? 1.f : 0.f;
           } else {
-            const float u = __uint_as_float((unsigned)(127 - e) << 23);  // 2^-e
+            const float u = __uint_as_float((unsigned)(127 - e) << 23) * least;  // 2^-e
             const float a = __double2float_rn(y[i].x) * u, b = __double2float_rn(y[i].y) * u;
             acc[j][i] = fmaf(a, a, fmaf(b, b, acc[j][i]));
           }
@@ -572,10 +577,10 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
 }
 
 // One warp per row: the large factors that must coincide with large elements
-// of every band (see exact_stats_kernel); half sum: the power shared with the
-// least band (kHalfPower).
+// of every band (see exact_stats_kernel); half sum: the least sum of squares
+// with any band (kHalfPower).
 template <int kForm>
-__global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const int* kend, int nf, int slabs, int per_seg) {
+__global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, int nf, int slabs, int per_seg) {
   chain_begin();
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= slabs * p.ng) return;
@@ -589,10 +594,9 @@ __global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, const 
     return sum;
   };
   if (Form<kForm>::kHalf) {
-    const int k = kend[row];
+    const int k = gx_limit<kForm>(p, g, i / p.ng);
     float sum = 0.f;
-    for (int s = lane; s * kExSeg < k; s += 32)
-      sum += st(s) * fminf(__int_as_float(ex.seg_pow[s]), (float)kExSeg) / (float)min(kExSeg, p.nc - s * kExSeg);
+    for (int s = lane; s * kExSeg < k; s += 32) sum += st(s);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0 && !(sum >= (float)k * kHalfPower)) ex_raise(ex);
@@ -673,8 +677,8 @@ cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, b
     e = launch_ff<kForm, false>(g, p, grid, s);
   }
   if (e != cudaSuccess) return e;
-  return launch_chained(gx_check_kernel<kForm>, (slabs * p.ng * 32 + 255) / 256, 256, 0, s, true, p, ex, g.stat, g.kend,
-                        g.nf, slabs, kExSeg / g.run);
+  return launch_chained(gx_check_kernel<kForm>, (slabs * p.ng * 32 + 255) / 256, 256, 0, s, true, p, ex, g.stat, g.nf,
+                        slabs, kExSeg / g.run);
 }
 
 }  // namespace
@@ -709,7 +713,7 @@ bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp
   gx_size(g.ex, q, igp_of, sms, g.nf, g.nf2, kend, &t);
   g.run = gx_run(g.ex, q.ng, sms);
   const size_t work = exact_work_bytes(g.ex), own = exact_own_bytes(g.ex);
-  if (cudaMalloc(&g.own, own + sizeof(int) * kend.size()) != cudaSuccess) g.own = nullptr;
+  if (cudaMalloc(&g.own, own) != cudaSuccess) g.own = nullptr;
   if (g.own && !shared_work && cudaMalloc(&g.work, work + gx_stat_bytes(g.ex, g.run)) != cudaSuccess) {
     cudaFree(g.own);
     g.own = g.work = nullptr;
@@ -724,12 +728,7 @@ bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp
   g.form = q.form;
   g.stat = reinterpret_cast<float*>(static_cast<char*>(w) + work);
   g.grid = sms;
-  cudaError_t e = exact_upload_tables(g.ex, t);
-  if (e == cudaSuccess && !kend.empty()) {
-    g.kend = reinterpret_cast<int*>(static_cast<char*>(g.own) + own);
-    e = cudaMemcpy(g.kend, kend.data(), sizeof(int) * kend.size(), cudaMemcpyHostToDevice);
-  }
-  if (e != cudaSuccess) {
+  if (exact_upload_tables(g.ex, t) != cudaSuccess) {
     cudaGetLastError();
     gpp_exact_destroy(g);
     return false;

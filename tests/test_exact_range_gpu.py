@@ -1,0 +1,41 @@
+"""The exact contractions (csrc/exact_gemm.cu, csrc/gpp_exact.cu) on operands at
+the edges of what they accept: an operand that they cannot hold has to reach
+the FP64 kernels behind them, whatever its neighbours.
+
+Bars as the FP64 parity tests: 1e-12 per achtemp / asxtemp / achstemp output
+and 1e-12 of the largest band value, against the oracle.
+"""
+import numpy as np
+import pytest
+
+import workload as W
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def _close(g, o):
+    g, o = np.atleast_1d(g), np.atleast_1d(o)
+    assert np.all(np.abs(g - o) <= TOL * np.abs(o)), np.abs(g - o) / np.abs(o)
+
+
+def _half_close(g, o):
+    _close(g[0], o[0])
+    _close(g[1], o[1])
+    assert np.abs(g[2] - o[2]).max() <= TOL * np.abs(o[2]).max()
+    if g[3] is not None:
+        _close(g[3], o[3])
+
+
+# ---- half sum: a factor far above its row's others meets a zero band element
+@pytest.mark.parametrize("p", [30, 40])
+def test_halfsum_large_factor_meets_zero_band_element(sigma_lib, p):
+    prob = W.gpp_random(64, 0, 4096, 16, 400 + p)
+    assert 3 * 64 * 16 * 4096 >= 1 << 23
+    for g in range(prob.ngpown):
+        k = 600 + 3 * g  # below every later igp
+        prob.wtilde_array[g, k] = prob.wx_array[g % 3] + 2.0 ** -p
+        prob.aqsntemp[:, k] = 0
+        prob.aqsmtemp[:, k] = 0
+    _half_close(sigma_lib.gpp_halfsum_host(prob, want_static=False), O.gpp_halfsum(prob))
