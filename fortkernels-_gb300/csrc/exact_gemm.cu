@@ -469,13 +469,6 @@ __global__ void __launch_bounds__(256) exact_slice_a_kernel(ExactPrep ex, const 
   }
 }
 
-// The larger part of (re, im) over 2^e, rounded towards zero to 20 bits (|x| < 2^e).
-__device__ __forceinline__ float ex_rel_mag(double re, double im, int e) {
-  const int d = max(__double2hiint(re) & 0x7FFFFFFF, __double2hiint(im) & 0x7FFFFFFF);
-  const int sh = 1023 + e - (d >> 20);
-  return sh < 100 ? __uint_as_float(((unsigned)(127 - sh) << 23) | ((unsigned)(d & 0xFFFFF) << 3)) : 0.f;
-}
-
 template <int S, int kCols, bool kReal>
 __global__ void __launch_bounds__(256) exact_slice_b_kernel(ExactPrep ex, const void* b0, int nb0, const void* b1,
                                                             int nb, int nc) {

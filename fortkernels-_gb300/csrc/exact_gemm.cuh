@@ -32,7 +32,7 @@
 // others were zero, the error would be 2^-39.5 of the sum's root mean square
 // with six digits, 2^-48 with seven; uniform inputs: 2^-51 with six).  Rows that fail, and values that are not finite, raise
 // ExactPrep::flag, and the callers' FP64 kernels run instead.  The half sum's
-// rows with factors near poles hold too few large elements for that count;
+// rows end at their igp and may hold few large elements (factors near poles);
 // they are checked against band_min, the least element of any band at each K
 // value (gx_check_kernel).
 #pragma once
@@ -179,6 +179,14 @@ __device__ __forceinline__ void ex_begin_counts(const ExactPrep& ex) {
 __device__ __forceinline__ void ex_raise(const ExactPrep& ex) {
   *ex.flag = 1;
   if (ex.any) *ex.any = 1;
+}
+
+// The larger part of (re, im) over 2^e, rounded towards zero to 20 bits (|x| < 2^e;
+// integer pipe).
+__device__ __forceinline__ float ex_rel_mag(double re, double im, int e) {
+  const int d = max(__double2hiint(re) & 0x7FFFFFFF, __double2hiint(im) & 0x7FFFFFFF);
+  const int sh = 1023 + e - (d >> 20);
+  return sh < 100 ? __uint_as_float(((unsigned)(127 - sh) << 23) | ((unsigned)(d & 0xFFFFF) << 3)) : 0.f;
 }
 
 // The S digits of x (|x| < 2^e; S = 6: of x 2^(52 - e), 7: x 2^(61 - e)) as

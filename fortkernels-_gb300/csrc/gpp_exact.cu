@@ -52,6 +52,7 @@ template <int kForm>
 struct Form {
   static constexpr bool kReal = kForm == kGxReal || kForm == kGxRealOcc, kRealOcc = kForm == kGxRealOcc;
   static constexpr bool kHalf = kForm == kGxHalf, kHalfOcc = kForm == kGxHalfOcc;
+  static constexpr bool kLeast = kHalf || kHalfOcc;  // checked against band_min
   static constexpr bool kF64 = kRealOcc || kHalf || kHalfOcc;  // factors in FP64, seven digits
   static constexpr int kSlabs = kHalf ? 4 : kReal ? kNW : 2 * kNW, kParts = kReal ? 1 : 2;  // the most slabs
 };
@@ -401,9 +402,9 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
 }
 
 // ---------------------------------------------------------------- half-sum factors
-// kGxHalf: least sums of squares per run; kGxHalfOcc (sch and ssx,
-// gppKerSeq.cpp:96-139) and kGxRealOcc (gppKer_real.cpp:20-60): large factors
-// per segment.
+// kGxHalf and kGxHalfOcc (sch and ssx, gppKerSeq.cpp:96-139): least sums of
+// squares per run; kGxRealOcc (gppKer_real.cpp:20-60): large factors per
+// segment.
 template <int kForm>
 struct F64 {
   static constexpr bool kOcc = kForm != kGxHalf, kReal = kForm == kGxRealOcc;
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
       for (int h = 0; h < kK / 32; ++h) {
         const int k = h * 32 + lane, ig = k0 + k;
         float least = 0.f;  // of any band at this g-vector, relative to its largest
-        if (!H::kOcc && ig < s_lim[1][pl]) least = fminf(ex.band_min[ig], 1.f);
+        if (Form<kForm>::kLeast && ig < s_lim[1][pl]) least = fminf(ex.band_min[ig], 1.f);
         double2 y[kSlabs];
 #pragma unroll
         for (int i = 0; i < kSlabs; ++i) y[i] = make_double2(0.0, 0.0);
@@ -540,13 +541,12 @@ __global__ void __launch_bounds__(kGxThreads, F64<kForm>::kK == 64 && !F64<kForm
           sm.v[0][i][pl][k] = y[i].x;
           if (!H::kReal) sm.v[H::kParts - 1][i][pl][k] = y[i].y;
           const int e = s_e[min(i, nf - 1)][pl];  // |e| < 64 unless flagged; a zero row is not checked
-          if (H::kOcc) {
+          if (!Form<kForm>::kLeast) {
             const int big = max(__double2hiint(y[i].x) & 0x7FFFFFFF, __double2hiint(y[i].y) & 0x7FFFFFFF);
             acc[j][i] += ig % kExSeg < kExCount && big >= (min(e, 1000) + 1022 - kExSlackA) << 20 ? 1.f : 0.f;
           } else {
-            const float u = __uint_as_float((unsigned)(127 - e) << 23) * least;  // 2^-e
-            const float a = __double2float_rn(y[i].x) * u, b = __double2float_rn(y[i].y) * u;
-            acc[j][i] = fmaf(a, a, fmaf(b, b, acc[j][i]));
+            const float a = ex_rel_mag(y[i].x, y[i].y, e) * least;
+            acc[j][i] = fmaf(a, a, acc[j][i]);
           }
         }
       }
@@ -593,23 +593,19 @@ __global__ void gx_check_kernel(GxDev p, ExactPrep ex, const float* stat, int nf
     for (int q = 0; q < per_seg; ++q) sum += v[q];
     return sum;
   };
-  if (Form<kForm>::kHalf) {
-    const int k = gx_limit<kForm>(p, g, i / p.ng);
+  if (Form<kForm>::kLeast) {
+    const int k = gx_limit<kForm>(p, g, Form<kForm>::kHalf ? i / p.ng : 0);
     float sum = 0.f;
     for (int s = lane; s * kExSeg < k; s += 32) sum += st(s);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0 && !(sum >= (float)k * kHalfPower)) ex_raise(ex);
   } else {
-    const int k = gx_limit<kForm>(p, g, 0);
-    // rows shorter than a segment (half sum, its first columns): the
-    // segment's counts say nothing of their few elements
-    if (k < min(kExSeg, p.nc)) return;
     int sum = 0;
-    for (int s = lane; s * kExSeg < k; s += 32)
+    for (int s = lane; s * kExSeg < p.nc; s += 32)
       sum += max(0, (int)st(s) + min(ex.seg_min[s], kExCount) - min(kExCount, p.nc - s * kExSeg));
     sum = __reduce_add_sync(0xffffffffu, sum);
-    if (lane == 0 && (long long)sum * kExOverlap < k) ex_raise(ex);
+    if (lane == 0 && (long long)sum * kExOverlap < p.nc) ex_raise(ex);
   }
 }
 

@@ -43,7 +43,7 @@ struct GppExact {
   ExactPrep ex{};
   GxForm form = kGxGpp;
   int nf = kNW, nf2 = 0;  // row slabs of ng columns: all bands', occupied bands'
-  float* stat = nullptr;  // [rows][runs] large factors per run (kGxHalf: least sums of squares with any band)
+  float* stat = nullptr;  // [rows][runs] large factors per run (half sum: least sums of squares with any band)
   int run = 0;            // g-vectors per factor item (a segment or a power-of-two part of it)
   int grid = 0;
   void *own = nullptr, *work = nullptr;  // work null when the caller's is used

@@ -39,3 +39,22 @@ def test_halfsum_large_factor_meets_zero_band_element(sigma_lib, p):
         prob.aqsntemp[:, k] = 0
         prob.aqsmtemp[:, k] = 0
     _half_close(sigma_lib.gpp_halfsum_host(prob, want_static=False), O.gpp_halfsum(prob))
+
+
+# ---- half sum, occupied bands: rows shorter than 512 g-vectors
+def _short_rows(scale, seed=41):
+    prob = W.gpp_random(8, 3, 4096, 128, seed)
+    assert 3 * 8 * 128 * 4096 >= 1 << 23
+    prob.inv_igp_index = (3 * np.arange(128) + 4).astype(np.int32)          # igp <= 385
+    prob.wtilde_array.real[:] = 0.5 + (prob.wtilde_array.real - 0.5) * (1.5 / 4.5)  # none within 0.5 of a frequency
+    prob.aqsntemp[:, 512:] *= scale
+    prob.aqsmtemp[:, 512:] *= scale
+    return prob
+
+
+@pytest.mark.parametrize("p", [0, 20, 30, 40])
+def test_halfsum_occupied_short_rows(sigma_lib, p):
+    prob = _short_rows(2.0 ** p)
+    g, o = sigma_lib.gpp_halfsum_host(prob, want_static=False), O.gpp_halfsum(prob)
+    _close(g[1], o[1])
+    assert np.abs(g[2] - o[2]).max() <= TOL * np.abs(o[2]).max()
