@@ -135,6 +135,10 @@ cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t);
 // 8 x (5 x 12) x 256 = 0.12 M takes 42 us, 67 us on the FP64 pipe.
 constexpr double kExactMin = 1 << 16;
 
+// The 64-bit integer sums hold K' products of the rows' largest elements (2^41
+// each) below K' = 2^22; longer sums stay with the FP64 kernels.
+constexpr bool exact_holds(int nc, bool cplx) { return (cplx ? 2LL : 1LL) * nc <= 1 << 21; }
+
 // One contraction, in order:
 //   exact_begin       clears the flag and the overlap counts
 //   launch_exact_b    band exponents, overlap counts and the B digits of bands

@@ -144,7 +144,8 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
     delete p;
     return SIGMA_ERR_CUDA;
   }
-  if (mode == SIGMA_FF_FP64 && (double)number_bands * ncouls * ngpown * nfreq >= kExactMin) {
+  if (mode == SIGMA_FF_FP64 && exact_holds(ncouls, true) &&
+      (double)number_bands * ncouls * ngpown * nfreq >= kExactMin) {
     ExactTables et;
     exact_size(p->ex, 6, number_bands, ncouls, ngpown, nfreq, true, sms, row_kend, &et);
     // without room for the digits the FP64 kernel keeps the work

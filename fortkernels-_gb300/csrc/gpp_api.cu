@@ -630,11 +630,12 @@ int gpp_host(int precision, int nb, int nvband, int nc, int ng, int nstart, int 
   char* a = static_cast<char*>(arena);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // The gated pipeline below pays when the FP64 pass takes much longer than the
-  // copies: large instances for whose contraction the device had no room.
+  // copies: large instances for whose contraction the device had no room, or
+  // whose sums are too long for it.
   // Small ones copy whole arrays and run the plan: 24 x 40 x 1024 takes 183 us
   // so, 531 us in ~30 pieces.
   if (precision == SIGMA_PREC_FP64 && plan->schy.n_items > 0 && !plan->exact &&
-      gpp_exact_fits(GxShape{kGxGpp, nb, nvband, nc, ng, false})) {
+      gpp_exact_pays(GxShape{kGxGpp, nb, nvband, nc, ng, false})) {
     // FP64 with the shared-frequency pass: the inputs travel on a copy
     // stream while the sum runs, each piece followed by a gate word the
     // pass's items wait for.  The items run with the K split slowest, and

@@ -685,13 +685,17 @@ cudaError_t launch_operands(const GppExact& g, const GxDev& p, cudaStream_t s, b
 // occupied bands and 50 / 66 without, real 16 x 20 x 512 (0.5 M) 105 / 138 and
 // 52 / 56; the half sum's two contractions 221 / 187 at 24 x 40 x 1024 (2.9 M),
 // 230 / 229 at 60 x 60 x 1024 (11 M), 315 / 372 at 60 x 60 x 2048.
-bool gpp_exact_fits(const GxShape& q) {
+bool gpp_exact_pays(const GxShape& q) {
   const double products = (double)kNW * q.ng * q.nb * q.nc;
   switch (q.form) {
     case kGxReal: return products >= 1 << 18;
     case kGxHalf: return products >= 1 << 23;
     default: return products >= 1 << 16;
   }
+}
+
+bool gpp_exact_fits(const GxShape& q) {
+  return gpp_exact_pays(q) && exact_holds(q.nc, q.form != kGxReal && q.form != kGxRealOcc);
 }
 
 size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms) {

@@ -65,6 +65,7 @@ struct GxShape {
 bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms,
                       void* shared_work = nullptr);
 bool gpp_exact_fits(const GxShape& q);
+bool gpp_exact_pays(const GxShape& q);  // large enough, whatever the sums' length
 size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms);
 void gpp_exact_destroy(GppExact& g);
 

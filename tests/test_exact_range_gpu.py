@@ -58,3 +58,22 @@ def test_halfsum_occupied_short_rows(sigma_lib, p):
     g, o = sigma_lib.gpp_halfsum_host(prob, want_static=False), O.gpp_halfsum(prob)
     _close(g[1], o[1])
     assert np.abs(g[2] - o[2]).max() <= TOL * np.abs(o[2]).max()
+
+
+# ---- sums over more g-vectors than the 64-bit integer sums hold
+def test_ff_long_coherent_sum(sigma_lib):
+    nc, x = 1 << 22, 0.96
+    z = np.full((1, nc), complex(x, x))
+    prob = W.FFProblem(1, nc, 1, 1, np.zeros(1, np.int32), np.arange(nc, dtype=np.int32), z.reshape(1, 1, nc),
+                       np.conj(z), np.ones((1, nc), np.complex128))
+    _close(sigma_lib.ff_host(prob, sigma_lib.FF_MODE_FP64), 2 * x * x * nc)
+
+
+def test_gpp_long_coherent_sum(sigma_lib):
+    nc = 1 << 23
+    one = np.ones((1, nc), np.complex128)
+    prob = W.GppProblem(1, 1, nc, 1, np.zeros(1, np.int32), np.arange(nc, dtype=np.int32), W.wx_frequencies(),
+                        one, one * (0.96 - 0.96j), one * (0.96 + 0.96j), one * 1.5, np.ones(nc))
+    g, o = sigma_lib.gpp_host(prob, sigma_lib.PREC_FP64), O.gpp(prob)
+    assert np.abs(g[0] - o[0]).max() <= TOL * np.abs(o[0]).max()
+    assert np.abs(g[1] - o[1]).max() <= TOL * np.abs(o[1]).max()
