@@ -88,7 +88,10 @@ __device__ __forceinline__ bool any_bits(double2 v) {
 
 // One CTA per column: exponents of its rows.  Squared magnitudes from FP32
 // values (c from exact FP32 halves), the guard taken somewhat wide on both
-// sides, with a 2^-8 margin; what FP32 cannot bound raises the flag.
+// sides, with a 2^-8 margin; what FP32 cannot bound raises the flag.  Squares
+// below 1e-36 count as 1e-36: an upper bound, so that no element exceeds its
+// row's exponent (one far above its row fails the overlap check).
+constexpr float kTinySq = 1e-36f;
 template <int kForm>
 __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep ex, int nf, int nf2) {
   using F = Form<kForm>;
@@ -99,11 +102,13 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
   const bool occ = F::kHalfOcc || F::kRealOcc || nf2 > 0;
   FF wx[kNW];
   float iwx4[kNW];
-  bool huge = false;  // |wx| or |wtilde| above 1e15: reciprocals may flush to 0
+  // |wtilde| or |I_eps| above 1e15 or not finite, |wx| outside 1e-9 .. 1e9:
+  // reciprocals and their squares may flush to 0
+  bool huge = false;
 #pragma unroll
   for (int iw = 0; iw < kNW; ++iw) {
     wx[iw] = ff_of(p.wx[iw]);
-    huge = huge || !(fabsf(wx[iw].hi) < 1e15f);
+    huge = huge || !(fabsf(wx[iw].hi) < 1e9f && fabsf(wx[iw].hi) > 1e-9f);
     const float i2 = rcp_approx(wx[iw].hi * wx[iw].hi);
     iwx4[iw] = i2 * i2;
   }
@@ -111,20 +116,24 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
 #pragma unroll
   for (int i = 0; i < F::kSlabs; ++i) m[i] = 0u;
   auto top = [](unsigned& v, float y) { v = max(v, __float_as_uint(y)); };
-  bool bad = false;
+  bool bad = false, bad_e = false;  // a nonzero factor, I_eps value below 1e-18
   const int k_end = gx_limit<kForm>(p, g, F::kSlabs - 1), k_freq = gx_limit<kForm>(p, g, 0);
   auto element = [&](int k, double2 w, double2 e) {
     const float er = f32_lead(e.x), ei = F::kReal ? 0.f : f32_lead(e.y);
     const float e2 = fmaf(er, er, ei * ei);
+    const bool any_e = any_bits(e);
     if (F::kHalf) {
       top(m[F::kSlabs - 1], e2);
+      bad_e = bad_e || (any_e && !(e2 > kTinySq));
       if (k >= k_freq || k % kIgBlk == kIgBlk - 1) return;
     }
     const FF a = ff_of(w.x);
     const float b = F::kReal ? 0.f : f32_lead(w.y), b2 = b * b;
-    const float s2 = fmaf(a.hi, a.hi, b2), g2 = s2 * e2;  // |wtilde|^2, |G|^2
-    huge = huge || !(s2 < 1e30f);
-    const bool any = any_bits(w) && any_bits(e);
+    const float s2 = fmaf(a.hi, a.hi, b2);  // |wtilde|^2
+    huge = huge || !(s2 + e2 < 1e30f);
+    const bool any = any_bits(w) && any_e;
+    const float g2 = any ? fmaxf(s2, kTinySq) * fmaxf(e2, kTinySq) : 0.f;  // |G|^2
+    const float least = fminf(s2, e2) > kTinySq ? kTinySq : INFINITY;       // factors from here on are not small ones
     // the guard's threshold, somewhat above and below
     const float up = fmaxf(0.2501f, s2 * 4.001e-6f), low = 0.2499f;
 #pragma unroll
@@ -134,7 +143,7 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
       if (!F::kRealOcc && (F::kHalf ? !(w2 > up) : !(w2 <= low))) {  // also NaN
         const float y = g2 * r;
         top(m[iw], y);
-        bad = bad || (any && !(y > 1e-36f));
+        bad = bad || (any && !(y > least));
       }
       if (!F::kHalf && (!F::kReal || F::kRealOcc) && occ) {
         const float z = (wx[iw].hi + a.hi) + (wx[iw].lo + a.lo);
@@ -143,7 +152,7 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
         // |Omega2 / (wx^2 - wtilde^2)|^2, |Omega2 / wx^2|^2
         if (!(w2 <= low)) y = fmaxf(y, s2 * g2 * (F::kHalfOcc ? r * rz : iwx4[iw]));
         top(m[F::kSlabs > kNW ? kNW + iw < F::kSlabs ? kNW + iw : 0 : iw], y);
-        bad = bad || (any && !(y > 1e-36f));
+        bad = bad || (any && !(y > least));
       }
     }
   };
@@ -161,6 +170,7 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
       if (k0 + q * kGxThreads < k_end) element(k0 + q * kGxThreads, w[q], e[q]);
   }
   bad = __syncthreads_or(bad);
+  if (F::kHalf) bad_e = __syncthreads_or(bad_e);
   huge = __syncthreads_or(huge);
 #pragma unroll
   for (int i = 0; i < F::kSlabs; ++i) {
@@ -173,7 +183,8 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
     for (int q = 0; q < kGxThreads / 32; ++q) v = max(v, s_m[tid][q]);
     const float f = sqrtf(__uint_as_float(v)) * (1.f + 1.f / 256.f);
     // a factor too small for FP32 may only be ignored beside large ones
-    if (huge || !(f < 1e18f) || (bad && !(f > 1e-6f)) || (v && f < 1e-18f)) ex_raise(ex);
+    const bool small = F::kHalf && tid == F::kSlabs - 1 ? bad_e : bad;
+    if (huge || !(f < 1e18f) || (small && !(f > 1e-6f)) || (v && f < 1e-18f)) ex_raise(ex);
     // float-float digits need a bit of room (ex_ff_digits)
     ex.ea[gx_row(ex, p.ng, nf, tid, g)] =
         v ? (int)(__float_as_uint(f) >> 23) - 126 + (F::kF64 ? 0 : 1) : kExZeroRow;

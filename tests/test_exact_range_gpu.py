@@ -77,3 +77,20 @@ def test_gpp_long_coherent_sum(sigma_lib):
     g, o = sigma_lib.gpp_host(prob, sigma_lib.PREC_FP64), O.gpp(prob)
     assert np.abs(g[0] - o[0]).max() <= TOL * np.abs(o[0]).max()
     assert np.abs(g[1] - o[1]).max() <= TOL * np.abs(o[1]).max()
+
+
+# ---- values whose squares leave the FP32 range of the row bounds
+def test_halfsum_static_of_tiny_inverse_dielectric_values(sigma_lib):
+    prob = W.gpp_random(64, 0, 4096, 16, 44)
+    prob.I_eps_array *= 1e-30
+    prob.wtilde_array.real[:] = 0.5 + (prob.wtilde_array.real - 0.5) * (1.5 / 4.5)
+    _close(sigma_lib.gpp_halfsum_host(prob)[3], O.gpp_halfsum(prob)[3])
+
+
+def test_gpp_tiny_inverse_dielectric_value_at_large_pole(sigma_lib):
+    prob = W.gpp_random(45, 2, 3001, 37, 45)
+    prob.I_eps_array[3, 100] = 1e-24
+    prob.wtilde_array[3, 100] = 1e14
+    g, o = sigma_lib.gpp_host(prob, sigma_lib.PREC_FP64), O.gpp(prob)
+    _close(g[0], o[0])
+    _close(g[1], o[1])
