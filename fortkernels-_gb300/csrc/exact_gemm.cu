@@ -860,6 +860,7 @@ cudaError_t launch_exact_a(const ExactPrep& ex, const double2* a, int rows, int 
 }
 
 cudaError_t launch_exact_gemm(const ExactPrep& ex, int grid, int* status, cudaStream_t s) {
+  if (ex.n_items == 0) return cudaSuccess;  // every row is zero: the epilogue sums no pieces
   auto* kernel = ex.slices == 7    ? exact_gemm_kernel<7, 64>
                  : ex.cols == 80 ? exact_gemm_kernel<6, 80>
                  : ex.cols == 64 ? exact_gemm_kernel<6, 64>

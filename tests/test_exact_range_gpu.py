@@ -60,6 +60,26 @@ def test_halfsum_occupied_short_rows(sigma_lib, p):
     assert np.abs(g[2] - o[2]).max() <= TOL * np.abs(o[2]).max()
 
 
+# ---- half sum: no g-vector below any igp (no work for the contractions)
+@pytest.mark.parametrize("static", [True, False], ids=["static", "nostatic"])
+@pytest.mark.parametrize("igps", [[0], [1], [0, 1, -1], [-1, -1]], ids=str)
+@pytest.mark.parametrize("nvb", [0, 2])
+def test_halfsum_without_pairs(sigma_lib, igps, nvb, static):
+    ng = len(igps)
+    prob = W.gpp_random(512, nvb, 8192, ng, 43)
+    assert 3 * 512 * ng * 8192 >= 1 << 23
+    prob.inv_igp_index = np.arange(ng, dtype=np.int32)
+    prob.indinv = np.arange(8192, dtype=np.int32)
+    prob.indinv[:ng] = igps
+    g, o = sigma_lib.gpp_halfsum_host(prob, want_static=static), O.gpp_halfsum(prob)
+    scale = max(np.abs(o[0]).max(), 1e-300)
+    assert np.abs(g[0] - o[0]).max() <= TOL * scale
+    assert np.abs(g[1] - o[1]).max() <= TOL * max(np.abs(o[1]).max(), 1e-300)
+    assert np.abs(g[2] - o[2]).max() <= TOL * max(np.abs(o[2]).max(), 1e-300)
+    if static:
+        assert abs(g[3] - o[3]) <= TOL * max(abs(o[3]), 1e-300)
+
+
 # ---- sums over more g-vectors than the 64-bit integer sums hold
 def test_ff_long_coherent_sum(sigma_lib):
     nc, x = 1 << 22, 0.96
