@@ -216,10 +216,10 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
           bulk_load(dst + kABytes, b + (size_t)s * kBBytes, kBBytes, bar);
         }
       }
-      // after a failure: the copies still landing end before the CTA does
-      if (!ok)
-        for (uint32_t t = g > (uint32_t)kStagesEx ? g - kStagesEx : 0u; t < g; ++t)
-          mbar_wait_own(full0 + 8u * (t % kStagesEx), (t / kStagesEx) & 1u);
+      // the last copies land before the CTA ends, also when another warp's wait
+      // gave up and nothing consumes them
+      for (uint32_t t = g > (uint32_t)kStagesEx ? g - kStagesEx : 0u; t < g; ++t)
+        mbar_wait_own(full0 + 8u * (t % kStagesEx), (t / kStagesEx) & 1u);
     }
     __syncwarp();
   } else if (warp == kGateWarpEx) {
@@ -311,9 +311,9 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
         __syncwarp();
       }
     }
-    // after a failure: the MMAs already issued end before the tensor memory
-    // is released
-    if (lane == 0 && failed) {
+    // the MMAs issued end before the tensor memory is released, also when the
+    // wait of a warp that reads them gave up
+    if (lane == 0) {
       mma_commit(done0);
       mbar_wait_own(done0, 0);
     }

@@ -161,11 +161,11 @@ __global__ void __launch_bounds__(kOzThreads, 1) ozaki_gemm_kernel(FfDev p, FfWo
           bulk_load(dst + kOperandBytes, b_src + (size_t)s * kOperandBytes, kOperandBytes, bar);
         }
       }
-      // after a failure: the copies of the last (up to kStages) tiles may
-      // still be landing; wait for them before the CTA releases its ring
-      if (!ok)
-        for (uint32_t t = g > (uint32_t)kStages ? g - kStages : 0u; t < g; ++t)
-          mbar_wait_own(full0 + 8u * (t % kStages), (t / kStages) & 1u);
+      // the copies of the last (up to kStages) tiles land before the CTA
+      // releases its ring, also when another warp's wait gave up and nothing
+      // consumes them
+      for (uint32_t t = g > (uint32_t)kStages ? g - kStages : 0u; t < g; ++t)
+        mbar_wait_own(full0 + 8u * (t % kStages), (t / kStages) & 1u);
     }
     __syncwarp();
   } else if (warp == kGateWarp) {
@@ -276,9 +276,9 @@ __global__ void __launch_bounds__(kOzThreads, 1) ozaki_gemm_kernel(FfDev p, FfWo
         __syncwarp();
       }
     }
-    // after a failure: the MMAs already issued complete before the tensor
-    // memory is released
-    if (lane == 0 && failed) {
+    // the MMAs issued complete before the tensor memory is released, also
+    // when the wait of a warp that reads them gave up
+    if (lane == 0) {
       mma_commit(done0);
       mbar_wait_own(done0, 0);
     }
