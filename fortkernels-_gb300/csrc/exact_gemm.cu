@@ -173,7 +173,9 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
   __shared__ __align__(8) unsigned long long bars[2 * kStagesEx + 5];
   __shared__ uint32_t tmem_slot;
   chain_begin();
-  if (*ex.flag) return;  // operands outside the split's range: the FP64 kernel runs instead
+  // operands outside the split's range: the FP64 kernel runs instead (one
+  // read for the CTA: another CTA may raise the flag below)
+  if (__syncthreads_or(threadIdx.x == 0 && *ex.flag)) return;
 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -362,6 +364,8 @@ __global__ void __launch_bounds__(kThreadsEx, 1) exact_gemm_kernel(ExactPrep ex,
 
   tc_fence_before();
   __syncthreads();
+  // a wait gave up: the sums are incomplete, the FP64 kernels form them
+  if (tid == 0 && status_set(status)) ex_raise(ex);
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 

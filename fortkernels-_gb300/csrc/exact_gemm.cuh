@@ -146,7 +146,8 @@ constexpr bool exact_holds(int nc, bool cplx) { return (cplx ? 2LL : 1LL) * nc <
 //                     real with halves = 1)
 //   launch_exact_a    row exponents, overlap check and the A digits of
 //                     complex rows (or the caller's own producer of both)
-//   launch_exact_gemm the digit products
+//   launch_exact_gemm the digit products; a wait that gives up also raises
+//                     the flag (the status word records it)
 //   launch_exact_finish  FP64 sums of the row groups per band, into out[n][f]
 //                     (complex; halves = 1: FfDev::aqsm holds real values and
 //                     the imaginary parts are zero); FfDev::nf, nb and vfac

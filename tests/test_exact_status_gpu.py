@@ -26,3 +26,10 @@ def check_output(tmp_path_factory):
 
 def test_contraction_that_gives_up_returns(check_output):
     assert "0 bad" in check_output
+
+
+def test_contraction_that_gives_up_raises_its_flag(check_output):
+    """Its sums are then left to the FP64 kernels, also in the real-valued and
+    half-sum forms, which report no status."""
+    for slices in (6, 7):
+        assert f"slices {slices}: flag 0, 1 with a set status, 0\n" in check_output
