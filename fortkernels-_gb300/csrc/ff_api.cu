@@ -149,8 +149,8 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
     ExactTables et;
     exact_size(p->ex, 6, number_bands, ncouls, ngpown, nfreq, true, sms, row_kend, &et);
     // without room for the digits the FP64 kernel keeps the work
-    const size_t work = exact_work_bytes(p->ex);
-    if (cudaMalloc(&p->ex_block, work + exact_own_bytes(p->ex)) != cudaSuccess) {
+    const size_t work = exact_work_bytes(p->ex), all = work + exact_own_bytes(p->ex);
+    if (!room_for_optional(all) || cudaMalloc(&p->ex_block, all) != cudaSuccess) {
       cudaGetLastError();
       p->ex_block = nullptr;
     } else {
@@ -167,6 +167,14 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
   }
   *out = p;
   return SIGMA_OK;
+}
+
+bool ff_plan_drop_exact(sigma_ff_plan p) {
+  if (!p->ex_block) return false;
+  cudaFree(p->ex_block);
+  p->ex_block = nullptr;
+  p->work.run_if = nullptr;
+  return true;
 }
 
 }  // namespace sigma
@@ -375,14 +383,16 @@ extern "C" int sigma_ff_schdt(int number_bands, int ncouls, int ngpown, int nfre
     return SIGMA_ERR_NO_DEVICE;
   }
   sigma_ff_plan plan = nullptr;
-  st = sigma_ff_plan_create(&plan, number_bands, ncouls, ngpown, nfreq, inv_igp_index, indinv, mode);
+  st = with_reclaim([&] {
+    return sigma_ff_plan_create(&plan, number_bands, ncouls, ngpown, nfreq, inv_igp_index, indinv, mode);
+  });
   if (st != SIGMA_OK) return st;
   const size_t eps_b = sizeof(sigma_complex128) * (size_t)nfreq * ngpown * ncouls;
   const size_t band_b = sizeof(sigma_complex128) * (size_t)number_bands * ncouls;
   const size_t out_b = sizeof(sigma_complex128) * (size_t)number_bands * nfreq;
   const size_t o1 = up256(eps_b), o2 = o1 + up256(band_b), o3 = o2 + up256(band_b);
   void* arena = nullptr;
-  st = arena_get(kArenaFfInputs, o3 + up256(out_b), &arena);
+  st = arena_beside(kArenaFfInputs, o3 + up256(out_b), &arena, [&] { return ff_plan_drop_exact(plan); });
   if (st != SIGMA_OK) {
     sigma_ff_plan_destroy(plan);
     return st;

@@ -25,6 +25,10 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
                   const int* row_kend = nullptr, int split_tiles_hint = 0, int items_per_cta = 0);
 int ff_plan_tile_bytes(int number_bands, int ncouls, int ngpown, int nfreq, size_t* bytes);
 
+// Gives back the exact contraction's workspace of an FP64 plan with no
+// execution in flight (the FP64 kernels then run); false if it has none.
+bool ff_plan_drop_exact(sigma_ff_plan plan);
+
 // The split-BF16 plan's operand layout (slice images, K tiles, row limits),
 // for kernels that write the A slices themselves and then execute with
 // reuse_a; nullptr for an FP64 plan.

@@ -347,8 +347,10 @@ extern "C" int sigma_ff_sigma(int number_bands, int nvband, int ncouls, int ngpo
       if (!(dFreqGrid[f + 1] > dFreqGrid[f])) return SIGMA_ERR_INVALID_SHAPE;  // ascending grid
   std::lock_guard<std::mutex> lk(api_mutex());
   sigma_ff_sigma_plan plan = nullptr;
-  int st = sigma_ff_sigma_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nfreq, nfreqeval,
-                                      inv_igp_index, indinv, mode);
+  int st = with_reclaim([&] {
+    return sigma_ff_sigma_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nfreq, nfreqeval, inv_igp_index,
+                                      indinv, mode);
+  });
   if (st != SIGMA_OK) return st;
   const int nb = number_bands, nf = nfreq, ne = nfreqeval;
   const size_t eps_b = sizeof(sigma_complex128) * (size_t)nf * ngpown * ncouls;
@@ -366,7 +368,7 @@ extern "C" int sigma_ff_sigma(int number_bands, int nvband, int ncouls, int ngpo
                o_pref = take(sizeof(double) * nf), o_sd = take(mat_b),
                o_out = take(sizeof(double2) * (1 + kOut * ne));
   void* arena = nullptr;
-  st = arena_get(kArenaFfInputs, off, &arena);
+  st = arena_beside(kArenaFfInputs, off, &arena, [&] { return ff_plan_drop_exact(plan->ff); });
   if (st != SIGMA_OK) {
     sigma_ff_sigma_plan_destroy(plan);
     return st;

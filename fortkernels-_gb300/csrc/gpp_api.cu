@@ -566,8 +566,21 @@ void drop_cached_plan() {
   drop_lane();
 }
 
+// The cached plan's contraction workspace; without it the plan's FP64 kernels run.
+void drop_cached_workspace() {
+  if (!g_cached_plan || !g_cached_plan->exact) return;
+  int cur = 0;
+  cudaGetDevice(&cur);
+  cudaSetDevice(g_cached_plan->device);
+  gpp_exact_destroy(g_cached_plan->exact);
+  cudaSetDevice(cur);
+}
+
 struct HookOnce {
-  HookOnce() { register_shutdown_hook(drop_cached_plan); }
+  HookOnce() {
+    register_shutdown_hook(drop_cached_plan);
+    register_reclaim_hook(drop_cached_workspace);
+  }
 };
 
 int cached_plan(int nb, int nvband, int nc, int ng, const int* inv, const int* indinv,

@@ -301,7 +301,7 @@ void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std
   size_t ws = 0;
   for (int i = 0; i < b->n; ++i)
     if (gpp_exact_fits(shape(i))) ws = std::max(ws, gpp_exact_work_bytes(shape(i), igp[i], sms));
-  if (ws == 0) return;
+  if (ws == 0 || !room_for_optional(ws)) return;
   if (cudaMalloc(&b->exact_ws, ws) != cudaSuccess) {
     cudaGetLastError();
     b->exact_ws = nullptr;

@@ -29,6 +29,7 @@
 
 #include "gpp_exact.cuh"
 #include "floatfloat.cuh"
+#include "runtime.h"
 
 namespace sigma {
 namespace {
@@ -724,8 +725,13 @@ bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp
   gx_size(g.ex, q, igp_of, sms, g.nf, g.nf2, kend, &t);
   g.run = gx_run(g.ex, q.ng, sms);
   const size_t work = exact_work_bytes(g.ex), own = exact_own_bytes(g.ex);
+  const size_t stat = gx_stat_bytes(g.ex, g.run);
+  if (!shared_work && !room_for_optional(work + stat)) {
+    g = GppExact();
+    return false;
+  }
   if (cudaMalloc(&g.own, own) != cudaSuccess) g.own = nullptr;
-  if (g.own && !shared_work && cudaMalloc(&g.work, work + gx_stat_bytes(g.ex, g.run)) != cudaSuccess) {
+  if (g.own && !shared_work && cudaMalloc(&g.work, work + stat) != cudaSuccess) {
     cudaFree(g.own);
     g.own = g.work = nullptr;
   }

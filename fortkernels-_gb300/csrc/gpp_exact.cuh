@@ -59,7 +59,8 @@ struct GxShape {
 };
 
 // Sizes, allocates and fills the contraction of one instance; false (with
-// nothing allocated) when the device has no room: the FP64 kernels keep the
+// nothing allocated) when the device has no room, or the workspace would take
+// more than half of its free memory: the FP64 kernels keep the
 // work, as for problems too small for it (gpp_exact_fits).  With shared_work set
 // (at least gpp_exact_work_bytes) the instance has no workspace of its own.
 bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms,

@@ -1450,8 +1450,10 @@ int halfsum_host(bool tensor, int number_bands, int nvband, int ncouls, int ngpo
   sigma_gpp_halfsum_plan plan = nullptr;
   const int flags = SIGMA_HALFSUM_GVEC_MAJOR | (achstemp ? SIGMA_HALFSUM_STATIC : 0) |
                     (tensor ? SIGMA_HALFSUM_TENSOR : 0);
-  st = sigma_gpp_halfsum_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend,
-                                     inv_igp_index, indinv, ncouls, flags);
+  st = with_reclaim([&] {
+    return sigma_gpp_halfsum_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index,
+                                         indinv, ncouls, flags);
+  });
   if (st != SIGMA_OK) return st;
   const size_t bb = sizeof(sigma_complex128) * (size_t)number_bands * ncouls;
   const size_t cb = sizeof(sigma_complex128) * (size_t)ngpown * ncouls;
@@ -1465,7 +1467,12 @@ int halfsum_host(bool tensor, int number_bands, int nvband, int ncouls, int ngpo
                o_v = take(sizeof(double) * ncouls), o_x = take(sizeof(double) * kNW),
                o_out = take(sizeof(sigma_complex128) * (2 * kNW + 1 + (size_t)number_bands));
   void* arena = nullptr;
-  st = arena_get(kArenaMisc, off, &arena);
+  st = arena_beside(kArenaMisc, off, &arena, [&] {
+    const bool any = static_cast<bool>(plan->exact);
+    gpp_exact_destroy(plan->exact);
+    gpp_exact_destroy(plan->exact_occ);
+    return any;
+  });
   if (st != SIGMA_OK) {
     sigma_gpp_halfsum_plan_destroy(plan);
     return st;

@@ -510,8 +510,10 @@ extern "C" int sigma_gpp_real_fp64(int number_bands, int nvband, int ncouls, int
   if (st != SIGMA_OK) return st;
   std::lock_guard<std::mutex> lk(api_mutex());
   sigma_gpp_real_plan plan = nullptr;
-  st = sigma_gpp_real_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend,
-                                  inv_igp_index, indinv, ncouls);
+  st = with_reclaim([&] {
+    return sigma_gpp_real_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index, indinv,
+                                      ncouls);
+  });
   if (st != SIGMA_OK) return st;
   const size_t bb = sizeof(double) * (size_t)number_bands * ncouls;
   const size_t cb = sizeof(double) * (size_t)ngpown * ncouls;
@@ -526,7 +528,12 @@ extern "C" int sigma_gpp_real_fp64(int number_bands, int nvband, int ncouls, int
                o_a = take(sizeof(double) * kNW), o_s = take(sizeof(double) * kNW),
                o_1 = take(sizeof(double) * number_bands);
   void* arena = nullptr;
-  st = arena_get(kArenaMisc, off, &arena);
+  st = arena_beside(kArenaMisc, off, &arena, [&] {
+    const bool any = static_cast<bool>(plan->exact);
+    gpp_exact_destroy(plan->exact);
+    gpp_exact_destroy(plan->exact_occ);
+    return any;
+  });
   if (st != SIGMA_OK) {
     sigma_gpp_real_plan_destroy(plan);
     return st;

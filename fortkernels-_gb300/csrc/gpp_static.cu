@@ -98,7 +98,8 @@ extern "C" int sigma_gpp_achstemp(int number_bands, int ncouls, int ngpown, cons
   }
   std::lock_guard<std::mutex> lk(api_mutex());
   sigma_ff_plan plan = nullptr;
-  int st = static_plan(&plan, number_bands, ncouls, ngpown, inv_igp_index, indinv, mode);
+  int st = with_reclaim(
+      [&] { return static_plan(&plan, number_bands, ncouls, ngpown, inv_igp_index, indinv, mode); });
   if (st != SIGMA_OK) return st;
   const size_t eps_b = sizeof(sigma_complex128) * (size_t)ngpown * ncouls;
   const size_t band_b = sizeof(sigma_complex128) * (size_t)number_bands * ncouls;
@@ -107,7 +108,7 @@ extern "C" int sigma_gpp_achstemp(int number_bands, int ncouls, int ngpown, cons
   const size_t o1 = up256(eps_b), o2 = o1 + up256(band_b), o3 = o2 + up256(band_b),
                o4 = o3 + up256(v_b), o5 = o4 + up256(out_b);
   void* arena = nullptr;
-  st = arena_get(kArenaFfInputs, o5 + 256, &arena);
+  st = arena_beside(kArenaFfInputs, o5 + 256, &arena, [&] { return ff_plan_drop_exact(plan); });
   if (st != SIGMA_OK) {
     sigma_ff_plan_destroy(plan);
     return st;

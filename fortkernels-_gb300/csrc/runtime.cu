@@ -58,6 +58,10 @@ std::vector<Arena>& arenas() {
   static std::vector<Arena> a(64 * kArenaSlots);
   return a;
 }
+std::vector<ReclaimHook>& reclaim_hooks() {
+  static std::vector<ReclaimHook> h;
+  return h;
+}
 std::vector<ShutdownHook>& hooks() {
   static std::vector<ShutdownHook> h;
   return h;
@@ -82,6 +86,11 @@ int arena_get(int slot, size_t bytes, void** out) {
     cudaError_t e = cudaMalloc(&a.ptr, want);
     if (e != cudaSuccess) {
       cudaGetLastError();
+      reclaim_caches();
+      e = cudaMalloc(&a.ptr, want);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
       set_last_cuda_error(e, "cudaMalloc(arena)", __LINE__);
       a.ptr = nullptr;
       return SIGMA_ERR_ALLOC;
@@ -92,7 +101,20 @@ int arena_get(int slot, size_t bytes, void** out) {
   return SIGMA_OK;
 }
 
+bool room_for_optional(size_t bytes) {
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= free_bytes / 2;
+}
+
 void register_shutdown_hook(ShutdownHook h) { hooks().push_back(h); }
+void register_reclaim_hook(ReclaimHook h) { reclaim_hooks().push_back(h); }
+void reclaim_caches() {
+  for (auto& h : reclaim_hooks()) h();
+}
 
 }  // namespace sigma
 

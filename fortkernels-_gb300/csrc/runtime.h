@@ -4,6 +4,8 @@
 #include <cstddef>
 #include <mutex>
 
+#include "sigma_common.h"
+
 namespace sigma {
 
 // Serialises the host-pointer entry points (they share cached buffers).
@@ -17,6 +19,32 @@ int device_sm_count();
 constexpr int kArenaSlots = 4;
 enum ArenaSlot { kArenaGppInputs = 0, kArenaFfInputs = 1, kArenaBatched = 2, kArenaMisc = 3 };
 int arena_get(int slot, size_t bytes, void** out);
+
+// Whether an optional workspace may be taken: it leaves at least as much of
+// the current device's free memory as it takes.
+bool room_for_optional(size_t bytes);
+
+// Functions that give back the optional workspaces of plan caches; run (and
+// the allocation tried again) when an arena, or a host call's plan, finds no
+// memory.  The caller holds api_mutex().
+typedef void (*ReclaimHook)();
+void register_reclaim_hook(ReclaimHook h);
+void reclaim_caches();
+
+// A host call's plan (create returns a status), and its arena with the
+// plan's own optional workspace (drop gives it up, false if it has none).
+template <class F>
+int with_reclaim(F create) {
+  const int st = create();
+  if (st != SIGMA_ERR_ALLOC) return st;
+  reclaim_caches();
+  return create();
+}
+template <class F>
+int arena_beside(int slot, size_t bytes, void** out, F drop) {
+  const int st = arena_get(slot, bytes, out);
+  return st == SIGMA_ERR_ALLOC && drop() ? arena_get(slot, bytes, out) : st;
+}
 
 void set_last_error_text(const char* text);
 

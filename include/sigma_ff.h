@@ -48,7 +48,11 @@ int sigma_ff_schdt(int number_bands, int ncouls, int ngpown, int nfreq,
 
 /* Device-resident plan: validates the index maps on the host, owns the
  * partial-sum (and, for the Ozaki mode, BF16 slice) buffers.  Execution is
- * asynchronous and allocates nothing; arrays are device pointers. */
+ * asynchronous and allocates nothing; arrays are device pointers.  An FP64
+ * plan whose sum is large enough also keeps its operands' digits for the exact
+ * contraction (about 24 B per I_epsR element and per band and g-vector: 5.8 GB at 512 x
+ * (15 x 820) x 16384) while they are at most half of the device's free
+ * memory at its creation, else it runs the FP64 kernel. */
 typedef struct sigma_ff_plan_s* sigma_ff_plan;
 
 int sigma_ff_plan_create(sigma_ff_plan* plan, int number_bands, int ncouls, int ngpown, int nfreq,

@@ -64,7 +64,8 @@ extern "C" {
  * between devices or shapes re-plans on every call: use one process per
  * device (the replica layout), or the plan API (sigma_gpp_plan_create /
  * sigma_gpp_execute), which keeps one plan per shape and device.
- * sigma_shutdown() frees the cached state.
+ * sigma_shutdown() frees the cached state, the plan's contraction workspace
+ * (below) included.
  * ------------------------------------------------------------------------- */
 int sigma_gpp_fp64(int number_bands, int nvband, int ncouls, int ngpown, int nstart, int nend,
                    const int* inv_igp_index, const int* indinv, const double* wx_array,
@@ -123,6 +124,16 @@ int sigma_gpp_tensor(int number_bands, int nvband, int ncouls, int ngpown, int n
  * graph.  Inputs and outputs of sigma_gpp_execute are device pointers.
  * One plan may be executed by one stream at a time (its partial buffers are
  * reused by every execution).
+ *
+ * Memory.  An FP64 plan whose sums are large enough keeps its operands' digits
+ * for the exact contraction of one frequency set, about 24 B per slab, column
+ * and g-vector (three slabs for the bands, three for the occupied ones) and
+ * 24 B per band and g-vector: 9.0 GB at 512 bands x 1638 columns x 32768
+ * g-vectors (real-valued 5.1 GB, half sum 18 GB).  It takes them at creation,
+ * and only while they are at most half of the device's free memory; without
+ * them it runs the FP64 kernels (150 ms instead of 12 at that size).  Executions
+ * with per-band frequencies, and sigma_gpp_fp64_noalloc, do not use them.  The
+ * host calls give them up where their inputs need the memory.
  * ------------------------------------------------------------------------- */
 typedef struct sigma_gpp_plan_s* sigma_gpp_plan;
 

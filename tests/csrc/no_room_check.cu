@@ -1,0 +1,203 @@
+// The host calls on a device with little free memory, simulated: the linker
+// routes the library's cudaMalloc, cudaFree and cudaMemGetInfo through the
+// functions below, which keep to a budget.  An optional workspace (the exact
+// contractions') must never make a call fail that its mandatory memory allows,
+// and every way of doing without it must give the same results.
+#include <cmath>
+#include <cstdio>
+#include <functional>
+#include <map>
+#include <string>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+#include "sigma_ff.h"
+#include "sigma_gpp.h"
+
+extern "C" {
+cudaError_t __real_cudaMalloc(void** p, size_t n);
+cudaError_t __real_cudaFree(void* p);
+}
+static size_t g_budget = ~size_t(0) / 4, g_used = 0, g_peak = 0;
+static bool g_report_none = false;  // cudaMemGetInfo reports no free memory
+static std::map<void*, size_t> g_size;
+extern "C" cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
+  if (g_used + n > g_budget) return cudaErrorMemoryAllocation;
+  const cudaError_t e = __real_cudaMalloc(p, n);
+  if (e != cudaSuccess) return e;
+  g_size[*p] = n;
+  g_used += n;
+  g_peak = g_used > g_peak ? g_used : g_peak;
+  return e;
+}
+extern "C" cudaError_t __wrap_cudaFree(void* p) {
+  const auto it = g_size.find(p);
+  if (it != g_size.end()) {
+    g_used -= it->second;
+    g_size.erase(it);
+  }
+  return __real_cudaFree(p);
+}
+extern "C" cudaError_t __wrap_cudaMemGetInfo(size_t* f, size_t* t) {
+  *f = g_report_none || g_used > g_budget ? 0 : g_budget - g_used;
+  *t = g_budget;
+  return cudaSuccess;
+}
+
+using cd = sigma_complex128;
+static unsigned long long g_rng = 1;
+static double uni(double lo, double hi) {
+  g_rng = g_rng * 6364136223846793005ull + 1442695040888963407ull;
+  return lo + (hi - lo) * (double)(g_rng >> 11) * 0x1p-53;
+}
+static std::vector<cd> cplx(size_t n, double lo = -1, double hi = 1, double ilo = -1, double ihi = 1) {
+  std::vector<cd> v(n);
+  for (auto& x : v) x = cd{uni(lo, hi), uni(ilo, ihi)};
+  return v;
+}
+static std::vector<double> real(size_t n, double lo, double hi) {
+  std::vector<double> v(n);
+  for (auto& x : v) x = uni(lo, hi);
+  return v;
+}
+
+using Call = std::function<int(std::vector<double>&)>;
+static int g_bad = 0;
+
+// The call without limits, with no optional memory, and over budgets from its
+// mandatory memory on.
+static void check(const std::string& name, const Call& call) {
+  std::vector<double> want, got;
+  auto run = [&](size_t budget, bool none, std::vector<double>& out) {
+    sigma_shutdown();
+    g_budget = budget;
+    g_report_none = none;
+    g_peak = g_used;
+    return call(out);
+  };
+  auto same = [&]() {
+    double worst = 0, top = 0;
+    for (double x : want) top = std::max(top, std::fabs(x));
+    for (size_t i = 0; i < want.size(); ++i) worst = std::max(worst, std::fabs(want[i] - got[i]));
+    return want.size() == got.size() && worst <= 1e-12 * top;  // NaN fails
+  };
+  const size_t all = ~size_t(0) / 4;
+  int st = run(all, false, want);
+  const size_t full = g_peak;
+  if (st != 0) g_bad++, printf("%s: status %d\n", name.c_str(), st);
+  st = run(all, true, got);
+  const size_t least = g_peak;
+  if (st != 0 || !same()) g_bad++, printf("%s without optional memory: status %d, results %d\n", name.c_str(), st, (int)same());
+  printf("%s: %zu MB with the contraction, %zu MB without\n", name.c_str(), full >> 20, least >> 20);
+  if (full <= least) g_bad++, printf("%s: no contraction ran\n", name.c_str());
+  size_t last = 0;
+  for (int k = 0; k <= 16; ++k) {
+    const size_t budget = least + (2 * full - least) / 16 * k;
+    st = run(budget, false, got);
+    if (st != 0 || !same() || g_peak > budget)
+      g_bad++, printf("%s with %zu MB: status %d, results %d\n", name.c_str(), budget >> 20, st, (int)same());
+    if (k == 16) last = g_peak;
+    // the same call again, from its caches
+    st = call(got);
+    if (st != 0 || !same()) g_bad++, printf("%s again with %zu MB: status %d, results %d\n", name.c_str(), budget >> 20, st, (int)same());
+  }
+  if (last != full) g_bad++, printf("%s: %zu MB of %zu at the largest budget\n", name.c_str(), last >> 20, full >> 20);
+}
+
+int main() {
+  const int nb = 71, nvb = 3, nc = 4099, ng = 203;  // nothing divides
+  std::vector<int> inv(ng), ind(nc), iota(nc);
+  for (int g = 0; g < ng; ++g) inv[g] = (g + 1) * (nc - 1) / ng;
+  for (int k = 0; k < nc; ++k) ind[k] = iota[k] = k;
+  const std::vector<double> wx = {3.0, 4.0, 5.0}, v = real(nc, 0.1, 10);
+  const auto am = cplx((size_t)nb * nc), an = cplx((size_t)nb * nc), ie = cplx((size_t)ng * nc),
+             wt = cplx((size_t)ng * nc, 0.5, 5, -0.1, 0.1);
+  const auto rm = real((size_t)nb * nc, -1, 1), rn = real((size_t)nb * nc, -1, 1), re = real((size_t)ng * nc, -1, 1),
+             rw = real((size_t)ng * nc, 0.5, 5);
+  auto put = [](std::vector<double>& out, const std::vector<cd>& z) {
+    for (const cd& x : z) out.insert(out.end(), {x.re, x.im});
+  };
+  check("GPP", [&](std::vector<double>& out) {
+    std::vector<cd> ach(3), asx(3), n1(nb);
+    const int st = sigma_gpp_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, am.data(), an.data(),
+                                  ie.data(), wt.data(), v.data(), ach.data(), asx.data(), n1.data(), nullptr);
+    out.clear();
+    put(out, ach), put(out, asx), put(out, n1);
+    return st;
+  });
+  check("real GPP", [&](std::vector<double>& out) {
+    std::vector<double> ach(3), asx(3), n1(nb);
+    const int st =
+        sigma_gpp_real_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, rm.data(), rn.data(),
+                            re.data(), rw.data(), v.data(), ach.data(), asx.data(), n1.data(), nullptr);
+    out = ach;
+    out.insert(out.end(), asx.begin(), asx.end());
+    out.insert(out.end(), n1.begin(), n1.end());
+    return st;
+  });
+  check("half sum", [&](std::vector<double>& out) {
+    std::vector<cd> ach(3), asx(3), n1(nb), st1(1);
+    const int st = sigma_gpp_halfsum_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, am.data(),
+                                          an.data(), ie.data(), wt.data(), v.data(), ach.data(), asx.data(), n1.data(),
+                                          st1.data(), nullptr);
+    out.clear();
+    put(out, ach), put(out, asx), put(out, n1), put(out, st1);
+    return st;
+  });
+  check("static remainder", [&](std::vector<double>& out) {
+    std::vector<cd> a(1), n1(nb);
+    const int st = sigma_gpp_achstemp(nb, nc, ng, inv.data(), ind.data(), am.data(), an.data(), ie.data(), v.data(),
+                                      a.data(), n1.data(), SIGMA_FF_FP64, nullptr);
+    out.clear();
+    put(out, a), put(out, n1);
+    return st;
+  });
+  const int nf = 4, ne = 5, ngf = 57;
+  const auto er = cplx((size_t)nf * ngf * nc), ea = cplx((size_t)nf * ngf * nc), brd = cplx(nf, 0, 0, 0.1, 0.2);
+  check("FF", [&](std::vector<double>& out) {
+    std::vector<cd> s((size_t)nb * nf);
+    const int st = sigma_ff_schdt(nb, nc, ngf, nf, iota.data(), iota.data(), er.data(), an.data(), am.data(), s.data(),
+                                  SIGMA_FF_FP64, nullptr);
+    out.clear();
+    put(out, s);
+    return st;
+  });
+  std::vector<double> ekq(nb), grid = {0, 1, 2.5, 4}, pref(nf, 0.3);
+  for (int n = 0; n < nb; ++n) ekq[n] = -3.0 + 0.1 * n;
+  check("FF band loop", [&](std::vector<double>& out) {
+    std::vector<cd> a0(1), a1(ne), a2(ne), a3(ne), a4(ne), a5(ne);
+    const int st = sigma_ff_sigma(nb, nvb, nc, ngf, nf, ne, iota.data(), iota.data(), am.data(), an.data(), er.data(),
+                                  ea.data(), v.data(), ekq.data(), grid.data(), brd.data(), pref.data(), 0.16, 0.0, 0.5,
+                                  1.0, nullptr, a0.data(), a1.data(), a2.data(), a3.data(), a4.data(), a5.data(),
+                                  SIGMA_FF_FP64, nullptr);
+    out.clear();
+    put(out, a0), put(out, a1), put(out, a2), put(out, a3), put(out, a4), put(out, a5);
+    return st;
+  });
+  // a plan cache left by one call gives way to another call's inputs
+  {
+    sigma_shutdown();
+    g_budget = ~size_t(0) / 4;
+    g_report_none = false;
+    std::vector<cd> ach(3), asx(3), s((size_t)nb * nf);
+    auto gpp = [&] {
+      return sigma_gpp_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, am.data(), an.data(),
+                            ie.data(), wt.data(), v.data(), ach.data(), asx.data(), nullptr, nullptr);
+    };
+    int st = gpp();
+    const size_t kept = g_used;
+    g_budget = kept + (8u << 20);  // less than the FF call's inputs
+    st = st ? st
+            : sigma_ff_schdt(nb, nc, ngf, nf, iota.data(), iota.data(), er.data(), an.data(), am.data(), s.data(),
+                             SIGMA_FF_FP64, nullptr);
+    if (st != 0) g_bad++, printf("FF after GPP: status %d\n", st);
+    const cd before = ach[0];
+    st = gpp();
+    if (st != 0 || std::hypot(ach[0].re - before.re, ach[0].im - before.im) > 1e-12 * std::hypot(before.re, before.im))
+      g_bad++, printf("GPP after FF: status %d\n", st);
+  }
+  sigma_shutdown();
+  printf("%d bad\n", g_bad);
+  return g_bad != 0;
+}
