@@ -2,7 +2,9 @@
 // routes the library's cudaMalloc, cudaFree and cudaMemGetInfo through the
 // functions below, which keep to a budget.  An optional workspace (the exact
 // contractions') must never make a call fail that its mandatory memory allows,
-// and every way of doing without it must give the same results.
+// and every way of doing without it must give the same results: the same bits
+// where an operand outside the contraction's range sends the call to the FP64
+// kernels anyway, others (the contraction's) where none does.
 #include <cmath>
 #include <cstdio>
 #include <functional>
@@ -67,7 +69,8 @@ static int g_bad = 0;
 
 // The call without limits, with no optional memory, and over budgets from its
 // mandatory memory on.
-static void check(const std::string& name, const Call& call) {
+enum Range { kInside, kOutside, kPartly };  // the operands, of every contraction or of some
+static void check(const std::string& name, const Call& call, Range range = kInside) {
   std::vector<double> want, got;
   auto run = [&](size_t budget, bool none, std::vector<double>& out) {
     sigma_shutdown();
@@ -89,6 +92,9 @@ static void check(const std::string& name, const Call& call) {
   st = run(all, true, got);
   const size_t least = g_peak;
   if (st != 0 || !same()) g_bad++, printf("%s without optional memory: status %d, results %d\n", name.c_str(), st, (int)same());
+  if (range != kPartly && (want == got) != (range == kOutside))
+    g_bad++, printf("%s: the contraction's range check\n", name.c_str());
+  if (range != kInside) return;
   printf("%s: %zu MB with the contraction, %zu MB without\n", name.c_str(), full >> 20, least >> 20);
   if (full <= least) g_bad++, printf("%s: no contraction ran\n", name.c_str());
   size_t last = 0;
@@ -111,22 +117,22 @@ int main() {
   for (int g = 0; g < ng; ++g) inv[g] = (g + 1) * (nc - 1) / ng;
   for (int k = 0; k < nc; ++k) ind[k] = iota[k] = k;
   const std::vector<double> wx = {3.0, 4.0, 5.0}, v = real(nc, 0.1, 10);
-  const auto am = cplx((size_t)nb * nc), an = cplx((size_t)nb * nc), ie = cplx((size_t)ng * nc),
+  auto am = cplx((size_t)nb * nc), an = cplx((size_t)nb * nc), ie = cplx((size_t)ng * nc),
              wt = cplx((size_t)ng * nc, 0.5, 5, -0.1, 0.1);
-  const auto rm = real((size_t)nb * nc, -1, 1), rn = real((size_t)nb * nc, -1, 1), re = real((size_t)ng * nc, -1, 1),
+  auto rm = real((size_t)nb * nc, -1, 1), rn = real((size_t)nb * nc, -1, 1), re = real((size_t)ng * nc, -1, 1),
              rw = real((size_t)ng * nc, 0.5, 5);
   auto put = [](std::vector<double>& out, const std::vector<cd>& z) {
     for (const cd& x : z) out.insert(out.end(), {x.re, x.im});
   };
-  check("GPP", [&](std::vector<double>& out) {
+  const Call gpp_call = [&](std::vector<double>& out) {
     std::vector<cd> ach(3), asx(3), n1(nb);
     const int st = sigma_gpp_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, am.data(), an.data(),
                                   ie.data(), wt.data(), v.data(), ach.data(), asx.data(), n1.data(), nullptr);
     out.clear();
     put(out, ach), put(out, asx), put(out, n1);
     return st;
-  });
-  check("real GPP", [&](std::vector<double>& out) {
+  };
+  const Call real_call = [&](std::vector<double>& out) {
     std::vector<double> ach(3), asx(3), n1(nb);
     const int st =
         sigma_gpp_real_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, rm.data(), rn.data(),
@@ -135,8 +141,8 @@ int main() {
     out.insert(out.end(), asx.begin(), asx.end());
     out.insert(out.end(), n1.begin(), n1.end());
     return st;
-  });
-  check("half sum", [&](std::vector<double>& out) {
+  };
+  const Call half_call = [&](std::vector<double>& out) {
     std::vector<cd> ach(3), asx(3), n1(nb), st1(1);
     const int st = sigma_gpp_halfsum_fp64(nb, nvb, nc, ng, 0, 3, inv.data(), ind.data(), wx.data(), 1.0, am.data(),
                                           an.data(), ie.data(), wt.data(), v.data(), ach.data(), asx.data(), n1.data(),
@@ -144,28 +150,28 @@ int main() {
     out.clear();
     put(out, ach), put(out, asx), put(out, n1), put(out, st1);
     return st;
-  });
-  check("static remainder", [&](std::vector<double>& out) {
+  };
+  const Call static_call = [&](std::vector<double>& out) {
     std::vector<cd> a(1), n1(nb);
     const int st = sigma_gpp_achstemp(nb, nc, ng, inv.data(), ind.data(), am.data(), an.data(), ie.data(), v.data(),
                                       a.data(), n1.data(), SIGMA_FF_FP64, nullptr);
     out.clear();
     put(out, a), put(out, n1);
     return st;
-  });
+  };
   const int nf = 4, ne = 5, ngf = 57;
-  const auto er = cplx((size_t)nf * ngf * nc), ea = cplx((size_t)nf * ngf * nc), brd = cplx(nf, 0, 0, 0.1, 0.2);
-  check("FF", [&](std::vector<double>& out) {
+  auto er = cplx((size_t)nf * ngf * nc), ea = cplx((size_t)nf * ngf * nc), brd = cplx(nf, 0, 0, 0.1, 0.2);
+  const Call ff_call = [&](std::vector<double>& out) {
     std::vector<cd> s((size_t)nb * nf);
     const int st = sigma_ff_schdt(nb, nc, ngf, nf, iota.data(), iota.data(), er.data(), an.data(), am.data(), s.data(),
                                   SIGMA_FF_FP64, nullptr);
     out.clear();
     put(out, s);
     return st;
-  });
+  };
   std::vector<double> ekq(nb), grid = {0, 1, 2.5, 4}, pref(nf, 0.3);
   for (int n = 0; n < nb; ++n) ekq[n] = -3.0 + 0.1 * n;
-  check("FF band loop", [&](std::vector<double>& out) {
+  const Call loop_call = [&](std::vector<double>& out) {
     std::vector<cd> a0(1), a1(ne), a2(ne), a3(ne), a4(ne), a5(ne);
     const int st = sigma_ff_sigma(nb, nvb, nc, ngf, nf, ne, iota.data(), iota.data(), am.data(), an.data(), er.data(),
                                   ea.data(), v.data(), ekq.data(), grid.data(), brd.data(), pref.data(), 0.16, 0.0, 0.5,
@@ -174,7 +180,31 @@ int main() {
     out.clear();
     put(out, a0), put(out, a1), put(out, a2), put(out, a3), put(out, a4), put(out, a5);
     return st;
-  });
+  };
+  const std::vector<std::pair<std::string, const Call*>> calls = {
+      {"GPP", &gpp_call}, {"real GPP", &real_call}, {"half sum", &half_call}, {"static remainder", &static_call},
+      {"FF", &ff_call},   {"FF band loop", &loop_call}};
+  for (const auto& c : calls) check(c.first, *c.second);
+  // one operand element 2^40 above its row
+  const double up = 0x1p40;
+  auto outlier = [&](cd& x, std::initializer_list<int> which, const char* what, Range range = kOutside) {
+    const cd keep = x;
+    x = cd{keep.re * up, keep.im * up};
+    for (int i : which) check(calls[i].first + ", " + what, *calls[i].second, range);
+    x = keep;
+  };
+  outlier(an[(size_t)17 * nc + 33], {0, 2, 3, 4, 5}, "outlier in aqsn");
+  outlier(am[(size_t)1 * nc + 34], {2}, "outlier in an occupied band's aqsm");
+  outlier(ie[(size_t)150 * nc + 35], {0, 3}, "outlier in I_eps");
+  outlier(ie[(size_t)150 * nc + 35], {2}, "outlier in I_eps", kPartly);  // every band is large beside it
+  outlier(er[(size_t)100 * nc + 36], {4, 5}, "outlier in I_epsR");
+  outlier(ea[(size_t)100 * nc + 36], {5}, "outlier in I_epsA", kPartly);
+  for (double* x : {&rn[(size_t)17 * nc + 33], &rn[(size_t)1 * nc + 33], &re[(size_t)150 * nc + 35]}) {
+    const double keep = *x;
+    *x *= up;
+    check("real GPP, outlier", real_call, kOutside);
+    *x = keep;
+  }
   // a plan cache left by one call gives way to another call's inputs
   {
     sigma_shutdown();

@@ -1,6 +1,7 @@
 """Every FP64 host call where the device has no room, or only some, for the
 exact contractions' workspaces: same results, and no call refused that its
-inputs and partial sums fit.  Free memory is simulated (csrc/no_room_check.cu,
+inputs and partial sums fit; and every form with an operand outside the
+contractions' range, which gives the FP64 kernels' bits.  Free memory is simulated (csrc/no_room_check.cu,
 linked with the library's objects); with too little of it the calls take the
 gated copies of the GPP drop-in and each form's FP64 kernels."""
 import pathlib
