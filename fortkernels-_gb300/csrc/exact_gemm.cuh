@@ -263,10 +263,13 @@ __device__ __forceinline__ void ex_put(unsigned char* tile, uint32_t slice_bytes
 }
 
 // The six digits of two values hi + lo (|lo| at most half an ulp of hi) in
-// units of 2^(7 - e), for |hi| < 2^(e - 1): FP32 operations on both lanes of
+// units of 2^(7 - e), for |hi| < 2^e: FP32 operations on both lanes of
 // paired instructions.  Every step is exact but the last addition, which
 // rounds at 2^-60 of 2^e (lo joins the third remainder by TwoSum; its
-// rounding error, 2^-51, joins the fourth).  neg_scale = -2^(7 - e): the
+// rounding error, 2^-51, joins the fourth).  The second digit is rounded with lo
+// in the remainder: beside a remainder of 1/2 lo would put the third at 257,
+// which BF16 does not hold (a bit more room in e avoids that too, at twice the
+// error of every product).  neg_scale = -2^(7 - e): the
 // digits of the negated value come out negated, kM - (x + kM), without an
 // instruction of their own.
 __device__ __forceinline__ void ex_ff_digits(float2 hi, float2 lo, float neg_scale, float2 (&d)[6]) {
@@ -276,7 +279,8 @@ __device__ __forceinline__ void ex_ff_digits(float2 hi, float2 lo, float neg_sca
   const float2 u = __fmul2_rn(hi, make_float2(neg_scale, neg_scale)), w = __fmul2_rn(lo, make_float2(w0, w0));
   d[0] = __ffma2_rn(__fadd2_rn(u, kM), m1, kM);
   float2 r = __fadd2_rn(u, d[0]);
-  d[1] = __ffma2_rn(__ffma2_rn(r, k512, kM), m1, kM);
+  const float2 rw = __ffma2_rn(w, make_float2(1.f / 262144.f, 1.f / 262144.f), r);
+  d[1] = __ffma2_rn(__ffma2_rn(rw, k512, kM), m1, kM);
   r = __ffma2_rn(r, k512, d[1]);
   d[2] = __ffma2_rn(__fadd2_rn(__ffma2_rn(r, k512, w), kM), m1, kM);
   r = __ffma2_rn(r, k512, d[2]);

@@ -184,6 +184,13 @@ __device__ __forceinline__ FF ff_rcp_raw(FF x) {
   const float r0 = rcp_f32(x.hi);
   return FF{r0, r0 * (fmaf(-x.hi, r0, 1.0f) - x.lo * r0)};
 }
+// The same with the correction's second-order term, which is one-signed
+// (2^-49 on average): within 2^-48.
+__device__ __forceinline__ FF ff_rcp2_raw(FF x) {
+  const float r0 = rcp_f32(x.hi);
+  const float t = fmaf(-x.lo, r0, fmaf(-x.hi, r0, 1.0f));
+  return FF{r0, r0 * fmaf(t, t, t)};
+}
 
 // Paired FP32 (f32x2) helpers: halves of a float4, and ff_add of two
 // independent float-float accumulators (hi.x, lo.x) += x.x, (hi.y, lo.y) +=

@@ -186,9 +186,7 @@ __global__ void __launch_bounds__(kGxThreads) gx_max_kernel(GxDev p, ExactPrep e
     // a factor too small for FP32 may only be ignored beside large ones
     const bool small = F::kHalf && tid == F::kSlabs - 1 ? bad_e : bad;
     if (huge || !(f < 1e18f) || (small && !(f > 1e-6f)) || (v && f < 1e-18f)) ex_raise(ex);
-    // float-float digits need a bit of room (ex_ff_digits)
-    ex.ea[gx_row(ex, p.ng, nf, tid, g)] =
-        v ? (int)(__float_as_uint(f) >> 23) - 126 + (F::kF64 ? 0 : 1) : kExZeroRow;
+    ex.ea[gx_row(ex, p.ng, nf, tid, g)] = v ? (int)(__float_as_uint(f) >> 23) - 126 : kExZeroRow;
   }
 }
 
@@ -274,17 +272,17 @@ __device__ __forceinline__ void gx_factors(const FF (&wx)[kNW], const FF (&iwx2)
     }
     const FF c = ff_split_in_range(cd);
     if (F::kReal) {
-      const FF y = ff_mul(gx, gx_norm(ff_rcp_raw(c)));
+      const FF y = ff_mul(gx, gx_norm(ff_rcp2_raw(c)));
       put(iw, keep ? y : zero, zero);
     } else {
-      const FF r = gx_norm(ff_rcp_raw(ff_split_in_range(wv)));
+      const FF r = gx_norm(ff_rcp2_raw(ff_split_in_range(wv)));
       const FF yx = ff_mul(gx_norm(ff_dot2_raw(gx, c, gy, b)), r);
       const FF yy = ff_mul(gx_norm(ff_dot2_raw(gy, c, ff_neg(gx), b)), r);
       put(iw, keep ? yx : zero, keep ? yy : zero);
       if (kOcc) {
         // Omega2 / wx^2 or -G conj(z) / (2 |z|^2), z = wx + wtilde
         const FF z = ff_add(wx[iw], a);
-        const FF rz = gx_norm(ff_rcp_raw(ff_sq_add(z, b2)));
+        const FF rz = gx_norm(ff_rcp2_raw(ff_sq_add(z, b2)));
         const FF tx = gx_norm(ff_dot2_raw(gx, z, gy, ff_neg(b))), ty = gx_norm(ff_dot2_raw(gy, z, gx, b));
         const FF m = keep ? iwx2[iw] : FF{-0.5f * rz.hi, -0.5f * rz.lo};
         const FF sx = ff_mul(keep ? ox : tx, m), sy = ff_mul(keep ? oy : ty, m);
@@ -334,9 +332,9 @@ __global__ void __launch_bounds__(kGxThreads, 4) gx_ff_kernel(GxDev p, ExactPrep
   if (tid < kSlabs * kGxCols) {
     const int i = tid / kGxCols, pl = tid % kGxCols, g = p0 + pl, R = gx_row(ex, p.ng, nf, i, g);
     const int e = g < p.ng ? ex.ea[R] : kExZeroRow;
-    // -2^(7 - e) and 2^(e - 2 - slack) (|e| < 64 unless flagged; a zero row's values are zero)
+    // -2^(7 - e) and 2^(e - 1 - slack) (|e| < 64 unless flagged; a zero row's values are zero)
     s_scale[i][pl] = e == kExZeroRow ? 0.f : -__uint_as_float((unsigned)(134 - e) << 23);
-    s_thr[i][pl] = e == kExZeroRow ? INFINITY : __uint_as_float((unsigned)(125 - kExSlackA + e) << 23);
+    s_thr[i][pl] = e == kExZeroRow ? INFINITY : __uint_as_float((unsigned)(126 - kExSlackA + e) << 23);
     if (i == 0) s_lim[pl] = g < p.ng ? gx_limit<kForm>(p, g, 0) : 0;
     const bool last = i == nf - 1 || i == kSlabs - 1;
     if ((g < p.ng || last) && R < gx_rows_end(ex, nf, i)) atomicMax(&s_need, ex.kt_lim[R / kExRows] * kExKTile);
