@@ -30,6 +30,7 @@
 // issuing thread polls no shared memory, which would stall the tensor pipe).
 #include <algorithm>
 #include <climits>
+#include <cstring>
 
 #include "exact_gemm.cuh"
 
@@ -786,7 +787,7 @@ size_t exact_work_bytes(const ExactPrep& ex) {
 }
 size_t exact_own_bytes(const ExactPrep& ex) {
   const ExSizes z = ex_sizes(ex);
-  return z.flag + z.ent + 2 * z.pcs + 256;
+  return z.flag + z.ent + 2 * z.pcs;
 }
 
 void exact_bind(ExactPrep& ex, void* work, void* own) {
@@ -819,14 +820,20 @@ void exact_bind(ExactPrep& ex, void* work, void* own) {
   ex.any = nullptr;
 }
 
+void exact_pack_own(const ExactPrep& ex, const ExactTables& t, char* host) {
+  const ExSizes z = ex_sizes(ex);
+  std::memset(host, 0, z.flag);
+  host += z.flag;
+  if (!t.entries.empty()) std::memcpy(host, t.entries.data(), sizeof(int4) * t.entries.size());
+  std::memcpy(host + z.ent, t.pieces.data(), sizeof(int) * t.pieces.size());
+  std::memcpy(host + z.ent + z.pcs, t.kt_lim.data(), sizeof(int) * t.kt_lim.size());
+}
 cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t) {
-  auto up = [](const void* dst, const void* src, size_t n) {
-    return n ? cudaMemcpy(const_cast<void*>(dst), src, n, cudaMemcpyHostToDevice) : cudaSuccess;
-  };
-  cudaError_t e = up(ex.entries, t.entries.data(), sizeof(int4) * t.entries.size());
-  if (e == cudaSuccess) e = up(ex.pieces, t.pieces.data(), sizeof(int) * t.pieces.size());
-  if (e == cudaSuccess) e = up(ex.kt_lim, t.kt_lim.data(), sizeof(int) * t.kt_lim.size());
-  return e;
+  std::vector<char> host(exact_own_bytes(ex));
+  exact_pack_own(ex, t, host.data());
+  // own begins 256 bytes, the flag's, before its first table
+  return cudaMemcpy(const_cast<char*>(reinterpret_cast<const char*>(ex.entries)) - 256, host.data(), host.size(),
+                    cudaMemcpyHostToDevice);
 }
 
 cudaError_t exact_begin_flag(const ExactPrep& ex, cudaStream_t s) {

@@ -125,10 +125,13 @@ __host__ __device__ __forceinline__ size_t ex_block_index(const ExactPrep& ex, i
 void exact_size(ExactPrep& ex, int slices, int nb, int nc, int ng, int nf, bool cplx, int grid, const int* row_kend,
                 ExactTables* tables, int nf2 = 0, int nb2 = 0);
 // Buffers: `work` (digits, exponents, raw sums) may be shared by contractions
-// that run one after another on one stream; `own` (flag and tables) may not.
+// that run one after another on one stream; `own` (flag and tables; from a
+// 256-byte boundary) may not.  exact_pack_own writes own's contents, the flag
+// down, into host memory; exact_upload_tables copies them.
 size_t exact_work_bytes(const ExactPrep& ex);
 size_t exact_own_bytes(const ExactPrep& ex);
 void exact_bind(ExactPrep& ex, void* work, void* own);
+void exact_pack_own(const ExactPrep& ex, const ExactTables& t, char* host);
 cudaError_t exact_upload_tables(const ExactPrep& ex, const ExactTables& t);
 
 // FF plans take the exact form from this many products on (rows x bands x K):

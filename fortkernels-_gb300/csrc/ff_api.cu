@@ -19,6 +19,7 @@ struct sigma_ff_plan_s {
   sigma::OzakiPrep oz{};
   sigma::ExactPrep ex{};       // FP64 form on the tensor cores (ex_block set)
   void* ex_block = nullptr;
+  bool ex_arena = false;       // ex_block is an arena's
   void* block = nullptr;
   bool timing = false;
   std::vector<cudaEvent_t> events;  // 3 per recorded execution
@@ -58,7 +59,7 @@ namespace sigma {
 // left out).  Shared by the FF contraction and the static remainders.
 int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, int nfreq,
                   const std::vector<int>& igp_of, int mode, void* shared_tiles,
-                  const int* row_kend, int split_tiles_hint, int items_per_cta) {
+                  const int* row_kend, int split_tiles_hint, int items_per_cta, bool host_call) {
   *out = nullptr;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
@@ -150,7 +151,9 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
     exact_size(p->ex, 6, number_bands, ncouls, ngpown, nfreq, true, sms, row_kend, &et);
     // without room for the digits the FP64 kernel keeps the work
     const size_t work = exact_work_bytes(p->ex), all = work + exact_own_bytes(p->ex);
-    if (!room_for_optional(all) || cudaMalloc(&p->ex_block, all) != cudaSuccess) {
+    p->ex_block = host_call ? arena_optional(kArenaExact, all) : nullptr;
+    p->ex_arena = p->ex_block != nullptr;
+    if (!p->ex_block && (!room_for_optional(all) || cudaMalloc(&p->ex_block, all) != cudaSuccess)) {
       cudaGetLastError();
       p->ex_block = nullptr;
     } else {
@@ -169,20 +172,14 @@ int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, 
   return SIGMA_OK;
 }
 
-bool ff_plan_drop_exact(sigma_ff_plan p) {
-  if (!p->ex_block) return false;
-  cudaFree(p->ex_block);
+void ff_plan_drop_exact(sigma_ff_plan p) {
+  if (p->ex_block && !p->ex_arena) cudaFree(p->ex_block);
   p->ex_block = nullptr;
   p->work.run_if = nullptr;
-  return true;
 }
 
-}  // namespace sigma
-
-extern "C" int sigma_ff_plan_create(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown,
-                                    int nfreq, const int* inv_igp_index, const int* indinv,
-                                    int mode) {
-  using namespace sigma;
+int ff_plan_create(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, int nfreq,
+                   const int* inv_igp_index, const int* indinv, int mode, bool host_call) {
   if (!out || !inv_igp_index || !indinv) return SIGMA_ERR_NULL;
   *out = nullptr;
   int st = ff_check_shape(number_bands, ncouls, ngpown, nfreq);
@@ -191,7 +188,15 @@ extern "C" int sigma_ff_plan_create(sigma_ff_plan* out, int number_bands, int nc
   std::vector<int> igp_of;
   st = ff_map_columns(ncouls, ngpown, inv_igp_index, indinv, igp_of);
   if (st != SIGMA_OK) return st;
-  return ff_plan_build(out, number_bands, ncouls, ngpown, nfreq, igp_of, mode);
+  return ff_plan_build(out, number_bands, ncouls, ngpown, nfreq, igp_of, mode, nullptr, nullptr, 0, 0, host_call);
+}
+
+}  // namespace sigma
+
+extern "C" int sigma_ff_plan_create(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown,
+                                    int nfreq, const int* inv_igp_index, const int* indinv,
+                                    int mode) {
+  return sigma::ff_plan_create(out, number_bands, ncouls, ngpown, nfreq, inv_igp_index, indinv, mode, false);
 }
 
 extern "C" int sigma_ff_plan_destroy(sigma_ff_plan plan) {
@@ -201,7 +206,7 @@ extern "C" int sigma_ff_plan_destroy(sigma_ff_plan plan) {
   cudaSetDevice(plan->device);
   for (cudaEvent_t ev : plan->events) cudaEventDestroy(ev);
   if (plan->block) cudaFree(plan->block);
-  if (plan->ex_block) cudaFree(plan->ex_block);
+  sigma::ff_plan_drop_exact(plan);
   cudaSetDevice(cur);
   delete plan;
   return SIGMA_OK;
@@ -384,7 +389,7 @@ extern "C" int sigma_ff_schdt(int number_bands, int ncouls, int ngpown, int nfre
   }
   sigma_ff_plan plan = nullptr;
   st = with_reclaim([&] {
-    return sigma_ff_plan_create(&plan, number_bands, ncouls, ngpown, nfreq, inv_igp_index, indinv, mode);
+    return ff_plan_create(&plan, number_bands, ncouls, ngpown, nfreq, inv_igp_index, indinv, mode, true);
   });
   if (st != SIGMA_OK) return st;
   const size_t eps_b = sizeof(sigma_complex128) * (size_t)nfreq * ngpown * ncouls;
@@ -392,7 +397,7 @@ extern "C" int sigma_ff_schdt(int number_bands, int ncouls, int ngpown, int nfre
   const size_t out_b = sizeof(sigma_complex128) * (size_t)number_bands * nfreq;
   const size_t o1 = up256(eps_b), o2 = o1 + up256(band_b), o3 = o2 + up256(band_b);
   void* arena = nullptr;
-  st = arena_beside(kArenaFfInputs, o3 + up256(out_b), &arena, [&] { return ff_plan_drop_exact(plan); });
+  st = arena_beside(kArenaFfInputs, o3 + up256(out_b), &arena, [&] { ff_plan_drop_exact(plan); });
   if (st != SIGMA_OK) {
     sigma_ff_plan_destroy(plan);
     return st;

@@ -20,14 +20,20 @@ namespace sigma {
 // split_tiles_hint (split-BF16 form, > 0): K' tiles per work split, so
 // that the plans of a group have items of about the same size; otherwise
 // items_per_cta (> 0; default 20) GEMM items per resident CTA.
+// host_call: the plan lives for one host call (its optional workspace may come
+// from an arena).
 int ff_plan_build(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, int nfreq,
                   const std::vector<int>& igp_of, int mode, void* shared_tiles = nullptr,
-                  const int* row_kend = nullptr, int split_tiles_hint = 0, int items_per_cta = 0);
+                  const int* row_kend = nullptr, int split_tiles_hint = 0, int items_per_cta = 0,
+                  bool host_call = false);
 int ff_plan_tile_bytes(int number_bands, int ncouls, int ngpown, int nfreq, size_t* bytes);
 
 // Gives back the exact contraction's workspace of an FP64 plan with no
-// execution in flight (the FP64 kernels then run); false if it has none.
-bool ff_plan_drop_exact(sigma_ff_plan plan);
+// execution in flight (the FP64 kernels then run).
+void ff_plan_drop_exact(sigma_ff_plan plan);
+// sigma_ff_plan_create of a plan that lives for one host call.
+int ff_plan_create(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, int nfreq,
+                   const int* inv_igp_index, const int* indinv, int mode, bool host_call);
 
 // The split-BF16 plan's operand layout (slice images, K tiles, row limits),
 // for kernels that write the A slices themselves and then execute with

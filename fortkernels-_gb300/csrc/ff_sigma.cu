@@ -189,10 +189,10 @@ struct sigma_ff_sigma_plan_s {
   double2 *cr = nullptr, *ca = nullptr, *sd = nullptr, *per = nullptr;
 };
 
-extern "C" int sigma_ff_sigma_plan_create(sigma_ff_sigma_plan* out, int number_bands, int nvband,
-                                          int ncouls, int ngpown, int nfreq, int nfreqeval,
-                                          const int* inv_igp_index, const int* indinv, int mode) {
-  using namespace sigma;
+namespace sigma {
+namespace {
+int ff_sigma_plan_create(sigma_ff_sigma_plan* out, int number_bands, int nvband, int ncouls, int ngpown, int nfreq,
+                         int nfreqeval, const int* inv_igp_index, const int* indinv, int mode, bool host_call) {
   if (!out || !inv_igp_index || !indinv) return SIGMA_ERR_NULL;
   *out = nullptr;
   if (number_bands <= 0 || ncouls <= 0 || ngpown <= 0 || ngpown > ncouls || nfreq < 2 ||
@@ -209,7 +209,7 @@ extern "C" int sigma_ff_sigma_plan_create(sigma_ff_sigma_plan* out, int number_b
     igp_of[g] = (igp < 0 || igp >= ncouls) ? -1 : igp;
   }
   auto* p = new sigma_ff_sigma_plan_s();
-  int st = ff_plan_build(&p->ff, number_bands, ncouls, ngpown, nfreq, igp_of, mode);
+  int st = ff_plan_build(&p->ff, number_bands, ncouls, ngpown, nfreq, igp_of, mode, nullptr, nullptr, 0, 0, host_call);
   if (st != SIGMA_OK) {
     delete p;
     return st;
@@ -236,6 +236,15 @@ extern "C" int sigma_ff_sigma_plan_create(sigma_ff_sigma_plan* out, int number_b
   p->per = reinterpret_cast<double2*>(b + 3 * mat);
   *out = p;
   return SIGMA_OK;
+}
+}  // namespace
+}  // namespace sigma
+
+extern "C" int sigma_ff_sigma_plan_create(sigma_ff_sigma_plan* out, int number_bands, int nvband,
+                                          int ncouls, int ngpown, int nfreq, int nfreqeval,
+                                          const int* inv_igp_index, const int* indinv, int mode) {
+  return sigma::ff_sigma_plan_create(out, number_bands, nvband, ncouls, ngpown, nfreq, nfreqeval, inv_igp_index, indinv,
+                                     mode, false);
 }
 
 extern "C" int sigma_ff_sigma_plan_destroy(sigma_ff_sigma_plan p) {
@@ -348,8 +357,8 @@ extern "C" int sigma_ff_sigma(int number_bands, int nvband, int ncouls, int ngpo
   std::lock_guard<std::mutex> lk(api_mutex());
   sigma_ff_sigma_plan plan = nullptr;
   int st = with_reclaim([&] {
-    return sigma_ff_sigma_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nfreq, nfreqeval, inv_igp_index,
-                                      indinv, mode);
+    return ff_sigma_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nfreq, nfreqeval, inv_igp_index, indinv,
+                                mode, true);
   });
   if (st != SIGMA_OK) return st;
   const int nb = number_bands, nf = nfreq, ne = nfreqeval;
@@ -368,7 +377,7 @@ extern "C" int sigma_ff_sigma(int number_bands, int nvband, int ncouls, int ngpo
                o_pref = take(sizeof(double) * nf), o_sd = take(mat_b),
                o_out = take(sizeof(double2) * (1 + kOut * ne));
   void* arena = nullptr;
-  st = arena_beside(kArenaFfInputs, off, &arena, [&] { return ff_plan_drop_exact(plan->ff); });
+  st = arena_beside(kArenaFfInputs, off, &arena, [&] { ff_plan_drop_exact(plan->ff); });
   if (st != SIGMA_OK) {
     sigma_ff_sigma_plan_destroy(plan);
     return st;

@@ -638,7 +638,7 @@ int gpp_host(int precision, int nb, int nvband, int nc, int ng, int nstart, int 
     total += align_up(sizes[i], 256);
   }
   void* arena = nullptr;
-  st = arena_get(kArenaGppInputs, total, &arena);
+  st = arena_beside(kArenaGppInputs, total, &arena, [] {});  // (the cached plan's workspace: drop_cached_workspace)
   if (st != SIGMA_OK) return st;
   char* a = static_cast<char*>(arena);
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -292,30 +292,48 @@ int build_tensor_group(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst,
 }
 
 // FP64 with shared frequencies: an exact contraction per instance that is
-// large enough, when the device has room for the largest one's workspace.
+// large enough, when the device has room for the largest one's workspace (and
+// the tables, which follow it).
 void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std::vector<std::vector<int>>& igp,
                  int sms) {
   auto shape = [&](int i) {
     return GxShape{kGxGpp, inst[i].number_bands, inst[i].nvband, inst[i].ncouls, inst[i].ngpown, false};
   };
-  size_t ws = 0;
+  size_t ws = 0, own = 0;
+  std::vector<size_t> own_off(b->n);
   for (int i = 0; i < b->n; ++i)
-    if (gpp_exact_fits(shape(i))) ws = std::max(ws, gpp_exact_work_bytes(shape(i), igp[i], sms));
-  if (ws == 0 || !room_for_optional(ws)) return;
-  if (cudaMalloc(&b->exact_ws, ws) != cudaSuccess) {
+    if (gpp_exact_fits(shape(i))) {
+      size_t bytes = 0;
+      ws = std::max(ws, gpp_exact_work_bytes(shape(i), igp[i], sms, &bytes));
+      own_off[i] = own;
+      own += bytes;
+    }
+  ws = up256(ws);
+  if (ws == 0 || !room_for_optional(ws + own)) return;
+  if (cudaMalloc(&b->exact_ws, ws + own) != cudaSuccess) {
     cudaGetLastError();
     b->exact_ws = nullptr;
     return;
   }
+  char* own_dev = static_cast<char*>(b->exact_ws) + ws;
+  std::vector<char> own_host(own);
   b->exact.resize(b->n);
   bool all = true;
   for (int i = 0; i < b->n; ++i) {
-    if (!gpp_exact_fits(shape(i)) || !gpp_exact_create(b->exact[i], shape(i), igp[i], sms, b->exact_ws)) {
+    if (!gpp_exact_fits(shape(i))) {
       all = false;
       continue;
     }
+    gpp_exact_create(b->exact[i], shape(i), igp[i], sms,
+                     GxShared{b->exact_ws, own_dev + own_off[i], own_host.data() + own_off[i]});
     b->sch[i].run_if = b->ssx[i].run_if = b->exact[i].ex.flag;
     b->exact[i].ex.any = b->counters + 3;
+  }
+  if (cudaMemcpy(own_dev, own_host.data(), own, cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaGetLastError();
+    for (int i = 0; i < b->n; ++i) b->sch[i].run_if = b->ssx[i].run_if = nullptr;
+    b->exact.clear();
+    return;
   }
   // no instance needs the queue's passes unless some flag is raised
   if (all) b->sch_view.run_if = b->counters + 3;
@@ -757,7 +775,6 @@ extern "C" int sigma_gpp_batch_destroy(sigma_gpp_batch b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   for (sigma_ff_plan f : b->ff)
     if (f) sigma_ff_plan_destroy(f);
-  for (sigma::GppExact& x : b->exact) sigma::gpp_exact_destroy(x);
   if (b->exact_ws) cudaFree(b->exact_ws);
   if (b->tensor_ws) cudaFree(b->tensor_ws);
   if (b->group_block) cudaFree(b->group_block);

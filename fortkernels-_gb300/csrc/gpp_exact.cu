@@ -708,52 +708,67 @@ bool gpp_exact_fits(const GxShape& q) {
   return gpp_exact_pays(q) && exact_holds(q.nc, q.form != kGxReal && q.form != kGxRealOcc);
 }
 
-size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms) {
+size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms, size_t* own) {
   ExactPrep ex{};
   std::vector<int> kend;
   int nf, nf2;
   gx_size(ex, q, igp_of, sms, nf, nf2, kend, nullptr);
+  if (own) *own = exact_own_bytes(ex);
   return exact_work_bytes(ex) + gx_stat_bytes(ex, gx_run(ex, q.ng, sms));
 }
 
-bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, void* shared_work) {
+namespace {
+
+// Sizes g; returns its tables.
+ExactTables gx_plan(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms) {
   g = GppExact();
   ExactTables t;
   std::vector<int> kend;
   gx_size(g.ex, q, igp_of, sms, g.nf, g.nf2, kend, &t);
   g.run = gx_run(g.ex, q.ng, sms);
-  const size_t work = exact_work_bytes(g.ex), own = exact_own_bytes(g.ex);
-  const size_t stat = gx_stat_bytes(g.ex, g.run);
-  if (!shared_work && !room_for_optional(work + stat)) {
-    g = GppExact();
-    return false;
-  }
-  if (cudaMalloc(&g.own, own) != cudaSuccess) g.own = nullptr;
-  if (g.own && !shared_work && cudaMalloc(&g.work, work + stat) != cudaSuccess) {
-    cudaFree(g.own);
-    g.own = g.work = nullptr;
-  }
-  if (!g.own) {
-    cudaGetLastError();
-    g = GppExact();
-    return false;
-  }
-  void* w = shared_work ? shared_work : g.work;
-  exact_bind(g.ex, w, g.own);
   g.form = q.form;
-  g.stat = reinterpret_cast<float*>(static_cast<char*>(w) + work);
   g.grid = sms;
+  return t;
+}
+void gx_bind(GppExact& g, void* work, void* own) {
+  exact_bind(g.ex, work, own);
+  g.stat = reinterpret_cast<float*>(static_cast<char*>(work) + exact_work_bytes(g.ex));
+}
+
+}  // namespace
+
+bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, int arena_slot) {
+  const ExactTables t = gx_plan(g, q, igp_of, sms);
+  const size_t work = (exact_work_bytes(g.ex) + gx_stat_bytes(g.ex, g.run) + 255) / 256 * 256;
+  const size_t all = work + exact_own_bytes(g.ex);
+  void* block = arena_slot >= 0 ? arena_optional(arena_slot, all) : nullptr;
+  if (!block) {
+    if (!room_for_optional(all) || cudaMalloc(&g.block, all) != cudaSuccess) {
+      cudaGetLastError();
+      g = GppExact();
+      return false;
+    }
+    block = g.block;
+  }
+  gx_bind(g, block, static_cast<char*>(block) + work);
   if (exact_upload_tables(g.ex, t) != cudaSuccess) {
     cudaGetLastError();
     gpp_exact_destroy(g);
     return false;
   }
+  g.ready = true;
   return true;
 }
 
+void gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, const GxShared& m) {
+  const ExactTables t = gx_plan(g, q, igp_of, sms);
+  gx_bind(g, m.work, m.own);
+  exact_pack_own(g.ex, t, m.own_host);
+  g.ready = true;
+}
+
 void gpp_exact_destroy(GppExact& g) {
-  if (g.own) cudaFree(g.own);
-  if (g.work) cudaFree(g.work);
+  if (g.block) cudaFree(g.block);
   g = GppExact();
 }
 

@@ -46,8 +46,17 @@ struct GppExact {
   float* stat = nullptr;  // [rows][runs] large factors per run (half sum: least sums of squares with any band)
   int run = 0;            // g-vectors per factor item (a segment or a power-of-two part of it)
   int grid = 0;
-  void *own = nullptr, *work = nullptr;  // work null when the caller's is used
-  explicit operator bool() const { return own != nullptr; }
+  void* block = nullptr;  // its allocation; null when the caller's memory is used
+  bool ready = false;
+  explicit operator bool() const { return ready; }
+};
+
+// Memory of a caller that runs several contractions one after another on one
+// stream: one workspace (at least gpp_exact_work_bytes of each), and tables
+// (gpp_exact_own_bytes each), packed into host memory for one copy.
+struct GxShared {
+  void *work, *own;  // device
+  char* own_host;
 };
 
 // The contraction's shape: nb bands (kGxRealOcc, kGxHalfOcc: the occupied ones),
@@ -61,13 +70,14 @@ struct GxShape {
 // Sizes, allocates and fills the contraction of one instance; false (with
 // nothing allocated) when the device has no room, or the workspace would take
 // more than half of its free memory: the FP64 kernels keep the
-// work, as for problems too small for it (gpp_exact_fits).  With shared_work set
-// (at least gpp_exact_work_bytes) the instance has no workspace of its own.
-bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms,
-                      void* shared_work = nullptr);
+// work, as for problems too small for it (gpp_exact_fits).
+// A plan that lives for one host call takes its memory from an arena slot
+// (ArenaSlot) where it may.
+bool gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, int arena_slot = -1);
+void gpp_exact_create(GppExact& g, const GxShape& q, const std::vector<int>& igp_of, int sms, const GxShared& m);
 bool gpp_exact_fits(const GxShape& q);
 bool gpp_exact_pays(const GxShape& q);  // large enough, whatever the sums' length
-size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms);
+size_t gpp_exact_work_bytes(const GxShape& q, const std::vector<int>& igp_of, int sms, size_t* own = nullptr);
 void gpp_exact_destroy(GppExact& g);
 
 // launch_gpp_exact_operands forms the operands and raises g.ex.flag for

@@ -1120,11 +1120,11 @@ struct sigma_gpp_halfsum_plan_s {
   double2 *t3 = nullptr, *u3 = nullptr, *ts = nullptr, *us = nullptr;  // [nb][3], [nb][1]
 };
 
-extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int number_bands,
-                                             int nvband, int ncouls, int ngpown, int nstart,
-                                             int nend, const int* inv_igp_index,
-                                             const int* indinv, int indinv_len, int flags) {
-  using namespace sigma;
+namespace sigma {
+namespace {
+int halfsum_plan_create(sigma_gpp_halfsum_plan* out, int number_bands, int nvband, int ncouls, int ngpown, int nstart,
+                        int nend, const int* inv_igp_index, const int* indinv, int indinv_len, int flags,
+                        bool host_call) {
   if (!out || !inv_igp_index || !indinv) return SIGMA_ERR_NULL;
   *out = nullptr;
   if (flags & ~(SIGMA_HALFSUM_STATIC | SIGMA_HALFSUM_GVEC_MAJOR | SIGMA_HALFSUM_TENSOR))
@@ -1256,7 +1256,7 @@ extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int nu
     }
   }
   const GxShape q{kGxHalf, number_bands, nvband, ncouls, ngpown, (flags & SIGMA_HALFSUM_STATIC) != 0};
-  if (!tensor && gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms)) {
+  if (!tensor && gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms, host_call ? kArenaExact : -1)) {
     const size_t n = 2 * (size_t)number_bands * p->exact.nf, n_occ = 2 * (size_t)nvband * 2 * kNW;
     if (cudaMalloc(&p->tblock, sizeof(double2) * (n + n_occ)) != cudaSuccess) {
       cudaGetLastError();
@@ -1267,11 +1267,22 @@ extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int nu
       p->tu_occ = p->tu + n;
       p->exact.ex.flag = p->counters + 3;  // cleared with the counters
       const GxShape qo{kGxHalfOcc, nvband, nvband, ncouls, ngpown, false};
-      if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->counters + 3;
+      if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms, host_call ? kArenaExactOcc : -1))
+        p->exact_occ.ex.flag = p->counters + 3;
     }
   }
   *out = p;
   return SIGMA_OK;
+}
+}  // namespace
+}  // namespace sigma
+
+extern "C" int sigma_gpp_halfsum_plan_create(sigma_gpp_halfsum_plan* out, int number_bands,
+                                             int nvband, int ncouls, int ngpown, int nstart,
+                                             int nend, const int* inv_igp_index,
+                                             const int* indinv, int indinv_len, int flags) {
+  return sigma::halfsum_plan_create(out, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index, indinv,
+                                    indinv_len, flags, false);
 }
 
 extern "C" int sigma_gpp_halfsum_plan_destroy(sigma_gpp_halfsum_plan p) {
@@ -1451,8 +1462,8 @@ int halfsum_host(bool tensor, int number_bands, int nvband, int ncouls, int ngpo
   const int flags = SIGMA_HALFSUM_GVEC_MAJOR | (achstemp ? SIGMA_HALFSUM_STATIC : 0) |
                     (tensor ? SIGMA_HALFSUM_TENSOR : 0);
   st = with_reclaim([&] {
-    return sigma_gpp_halfsum_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index,
-                                         indinv, ncouls, flags);
+    return halfsum_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index, indinv, ncouls,
+                               flags, true);
   });
   if (st != SIGMA_OK) return st;
   const size_t bb = sizeof(sigma_complex128) * (size_t)number_bands * ncouls;
@@ -1468,10 +1479,8 @@ int halfsum_host(bool tensor, int number_bands, int nvband, int ncouls, int ngpo
                o_out = take(sizeof(sigma_complex128) * (2 * kNW + 1 + (size_t)number_bands));
   void* arena = nullptr;
   st = arena_beside(kArenaMisc, off, &arena, [&] {
-    const bool any = static_cast<bool>(plan->exact);
     gpp_exact_destroy(plan->exact);
     gpp_exact_destroy(plan->exact_occ);
-    return any;
   });
   if (st != SIGMA_OK) {
     sigma_gpp_halfsum_plan_destroy(plan);

@@ -360,11 +360,10 @@ struct sigma_gpp_real_plan_s {
   double2* outc = nullptr;     // achtemp[3], asxtemp[3], acht_n1_loc[nb] (complex workspace)
 };
 
-extern "C" int sigma_gpp_real_plan_create(sigma_gpp_real_plan* out, int number_bands, int nvband,
-                                          int ncouls, int ngpown, int nstart, int nend,
-                                          const int* inv_igp_index, const int* indinv,
-                                          int indinv_len) {
-  using namespace sigma;
+namespace sigma {
+namespace {
+int real_plan_create(sigma_gpp_real_plan* out, int number_bands, int nvband, int ncouls, int ngpown, int nstart,
+                     int nend, const int* inv_igp_index, const int* indinv, int indinv_len, bool host_call) {
   if (!out || !inv_igp_index || !indinv) return SIGMA_ERR_NULL;
   *out = nullptr;
   int st = gpp_check_shape(number_bands, nvband, ncouls, ngpown, nstart, nend);
@@ -422,13 +421,24 @@ extern "C" int sigma_gpp_real_plan_create(sigma_gpp_real_plan* out, int number_b
     return SIGMA_ERR_CUDA;
   }
   const GxShape q{kGxReal, number_bands, nvband, ncouls, ngpown, false};
-  if (gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms)) {
+  if (gpp_exact_fits(q) && gpp_exact_create(p->exact, q, igp_of, sms, host_call ? kArenaExact : -1)) {
     p->exact.ex.flag = p->counters + 3;  // cleared with the counters
     const GxShape qo{kGxRealOcc, nvband, nvband, ncouls, ngpown, false};
-    if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms)) p->exact_occ.ex.flag = p->counters + 3;
+    if (nvband > 0 && gpp_exact_create(p->exact_occ, qo, igp_of, sms, host_call ? kArenaExactOcc : -1))
+      p->exact_occ.ex.flag = p->counters + 3;
   }
   *out = p;
   return SIGMA_OK;
+}
+}  // namespace
+}  // namespace sigma
+
+extern "C" int sigma_gpp_real_plan_create(sigma_gpp_real_plan* out, int number_bands, int nvband,
+                                          int ncouls, int ngpown, int nstart, int nend,
+                                          const int* inv_igp_index, const int* indinv,
+                                          int indinv_len) {
+  return sigma::real_plan_create(out, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index, indinv,
+                                 indinv_len, false);
 }
 
 extern "C" int sigma_gpp_real_plan_destroy(sigma_gpp_real_plan p) {
@@ -511,8 +521,8 @@ extern "C" int sigma_gpp_real_fp64(int number_bands, int nvband, int ncouls, int
   std::lock_guard<std::mutex> lk(api_mutex());
   sigma_gpp_real_plan plan = nullptr;
   st = with_reclaim([&] {
-    return sigma_gpp_real_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index, indinv,
-                                      ncouls);
+    return real_plan_create(&plan, number_bands, nvband, ncouls, ngpown, nstart, nend, inv_igp_index, indinv, ncouls,
+                            true);
   });
   if (st != SIGMA_OK) return st;
   const size_t bb = sizeof(double) * (size_t)number_bands * ncouls;
@@ -529,10 +539,8 @@ extern "C" int sigma_gpp_real_fp64(int number_bands, int nvband, int ncouls, int
                o_1 = take(sizeof(double) * number_bands);
   void* arena = nullptr;
   st = arena_beside(kArenaMisc, off, &arena, [&] {
-    const bool any = static_cast<bool>(plan->exact);
     gpp_exact_destroy(plan->exact);
     gpp_exact_destroy(plan->exact_occ);
-    return any;
   });
   if (st != SIGMA_OK) {
     sigma_gpp_real_plan_destroy(plan);

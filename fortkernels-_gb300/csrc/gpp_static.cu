@@ -36,7 +36,7 @@ __global__ void band_total_kernel(const double2* n1v, int nb, double2* total) {
 }
 
 int static_plan(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, const int* inv_igp_index,
-                const int* indinv, int mode) {
+                const int* indinv, int mode, bool host_call) {
   using namespace sigma;
   int st = gpp_check_shape(number_bands, 0, ncouls, ngpown, 0, kNW);
   if (st != SIGMA_OK) return st;
@@ -45,7 +45,7 @@ int static_plan(sigma_ff_plan* out, int number_bands, int ncouls, int ngpown, co
   int valid = 0;
   st = gpp_map_columns(ncouls, ngpown, inv_igp_index, indinv, ncouls, igp_of, valid);
   if (st != SIGMA_OK) return st;
-  return ff_plan_build(out, number_bands, ncouls, ngpown, 1, igp_of, mode);
+  return ff_plan_build(out, number_bands, ncouls, ngpown, 1, igp_of, mode, nullptr, nullptr, 0, 0, host_call);
 }
 }  // namespace
 
@@ -54,7 +54,7 @@ extern "C" int sigma_gpp_static_plan_create(sigma_ff_plan* plan, int number_band
                                             int mode) {
   if (!plan || !inv_igp_index || !indinv) return SIGMA_ERR_NULL;
   *plan = nullptr;
-  return static_plan(plan, number_bands, ncouls, ngpown, inv_igp_index, indinv, mode);
+  return static_plan(plan, number_bands, ncouls, ngpown, inv_igp_index, indinv, mode, false);
 }
 
 extern "C" int sigma_gpp_static_execute(sigma_ff_plan plan, const sigma_complex128* aqsmtemp,
@@ -99,7 +99,7 @@ extern "C" int sigma_gpp_achstemp(int number_bands, int ncouls, int ngpown, cons
   std::lock_guard<std::mutex> lk(api_mutex());
   sigma_ff_plan plan = nullptr;
   int st = with_reclaim(
-      [&] { return static_plan(&plan, number_bands, ncouls, ngpown, inv_igp_index, indinv, mode); });
+      [&] { return static_plan(&plan, number_bands, ncouls, ngpown, inv_igp_index, indinv, mode, true); });
   if (st != SIGMA_OK) return st;
   const size_t eps_b = sizeof(sigma_complex128) * (size_t)ngpown * ncouls;
   const size_t band_b = sizeof(sigma_complex128) * (size_t)number_bands * ncouls;
@@ -108,7 +108,7 @@ extern "C" int sigma_gpp_achstemp(int number_bands, int ncouls, int ngpown, cons
   const size_t o1 = up256(eps_b), o2 = o1 + up256(band_b), o3 = o2 + up256(band_b),
                o4 = o3 + up256(v_b), o5 = o4 + up256(out_b);
   void* arena = nullptr;
-  st = arena_beside(kArenaFfInputs, o5 + 256, &arena, [&] { return ff_plan_drop_exact(plan); });
+  st = arena_beside(kArenaFfInputs, o5 + 256, &arena, [&] { ff_plan_drop_exact(plan); });
   if (st != SIGMA_OK) {
     sigma_ff_plan_destroy(plan);
     return st;

@@ -50,6 +50,7 @@ int device_sm_count() {
 
 // ---------------------------------------------------------------- device arena
 namespace {
+constexpr size_t kOptionalUnasked = size_t(256) << 20;
 struct Arena {
   void* ptr = nullptr;
   size_t bytes = 0;
@@ -102,12 +103,40 @@ int arena_get(int slot, size_t bytes, void** out) {
 }
 
 bool room_for_optional(size_t bytes) {
+  if (bytes <= kOptionalUnasked) return true;
   size_t free_bytes = 0, total = 0;
   if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   return bytes <= free_bytes / 2;
+}
+
+void* arena_optional(int slot, size_t bytes) {
+  void* p = nullptr;
+  int dev = 0;
+  if (bytes > kOptionalUnasked || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  Arena& a = arenas()[dev * kArenaSlots + slot];
+  if (a.bytes >= bytes) return a.ptr;
+  if (a.ptr) cudaFree(a.ptr);
+  const size_t step = size_t(32) << 20, want = (bytes + step - 1) / step * step;
+  if (cudaMalloc(&p, want) != cudaSuccess) {
+    cudaGetLastError();
+    p = nullptr;
+  }
+  a.ptr = p;
+  a.bytes = p ? want : 0;
+  return p;
+}
+void drop_optional_arenas() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  for (int slot : {kArenaExact, kArenaExactOcc}) {
+    Arena& a = arenas()[dev * kArenaSlots + slot];
+    if (a.ptr) cudaFree(a.ptr);
+    a.ptr = nullptr;
+    a.bytes = 0;
+  }
 }
 
 void register_shutdown_hook(ShutdownHook h) { hooks().push_back(h); }

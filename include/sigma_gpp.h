@@ -133,7 +133,8 @@ int sigma_gpp_tensor(int number_bands, int nvband, int ncouls, int ngpown, int n
  * and only while they are at most half of the device's free memory; without
  * them it runs the FP64 kernels (150 ms instead of 12 at that size).  Executions
  * with per-band frequencies, and sigma_gpp_fp64_noalloc, do not use them.  The
- * host calls give them up where their inputs need the memory.
+ * host calls give them up where their inputs need the memory, and keep those of
+ * up to 256 MB (two for the real-valued and the half sum) between calls.
  * ------------------------------------------------------------------------- */
 typedef struct sigma_gpp_plan_s* sigma_gpp_plan;
 
