@@ -28,6 +28,7 @@
 // The FP64 and mixed forms reduce all instances with the grouped reduction
 // (two launches).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <numeric>
 #include <vector>
@@ -291,20 +292,45 @@ int build_tensor_group(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst,
   return SIGMA_OK;
 }
 
-// FP64 with shared frequencies: an exact contraction per instance that is
-// large enough, when the device has room for the largest one's workspace (and
-// the tables, which follow it).
+// Which instances take an exact contraction.  A contraction is a chain of
+// eight launches, 45 us for the smallest instance and 60 at 24 x 40 x 1024;
+// the queue's passes take all instances at once, 100 us and more for the first
+// but only 6 and 33 us for each further one of these.  Below 1.5e7 products an
+// instance costs the contraction up to 40 us more than the queue; where
+// those add up to more than the queue's own start, or the queue runs
+// anyway for an instance too small for a contraction, such instances stay with
+// it (batches of 8: 16 x 20 x 512 in 141 us, 393 in contractions; 24 x 40 x 1024
+// 316 and 489; 60 x 60 x 2048 1102 and 714).
+constexpr double kQueueBelow = 1.5e7, kQueueGain = 40.0, kQueueStart = 85.0;
+std::vector<bool> exact_choice(const std::vector<GxShape>& q) {
+  std::vector<bool> take(q.size());
+  double gain = 0.0;
+  bool queue = false;
+  auto products = [&](size_t i) { return (double)kNW * q[i].nb * q[i].ng * q[i].nc; };
+  for (size_t i = 0; i < q.size(); ++i) {
+    take[i] = gpp_exact_fits(q[i]);
+    queue = queue || !take[i];
+    gain += kQueueGain * std::max(0.0, 1.0 - std::sqrt(products(i) / kQueueBelow));
+  }
+  if (queue || gain > kQueueStart)
+    for (size_t i = 0; i < q.size(); ++i) take[i] = take[i] && products(i) >= kQueueBelow;
+  return take;
+}
+
+// FP64 with shared frequencies: exact contractions, when the device has room
+// for the largest one's workspace (and the tables, which follow it).
 void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std::vector<std::vector<int>>& igp,
                  int sms) {
-  auto shape = [&](int i) {
-    return GxShape{kGxGpp, inst[i].number_bands, inst[i].nvband, inst[i].ncouls, inst[i].ngpown, false};
-  };
+  std::vector<GxShape> q;
+  for (int i = 0; i < b->n; ++i)
+    q.push_back({kGxGpp, inst[i].number_bands, inst[i].nvband, inst[i].ncouls, inst[i].ngpown, false});
+  const std::vector<bool> take = exact_choice(q);
   size_t ws = 0, own = 0;
   std::vector<size_t> own_off(b->n);
   for (int i = 0; i < b->n; ++i)
-    if (gpp_exact_fits(shape(i))) {
+    if (take[i]) {
       size_t bytes = 0;
-      ws = std::max(ws, gpp_exact_work_bytes(shape(i), igp[i], sms, &bytes));
+      ws = std::max(ws, gpp_exact_work_bytes(q[i], igp[i], sms, &bytes));
       own_off[i] = own;
       own += bytes;
     }
@@ -320,11 +346,11 @@ void build_exact(sigma_gpp_batch_s* b, const sigma_gpp_instance* inst, const std
   b->exact.resize(b->n);
   bool all = true;
   for (int i = 0; i < b->n; ++i) {
-    if (!gpp_exact_fits(shape(i))) {
+    if (!take[i]) {
       all = false;
       continue;
     }
-    gpp_exact_create(b->exact[i], shape(i), igp[i], sms,
+    gpp_exact_create(b->exact[i], q[i], igp[i], sms,
                      GxShared{b->exact_ws, own_dev + own_off[i], own_host.data() + own_off[i]});
     b->sch[i].run_if = b->ssx[i].run_if = b->exact[i].ex.flag;
     b->exact[i].ex.any = b->counters + 3;
