@@ -314,7 +314,7 @@ EXACT_BF16_FLOP_PER_TERM = 2.0 * 4 * 21
 # A's tiles in L2, so the traffic of a launch is A's digits once per pass over
 # its bands.
 EXACT_DRAM_BYTES_PER_A_BYTE = 1.06
-EXACT_TENSOR_PIPE_ACTIVE_NCU = 0.673
+EXACT_TENSOR_PIPE_ACTIVE_NCU = 0.718
 # FP32 pipe operations of sch_mixedy_kernel per term: 4 FFMA (complex
 # multiply-add) + the float-float fold of each accumulator every 8 g-vectors
 # (2 x 7 operations / 8) + the shared frequency factor (~10 per column,

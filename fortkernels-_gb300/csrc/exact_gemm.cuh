@@ -16,25 +16,29 @@
 // s <= 5 go to six FP32 accumulators, one per s.  Over 128 K values the sums
 // stay below 2^24 (s <= 2: 128 (2 2^15 + 2^16) = 2^24 at most), so the FP32
 // accumulation is exact whatever the data; s = 3 .. 5 carry weights of 2^-41
-// and below of the row maxima and may round in the all-equal worst case only.
-// Dropped products (s >= 6) and the digits' own rounding are 2^-53 of the
-// product of the row maxima.
+// and below of the row maxima and may round where the data are all alike.
+// Dropped products (s >= 6) come to 2^-52 rms of the product of the row maxima,
+// the digits' own rounding to 2^-54.
 //
 // Seven digits (28 products) serve operands whose rows hold a few elements
 // far above the rest: the half sum's factors near poles.
 //
 // Over random digits a product's error is 2^-52 (six digits) or 2^-61 (seven)
 // rms of the product of its rows' largest elements, and that of a sum of K
-// products sqrt(K) times it, whatever the elements' own size.  So every row pair
-// is checked for a sum of squares that is large enough beside it.  The
+// products sqrt(K) times it, whatever the elements' own size.  So every row
+// pair is checked for a sum of squares that is large enough beside it.  The
 // statistics passes count that elements within 2^-5 (A) and 2^-4 (B) of their
-// rows' largest meet in at least K / 128 places of every row pair (if all
-// others were zero, the error would be 2^-39.5 of the sum's root mean square
-// with six digits, 2^-48 with seven; uniform inputs: 2^-51 with six).  Rows that fail, and values that are not finite, raise
-// ExactPrep::flag, and the callers' FP64 kernels run instead.  The half sum's
-// rows end at their igp and may hold few large elements (factors near poles);
-// they are checked against band_min, the least element of any band at each K
-// value (gx_check_kernel).
+// rows' largest meet in at least K / 128 places of every row pair: if all others
+// were zero, the error would be 2^-39.5 of the sum's root mean square with six
+// digits and 2^-48 with seven (uniform inputs: 2^-51 with six).  Rows that fail,
+// and values that are not finite, raise ExactPrep::flag, and the callers' FP64
+// kernels run instead.  The half sum's rows end at their igp and may hold few
+// large elements (factors near poles); they are checked against band_min, the
+// least element of any band at each K value (gx_check_kernel).
+//
+// The splitting is the error-free transformation of matrix products of Ozaki,
+// Ogita, Oishi and Rump (Numerical Algorithms 59, 2012), here with one exponent
+// per row, digits fixed by BF16's significand and integer sums.
 #pragma once
 
 #include <vector>

@@ -11,13 +11,14 @@
 // gx_max_kernel bounds the factors per row (the digits' exponent) from FP32
 // values, one pass over the inputs at memory speed.
 // gx_ff_kernel forms them from FP64 numerators in float-float arithmetic (FP32
-// pairs: ~2^-48 rms, below the float-float terms it replaces), cuts them into
+// pairs: ~2^-48 rms), cuts them into
 // digits with paired FP32 operations and writes each row's digits as 16-byte
 // chunks: 16 columns x 32 g-vectors staged in shared memory, four CTAs per SM.
-// Bound by issue slots (69 % issuing, FP64 pipe 52 %, FMA 48 %): 2.43 ms at
-// 1638 x 32768 with the occupied bands' factors (2.38 ms with the next tile
-// prefetched to L2), 2.74 ms with digits of one
-// value per instruction, the general FP64 split and all large factors counted.
+// Bound by issue slots (69 % issuing, FP64 pipe 53 %, FMA 49 %): 2.42 ms at
+// 1638 x 32768 with the occupied bands' factors (2.38 ms with the reciprocal's
+// first-order correction and an exponent bit to spare, whose band sums' errors
+// were 7.4e-15 instead of 4.8e-15; 2.74 ms with digits of one
+// value per instruction, the general FP64 split and all large factors counted).
 // Factors of two elements per instruction need 80 registers or spill at two
 // or three CTAs per SM: 3.13 and 3.35 ms.
 // (The factors in FP64, 34 operations per column and g-vector, ran at the FP64

@@ -3,8 +3,9 @@
 // Some callers cannot call cudaMalloc: code running inside a framework whose
 // memory pool owns the whole device, a plug-in loaded into a process that
 // forbids allocations after start-up, or a hard real-time loop where an
-// allocation could stall.  sigma_gpp_fp64_noalloc serves them.  It runs the
-// same FP64 kernels as sigma_gpp_execute, but every scratch buffer they need
+// allocation could stall.  sigma_gpp_fp64_noalloc serves them.  It runs
+// sigma_gpp_execute's FP64 kernels (not the exact contraction, whose digits take
+// gigabytes: 150 ms instead of 12 at 512 x 1638 x 32768), but every scratch buffer they need
 // (item counters, the column map, per-item partial sums, per-band results)
 // lives in one file-scope __device__ array of fixed size, so the call makes
 // no allocation of any kind.  Every GPU that loads the library holds that

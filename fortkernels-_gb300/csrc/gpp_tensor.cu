@@ -85,7 +85,7 @@ struct FactorSmem {
 __host__ __device__ constexpr size_t factor_acc_bytes(int nvband) {
   return sizeof(float4) * (size_t)(nvband < kFusedBands ? nvband : kFusedBands) * kNW * kFacCols * 4;
 }
-// ssx sums: output o = r * 64 + 8 * warp + lane / 4 is computed by the four
+// ssx sums: output o = r * 32 + 8 * warp + lane / 4 is computed by the four
 // lanes 4 (lane / 4) + q (q = 0..3, 8 g-vectors each) in round r, so every
 // warp takes part; each lane owns the accumulator acc[4 o + q]
 constexpr int kSsxRounds = (kFusedBands * kNW * kFacCols * 4 + kFacThreads - 1) / kFacThreads;

@@ -131,10 +131,22 @@ int sigma_gpp_tensor(int number_bands, int nvband, int ncouls, int ngpown, int n
  * 24 B per band and g-vector: 9.0 GB at 512 bands x 1638 columns x 32768
  * g-vectors (real-valued 5.1 GB, half sum 18 GB).  It takes them at creation,
  * and only while they are at most half of the device's free memory; without
- * them it runs the FP64 kernels (150 ms instead of 12 at that size).  Executions
- * with per-band frequencies, and sigma_gpp_fp64_noalloc, do not use them.  The
- * host calls give them up where their inputs need the memory, and keep those of
- * up to 256 MB (two for the real-valued and the half sum) between calls.
+ * them it runs the FP64 kernels (150 ms instead of 12 at that size).
+ * Executions with per-band frequencies, and sigma_gpp_fp64_noalloc, do not use
+ * them.  The host calls give them up where their inputs need the memory, and
+ * keep those of up to 256 MB (two for the real-valued and the half sum) between
+ * calls.
+ *
+ * Operands.  The contraction holds each operand row (a band's aqsn, a column's
+ * factors of one frequency) in fixed point below its largest element; an
+ * execution whose rows it could not sum to about 1e-12 runs the FP64 kernels
+ * instead, after the passes that find it out (3.8 ms instead of 0.46 at 128 x
+ * 409 x 8192, 154 instead of 12 at 512 x 1638 x 32768; 1 to 10 % above the FP64
+ * kernels alone).  These are rows whose large elements are few: fewer than one
+ * in 128 places where it is certain that a column's factor within 2^-5 and a
+ * band's element within 2^-4 of their row's largest meet (one element of 1
+ * beside others below 0.03 makes such a row), values that are not finite,
+ * |wtilde| or |I_eps| above 1e15, and frequencies outside 1e-9 .. 1e9.
  * ------------------------------------------------------------------------- */
 typedef struct sigma_gpp_plan_s* sigma_gpp_plan;
 
@@ -215,10 +227,15 @@ typedef struct sigma_gpp_instance {
 typedef struct sigma_gpp_batch_s* sigma_gpp_batch;
 
 /* Validates every instance like sigma_gpp_plan_create and sizes the queues.
- * tile_shape (may be NULL) picks the FP64 main-pass tile per instance, -1
- * for the library's choice (least padding).  A batch whose instances all
- * share one frequency set per instance (wx_band_stride 0) runs the
- * shared-frequency kernel: tiles 3 = 64 bands x 32 columns, 4 = 32 x 64,
+ * An FP64 batch whose instances all share one frequency set per instance
+ * (wx_band_stride 0) runs an exact contraction per instance, over one workspace
+ * of the largest instance's size (taken as a plan takes its own), and
+ * the queue's main and occupied-band passes for the rest: instances too small,
+ * many small ones together, out-of-range operands (below), and every instance of
+ * other batches.
+ * tile_shape (may be NULL) picks the tile of that FP64 main pass per instance, -1
+ * for the library's choice (least padding).  With shared frequencies it is the
+ * shared-frequency kernel's: tiles 3 = 64 bands x 32 columns, 4 = 32 x 64,
  * 5 = 32 x 32, 6 = 64 x 16 (5 and 6: two CTAs per SM when every instance
  * takes one of them); otherwise the per-band kernel: 0 = 32 x 32,
  * 1 = 16 x 64, 2 = 64 x 16.  A tile of the other family is
@@ -236,8 +253,8 @@ int sigma_gpp_batch_create(sigma_gpp_batch* batch, int n_instances, const sigma_
                            int precision, const int* tile_shape);
 
 /* sigma_gpp_batch_create with the work sizing given (0 for the default of
- * each): items_per_cta, the FP64 and mixed main pass's work items per
- * resident CTA (each item a band block x column block x g-vector split;
+ * each): items_per_cta, the FP64 and mixed main pass's work items (in FP64 those
+ * of the instances without a contraction) per resident CTA (each item a band block x column block x g-vector split;
  * default 16), and tensor_split_tiles, the tensor form's contraction items'
  * length in K tiles of 32 g-vectors (real and imaginary halves counted
  * apart), the same for every instance (default: each instance's items
@@ -274,8 +291,8 @@ int sigma_gpp_batched(int n_instances, const sigma_gpp_instance* inst, int preci
  * plug-in in a process that forbids allocation after start-up, or a
  * real-time loop where an allocation could stall.
  *
- * Same result as sigma_gpp_execute with an FP64 plan (within 1e-12 relative;
- * the g-vector split differs), same arrays, all device pointers except the
+ * Same result as sigma_gpp_execute with an FP64 plan (within 1e-12 relative; it
+ * runs the FP64 kernels, without the exact contraction), same arrays, all device pointers except the
  * host index maps (indinv with ncouls entries; wx_array: 3 device doubles
  * shared by every band).  Its scratch (item counters, column map, partial
  * sums) is one fixed 32 MiB __device__ array inside the library, held by
